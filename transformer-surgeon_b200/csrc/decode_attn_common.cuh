@@ -99,6 +99,64 @@ __device__ __forceinline__ float v_elem(const uint8_t* __restrict__ rec, int fmt
   return e2m1_nibble_to_f32(b >> ((e & 1) * 4)) * e4m3_byte_to_f32(rec[16 * (D / 2) + (e >> 4) * 16 + t]);
 }
 
+// The last CTA of a (sequence, kv head, head chunk) merges its S partials, in split order:
+//   out[h][e] = sum_s acc_s[e] c_s / sum_s l_s c_s,  c_s = exp(m_s - max m).
+// `part` = partials of the chunk's first head ([heads][S][2 + D], consecutive), `out` = its outputs, `sm` = shared scratch of
+// 2 heads * S + heads floats.  Bound by the round trips to partials that other SMs have just written: every (m, l) is fetched
+// once, all in flight together (it was two dependent loads per split and output element: 75 us of an 83 us launch at 63 splits,
+// batch 1, 7 heads), the coefficients come from shared memory, and kFly partials of an element pair are in flight at once.
+template <typename T, int D>
+__device__ __forceinline__ void merge_splits(const float* __restrict__ part, int heads, int S, float* sm, T* __restrict__ out) {
+  constexpr int kFly = 16;
+  float* sc = sm;                                     // [heads][S] m, then c
+  float* sl = sm + heads * S;                         // [heads][S] l
+  float* ssum = sl + heads * S;                       // [heads]
+  for (int i = threadIdx.x; i < heads * S; i += blockDim.x) {
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(part + (size_t)i * (2 + D)));
+    sc[i] = ml.x;
+    sl[i] = ml.y;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int h = warp; h < heads; h += blockDim.x >> 5) {
+    float mm = -INFINITY;
+    for (int s = lane; s < S; s += 32) mm = fmaxf(mm, sc[h * S + s]);
+    mm = warp_max(mm);
+    for (int s = lane; s < S; s += 32) {
+      const float ms = sc[h * S + s];
+      sc[h * S + s] = ms == -INFINITY ? 0.f : __expf(ms - mm);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      float ll = 0.f;
+      for (int s = 0; s < S; ++s) ll += sl[h * S + s] * sc[h * S + s];
+      ssum[h] = ll;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x) {
+    const int h = i / (D / 2), e = i % (D / 2) * 2;
+    const float* p = part + (size_t)h * S * (2 + D) + 2 + e;
+    const float* c = sc + h * S;
+    float a0 = 0.f, a1 = 0.f;
+    for (int s0 = 0; s0 < S; s0 += kFly) {
+      float2 v[kFly];
+#pragma unroll
+      for (int u = 0; u < kFly; ++u)
+        if (s0 + u < S) v[u] = __ldcg(reinterpret_cast<const float2*>(p + (size_t)(s0 + u) * (2 + D)));
+#pragma unroll
+      for (int u = 0; u < kFly; ++u)
+        if (s0 + u < S) {
+          a0 += v[u].x * c[s0 + u];
+          a1 += v[u].y * c[s0 + u];
+        }
+    }
+    const float ll = ssum[h];
+    out[h * D + e] = from_f32<T>(ll > 0.f ? a0 / ll : 0.f);
+    out[h * D + e + 1] = from_f32<T>(ll > 0.f ? a1 / ll : 0.f);
+  }
+}
+
 int validate_kv(const tsb200_kv_desc* kv, bool need_table);
 
 }  // namespace tsb

@@ -423,21 +423,8 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int idx = threadIdx.x; idx < g * D; idx += blockDim.x) {
-    const int i = idx / D, e = idx % D;
-    const int64_t bh = (int64_t)b * H + hk * g + i;
-    const float* pr = ws + bh * S * (2 + D);
-    float mm = -INFINITY;
-    for (int sp = 0; sp < S; ++sp) mm = fmaxf(mm, __ldcg(pr + sp * (2 + D)));
-    float ll = 0.f, a = 0.f;
-    for (int sp = 0; sp < S; ++sp) {
-      const float ms = __ldcg(pr + sp * (2 + D));
-      const float c = ms == -INFINITY ? 0.f : __expf(ms - mm);
-      ll += __ldcg(pr + sp * (2 + D) + 1) * c;
-      a += __ldcg(pr + sp * (2 + D) + 2 + e) * c;
-    }
-    out[bh * D + e] = from_f32<T>(ll > 0.f ? a / ll : 0.f);
-  }
+  const int64_t bh0 = (int64_t)b * H + hk * g;
+  merge_splits<T, D>(ws + bh0 * S * (2 + D), g, S, reinterpret_cast<float*>(smem), out + bh0 * D);
   if (threadIdx.x == 0) *ctr = 0;
 }
 
