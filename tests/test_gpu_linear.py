@@ -108,6 +108,27 @@ def test_prompt_sized_token_counts(cuda, p, M, K, N, r):
     assert torch.equal(lin(x.to(cuda)), y)
 
 
+@pytest.mark.parametrize("p", [4, 8, 2, "binary"])
+@pytest.mark.parametrize("M,K,N,r", [(1, 72, 37, 0),            # one partial K block per chain pair, rows beyond the last tile
+                                     (8, 4096, 256, 0),         # 16 K splits over a cluster, full token tile
+                                     (9, 1000, 4100, 136),      # second token tile with one token; K and rank end inside a block; odd block counts
+                                     (16, 14336, 520, 0),       # most splits, uneven last split, N not a multiple of 16
+                                     (13, 8, 8, 8)])            # smallest
+def test_decode_sized_token_counts(cuda, p, M, K, N, r):
+    """At most 16 tokens: warp-level kernel with one accumulation chain per warp; every output within 1e-2 of the fp32
+    result on the dequantized factors, and a second call returns the same bits."""
+    from transformer_surgeon_b200 import ops
+    x, U, V, b = _case(M, K, N, r, p, "bf16", seed=9)
+    fu = ops.Factor.quantize(U.to(cuda), p)
+    fv = ops.Factor.quantize(V.to(cuda), p) if r else None
+    ref32 = olin.linear_compressed_fp32(x, fu.reconstruct(torch.bfloat16).cpu(), b, fv.reconstruct(torch.bfloat16).cpu() if r else None)
+    lin = ops.PackedLinear(fu, fv, b.to(cuda), torch.bfloat16)
+    y = lin(x.to(cuda))
+    err = (y.cpu().float() - ref32.float()).abs()
+    assert (err <= 2e-2 * ref32.float().abs() + 1e-2 * ref32.float().abs().max()).all()
+    assert torch.equal(lin(x.to(cuda)), y)
+
+
 def test_config2_shape_sweep(cuda):
     """x [M, 4096], W 4096x4096 factored at r in {256, 1024}, 8/4-bit + binary factors, bf16:
     compared with the dequantized fp32 result (max-rel-err <= 1e-2)."""

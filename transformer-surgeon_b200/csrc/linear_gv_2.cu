@@ -1,0 +1,8 @@
+// The decode-sized packed GEMM on 2-bit codes (one file per container: they compile side by side).
+#include "linear_gv_launch.cuh"
+
+namespace tsb {
+namespace gv {
+template cudaError_t launch<2>(const Params&, const Plan&, bool, bool, cudaStream_t);
+}  // namespace gv
+}  // namespace tsb

@@ -340,8 +340,8 @@ int gemm_tc(const void* W, int bits, const float* scale, const void* bias, const
 }
 
 // 1-bit rows are 8 bytes per 64 columns: the copy engine wants a 16-byte row pitch
-bool tc_supported_factor(int bits, int64_t K) {
-  if (bits == 1) return K % 128 == 0;
+bool tc_supported_factor(int bits, int64_t K, int64_t M) {
+  if (bits == 1) return K % 128 == 0 || (M <= kGvTokens && K % 8 == 0);
   return (bits == 2 || bits == 4 || bits == 8 || bits == 16) && (K % 8) == 0;
 }
 
@@ -368,8 +368,8 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
               cudaStream_t s) {
   if (d->act_dtype != TSB200_BF16) return TSB200_ERR_UNSUPPORTED;
   const int64_t ku = d->rank > 0 ? d->rank : d->in_features;
-  if (!tc_supported_factor(d->u_bits, ku)) return TSB200_ERR_UNSUPPORTED;
-  if (d->rank > 0 && !tc_supported_factor(d->v_bits, d->in_features)) return TSB200_ERR_UNSUPPORTED;
+  if (!tc_supported_factor(d->u_bits, ku, M)) return TSB200_ERR_UNSUPPORTED;
+  if (d->rank > 0 && !tc_supported_factor(d->v_bits, d->in_features, M)) return TSB200_ERR_UNSUPPORTED;
   if (!aligned(x, 16) || !aligned(y, 2)) return TSB200_ERR_ARG;
   if (!workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
   if (workspace_bytes < tsb200_linear_workspace_bytes(d, M)) return TSB200_ERR_WORKSPACE;
@@ -379,11 +379,28 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
   void* h = ws + kWsHeader;
   const size_t hbytes = ((size_t)M * (size_t)(d->rank > 0 ? d->rank : 0) * 2 + 255) / 256 * 256;
   float* partial = (float*)(ws + kWsHeader + hbytes);
+  // decode-sized token counts on packed factors: one launch per factor, the second chained to the first
+  auto small = [&](const void* W, int bits, const float* scale, const void* bias, const void* in, void* out, int64_t K, int64_t N,
+                   bool pdl, const GvSpan* ahead) {
+    if (bits > 8 || M > kGvTokens) return (int)TSB200_ERR_UNSUPPORTED;
+    PhaseSpec ps;
+    ps.nsub = 1; ps.gated = 0;
+    ps.g[0] = GemmSpec{W, scale, bias, in, out, N, K};
+    return gv_gemm(ps, bits, M, pdl, ahead, ahead ? 1 : 0, s);
+  };
   auto gemm = [&](const void* W, int bits, const float* scale, const void* bias, const void* in, void* out, int64_t K,
                   int64_t N) {
-    return bits == 16 ? gemm_tc(W, bits, scale, bias, in, out, M, K, N, partial, status, s)
-                      : gemm_tcq(W, bits, scale, bias, in, out, M, K, N, partial, counters, status, s);
+    if (bits == 16) return gemm_tc(W, bits, scale, bias, in, out, M, K, N, partial, status, s);
+    const int st = small(W, bits, scale, bias, in, out, K, N, g_pdl != 0, nullptr);
+    if (st != TSB200_ERR_UNSUPPORTED) return st;
+    return gemm_tcq(W, bits, scale, bias, in, out, M, K, N, partial, counters, status, s);
   };
+  if (d->rank > 0 && d->u_bits <= 8 && d->v_bits <= 8 && M <= kGvTokens && gv_supported(d->u_bits, M, d->out_features, ku)) {
+    const GvSpan u{d->u, (size_t)d->out_features * tsb200_packed_row_bytes(ku, d->u_bits)};
+    int st = small(d->v, d->v_bits, d->v_scale, nullptr, x, h, d->in_features, d->rank, g_pdl != 0, &u);
+    if (st == TSB200_OK) st = small(d->u, d->u_bits, d->u_scale, d->bias, h, y, ku, d->out_features, true, nullptr);
+    if (st != TSB200_ERR_UNSUPPORTED) return st;
+  }
   if (d->rank > 0 && d->u_bits == d->v_bits && d->u_bits <= 8) {
     // both factors packed alike: V then U as two phases of ONE launch (grid barrier in between);
     // the rank-r intermediate is produced and consumed through L2

@@ -1026,7 +1026,6 @@ int run_program_tcq(const PhaseSpec* specs, int n_phases, int bits, int64_t M, u
     coresident = coresident || ph.scatter;
   }
   switch (tn) {
-    case 16: return launch_q_bits<16>(bits, prog, grid, coresident, s);
     case 32: return launch_q_bits<32>(bits, prog, grid, coresident, s);
     case 64: return launch_q_bits<64>(bits, prog, grid, coresident, s);
     case 256: return launch_q_bits<256>(bits, prog, grid, coresident, s);

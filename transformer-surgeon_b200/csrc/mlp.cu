@@ -30,6 +30,14 @@ bool fusable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, const tsb
   if (tiles < tc::kPlanSMs * 3 / 8) return false;
   return true;
 }
+// Few enough tokens for the chain of decode-sized launches (linear_gv.cu); its results are those of the one-launch block.
+bool chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, const tsb200_linear_desc* d, int64_t M) {
+  const int b = g->u_bits;
+  return M <= kGvTokens && (g->rank == 0 || gv_supported(b, M, g->rank, g->in_features)) &&
+         gv_supported(b, M, g->out_features, g->rank > 0 ? g->rank : g->in_features) &&
+         (d->rank == 0 || gv_supported(b, M, d->rank, d->in_features)) &&
+         gv_supported(b, M, d->out_features, d->rank > 0 ? d->rank : d->in_features);
+}
 }  // namespace
 
 // Workspace layout: [region 0 | gate out | up out | act | h0 | h1 | h2].  Region 0 starts with the
@@ -92,7 +100,53 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
   uint8_t* h1 = h0 + r_b;
   uint8_t* h2 = h1 + r_b;
 
-  if (fusable(gate, up, down, M)) {
+  const bool fused = fusable(gate, up, down, M);
+  if (fused && chainable(gate, up, down, M)) {
+    // [gate V | up V] -> [gate U, up U with SiLU(g) * u] -> [down V] -> [down U]: chained launches, the first one also requests
+    // the codes of the others into the L2
+    GvSpan ahead[3];
+    int na = 0;
+    const int64_t kgu = gate->rank > 0 ? gate->rank : gate->in_features, kd = down->rank > 0 ? down->rank : down->in_features;
+    auto span = [&](const void* p, int bits, int64_t rows, int64_t cols) { ahead[na++] = GvSpan{p, (size_t)rows * tsb200_packed_row_bytes(cols, bits)}; };
+    PhaseSpec ps;
+    int st = TSB200_OK;
+    bool pdl = g_pdl != 0;
+    ps.g[1] = GemmSpec{};
+    const void* gx = x;
+    const void* ux = x;
+    if (gate->rank > 0) {
+      span(gate->u, gate->u_bits, gate->out_features, kgu);
+      span(up->u, up->u_bits, up->out_features, kgu);
+      span(down->rank > 0 ? down->v : down->u, down->rank > 0 ? down->v_bits : down->u_bits, down->rank > 0 ? down->rank : down->out_features, down->in_features);
+      ps.nsub = 2; ps.gated = 0;
+      ps.g[0] = GemmSpec{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features};
+      ps.g[1] = GemmSpec{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features};
+      st = gv_gemm(ps, gate->v_bits, M, pdl, ahead, na, s);
+      gx = h0; ux = h1;
+      pdl = true;
+    }
+    if (st == TSB200_OK) {
+      na = 0;
+      span(down->u, down->u_bits, down->out_features, kd);
+      ps.nsub = 2; ps.gated = 1;
+      ps.g[0] = GemmSpec{gate->u, gate->u_scale, gate->bias, gx, buf_g, gate->out_features, kgu};
+      ps.g[1] = GemmSpec{up->u, up->u_scale, up->bias, ux, buf_g, up->out_features, kgu};
+      st = gv_gemm(ps, gate->u_bits, M, pdl, ahead, na, s);
+    }
+    ps.nsub = 1; ps.gated = 0;
+    const void* dx = buf_g;
+    if (st == TSB200_OK && down->rank > 0) {
+      ps.g[0] = GemmSpec{down->v, down->v_scale, nullptr, buf_g, h2, down->rank, down->in_features};
+      st = gv_gemm(ps, down->v_bits, M, true, nullptr, 0, s);
+      dx = h2;
+    }
+    if (st == TSB200_OK) {
+      ps.g[0] = GemmSpec{down->u, down->u_scale, down->bias, dx, y, down->out_features, kd};
+      st = gv_gemm(ps, down->u_bits, M, true, nullptr, 0, s);
+    }
+    if (st != TSB200_ERR_UNSUPPORTED) return st;
+  }
+  if (fused) {
     PhaseSpec ps[4];
     int n = 0;
     const void* gx = x;

@@ -35,10 +35,7 @@ inline GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int nsub = 1, bool no
   // above 128 tokens a 256-token tile with two k-blocks per stage: every widened weight tile then meets twice as many
   // tokens, and one M128 x N256 x K16 MMA (128 cycles of the tensor pipe) outlasts the ~115 cycles its lane needs to
   // issue it (M = 2048, rank 1024, int4: 524 -> 566 TFLOP/s; with one k-block per stage it was slower than 128)
-  g.tn = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256)));
-#ifdef TSB_FORCE_TN128
-  if (g.tn == 256) g.tn = 128;
-#endif
+  g.tn = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
   g.kb_total = (int)((K + BK - 1) / BK);
   const int64_t n_tiles = (N + BM - 1) / BM, m_tiles = (M + g.tn - 1) / g.tn;
   const int64_t base = n_tiles * m_tiles * nsub;
@@ -242,5 +239,17 @@ struct PhaseSpec {
 int run_program_tcq(const PhaseSpec* specs, int n_phases, int bits, int64_t M, uint8_t* scratch, int* counters, int* grid_bar,
                     int* status, cudaStream_t s);
 size_t phase_scratch_bytes(int64_t M, int64_t N, int64_t K, int nsub, bool gated);
+
+// Decode-sized packed GEMM (linear_gv.cu): one phase, one launch, no workspace.  `ahead`: constants of the launches that follow,
+// requested into the L2 while this one runs.
+// Token counts it serves.  Above 16 tokens the tcgen05 kernel is as fast: 32 tokens through 4096 x 4096 take 9.8 us there and
+// 10.1 here, through 4096 x 6144 11.7 and 20.5 (its MMAs take 32 tokens at the price of 16; these pay per 8).
+constexpr int64_t kGvTokens = 16;
+struct GvSpan {
+  const void* p;
+  size_t bytes;
+};
+bool gv_supported(int bits, int64_t M, int64_t N, int64_t K);
+int gv_gemm(const PhaseSpec& ps, int bits, int64_t M, bool pdl, const GvSpan* ahead, int n_ahead, cudaStream_t s);
 
 }  // namespace tsb
