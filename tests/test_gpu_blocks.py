@@ -66,3 +66,19 @@ def test_swiglu_prompt_sized_equals_elementwise_form(cuda):
     assert torch.equal(y, y_ref)
     ref = oatt.swiglu(gu[:, :n].cpu(), gu[:, n:].cpu())
     torch.testing.assert_close(y.cpu(), ref, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("hidden", [8, 1024, 1028 * 2, 4096, 4104])
+def test_rmsnorm_row_lengths(cuda, name, hidden):
+    """One, two and four pieces per thread, rows that end inside a thread block's pass, and rows too long for registers."""
+    from transformer_surgeon_b200 import ops
+    dt = {"fp32": torch.float32, "bf16": torch.bfloat16}[name]
+    g = torch.Generator().manual_seed(hidden)
+    r, d, w = (torch.randn(n, generator=g).to(dt) for n in ((3, hidden), (3, hidden), (hidden,)))
+    res = r.to(cuda).clone()
+    y = ops.add_rmsnorm(res, d.to(cuda), w.to(cuda), eps=1e-6, variant=0)
+    s = r + d
+    tol = dict(rtol=1e-5, atol=1e-5) if name == "fp32" else dict(rtol=1e-2, atol=1e-2)
+    assert torch.equal(res.cpu(), s)
+    torch.testing.assert_close(y.cpu(), oatt.rmsnorm_hf(s, w, 1e-6), **tol)

@@ -93,72 +93,108 @@ __global__ void add_rmsnorm_kernel(T* __restrict__ residual, const T* __restrict
   }
 }
 
-// Hugging Face variant, bf16, hidden % 8 == 0 and hidden <= 8192: one pass over global memory with
-// 16-byte loads; the row stays in registers between the statistic and the scaling.
+// Sum over the CTA (256 threads), every thread gets it; used once per launch.
+__device__ __forceinline__ float block_sum_once(float v, float* sh) {
+  v = warp_sum(v);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) sh[w] = v;
+  __syncthreads();
+  return warp_sum(l < (int)(blockDim.x >> 5) ? sh[l] : 0.f);
+}
+
+// 16 bytes of a row as fp32 and back.
+template <typename T> struct Vec16;
+template <> struct Vec16<float> {
+  static constexpr int N = 4;
+  __device__ static void unpack(const uint4& a, float (&v)[4]) {
+    v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
+  }
+  __device__ static uint4 pack(const float (&v)[4]) {
+    return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  }
+};
+template <> struct Vec16<__nv_bfloat16> {
+  static constexpr int N = 8;
+  __device__ static void unpack(const uint4& a, float (&v)[8]) {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&a);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(p[j]);
+      v[2 * j] = f.x; v[2 * j + 1] = f.y;
+    }
+  }
+  __device__ static uint4 pack(const float (&v)[8]) {
+    uint4 o;
+    __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+    return o;
+  }
+};
+
+// Hugging Face variant, rows of whole 16-byte pieces, at most IT * 256 of them: one pass over global memory; the row stays in
+// registers between the statistic and the scaling.  With a decode batch the launch is a chain of latencies (launch, row, sum, row
+// out): the weights, constants, are requested ahead of the dependency wait so that they are no link of it.
+template <typename T, int IT>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_hf_bf16_kernel(__nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ delta,
-                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int hidden, float eps) {
+add_rmsnorm_hf_kernel(T* __restrict__ residual, const T* __restrict__ delta, const T* __restrict__ w, T* __restrict__ y, int hidden, float eps) {
+  using V = Vec16<T>;
   __shared__ float sh[32];
   pdl_launch_dependents();
-  pdl_wait();
   const int64_t row = blockIdx.x;
-  const int nvec = hidden >> 3;
+  const int nvec = hidden / V::N;
+  const uint4* wv = reinterpret_cast<const uint4*>(w);
+  uint4 ww[IT];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int i = threadIdx.x + it * 256;
+    if (i < nvec) ww[it] = __ldg(wv + i);
+  }
+  pdl_wait();
   uint4* r = reinterpret_cast<uint4*>(residual + row * hidden);
   const uint4* dl = delta ? reinterpret_cast<const uint4*>(delta + row * hidden) : nullptr;
-  float v[4][8];
+  float v[IT][V::N];
   float ss = 0.f;
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int i = threadIdx.x + it * 256;
     if (i < nvec) {
-      uint4 a = r[i];
-      const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a);
+      V::unpack(r[i], v[it]);
       if (dl) {
-        const uint4 b = dl[i];
-        const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&b);
-        uint4 o;
-        __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+        float d[V::N];
+        V::unpack(dl[i], d);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 fa = __bfloat1622float2(ap[j]), fb = __bfloat1622float2(bp[j]);
-          op[j] = __floats2bfloat162_rn(__fadd_rn(fa.x, fb.x), __fadd_rn(fa.y, fb.y));
-          const float2 fo = __bfloat1622float2(op[j]);
-          v[it][2 * j] = fo.x; v[it][2 * j + 1] = fo.y;
-        }
-        r[i] = o;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 fa = __bfloat1622float2(ap[j]);
-          v[it][2 * j] = fa.x; v[it][2 * j + 1] = fa.y;
-        }
+        for (int j = 0; j < V::N; ++j) v[it][j] = rnd<T>(__fadd_rn(v[it][j], d[j]));
+        r[i] = V::pack(v[it]);
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss += v[it][j] * v[it][j];
+      for (int j = 0; j < V::N; ++j) ss += v[it][j] * v[it][j];
     }
   }
-  const float var = block_reduce_sum(ss, sh) / (float)hidden;
+  const float var = block_sum_once(ss, sh) / (float)hidden;
   const float inv = 1.0f / sqrtf(var + eps);
-  const uint4* wv = reinterpret_cast<const uint4*>(w);
   uint4* yo = reinterpret_cast<uint4*>(y + row * hidden);
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int i = threadIdx.x + it * 256;
     if (i < nvec) {
-      const uint4 ww = wv[i];
-      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&ww);
-      uint4 o;
-      __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+      float f[V::N], o[V::N];
+      V::unpack(ww[it], f);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 fw = __bfloat1622float2(wp[j]);
-        const __nv_bfloat162 n = __floats2bfloat162_rn(__fmul_rn(v[it][2 * j], inv), __fmul_rn(v[it][2 * j + 1], inv));
-        const float2 fn = __bfloat1622float2(n);
-        op[j] = __floats2bfloat162_rn(__fmul_rn(fw.x, fn.x), __fmul_rn(fw.y, fn.y));
-      }
-      yo[i] = o;
+      for (int j = 0; j < V::N; ++j) o[j] = __fmul_rn(f[j], rnd<T>(__fmul_rn(v[it][j], inv)));
+      yo[i] = V::pack(o);
     }
   }
+}
+
+template <typename T>
+int launch_rmsnorm_hf(void* residual, const void* delta, const void* w, void* y, int64_t M, int64_t hidden, float eps, cudaStream_t s) {
+  auto go = [&](auto* kernel) {
+    return launch_kernel(kernel, dim3((unsigned)M), dim3(256), 0, s, (T*)residual, (const T*)delta, (const T*)w, (T*)y, (int)hidden, eps);
+  };
+  const int64_t pieces = hidden / Vec16<T>::N;
+  TSB_CUDA(pieces <= 256 ? go(add_rmsnorm_hf_kernel<T, 1>) : (pieces <= 512 ? go(add_rmsnorm_hf_kernel<T, 2>) : go(add_rmsnorm_hf_kernel<T, 4>)));
+  return TSB200_OK;
 }
 
 template <typename T>
@@ -238,13 +274,11 @@ int tsb200_add_rmsnorm(void* residual, const void* delta, const void* w, void* y
   if (M == 0) return TSB200_OK;
   if (!residual || !w || !y) return TSB200_ERR_ARG;
   if (M > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
-  if (dtype == TSB200_BF16 && variant == 0 && hidden % 8 == 0 && hidden <= 8192 && aligned(residual, 16) &&
-      aligned(y, 16) && aligned(w, 16) && (!delta || aligned(delta, 16))) {
-    TSB_CUDA(launch_kernel(add_rmsnorm_hf_bf16_kernel, dim3((unsigned)M), dim3(256), 0, as_stream(stream),
-                           (__nv_bfloat16*)residual, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-                           (int)hidden, eps));
-    return TSB200_OK;
-  }
+  const int64_t elt = dtype == TSB200_F32 ? 4 : 2;
+  if ((dtype == TSB200_F32 || dtype == TSB200_BF16) && variant == 0 && hidden * elt % 16 == 0 && hidden * elt <= 16384 && aligned(residual, 16) &&
+      aligned(y, 16) && aligned(w, 16) && (!delta || aligned(delta, 16)))
+    return dtype == TSB200_F32 ? launch_rmsnorm_hf<float>(residual, delta, w, y, M, hidden, eps, as_stream(stream))
+                               : launch_rmsnorm_hf<__nv_bfloat16>(residual, delta, w, y, M, hidden, eps, as_stream(stream));
   if (dtype == TSB200_F32)
     add_rmsnorm_kernel<float><<<(unsigned)M, 256, 0, as_stream(stream)>>>((float*)residual, (const float*)delta, (const float*)w, (float*)y, hidden, eps, variant);
   else if (dtype == TSB200_BF16)
