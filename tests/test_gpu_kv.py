@@ -181,6 +181,27 @@ def test_decode_attention_against_oracle(cuda, fmt, name, H, Hkv, d, simt):
     assert np.all(np.abs(out - ref) <= tol), (np.abs(out - ref) / tol).max()
 
 
+@pytest.mark.parametrize("fmt", ["fp32", "bf16"])
+@pytest.mark.parametrize("H,Hkv,d", [(14, 2, 64), (9, 1, 128), (4, 4, 128)])
+@pytest.mark.parametrize("lens", [(1, 16, 17), (0, 129, 150), (700, 2049, 33)])
+def test_decode_attention_unquantized_pages(cuda, fmt, H, Hkv, d, lens):
+    """Unquantized pages: one split and several, empty and one-token sequences, a second chunk of query heads, stale slots; against
+    the one-lane-per-element cross-check kernel."""
+    from transformer_surgeon_b200 import ops
+    B, cap = len(lens), 2064
+    g = torch.Generator(device=cuda).manual_seed(3)
+    pages = cap // 16
+    bt = torch.randperm(B * pages, generator=g, device=cuda).to(torch.int32).reshape(B, pages)
+    seq = torch.zeros(B, dtype=torch.int32, device=cuda)
+    kv = ops.PagedKV(fmt, B * pages, Hkv, d, bt, seq, cuda)
+    k, v = (torch.randn((B, cap, Hkv, d), generator=g, device=cuda).to(DT[fmt]) for _ in range(2))
+    kv.append(k, v)
+    seq.copy_(torch.tensor(lens, dtype=torch.int32))
+    q = torch.randn((B, H, d), generator=g, device=cuda).to(DT[fmt])
+    out, ref = ops.paged_decode_attention(kv, q, max(lens)), ops.paged_decode_attention(kv, q, max(lens), simt=True)
+    torch.testing.assert_close(out, ref, rtol=1e-5 if fmt == "fp32" else 1e-2, atol=1e-5 if fmt == "fp32" else 1e-2)
+
+
 @pytest.mark.parametrize("fmt", FMTS)
 def test_decode_attention_config3_shape(cuda, fmt):
     """Llama-3-8B layout (32 q heads / 8 kv heads / d 128), batch 8, context 4096, seeded random

@@ -24,6 +24,8 @@ int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, 
                     int64_t B, float* ws, int* counters, void* out, int* status, cudaStream_t st);
 int validate_attn_args(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, int64_t B, int H,
                        int64_t max_seq_len, void* workspace, size_t workspace_bytes, bool& noop, size_t need_bytes);
+int attn_dense(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, int64_t qs, int64_t B, int H, float sm_scale,
+               int64_t max_seq_len, float* ws, int* counters, cudaStream_t s);
 
 namespace {
 
@@ -425,8 +427,6 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   if (st != TSB200_OK || noop) return st;
   const int64_t qs = q_batch_stride ? q_batch_stride : (int64_t)H * kv->head_dim;
   if (qs < (int64_t)H * kv->head_dim) return TSB200_ERR_ARG;
-  if (kv->format > TSB200_KV_NVFP4)    // unquantized pages: CUDA-core kernel (fp32 math)
-    return tsb200_paged_decode_attn_simt(kv, q, out, dtype, q_batch_stride, B, H, sm_scale, max_seq_len, workspace, workspace_bytes, stream);
   cudaStream_t s = as_stream(stream);
   const int S = choose_splits(B, kv->hkv, max_seq_len);
   int* counters = (int*)workspace;                               // zero between calls
@@ -437,6 +437,8 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   const bool fused = n_ctr < (int64_t)(kAttnCounterBytes / sizeof(int));           // else: separate reduction launch
   int* status = counters + kAttnStatusIndex;
   int r;
+  if (kv->format > TSB200_KV_NVFP4)    // unquantized pages: fp32 math (decode_attn_dense.cu)
+    return attn_dense(kv, q, out, dtype, qs, B, H, sm_scale, max_seq_len, ws, fused ? counters : nullptr, s);
   if (kv->format == TSB200_KV_FP8 && D == 128 && H / kv->hkv <= 4) {
     // e4m3 pages go to the tensor cores as FP8 (decode_attn_fp8.cu)
     int* ctr = fused ? counters : nullptr;
