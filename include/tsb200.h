@@ -144,6 +144,13 @@ int tsb200_linear(const tsb200_linear_desc* d, const void* x, void* y, int64_t M
 int tsb200_linear_simt(const tsb200_linear_desc* d, const void* x, void* y, int64_t M,
                        void* workspace, size_t workspace_bytes, void* stream);
 
+/* n layers that read the same x (q, k and v of a decoder layer): y[i] [M, out_i], equal to n calls of tsb200_linear in order.
+ * fp32 layers with alike factors (same rank and containers; n <= 4) run as one launch per factor.  `d` and `y` are host
+ * arrays.  The workspace follows the rules of tsb200_linear's. */
+size_t tsb200_linear_group_workspace_bytes(const tsb200_linear_desc* const* d, int n, int64_t M);
+int tsb200_linear_group(const tsb200_linear_desc* const* d, int n, const void* x, void* const* y, int64_t M,
+                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* Greedy head: tokens[m] = argmax_n (x . W^T + bias)[m, n] with the logits rounded to the act dtype first, i.e. the
  * token torch.argmax would pick from tsb200_linear's output (the first maximum on ties).
  * Replaces the final layer + argmax of a greedy decode step (export/common.py:167,175 for the blocks path; the

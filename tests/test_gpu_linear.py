@@ -129,6 +129,27 @@ def test_decode_sized_token_counts(cuda, p, M, K, N, r):
     assert torch.equal(lin(x.to(cuda)), y)
 
 
+@pytest.mark.parametrize("p", [None, 8, 4, 2, "binary"])
+@pytest.mark.parametrize("M,K,N,r", [(1, 8200, 37, 0),          # one token past a staged K tile, K split over the warps of a CTA
+                                     (2, 72, 300, 0), (3, 904, 1000, 40), (5, 2056, 64, 0), (9, 264, 130, 24),
+                                     (16, 40, 65, 8), (67, 264, 1000, 136), (130, 512, 4100, 0)])   # 64 x 64 tiles (dense), ragged in both directions
+def test_fp32_layers(cuda, p, M, K, N, r):
+    """fp32 activations: every token group (1, 2, 4, 8 tokens), ragged rows, pieces that end inside a word of codes; a group of
+    layers equals the layers one by one."""
+    from transformer_surgeon_b200 import ops
+    x, U, V, b = _case(M, K, N, r, p, "fp32", seed=4)
+    mk = (lambda w: ops.Factor.dense(w.to(cuda))) if p is None else (lambda w: ops.Factor.quantize(w.to(cuda), p))
+    fu, fv = mk(U), mk(V) if r else None
+    ref = olin.linear_compressed_fp32(x, fu.reconstruct(torch.float32).cpu(), b, fv.reconstruct(torch.float32).cpu() if r else None)
+    lin = ops.PackedLinear(fu, fv, b.to(cuda), torch.float32)
+    y = lin(x.to(cuda))
+    assert rel_err(y.cpu(), ref) < 1e-5
+    small = ops.PackedLinear(mk(U[:5]), fv, None, torch.float32)
+    ya, yb = ops.LinearGroup([lin, small])(x.to(cuda))
+    torch.testing.assert_close(ya, y, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(yb, small(x.to(cuda)), rtol=1e-5, atol=1e-5)
+
+
 def test_config2_shape_sweep(cuda):
     """x [M, 4096], W 4096x4096 factored at r in {256, 1024}, 8/4-bit + binary factors, bf16:
     compared with the dequantized fp32 result (max-rel-err <= 1e-2)."""

@@ -1,0 +1,434 @@
+// LinearCompressed.forward with fp32 activations (transformersurgeon/blocks/linear_compressed.py:96-100): dense fp32 or packed
+// factors, fp32 accumulation on the FMA pipe (fp32 models keep fp32 products: no tensor-core path).
+//
+// What bounds it: one token is a stream of weights through launches of a few hundred KB, i.e. latency; a prompt is FMAs.  One
+// kernel serves both.  A warp owns R weight rows and MT tokens; its lanes walk K in 16-byte pieces (dense) or words (codes), and
+// the R x MT sums of the 32 lanes are reduced by a butterfly that halves the values with the lanes (31 shuffles for 32 sums
+// instead of 160).  Activations are staged in shared memory once per CTA and K tile and shared by its 8 warps.  With one token,
+// where the rows alone do not fill the machine, up to 8 warps split K.  Before the dependency wait of a programmatic launch every
+// warp requests its rows into the L2.
+//
+// Up to four matrices that share the reduction length run as one launch (q | k | v, gate | up), and the second factors of a gate /
+// up pair end in SiLU(g) * u (blocks/mlp.py:181-183).
+#include "tc_common.cuh"
+
+namespace tsb {
+namespace {
+
+constexpr int kWarps = 8;
+constexpr int kXFloats = 8192;               // staged activations: a K tile of this many floats over all tokens and matrices
+constexpr int kMaxSegs = 4;
+
+struct Seg {
+  const uint8_t* w;
+  const uint8_t* w2;                         // gated: the up matrix (w: gate)
+  const float *scale, *scale2, *bias, *bias2;
+  const float *x, *x2;
+  float* y;
+  int n, cta0;                               // rows; first CTA
+};
+struct F32Params {
+  Seg seg[kMaxSegs];
+  int nseg, M, K, ks_log2;
+  int64_t row_bytes;
+};
+
+// CNT consecutive weights of a lane: a 16-byte piece of a dense row (4) or one 32-bit word of codes (4 / 8 / 16 / 32).
+template <int BITS> struct Piece {
+  static constexpr int kCnt = BITS == 32 ? 4 : 32 / BITS;
+  static constexpr int kBytes = BITS == 32 ? 16 : 4;
+};
+template <int BITS> __device__ __forceinline__ void load_piece(const uint8_t* p, float (&v)[Piece<BITS>::kCnt]) {
+  if constexpr (BITS == 32) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  } else {
+    const unsigned w = __ldg(reinterpret_cast<const unsigned*>(p));
+    if constexpr (BITS == 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = (float)(int8_t)(w >> (8 * i));
+    } else if constexpr (BITS == 1) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[2 * i] = (float)(int)(((w >> i) & 1u) * 2u) - 1.0f;
+        v[2 * i + 1] = (float)(int)(((w >> (i + 16)) & 1u) * 2u) - 1.0f;
+      }
+    } else {
+      constexpr int half = 16 / BITS;          // pair-interleaved: field i = column 2 i, field i + half = column 2 i + 1
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        v[2 * i] = (float)sext((int)(w >> (BITS * i)), BITS);
+        v[2 * i + 1] = (float)sext((int)(w >> (BITS * i + 16)), BITS);
+      }
+    }
+  }
+}
+
+// Sums V values per lane over the 32 lanes; lane l returns the sum of value l % V (V a power of two up to 32).
+template <int V> __device__ __forceinline__ float reduce_scatter(float (&v)[V]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = V / 2; n > 0; n /= 2) {
+    const bool up = lane & n;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+    }
+  }
+  float s = v[0];
+#pragma unroll
+  for (int o = V; o < 32; o *= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+template <int BITS, int MT, int R, bool GATED>
+__global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_constant__ F32Params p) {
+  constexpr int MATS = GATED ? 2 : 1;
+  constexpr int CNT = Piece<BITS>::kCnt;
+  constexpr int V = MATS * R * MT;
+  constexpr int kKT = kXFloats / (MATS * MT);
+  static_assert(V <= 32 && (V & (V - 1)) == 0, "one sum per lane");
+  __shared__ __align__(16) float xs[MATS][MT][kKT];
+  __shared__ float red[kWarps][32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ks_n = 1 << p.ks_log2, ks = warp & (ks_n - 1);
+  int si = 0;
+  while (si + 1 < p.nseg && (int)blockIdx.x >= p.seg[si + 1].cta0) ++si;
+  const Seg& sg = p.seg[si];
+  const int row0 = (((int)blockIdx.x - sg.cta0) * (kWarps >> p.ks_log2) + (warp >> p.ks_log2)) * R;
+  const int m0 = blockIdx.y * MT;
+  const uint8_t* rows[MATS][R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t o = (int64_t)min(row0 + r, sg.n - 1) * p.row_bytes;          // beyond the matrix: the last row, never stored
+    rows[0][r] = sg.w + o;
+    if (GATED) rows[MATS - 1][r] = sg.w2 + o;
+  }
+  pdl_launch_dependents();
+  // One or two tokens: the first pieces of this warp's rows come ahead of the dependency wait (weights are constants), the rest of the
+  // rows into the L2
+  constexpr int kPre = MT <= 2 ? 16 / CNT / MATS : 0;           // 16 columns per row and matrix: 32 registers
+  float pre[kPre ? kPre : 1][MATS][R][CNT];
+  const int pre_end = (min(kKT, p.K) + CNT - 1) / CNT;
+#pragma unroll
+  for (int q = 0; q < kPre; ++q) {
+    const int i = lane + 32 * (ks + q * ks_n);
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (i < pre_end) load_piece<BITS>(rows[mat][r] + (int64_t)i * Piece<BITS>::kBytes, pre[q][mat][r]);
+  }
+  if (lane < MATS * R && ks == 0 && row0 < sg.n) {
+    const uint8_t* q = rows[0][0];
+#pragma unroll
+    for (int i = 0; i < MATS * R; ++i)
+      if (i == lane) q = rows[i / R][i % R];
+    const uintptr_t a = (reinterpret_cast<uintptr_t>(q) + 15) & ~(uintptr_t)15, e = (reinterpret_cast<uintptr_t>(q) + p.row_bytes) & ~(uintptr_t)15;
+    if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
+  }
+  pdl_wait();
+
+  float acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.f;
+  for (int k0 = 0; k0 < p.K; k0 += kKT) {
+    const int kt = min(kKT, p.K - k0);
+    __syncthreads();
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat) {
+      const float* x = mat ? sg.x2 : sg.x;
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const bool in = m0 + m < p.M;
+        const float* xr = x + (int64_t)(m0 + m) * p.K + k0;
+        const bool vec = (p.K & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+        const int stop = min(kKT, (kt + 31) & ~31);            // pieces of up to 32 columns are read beyond the end
+        if (vec) {
+          for (int i = tid * 4; i < stop; i += kWarps * 128) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in && i < kt) v = *reinterpret_cast<const float4*>(xr + i);
+            *reinterpret_cast<float4*>(&xs[mat][m][i]) = v;
+          }
+        } else {
+          for (int i = tid; i < stop; i += kWarps * 32) xs[mat][m][i] = in && i < kt ? xr[i] : 0.f;
+        }
+      }
+    }
+    __syncthreads();
+    // pieces of this warp: lane + 32 ks, then every 32 * ks_n; beyond the row's end the activations are zero, and no piece is read
+    const int pieces = (kt + CNT - 1) / CNT;
+    const int64_t b0 = (int64_t)k0 * Piece<BITS>::kBytes / CNT;
+    auto use = [&](int i, const float (&w)[MATS][R][CNT]) {
+#pragma unroll
+      for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+          for (int c = 0; c < CNT; c += 4) {
+            const float4 xv = *reinterpret_cast<const float4*>(&xs[mat][m][i * CNT + c]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              float& a = acc[(mat * R + r) * MT + m];
+              a += w[mat][r][c] * xv.x;
+              a += w[mat][r][c + 1] * xv.y;
+              a += w[mat][r][c + 2] * xv.z;
+              a += w[mat][r][c + 3] * xv.w;
+            }
+          }
+    };
+    int i = lane + 32 * ks;
+    if (kPre && k0 == 0) {
+#pragma unroll
+      for (int q = 0; q < kPre; ++q, i += 32 * ks_n)
+        if (i < pieces) use(i, pre[q]);
+    }
+#pragma unroll(MT <= 2 ? 4 : 2)
+    for (; i < pieces; i += 32 * ks_n) {
+      float w[MATS][R][CNT];
+#pragma unroll
+      for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+        for (int r = 0; r < R; ++r) load_piece<BITS>(rows[mat][r] + b0 + (int64_t)i * Piece<BITS>::kBytes, w[mat][r]);
+      use(i, w);
+    }
+  }
+  float s = reduce_scatter<V>(acc);
+  if (ks_n > 1) {
+    red[warp][lane] = s;
+    __syncthreads();
+    if (ks) return;
+    for (int q = 1; q < ks_n; ++q) s += red[warp + q][lane];
+  }
+  // lane v: matrix v / (R MT), row v / MT % R, token v % MT
+  const int r = lane / MT % R, m = m0 + lane % MT, n = row0 + r;
+  const bool ok = lane < R * MT && n < sg.n && m < p.M;
+  if constexpr (GATED) {
+    const float u = __shfl_sync(0xffffffffu, s, (lane + R * MT) & 31);
+    if (ok) {
+      const float g = s * (sg.scale ? sg.scale[n] : 1.0f) + (sg.bias ? sg.bias[n] : 0.f);
+      const float uv = u * (sg.scale2 ? sg.scale2[n] : 1.0f) + (sg.bias2 ? sg.bias2[n] : 0.f);
+      sg.y[(int64_t)m * sg.n + n] = __fmul_rn(g / (1.0f + expf(-g)), uv);
+    }
+  } else if (ok) {
+    sg.y[(int64_t)m * sg.n + n] = s * (sg.scale ? sg.scale[n] : 1.0f) + (sg.bias ? sg.bias[n] : 0.f);
+  }
+}
+
+// Prompt-sized token counts on dense factors: 64 tokens x 64 rows per CTA, 4 x 4 sums per thread, K in steps of 32 through shared
+// memory (k-major, so that a thread's operands are two 16-byte reads per k and matrix); the next step is fetched into registers
+// while this one is used.  The kernel above reduces over the lanes and pays 31 shuffles per 32 sums, which at a rank of 128 is as
+// much as the products: 128 tokens, gate | up 4864 x 128: 120 us there, 16 here.
+constexpr int kTM = 64, kTN = 64, kTK = 32;
+template <bool GATED>
+__global__ void __launch_bounds__(256) linear_f32_tile_kernel(const __grid_constant__ F32Params p) {
+  constexpr int MATS = GATED ? 2 : 1;
+  __shared__ __align__(16) float sx[MATS][kTK][kTM + 4], sw[MATS][kTK][kTN + 4];
+  int si = 0;
+  while (si + 1 < p.nseg && (int)blockIdx.x >= p.seg[si + 1].cta0) ++si;
+  const Seg& sg = p.seg[si];
+  const int n0 = ((int)blockIdx.x - sg.cta0) * kTN, m0 = blockIdx.y * kTM;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;         // rows 4 tx .., tokens 4 ty ..
+  pdl_launch_dependents();
+  // a thread fetches 16-byte pieces lk of tile rows lr and lr + 32, of x and of W
+  const int lk = (tid & 7) * 4, lr = tid >> 3;
+  float4 fx[MATS][2], fw[MATS][2];
+  auto fetch_w = [&](int k0) {
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float* w = reinterpret_cast<const float*>(mat ? sg.w2 : sg.w) + (int64_t)min(n0 + lr + 32 * h, sg.n - 1) * p.K;
+        fw[mat][h] = k0 + lk < p.K ? __ldg(reinterpret_cast<const float4*>(w + k0 + lk)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+  };
+  auto fetch_x = [&](int k0) {
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float* x = (mat ? sg.x2 : sg.x) + (int64_t)min(m0 + lr + 32 * h, p.M - 1) * p.K;
+        fx[mat][h] = k0 + lk < p.K ? *reinterpret_cast<const float4*>(x + k0 + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+  };
+  fetch_w(0);
+  pdl_wait();
+  fetch_x(0);
+  float acc[MATS][4][4] = {};
+  for (int k0 = 0; k0 < p.K; k0 += kTK) {
+    __syncthreads();
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float a[4] = {fx[mat][h].x, fx[mat][h].y, fx[mat][h].z, fx[mat][h].w};
+        const float b[4] = {fw[mat][h].x, fw[mat][h].y, fw[mat][h].z, fw[mat][h].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sx[mat][lk + j][lr + 32 * h] = a[j];
+          sw[mat][lk + j][lr + 32 * h] = b[j];
+        }
+      }
+    __syncthreads();
+    if (k0 + kTK < p.K) { fetch_w(k0 + kTK); fetch_x(k0 + kTK); }
+#pragma unroll
+    for (int k = 0; k < kTK; ++k)
+#pragma unroll
+      for (int mat = 0; mat < MATS; ++mat) {
+        const float4 xa = *reinterpret_cast<const float4*>(&sx[mat][k][ty * 4]), wa = *reinterpret_cast<const float4*>(&sw[mat][k][tx * 4]);
+        const float xv[4] = {xa.x, xa.y, xa.z, xa.w}, wv[4] = {wa.x, wa.y, wa.z, wa.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[mat][i][j] += xv[i] * wv[j];
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    if (m >= p.M) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + tx * 4 + j;
+      if (n >= sg.n) break;
+      float v = acc[0][i][j] + (sg.bias ? sg.bias[n] : 0.f);
+      if (GATED) v = __fmul_rn(v / (1.0f + expf(-v)), acc[MATS - 1][i][j] + (sg.bias2 ? sg.bias2[n] : 0.f));
+      sg.y[(int64_t)m * sg.n + n] = v;
+    }
+  }
+}
+
+template <int BITS, int MT, int R, bool GATED>
+int launch_cfg(F32Params& p, bool pdl, cudaStream_t s) {
+  // K split: enough CTAs for the machine with one token (148 SMs x 2), at least one piece per lane and warp
+  int rows = 0;
+  for (int i = 0; i < p.nseg; ++i) rows += p.seg[i].n;
+  const int groups = (p.M + MT - 1) / MT;
+  int ks = 0;
+  while (ks < 3 && (int64_t)((rows + (kWarps >> ks) * R - 1) / ((kWarps >> ks) * R)) * groups < 296 &&
+         p.K >= (64 << ks) * Piece<BITS>::kCnt)
+    ++ks;
+  p.ks_log2 = ks;
+  const int per = (kWarps >> ks) * R;
+  int ctas = 0;
+  for (int i = 0; i < p.nseg; ++i) {
+    p.seg[i].cta0 = ctas;
+    ctas += (p.seg[i].n + per - 1) / per;
+  }
+  if (groups > 65535) return TSB200_ERR_UNSUPPORTED;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas, (unsigned)groups);
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, linear_f32_kernel<BITS, MT, R, GATED>, p));
+  return TSB200_OK;
+}
+
+template <int BITS>
+int launch_bits(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
+  // tokens per warp, and rows so that 32 sums fill the lanes where the tokens do not (few tokens: fewer rows, more warps)
+  if (gated) {
+    if (p.M == 1) return launch_cfg<BITS, 1, 2, true>(p, pdl, s);
+    if (p.M <= 2) return launch_cfg<BITS, 2, 2, true>(p, pdl, s);
+    if (p.M <= 4) return launch_cfg<BITS, 4, 2, true>(p, pdl, s);
+    return launch_cfg<BITS, 8, 2, true>(p, pdl, s);
+  }
+  if (p.M == 1) return launch_cfg<BITS, 1, 2, false>(p, pdl, s);
+  if (p.M <= 2) return launch_cfg<BITS, 2, 2, false>(p, pdl, s);
+  if (p.M <= 4) return launch_cfg<BITS, 4, 4, false>(p, pdl, s);
+  return launch_cfg<BITS, 8, 4, false>(p, pdl, s);
+}
+
+// Tiles pay where K is short (up to two staged steps of the lanes) or where they fill most of the machine: with few tiles and a long
+// K the lane kernel has more warps (128 tokens, 384 x 896: 13 us there, 20 in 12 tiles).
+bool use_tiles(const F32Params& p, int bits) {
+  if (bits != 32 || p.M < 16) return false;
+  int64_t tiles = 0;
+  for (int i = 0; i < p.nseg; ++i) {
+    tiles += (p.seg[i].n + kTN - 1) / kTN;
+    if (!aligned(p.seg[i].x, 16) || (p.seg[i].x2 && !aligned(p.seg[i].x2, 16))) return false;
+  }
+  return p.K <= 256 || tiles * ((p.M + kTM - 1) / kTM) >= 96;
+}
+int launch_tiles(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
+  int ctas = 0;
+  for (int i = 0; i < p.nseg; ++i) {
+    p.seg[i].cta0 = ctas;
+    ctas += (p.seg[i].n + kTN - 1) / kTN;
+  }
+  const int groups = (p.M + kTM - 1) / kTM;
+  if (groups > 65535) return TSB200_ERR_UNSUPPORTED;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas, (unsigned)groups);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  TSB_CUDA(gated ? cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<true>, p) : cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<false>, p));
+  return TSB200_OK;
+}
+
+int launch_any(F32Params& p, int bits, bool gated, bool pdl, cudaStream_t s) {
+  if (use_tiles(p, bits)) return launch_tiles(p, gated, pdl, s);
+  switch (bits) {
+    case 1: return launch_bits<1>(p, gated, pdl, s);
+    case 2: return launch_bits<2>(p, gated, pdl, s);
+    case 4: return launch_bits<4>(p, gated, pdl, s);
+    case 8: return launch_bits<8>(p, gated, pdl, s);
+    default: return launch_bits<32>(p, gated, pdl, s);
+  }
+}
+
+int64_t row_bytes(int64_t K, int bits) { return bits == 32 ? K * 4 : (int64_t)tsb200_packed_row_bytes(K, bits); }
+
+}  // namespace
+
+// n matrices [N_i, K] of one container as one launch; x[i] [M, K], y[i] [M, N_i].
+int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s) {
+  F32Params p = {};
+  if (n < 1 || n > kMaxSegs || M < 1 || M > 65535 * 8 || g[0].K > (1 << 30)) return TSB200_ERR_UNSUPPORTED;
+  for (int i = 0; i < n; ++i) {
+    if (g[i].K != g[0].K || g[i].N > (1 << 28)) return TSB200_ERR_UNSUPPORTED;
+    Seg& sg = p.seg[i];
+    sg.w = (const uint8_t*)g[i].W;
+    sg.scale = bits == 32 ? nullptr : g[i].scale;
+    sg.bias = (const float*)g[i].bias;
+    sg.x = (const float*)g[i].x;
+    sg.y = (float*)g[i].y;
+    sg.n = (int)g[i].N;
+  }
+  p.nseg = n;
+  p.M = (int)M;
+  p.K = (int)g[0].K;
+  p.row_bytes = row_bytes(g[0].K, bits);
+  return launch_any(p, bits, false, pdl, s);
+}
+
+// y = silu(x_gate . gate^T) * (x_up . up^T), both [N, K] of one container.
+int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s) {
+  F32Params p = {};
+  if (gate.K != up.K || gate.N != up.N || M < 1 || M > 65535 * 8 || gate.K > (1 << 30) || gate.N > (1 << 28)) return TSB200_ERR_UNSUPPORTED;
+  Seg& sg = p.seg[0];
+  sg.w = (const uint8_t*)gate.W; sg.w2 = (const uint8_t*)up.W;
+  sg.scale = bits == 32 ? nullptr : gate.scale; sg.scale2 = bits == 32 ? nullptr : up.scale;
+  sg.bias = (const float*)gate.bias; sg.bias2 = (const float*)up.bias;
+  sg.x = (const float*)gate.x; sg.x2 = (const float*)up.x;
+  sg.y = (float*)gate.y;
+  sg.n = (int)gate.N;
+  p.nseg = 1;
+  p.M = (int)M;
+  p.K = (int)gate.K;
+  p.row_bytes = row_bytes(gate.K, bits);
+  return launch_any(p, bits, true, pdl, s);
+}
+
+}  // namespace tsb

@@ -38,6 +38,18 @@ bool chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, const t
          (d->rank == 0 || gv_supported(b, M, d->rank, d->in_features)) &&
          gv_supported(b, M, d->out_features, d->rank > 0 ? d->rank : d->in_features);
 }
+// fp32 layers the FMA kernel takes as a chain: gate and up alike, dense or packed.
+bool f32_chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, const tsb200_linear_desc* d) {
+  auto ok = [](const tsb200_linear_desc* l) {
+    auto factor = [](int bits, const void* p, const float* scale, int64_t k) {
+      return (bits == 32 && k % 8 == 0 && p) || ((bits == 1 || bits == 2 || bits == 4 || bits == 8) && p && scale);
+    };
+    if (l->act_dtype != TSB200_F32 || l->in_features <= 0 || l->out_features <= 0 || l->rank < 0) return false;
+    if (l->rank > 0 && !(factor(l->v_bits, l->v, l->v_scale, l->in_features) && aligned(l->v, 16))) return false;
+    return factor(l->u_bits, l->u, l->u_scale, l->rank > 0 ? l->rank : l->in_features) && aligned(l->u, 16);
+  };
+  return ok(g) && ok(u) && ok(d) && g->u_bits == u->u_bits && g->rank == u->rank && (g->rank == 0 || g->v_bits == u->v_bits);
+}
 }  // namespace
 
 // Workspace layout: [region 0 | gate out | up out | act | h0 | h1 | h2].  Region 0 starts with the
@@ -178,6 +190,28 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
     }
     const int st = run_program_tcq(ps, n, gate->u_bits, M, ws + tc::kWsHeader, (int*)(ws + tc::kWsCounters),
                                    (int*)(ws + tc::kWsGridBar), (int*)ws, s);
+    if (st != TSB200_ERR_UNSUPPORTED) return st;
+  }
+  if (f32_chainable(gate, up, down)) {
+    // fp32: [gate V | up V] -> gated U -> down V -> down U on the FMA kernel, chained
+    const bool low = gate->rank > 0;
+    const int64_t kgu = low ? gate->rank : gate->in_features;
+    GemmSpec v[2] = {GemmSpec{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features},
+                     GemmSpec{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features}};
+    int st = low ? gemm_f32(v, 2, gate->v_bits, M, g_pdl != 0, s) : TSB200_OK;
+    if (st == TSB200_OK)
+      st = gemm_f32_gated(GemmSpec{gate->u, gate->u_scale, gate->bias, low ? h0 : x, buf_g, gate->out_features, kgu},
+                          GemmSpec{up->u, up->u_scale, up->bias, low ? h1 : x, buf_g, up->out_features, kgu}, gate->u_bits, M, low || g_pdl, s);
+    const void* dx = buf_g;
+    if (st == TSB200_OK && down->rank > 0) {
+      const GemmSpec dv{down->v, down->v_scale, nullptr, buf_g, h2, down->rank, down->in_features};
+      st = gemm_f32(&dv, 1, down->v_bits, M, true, s);
+      dx = h2;
+    }
+    if (st == TSB200_OK) {
+      const GemmSpec du{down->u, down->u_scale, down->bias, dx, y, down->out_features, down->rank > 0 ? down->rank : down->in_features};
+      st = gemm_f32(&du, 1, down->u_bits, M, true, s);
+    }
     if (st != TSB200_ERR_UNSUPPORTED) return st;
   }
   // composed path: three linear calls and the SwiGLU kernel; region 0 is their workspace

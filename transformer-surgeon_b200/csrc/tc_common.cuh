@@ -250,6 +250,9 @@ struct GvSpan {
   size_t bytes;
 };
 bool gv_supported(int bits, int64_t M, int64_t N, int64_t K);
+// fp32 activations (linear_f32.cu): n <= 4 matrices of one container and reduction length in one launch; a gate / up pair.
+int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s);
+int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s);
 int gv_gemm(const PhaseSpec& ps, int bits, int64_t M, bool pdl, const GvSpan* ahead, int n_ahead, cudaStream_t s);
 
 }  // namespace tsb

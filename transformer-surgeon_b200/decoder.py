@@ -48,6 +48,7 @@ class LayerWeights:
         self.ln1, self.ln2, self.o, self.gate, self.up, self.down = ln1, ln2, o, gate, up, down
         self.qkv, self.q, self.k, self.v = qkv, q, k, v
         self.mlp = ops.GatedMLP(gate, up, down)
+        self.qkv_group = None if qkv is not None else ops.LinearGroup([q, k, v])
 
 
 def fuse_rows(factors, biases, act_dtype):
@@ -115,6 +116,8 @@ class CompressedDecoder:
             for lin in (L.qkv, L.q, L.k, L.v, L.o, L.gate, L.up, L.down):
                 if lin is not None:
                     lin_ws = max(lin_ws, lin.workspace_bytes(B))
+            if L.qkv_group is not None:
+                lin_ws = max(lin_ws, L.qkv_group.workspace_bytes(B))
         lin_ws = max(lin_ws, lm_head.workspace_bytes(B))
         self.lin_ws = torch.zeros(lin_ws, dtype=torch.uint8, device=device)
         self.mlp_ws = torch.zeros(max(L.mlp.workspace_bytes(B) for L in layers), dtype=torch.uint8, device=device)
@@ -180,9 +183,7 @@ class CompressedDecoder:
                 k4 = self.qkv[:, H * d:(H + Hkv) * d].unflatten(1, (Hkv, d)).unsqueeze(1)
                 v4 = self.qkv[:, (H + Hkv) * d:].unflatten(1, (Hkv, d)).unsqueeze(1)
             else:
-                L.q(self.xn, out=self.qb, ws=self.lin_ws)
-                L.k(self.xn, out=self.kb, ws=self.lin_ws)
-                L.v(self.xn, out=self.vb, ws=self.lin_ws)
+                L.qkv_group(self.xn, (self.qb, self.kb, self.vb), ws=self.lin_ws)
                 n += sum(2 if l.rank else 1 for l in (L.q, L.k, L.v))
                 q4, k4, v4 = self.qb.view(B, 1, H, d), self.kb.view(B, 1, Hkv, d), self.vb.view(B, 1, Hkv, d)
             self.kv[li].rope_append(q4, k4, v4, rope, seq_lens=self.write_pos); n += 1
@@ -313,6 +314,9 @@ class CompressedDecoder:
         rope = (self.cos, self.sin)
         resid = self.embed[ids.reshape(-1)].contiguous()                # [B*T, hidden]
         delta = None
+        self.seq_lens.fill_(T)                                          # appends take their positions from `zeros`
+        status = self.attn_ws[ops.ATTN_STATUS_OFFSET:ops.ATTN_STATUS_OFFSET + 4]
+        sequences = ops.query_sequences(self.kv[0], B, T, T, self.seq_lens) if c.dtype == torch.float32 else None
         for li, L in enumerate(self.layers):
             xn = ops.add_rmsnorm(resid, delta, L.ln1, c.rms_eps, c.norm_variant)
             if L.qkv is not None:
@@ -321,15 +325,15 @@ class CompressedDecoder:
                 k4 = qkv[:, H * d:(H + Hkv) * d].unflatten(1, (Hkv, d)).unflatten(0, (B, T))
                 v4 = qkv[:, (H + Hkv) * d:].unflatten(1, (Hkv, d)).unflatten(0, (B, T))
             else:
-                q4, k4, v4 = L.q(xn).view(B, T, H, d), L.k(xn).view(B, T, Hkv, d), L.v(xn).view(B, T, Hkv, d)
+                q, k, v = L.qkv_group(xn)
+                q4, k4, v4 = q.view(B, T, H, d), k.view(B, T, Hkv, d), v.view(B, T, Hkv, d)
             q4, k4, v4 = q4.contiguous(), k4.contiguous(), v4.contiguous()
             kv = self.kv[li]
             if kv.k_scale is not None:
                 kv.set_fp8_scales(k4, v4, rope=rope, pos0=zeros)
             kv.rope_append(q4, k4, v4, rope, seq_lens=zeros)            # q4 rotated in place
-            self.seq_lens.fill_(T)
             # causal attention of the chunk over the DEQUANTIZED cache (what every attention read sees)
-            att = ops.prefill_attention(kv, q4, T, status=self.attn_ws[ops.ATTN_STATUS_OFFSET:ops.ATTN_STATUS_OFFSET + 4])
+            att = ops.prefill_attention(kv, q4, T, status=status, sequences=sequences)
             delta = L.o(att.view(B * T, H * d))
             xn = ops.add_rmsnorm(resid, delta, L.ln2, c.rms_eps, c.norm_variant)
             delta = L.mlp(xn)
@@ -339,7 +343,6 @@ class CompressedDecoder:
         ops.add_rmsnorm(self.resid, dl, self.final_norm, c.rms_eps, c.norm_variant, out=self.xn)
         self.lm_head(self.xn, out=self.logits, ws=self.lin_ws)
         torch.argmax(self.logits, dim=-1, out=self.next_tokens)
-        self.seq_lens.fill_(T)
         return self.logits
 
     @torch.no_grad()

@@ -313,6 +313,34 @@ class PackedLinear:
         return int(ws[:4].view(torch.int32).item())
 
 
+class LinearGroup:
+    """PackedLinear layers that read the same x (q, k, v of a decoder layer) behind one call; equal to calling them in turn."""
+
+    def __init__(self, layers):
+        self.layers = list(layers)
+        n = len(self.layers)
+        self._descs = (C.POINTER(LinearDesc) * n)(*(C.pointer(l.desc) for l in self.layers))
+        self._ptrs = C.c_void_p * n
+
+    def workspace_bytes(self, M):
+        return int(_lib.load().tsb200_linear_group_workspace_bytes(self._descs, len(self.layers), M))
+
+    def __call__(self, x, outs=None, ws=None):
+        x = _cuda(x, "x")
+        lead = x.shape[:-1]
+        M = lead.numel()
+        if any(x.dtype != l.act_dtype for l in self.layers):
+            raise TypeError(f"x is {x.dtype}, a layer was packed for another type")
+        if outs is None:
+            outs = [x.new_empty((*lead, l.out_features)) for l in self.layers]
+        if ws is None:
+            ws = workspace(x.device, self.workspace_bytes(M))
+        ptrs = self._ptrs(*(o.data_ptr() for o in outs))
+        check(_lib.load().tsb200_linear_group(self._descs, len(self.layers), x.data_ptr(), ptrs, M, ws.data_ptr(), ws.numel(), _stream()),
+              "tsb200_linear_group")
+        return outs
+
+
 class GatedMLP:
     """down(silu(gate(x)) * up(x)): MLPGated.forward (blocks/mlp.py:171-185) on three PackedLinear."""
 
@@ -432,12 +460,21 @@ def kv_gather(kv, L, dtype=torch.bfloat16, seq_lens=None):
     return k, v
 
 
-def prefill_attention(kv, q, L, sm_scale=None, out=None, status=None, seq_lens=None):
+def query_sequences(kv, B, T, L, seq_lens=None):
+    """Lengths and block-table rows that make every query token of a prompt chunk a one-token sequence of the paged decode kernel
+    (fp32 prompts): query i of a sequence attends over its first L - T + i + 1 positions.  The same for every layer of a model."""
+    base = kv.seq_lens if seq_lens is None else seq_lens
+    lens = torch.arange(L - T + 1, L + 1, dtype=torch.int32, device=base.device).repeat(B)             # [B * T]
+    return torch.minimum(lens, base.repeat_interleave(T)), kv.block_table.repeat_interleave(T, dim=0)
+
+
+def prefill_attention(kv, q, L, sm_scale=None, out=None, status=None, seq_lens=None, sequences=None):
     """Causal attention of a prompt chunk: q [B, T, H, d] (heads dense, tokens evenly strided; bf16) over the first
     L >= T positions of the cache `kv` (query i at position L - T + i), reading the dequantized cache
     (blocks/mha.py:9-103 for T > 1).  bf16: head-major gather + tcgen05 kernel.  fp32: every query token becomes a
     one-token "sequence" of the paged decode kernel (block-table rows repeated, lengths L - T + i + 1), which reads
-    the pages directly in fp32 math.  Returns out [B, T, H, d]."""
+    the pages directly in fp32 math; `sequences` = query_sequences(...), for callers with several layers.  Returns
+    out [B, T, H, d]."""
     lib = _lib.load()
     B, T, H, d = q.shape
     if sm_scale is None:
@@ -445,13 +482,10 @@ def prefill_attention(kv, q, L, sm_scale=None, out=None, status=None, seq_lens=N
     if out is None:
         out = torch.empty((B, T, H, d), dtype=q.dtype, device=q.device)
     if q.dtype == torch.float32:
-        lens = (torch.arange(L - T + 1, L + 1, dtype=torch.int32, device=q.device)).repeat(B)          # [B * T]
-        base = kv.seq_lens if seq_lens is None else seq_lens
-        lens = torch.minimum(lens, base.repeat_interleave(T))
+        lens, table = sequences if sequences is not None else query_sequences(kv, B, T, L, seq_lens)
         view = PagedKV.__new__(PagedKV)
         view.__dict__.update(kv.__dict__)
-        view.block_table = kv.block_table.repeat_interleave(T, dim=0).contiguous()
-        view.seq_lens = lens
+        view.block_table, view.seq_lens = table, lens
         if kv.k_scale is not None:
             view.k_scale, view.v_scale = kv.k_scale.repeat_interleave(T, dim=0).contiguous(), kv.v_scale.repeat_interleave(T, dim=0).contiguous()
         qq = q.reshape(B * T, H, d) if q.is_contiguous() else q.contiguous().reshape(B * T, H, d)
