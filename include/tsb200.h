@@ -163,6 +163,9 @@ size_t tsb200_linear_argmax_workspace_bytes(const tsb200_linear_desc* d, int64_t
 int tsb200_linear_argmax(const tsb200_linear_desc* d, const void* x, int64_t* tokens, int64_t M,
                          void* workspace, size_t workspace_bytes, void* stream);
 
+/* tokens[m] = the column of the first maximum of row m of y [M, N] (NaN counts as largest): torch.argmax(y, -1). */
+int tsb200_argmax(const void* y, int dtype, int64_t M, int64_t N, int64_t* tokens, void* stream);
+
 /* Gated MLP block: y = down(silu(gate(x)) * up(x)).
  * Replaces: blocks/mlp.py:171-185 (MLPGated.forward: up_proj, gate_proj, activation * up, down_proj)
  * with SiLU as the activation (the Qwen2 / Llama choice).  gate and up map in -> inter, down maps

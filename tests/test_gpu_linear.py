@@ -333,3 +333,20 @@ def test_split_k_launches_repeat_bit_for_bit(cuda):
     finally:
         ops.set_pdl(old)
     assert ops.PackedLinear.device_status(device=x.device) == 0
+
+
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("M,N", [(1, 1), (3, 7), (2, 4097), (5, 50257), (2, 64)])
+def test_argmax_of_rows(cuda, name, M, N):
+    """Rows shorter than a cluster, misaligned rows, ties (the first maximum), negative rows, NaN, both zeros."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator().manual_seed(N)
+    y = torch.randn(M, N, generator=g).to(DT[name])
+    y[0] = -y[0].abs() - 1
+    if M > 1:
+        y[1, N // 2:] = y[1].max()
+    if M > 2:
+        y[2] = 0.0
+        y[2, 0] = -0.0
+        y[2, N - 1] = float("nan") if N > 5 else 0.0
+    assert torch.equal(ops.argmax(y.to(cuda)).cpu(), torch.argmax(y.float(), -1))

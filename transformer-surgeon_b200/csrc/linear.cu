@@ -42,6 +42,15 @@ extern "C" int tsb200_linear_argmax(const tsb200_linear_desc* d, const void* x, 
   return argmax_rows(extra, d->act_dtype, M, d->out_features, tokens, s);
 }
 
+extern "C" int tsb200_argmax(const void* y, int dtype, int64_t M, int64_t N, int64_t* tokens, void* stream) {
+  TSB_REQUIRE_DEVICE();
+  if (M < 0 || N <= 0) return TSB200_ERR_ARG;
+  if (dtype != TSB200_F32 && dtype != TSB200_BF16) return TSB200_ERR_UNSUPPORTED;
+  if (M == 0) return TSB200_OK;
+  if (!y || !tokens) return TSB200_ERR_ARG;
+  return argmax_rows(y, dtype, M, N, tokens, as_stream(stream));
+}
+
 namespace {
 bool f32_factor(int bits) { return bits == 32 || (bits <= 8); }
 

@@ -226,32 +226,57 @@ __global__ void argmax_finalize_kernel(const float* __restrict__ val, const int*
   if (threadIdx.x == 0) out[m] = si[0] == 0x7fffffff ? 0 : si[0];
 }
 
-// Argmax over stored logits y [M, N] (the route for heads the fused epilogue does not serve).
+// Argmax over stored logits y [M, N]: the first maximum of a row, NaN counting as largest (torch.argmax).  A cluster of eight
+// CTAs shares a row, 16-byte loads, one 64-bit key per candidate (order-preserving value bits, then the complement of the column),
+// exchanged through distributed shared memory.  [32, 128256] bf16: 42 us with the library reduction, about 5 here.
+constexpr int kArgRanks = 8, kArgThreads = 1024;
+__device__ __forceinline__ unsigned long long argmax_key(float v, unsigned col) {
+  const unsigned b = __float_as_uint(v + 0.f);                       // -0 counts as +0
+  const unsigned o = v != v ? 0xffffffffu : ((b >> 31) ? ~b : (b | 0x80000000u));
+  return ((unsigned long long)o << 32) | (unsigned)~col;
+}
 template <typename T>
-__global__ void argmax_rows_kernel(const T* __restrict__ y, int64_t N, int64_t* __restrict__ out) {
+__global__ void __launch_bounds__(kArgThreads) argmax_rows_kernel(const T* __restrict__ y, int64_t N, int64_t* __restrict__ out) {
+  __shared__ unsigned long long sw[kArgThreads / 32], srank[kArgRanks];
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float sv[256];
-  __shared__ int si[256];
-  const int64_t m = blockIdx.x;
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int64_t n = threadIdx.x; n < N; n += blockDim.x) {
-    const float v = to_f32<T>(y[m * N + n]);
-    if (v > bv) { bv = v; bi = (int)n; }               // ascending per thread: the first maximum is kept
-  }
-  sv[threadIdx.x] = bv;
-  si[threadIdx.x] = bi;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) {
-      const float v = sv[threadIdx.x + s];
-      const int i = si[threadIdx.x + s];
-      if (v > sv[threadIdx.x] || (v == sv[threadIdx.x] && i < si[threadIdx.x])) { sv[threadIdx.x] = v; si[threadIdx.x] = i; }
+  constexpr int E = 16 / sizeof(T);
+  const unsigned rank = blockIdx.x % kArgRanks;
+  const T* row = y + (int64_t)(blockIdx.x / kArgRanks) * N;
+  const int64_t len = ((N + kArgRanks - 1) / kArgRanks + E - 1) / E * E;
+  const int64_t c0 = rank * len, c1 = min(N, c0 + len);
+  unsigned long long best = 0;                                       // below every key of a column
+  if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+#pragma unroll 4
+    for (int64_t c = c0 + threadIdx.x * E; c < c1; c += kArgThreads * E) {
+      if (c + E <= c1) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(row + c));
+        const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+        for (int j = 0; j < E; ++j) best = max(best, argmax_key(to_f32<T>(e[j]), (unsigned)(c + j)));
+      } else {
+        for (int64_t j = c; j < c1; ++j) best = max(best, argmax_key(to_f32<T>(row[j]), (unsigned)j));
+      }
     }
-    __syncthreads();
+  } else {
+    for (int64_t c = c0 + threadIdx.x; c < c1; c += kArgThreads) best = max(best, argmax_key(to_f32<T>(row[c]), (unsigned)c));
   }
-  if (threadIdx.x == 0) out[m] = si[0] == 0x7fffffff ? 0 : si[0];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < kArgThreads / 32; ++i) best = max(best, sw[i]);
+    unsigned dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"(smem_u32(&srank[rank])));
+    asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(dst), "l"(best) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    best = srank[0];
+    for (int i = 1; i < kArgRanks; ++i) best = max(best, srank[i]);
+    out[blockIdx.x / kArgRanks] = (int64_t)(unsigned)~(unsigned)best;
+  }
 }
 
 // fp32 split-K buffer -> bf16 output.
@@ -359,8 +384,22 @@ int linear_argmax_tc(const tsb200_linear_desc* d, const void* x, int64_t* tokens
   return gemm_tc(d->u, 16, nullptr, d->bias, x, nullptr, M, d->in_features, d->out_features, nullptr, status, s, tokens, amax);
 }
 int argmax_rows(const void* y, int dtype, int64_t M, int64_t N, int64_t* tokens, cudaStream_t s) {
-  if (dtype == TSB200_F32) TSB_CUDA(launch_kernel(argmax_rows_kernel<float>, dim3((unsigned)M), dim3(256), 0, s, (const float*)y, N, tokens));
-  else TSB_CUDA(launch_kernel(argmax_rows_kernel<__nv_bfloat16>, dim3((unsigned)M), dim3(256), 0, s, (const __nv_bfloat16*)y, N, tokens));
+  if (N > 0xfffffffell || M * kArgRanks > 0x7fffffffll) return TSB200_ERR_UNSUPPORTED;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(M * kArgRanks));
+  cfg.blockDim = dim3(kArgThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kArgRanks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_pdl ? 2 : 1;
+  if (dtype == TSB200_F32) TSB_CUDA(cudaLaunchKernelEx(&cfg, argmax_rows_kernel<float>, (const float*)y, N, tokens));
+  else TSB_CUDA(cudaLaunchKernelEx(&cfg, argmax_rows_kernel<__nv_bfloat16>, (const __nv_bfloat16*)y, N, tokens));
   return TSB200_OK;
 }
 

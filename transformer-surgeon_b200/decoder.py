@@ -11,7 +11,7 @@ The `variant=1` norm and rope base of the reference's own blocks path (blocks/de
 blocks/norm.py:8-23) are selectable through DecoderConfig.
 
 There is no CPU path: every tensor lives on the GPU and every op is a libtsb200 kernel, except
-the embedding gather, the final argmax and integer bookkeeping (torch).
+the embedding gather and integer bookkeeping (torch).
 """
 from dataclasses import dataclass
 
@@ -212,8 +212,8 @@ class CompressedDecoder:
             self.lm_head.argmax(self.xn, out=self.next_tokens, ws=self.head_ws); n += 2
             self.kernel_launches_per_step = n
             return None
-        self.lm_head(self.xn, out=self.logits, ws=self.lin_ws); n += 1
-        torch.argmax(self.logits, dim=-1, out=self.next_tokens)
+        self.lm_head(self.xn, out=self.logits, ws=self.lin_ws); n += 2
+        ops.argmax(self.logits, out=self.next_tokens)
         self.kernel_launches_per_step = n
         return self.logits
 
@@ -342,7 +342,7 @@ class CompressedDecoder:
         self.resid.copy_(last)
         ops.add_rmsnorm(self.resid, dl, self.final_norm, c.rms_eps, c.norm_variant, out=self.xn)
         self.lm_head(self.xn, out=self.logits, ws=self.lin_ws)
-        torch.argmax(self.logits, dim=-1, out=self.next_tokens)
+        ops.argmax(self.logits, out=self.next_tokens)
         return self.logits
 
     @torch.no_grad()

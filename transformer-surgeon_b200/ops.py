@@ -533,6 +533,16 @@ def paged_decode_attention(kv, q, max_seq_len, sm_scale=None, out=None, ws=None,
 
 
 # ---------------------------------------------------------------- small ops --------
+def argmax(y, out=None):
+    """Column of the first maximum of every row of y [M, N] (NaN counts as largest), int64 [M]: torch.argmax(y, -1)."""
+    y = _cuda(y, "y")
+    M, N = y.shape
+    if out is None:
+        out = torch.empty(M, dtype=torch.int64, device=y.device)
+    check(_lib.load().tsb200_argmax(y.data_ptr(), _dt(y), M, N, out.data_ptr(), _stream()), "tsb200_argmax")
+    return out
+
+
 def rope_(x, cos, sin, pos0=None):
     """In-place half-split RoPE on x [B, T, heads, d] (blocks/rope.py:140-173)."""
     lib = _lib.load()
