@@ -99,6 +99,13 @@ int tsb200_quantize_weight(const void* w, int dtype, int64_t rows, int64_t cols,
 int tsb200_pack_codes(const int8_t* codes, int64_t rows, int64_t cols, int bits,
                       uint8_t* packed, int32_t* zero_flag, void* stream);
 
+/* tsb200_quantize_weight and tsb200_pack_codes in one pass: the same codes and scales, without the codes in memory.  Rows of
+ * more than 32768 columns return TSB200_ERR_UNSUPPORTED (use the two calls).  packed: 8-byte aligned. */
+int tsb200_quantize_pack(const void* w, int dtype, int64_t rows, int64_t cols,
+                         int precision, int per_channel, float eps, int bits,
+                         uint8_t* packed, float* scales, int32_t* zero_flag,
+                         void* workspace, size_t workspace_bytes, void* stream);
+
 /* packed -> codes int8 [rows, cols]. */
 int tsb200_unpack_codes(const uint8_t* packed, int64_t rows, int64_t cols, int bits,
                         int8_t* codes, void* stream);

@@ -52,6 +52,32 @@ def test_quantize_large_matrix_against_oracle(cuda, name, p):
     assert np.array_equal(f.reconstruct(DT[name]).float().cpu().numpy(), wq.dequantize(q, s, name))
 
 
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("p", [8, 4, 3, 2, "binary"])
+@pytest.mark.parametrize("gran", ["per_channel", "per_tensor"])
+@pytest.mark.parametrize("cols", [1, 1024, 1027, 4096, 4104, 16392, 32769])
+def test_quantize_and_pack_in_one_pass(cuda, name, p, gran, cols):
+    """Every split of a row over threads (1024 / 4096 / 16384 / 32768 columns) and one column beyond, padding,
+    a zero row, divisors at the ends of the exponent range, rows that are not a multiple of a CTA's."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator().manual_seed(7)
+    w = (torch.randn(9, cols, generator=g) * 0.02).to(DT[name])
+    w[w == 0] = 0.01
+    w[3] *= 1e-22
+    w[4] *= 1e22
+    if cols != 1024:
+        w[5] = 0                                  # binary: the 2-bit container
+    f = ops.Factor.quantize(w.to(cuda), p, gran, 0.0 if cols == 4096 else 1e-6)
+    codes, scales = ops.quantize_weight(w.to(cuda), p, gran, 0.0 if cols == 4096 else 1e-6)
+    if cols != 4096:
+        q, s = wq.quantize_vanilla(w.float().numpy(), p, 1e-6, gran, name)
+        assert np.array_equal(codes.cpu().numpy(), q)
+    assert torch.equal(f.scales, scales)
+    q = codes.cpu().numpy()
+    assert f.bits == wq.container_bits(p, q)
+    assert np.array_equal(f.data.cpu().numpy(), wq.pack_codes(q, f.bits))
+
+
 def test_ragged_columns_and_empty(cuda):
     from transformer_surgeon_b200 import ops
     w = torch.randn(7, 100).to(cuda)                       # 100 columns -> padded to 128

@@ -52,6 +52,7 @@ SIGNATURES = {
     "tsb200_packed_row_bytes": (_sz, [_i64, _i32]),
     "tsb200_quantize_weight": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _f32, _vp, _vp, _vp, _sz, _vp]),
     "tsb200_pack_codes": (_i32, [_vp, _i64, _i64, _i32, _vp, _vp, _vp]),
+    "tsb200_quantize_pack": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _f32, _i32, _vp, _vp, _vp, _vp, _sz, _vp]),
     "tsb200_unpack_codes": (_i32, [_vp, _i64, _i64, _i32, _vp, _vp]),
     "tsb200_dequantize_weight": (_i32, [_vp, _vp, _i64, _i64, _i32, _i32, _vp, _vp]),
     "tsb200_linear_workspace_bytes": (_sz, [_LD, _i64]),

@@ -5,6 +5,7 @@
 // scale+eps, w/(scale+eps)) is rounded to bf16 before the next op, exactly as the
 // chain of torch ops does; rounding of the quotient to an integer is half-to-even.
 #include "common.cuh"
+#include <type_traits>
 
 namespace tsb {
 
@@ -155,6 +156,240 @@ __global__ void dequantize_kernel(const uint8_t* __restrict__ packed, const floa
   }
 }
 
+// ---- quantize and pack in one pass --------------------------------------------------------------------------------------
+// Bound by the weights' one trip from memory (a 14336 x 4096 bf16 matrix: 147 MB, 22 us) and, next to it, by the arithmetic: the
+// quotient that vanilla.py prescribes is an IEEE division per element.  TPR threads own a row and keep it in registers between the
+// statistic and the codes (IT units of 8 columns each), the codes never exist as bytes, and the quotient by a divisor that the
+// whole row shares comes from its correctly rounded reciprocal y: q = w y, r = w - d q (exact), q + r y - correctly rounded by
+// Markstein's theorem (Computation of elementary functions on the IBM RISC System/6000 processor, 1990) as long as nothing leaves
+// the normal range, which the divisor's range guarantees for every quotient that does not round to zero; other divisors divide.
+// Together with its packing launch the two-pass form took 177 us on that matrix; this one takes 36 us.  The row stays in the weights'
+// own type (as floats: 88 registers a thread, too few warps in flight, 108 us), and bf16 codes of up to four bits are rounded and
+// clamped in pairs.
+//
+// Eight columns in the weights' own type (bf16: as four packed pairs).
+template <typename T> struct Unit;
+template <> struct Unit<__nv_bfloat16> {
+  unsigned u[4];
+  __device__ __forceinline__ void load(const __nv_bfloat16* row, int64_t c, int64_t cols, bool vec) {
+    if (vec && c + 8 <= cols) {
+      const uint4 a = __ldg(reinterpret_cast<const uint4*>(row + c));
+      u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned lo = c + 2 * i < cols ? __bfloat16_as_ushort(row[c + 2 * i]) : 0, hi = c + 2 * i + 1 < cols ? __bfloat16_as_ushort(row[c + 2 * i + 1]) : 0;
+        u[i] = lo | (hi << 16);
+      }
+    }
+  }
+  __device__ __forceinline__ float at(int j) const { return __uint_as_float((j & 1) ? u[j >> 1] & 0xffff0000u : u[j >> 1] << 16); }
+  __device__ __forceinline__ float amax(float m) const {
+    __nv_bfloat162 a = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&u[0]));
+#pragma unroll
+    for (int i = 1; i < 4; ++i) a = __hmax2(a, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&u[i])));
+    return fmaxf(m, fmaxf(__low2float(a), __high2float(a)));
+  }
+};
+template <> struct Unit<float> {
+  float f[8];
+  __device__ __forceinline__ void load(const float* row, int64_t c, int64_t cols, bool vec) {
+    if (vec && c + 8 <= cols) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(row + c)), b = __ldg(reinterpret_cast<const float4*>(row + c + 4));
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = c + i < cols ? row[c + i] : 0.f;
+    }
+  }
+  __device__ __forceinline__ float at(int j) const { return f[j]; }
+  __device__ __forceinline__ float amax(float m) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(f[i]));
+    return m;
+  }
+};
+
+// The unit's codes in the low BITS bits of q[0..7] (the other bits are anything).  y: correctly rounded 1 / denom.
+template <typename T, int BITS, bool DIVIDE>
+__device__ __forceinline__ void unit_codes(const Unit<T>& v, float denom, float y, float qmax, unsigned (&q)[8]) {
+  float p[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float x = v.at(j);
+    if (DIVIDE) {
+      p[j] = __fdiv_rn(x, denom);
+    } else {
+      p[j] = x * y;
+      p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);                        // bf16: enough (exact where the quotient is; no other quotient of
+      if (sizeof(T) == 4) p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);    // two 8-bit numbers is within 2^-17 of a rounding boundary)
+    }
+  }
+  if constexpr (sizeof(T) == 2 && BITS < 8) {
+    // packed: round to bf16, clamp, and add 192: bf16 numbers of [128, 256) are whole, so the sum is rounded half-to-even to a whole
+    // number that stands in its low bits (|code| <= 7)
+    const __nv_bfloat162 hi = __float2bfloat162_rn(qmax), lo = __float2bfloat162_rn(-qmax), magic = __float2bfloat162_rn(192.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __nv_bfloat162 h = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+      h = __hadd2_rn(__hmin2(__hmax2(h, lo), hi), magic);
+      const unsigned b = *reinterpret_cast<unsigned*>(&h);
+      q[2 * i] = b;
+      q[2 * i + 1] = b >> 16;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)     // the bounds are whole numbers: clamping before or after rounding is the same; 1.5 * 2^23: half-to-even
+      q[j] = __float_as_uint(fminf(fmaxf(rnd<T>(p[j]), -qmax), qmax) + 12582912.0f);
+  }
+}
+
+// Reductions over the TPR threads of a row.
+template <int TPR> __device__ __forceinline__ float row_max(float v, float* sh) {
+  v = warp_max(v);
+  if (TPR > 32) {
+    const int w = threadIdx.x >> 5, w0 = w / (TPR / 32) * (TPR / 32);
+    if ((threadIdx.x & 31) == 0) sh[w] = v;
+    __syncthreads();
+    v = sh[w0];
+#pragma unroll
+    for (int i = 1; i < TPR / 32; ++i) v = fmaxf(v, sh[w0 + i]);
+  }
+  return v;
+}
+template <int TPR> __device__ __forceinline__ double row_sum(double v, double* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (TPR > 32) {
+    const int w = threadIdx.x >> 5, w0 = w / (TPR / 32) * (TPR / 32);
+    if ((threadIdx.x & 31) == 0) sh[w] = v;
+    __syncthreads();
+    v = sh[w0];
+#pragma unroll
+    for (int i = 1; i < TPR / 32; ++i) v += sh[w0 + i];
+  }
+  return v;
+}
+
+// The unit's eight codes (as bits of `bits` each) in the pair-interleaved order of the container word that holds them.
+template <int BITS> __device__ __forceinline__ unsigned place(const unsigned (&q)[8], int64_t c) {
+  constexpr unsigned mask = BITS == 8 ? 0xffu : (1u << BITS) - 1u;
+  constexpr int per = 32 / BITS;
+  const int f0 = (int)(c % per) >> 1;          // first field of the unit's even columns
+  unsigned w = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w |= ((q[2 * i] & mask) << (BITS * i)) | ((q[2 * i + 1] & mask) << (BITS * (i + per / 2)));
+  return BITS == 4 ? w : w << (BITS * f0);
+}
+
+template <typename T, int TPR, int IT, int BITS>
+__global__ void __launch_bounds__(256)
+quantize_pack_kernel(const T* __restrict__ w, int64_t rows, int64_t cols, int precision, int per_channel, float eps, int64_t row_bytes,
+                     uint8_t* __restrict__ packed, float* __restrict__ scales, const TensorStats* st, int32_t* zero_flag) {
+  __shared__ float shf[8];
+  __shared__ double shd[8];
+  const int64_t r = (int64_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
+  const int t = threadIdx.x % TPR;
+  const bool live = r < rows;                  // every thread takes part in the reductions
+  const T* row = w + (live ? r : rows - 1) * cols;
+  const bool vec = cols % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+  const int64_t units = row_bytes / BITS;      // of 8 columns, the padding to 64 columns included
+  Unit<T> v[IT];
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const int64_t u = t + (int64_t)i * TPR;
+    if (u < units) v[i].load(row, u * 8, cols, vec);
+    else v[i] = Unit<T>{};
+  }
+  float scale, denom = 1.f, y = 1.f;
+  const float qmax = (float)((1 << ((precision ? precision : 2) - 1)) - 1);
+  bool divide = false;
+  if (precision == 0) {
+    double s = 0.0;
+    if (per_channel) {
+#pragma unroll
+      for (int i = 0; i < IT; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += (double)fabsf(v[i].at(j));
+      s = row_sum<TPR>(s, shd) / (double)cols;
+    } else {
+      s = st->abs_sum / (double)(rows * cols);
+    }
+    scale = rnd<T>((float)s);
+  } else {
+    float m = 0.f;
+    if (per_channel) {
+#pragma unroll
+      for (int i = 0; i < IT; ++i)
+        m = v[i].amax(m);
+      m = row_max<TPR>(m, shf);
+    } else {
+      m = __uint_as_float(st->amax_bits);
+    }
+    scale = rnd<T>(__fdiv_rn(m, qmax));
+    denom = rnd<T>(__fadd_rn(scale, eps));
+    divide = !(denom >= 1e-18f && denom <= 1e18f);
+    y = __frcp_rn(denom);
+  }
+  if (!live) return;
+  if (t == 0) scales[r] = scale;
+  uint8_t* out = packed + r * row_bytes;
+  bool zero = false;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const int64_t u = t + (int64_t)i * TPR;
+    unsigned q[8];
+    if (precision == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float x = v[i].at(j);
+        const int sgn = (x > 0.f) - (x < 0.f);
+        if (BITS == 1) zero |= sgn == 0 && u < units && u * 8 + j < cols;
+        q[j] = BITS == 1 ? (unsigned)(sgn > 0) : (unsigned)sgn;
+      }
+    } else if (divide) {
+      unit_codes<T, BITS, true>(v[i], denom, y, qmax, q);
+    } else {
+      unit_codes<T, BITS, false>(v[i], denom, y, qmax, q);
+    }
+    if constexpr (BITS == 8) {
+      if (u < units) {
+        unsigned lo = 0, hi = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { lo |= (q[j] & 0xffu) << (8 * j); hi |= (q[4 + j] & 0xffu) << (8 * j); }
+        *reinterpret_cast<uint2*>(out + u * 8) = make_uint2(lo, hi);
+      }
+    } else {
+      unsigned word = u < units ? place<BITS>(q, u * 8) : 0u;
+      // a word of 2-bit codes is two units, one of 1-bit codes four: neighbouring lanes (units are a multiple of 8 per row)
+      if (BITS <= 2) word |= __shfl_xor_sync(0xffffffffu, word, 1);
+      if (BITS == 1) word |= __shfl_xor_sync(0xffffffffu, word, 2);
+      constexpr int per = BITS == 4 ? 1 : (BITS == 2 ? 2 : 4);
+      if (u < units && u % per == 0) *reinterpret_cast<unsigned*>(out + u * BITS) = word;
+    }
+  }
+  if (BITS == 1 && zero && zero_flag) *zero_flag = 1;
+}
+
+// False: rows too long for the registers of 256 threads.
+template <typename T, int BITS>
+bool launch_quantize_pack(const T* w, int64_t rows, int64_t cols, int precision, int per_channel, float eps, uint8_t* packed, float* scales,
+                          const TensorStats* st, int32_t* zero_flag, cudaStream_t s) {
+  const int64_t rb = (int64_t)tsb200_packed_row_bytes(cols, BITS), units = rb / BITS;
+  auto go = [&](auto tpr, auto it) {
+    constexpr int TPR = decltype(tpr)::value, IT = decltype(it)::value;
+    const int64_t blocks = (rows + 256 / TPR - 1) / (256 / TPR);
+    quantize_pack_kernel<T, TPR, IT, BITS><<<(unsigned)blocks, 256, 0, s>>>(w, rows, cols, precision, per_channel, eps, rb, packed, scales, st, zero_flag);
+    return true;
+  };
+  // as few threads per row as its units fit in registers, eight units to a thread where possible (64 registers)
+  if (units <= 32 * 4) return go(std::integral_constant<int, 32>{}, std::integral_constant<int, 4>{});
+  if (units <= 64 * 8) return go(std::integral_constant<int, 64>{}, std::integral_constant<int, 8>{});
+  if (units <= 256 * 8) return go(std::integral_constant<int, 256>{}, std::integral_constant<int, 8>{});
+  if (units <= 256 * 16) return go(std::integral_constant<int, 256>{}, std::integral_constant<int, 16>{});
+  return false;
+}
+
 inline int grid_for(int64_t n, int block) {
   int64_t g = (n + block - 1) / block;
   const int64_t cap = 148 * 16;
@@ -198,6 +433,43 @@ int tsb200_quantize_weight(const void* w, int dtype, int64_t rows, int64_t cols,
     quantize_rows_kernel<float><<<(unsigned)rows, 256, 0, s>>>((const float*)w, rows, cols, precision, per_channel, eps, codes, scales, st);
   else
     quantize_rows_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, s>>>((const __nv_bfloat16*)w, rows, cols, precision, per_channel, eps, codes, scales, st);
+  TSB_LAUNCH_CHECK();
+  return TSB200_OK;
+}
+
+int tsb200_quantize_pack(const void* w, int dtype, int64_t rows, int64_t cols, int precision, int per_channel, float eps, int bits,
+                         uint8_t* packed, float* scales, int32_t* zero_flag, void* workspace, size_t workspace_bytes, void* stream) {
+  TSB_REQUIRE_DEVICE();
+  if (rows < 0 || cols < 0) return TSB200_ERR_ARG;
+  if (!(precision == 0 || (precision >= 2 && precision <= 8))) return TSB200_ERR_UNSUPPORTED;
+  if (dtype != TSB200_F32 && dtype != TSB200_BF16) return TSB200_ERR_UNSUPPORTED;
+  if (!(bits == 1 || bits == 2 || bits == 4 || bits == 8) || (precision != 0 && bits < precision) || (bits == 1 && precision != 0)) return TSB200_ERR_UNSUPPORTED;
+  if (rows == 0 || cols == 0) return TSB200_OK;
+  if (!w || !packed || !scales || !aligned(packed, 8)) return TSB200_ERR_ARG;
+  if (rows > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
+  cudaStream_t s = as_stream(stream);
+  TensorStats* st = nullptr;
+  if (!per_channel) {
+    if (!workspace || !aligned(workspace, 8)) return TSB200_ERR_ARG;
+    if (workspace_bytes < sizeof(TensorStats)) return TSB200_ERR_WORKSPACE;
+    st = (TensorStats*)workspace;
+    TSB_CUDA(cudaMemsetAsync(st, 0, sizeof(TensorStats), s));
+    const int64_t n = rows * cols;
+    if (dtype == TSB200_F32) tensor_stats_kernel<float><<<grid_for(n, 256), 256, 0, s>>>((const float*)w, n, st);
+    else tensor_stats_kernel<__nv_bfloat16><<<grid_for(n, 256), 256, 0, s>>>((const __nv_bfloat16*)w, n, st);
+    TSB_LAUNCH_CHECK();
+  }
+  bool done;
+#define TSB_GO(TT)                                                                                                                         \
+  switch (bits) {                                                                                                                          \
+    case 1: done = launch_quantize_pack<TT, 1>((const TT*)w, rows, cols, precision, per_channel, eps, packed, scales, st, zero_flag, s); break; \
+    case 2: done = launch_quantize_pack<TT, 2>((const TT*)w, rows, cols, precision, per_channel, eps, packed, scales, st, zero_flag, s); break; \
+    case 4: done = launch_quantize_pack<TT, 4>((const TT*)w, rows, cols, precision, per_channel, eps, packed, scales, st, zero_flag, s); break; \
+    default: done = launch_quantize_pack<TT, 8>((const TT*)w, rows, cols, precision, per_channel, eps, packed, scales, st, zero_flag, s); break; \
+  }
+  if (dtype == TSB200_F32) { TSB_GO(float); } else { TSB_GO(__nv_bfloat16); }
+#undef TSB_GO
+  if (!done) return TSB200_ERR_UNSUPPORTED;
   TSB_LAUNCH_CHECK();
   return TSB200_OK;
 }

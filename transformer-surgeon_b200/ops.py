@@ -163,8 +163,23 @@ class Factor:
 
     @staticmethod
     def quantize(w, precision, granularity="per_channel", eps=1e-6):
-        codes, scales = quantize_weight(w, precision, granularity, eps)
-        return Factor.from_codes(codes, scales, precision)
+        w = _cuda(w, "w")
+        rows, cols = w.shape
+        code, bits = precision_code(precision), container_bits(precision)
+        per_channel = granularity == "per_channel"
+        scales = torch.empty(rows, dtype=torch.float32, device=w.device)
+        ws = None if per_channel else torch.empty(16, dtype=torch.uint8, device=w.device)
+        while True:
+            packed = torch.empty((rows, packed_row_bytes(cols, bits)), dtype=torch.uint8, device=w.device)
+            flag = torch.zeros(1, dtype=torch.int32, device=w.device) if bits == 1 else None
+            st = _lib.load().tsb200_quantize_pack(w.data_ptr(), _dt(w), rows, cols, code, int(per_channel), float(eps), bits, packed.data_ptr(),
+                                                  scales.data_ptr(), _p(flag), _p(ws), 16, _stream())
+            if st == _lib.ERR_UNSUPPORTED and rows and cols:         # rows too long for one pass
+                return Factor.from_codes(*quantize_weight(w, precision, granularity, eps), precision)
+            check(st, "tsb200_quantize_pack")
+            if flag is None or not bool(flag.item()):
+                return Factor(packed, scales, bits, rows, cols)
+            bits = container_bits(precision, has_zero=True)          # binary with zeros: the 2-bit container
 
     def codes(self):
         return unpack_codes(self.data, self.rows, self.cols, self.bits)
