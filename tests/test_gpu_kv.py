@@ -324,6 +324,41 @@ def test_rope_append_fused_equals_separate_calls(cuda, name):
     assert torch.equal(g1.k_pool, g2.k_pool) and torch.equal(g1.v_pool, g2.v_pool)
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("H,Hkv,d", [(14, 2, 64), (9, 9, 128)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_bulk_append_of_strided_prompts(cuda, fmt, name, H, Hkv, d, pad):
+    """Prompt chunks out of a fused projection buffer (pad: vectors off a 16-byte boundary), rotated with their queries: starts within
+    a page, ends within a page, pages covered whole and in part, more heads than warps."""
+    from transformer_surgeon_b200 import ops
+    rng = np.random.default_rng(19)
+    B, T = 4, 53
+    o, g = make_pair(fmt, B, 5, Hkv, d, cuda, rng)
+    start = np.array([0, 5, 16, 27], dtype=np.int32)
+    new_lens = np.array([53, 32, 16, 0], dtype=np.int32)
+    o.seq_lens[:] = start
+    g.seq_lens.copy_(torch.from_numpy(start))
+    cos, sin = oatt.rope_tables(d, 5e5, torch.arange(96))
+    rope = (cos.to(cuda), sin.to(cuda))
+    k, v = outlier_kv(rng, B, T, Hkv, d, DT[name])
+    q = torch.randn((B, T, H, d), generator=torch.Generator().manual_seed(3)).to(DT[name])
+    sync_scales(o, g, k, v, rope=rope)
+    buf = torch.zeros((B, T, (H + 2 * Hkv) * d + 2 * pad), dtype=DT[name], device=cuda)
+    q4 = buf[..., :H * d].unflatten(2, (H, d))
+    k4 = buf[..., H * d + pad:(H + Hkv) * d + pad].unflatten(2, (Hkv, d))
+    v4 = buf[..., (H + Hkv) * d + pad:(H + 2 * Hkv) * d + pad].unflatten(2, (Hkv, d))
+    q4.copy_(q); k4.copy_(k); v4.copy_(v)
+    g.rope_append(q4, k4, v4, rope, new_lens=torch.from_numpy(new_lens).to(cuda))
+    pos = torch.from_numpy(start.astype(np.int64))[:, None] + torch.arange(T)[None, :]
+    kr, qr = (torch.stack([oatt.apply_rope(x[b], cos[pos[b]], sin[pos[b]]) for b in range(B)]) for x in (k, q))
+    o.append(kr.float().numpy(), v.float().numpy(), new_lens=new_lens)
+    assert np.array_equal(g.k_pool.cpu().numpy(), o.k_pool)
+    assert np.array_equal(g.v_pool.cpu().numpy(), o.v_pool)
+    for b in range(B):
+        assert torch.equal(q4[b, :new_lens[b]].cpu(), qr[b, :new_lens[b]])
+
+
 def test_fp8_attention_after_append_under_dependent_launch(cuda):
     """One decode step's append -> attention pair with programmatic dependent launch on: the attention may fetch pages
     older than the newest token before the append has finished.  Lengths sit on, before and after page boundaries and

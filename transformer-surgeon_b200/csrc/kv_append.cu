@@ -202,160 +202,432 @@ __global__ void kv_append_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t q
   else quant_store<D, FMT, true>(x, lane, kv.v_pool + rec, slot, vscale);
 }
 
-// Bulk append (T >= 16 tokens per sequence, quantized formats): ONE CTA OWNS TWO consecutive PAGES of one (sequence, kv head).
-// Its 16 warps quantize the page's 16 tokens; K goes out token-major as above (one contiguous vector per warp).  V is
-// stored token-minor ([element][16 tokens], so that the decode kernels read consecutive tokens of one element from
-// consecutive bytes): written token by token that is one byte per 16-byte row and a partial sector per element.
-// Here the warps stage the page's V codes and scales in shared memory in the token-major form, and the CTA then
-// writes the record transposed, 16 bytes (one element row) per thread - whole sectors, fully coalesced.  A page the
-// append only partly covers (the first / last page of the range) keeps its other slots: those are written slot by slot.
-// Extra CTAs along x rotate the query heads in place.
-template <typename T, int D, int FMT>
-__global__ void __launch_bounds__(512)
-kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,
-                       const T* __restrict__ v, int64_t ks, int64_t vs_, int64_t Tn, const int32_t* __restrict__ new_lens,
-                       const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int64_t rope_rows,
-                       int64_t rec_bytes, int page_blocks) {
-  constexpr int VB = FMT == TSB200_KV_NVFP4 ? D / 2 : D;                  // bytes of V codes per token
-  constexpr int REC = FMT == TSB200_KV_INT8 ? 16 * D + 64 : (FMT == TSB200_KV_FP8 ? 16 * D : 9 * D);
-  __shared__ __align__(16) uint8_t stage[REC];                            // the page's V record in token-major form
-  pdl_launch_dependents();
-  pdl_wait();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t b = blockIdx.z;
-  const int h = blockIdx.y;
-  const int64_t n_b = new_lens ? min((int64_t)new_lens[b], Tn) : Tn;
-  const int64_t start = kv.seq_lens[b];
-  if ((int)blockIdx.x >= page_blocks) {
-    // ---- query rotation: 16 (token, head) vectors per CTA
-    if (q == nullptr || rope_cos == nullptr) return;
-    const int64_t idx = (((int64_t)blockIdx.x - page_blocks) * gridDim.y + blockIdx.y) * 16 + w;
-    if (idx >= Tn * qheads) return;
-    const int64_t j = idx / qheads;
-    const int qh = (int)(idx - j * qheads);
-    if (j >= n_b) return;
-    int64_t qp = start + j;
-    qp = qp < 0 ? 0 : (qp >= rope_rows ? rope_rows - 1 : qp);
-    float xq[D / 32];
-    T* dst = q + (b * Tn + j) * qs + (int64_t)qh * D;
-    load_vec<T, D>(dst, lane, xq, true, rope_cos + qp * (D / 2), rope_sin + qp * (D / 2));
+// ---- prompt chunks -------------------------------------------------------------------------------------------------------
+// Eight consecutive elements of a vector in the act dtype (bf16: as four packed pairs).
+template <typename T> struct Raw8;
+template <> struct Raw8<__nv_bfloat16> {
+  unsigned u[4];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, bool vec) {
+    if (vec) {
+      const uint4 a = *reinterpret_cast<const uint4*>(p);
+      u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < D / 32; ++i) dst[lane * (D / 32) + i] = from_f32<T>(xq[i]);
-    return;
-  }
-  // ---- pages 2 * blockIdx.x and 2 * blockIdx.x + 1 of the appended range (logical page start / 16 + ...), slot w.
-  // Both pages' vectors are requested before either is used (9 % faster for FP8 pages at 2048 tokens x batch 64; the
-  // exact divisions of the quantization rules are what bounds the kernel).
-  struct Page {
-    int64_t p;
-    bool valid, store, full;
-    uint8_t *krec, *vrec;
-  } pg[2];
-  float kscale = 1.f, vscale = 1.f;
-  if (FMT == TSB200_KV_FP8) {
-    kscale = kv.k_scale[b * kv.hkv + h];
-    vscale = kv.v_scale[b * kv.hkv + h];
-  }
-  const bool rope = rope_cos != nullptr;
-  float x[2][D / 32], xv[2][D / 32];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t lp = (start >> 4) + 2 * (int64_t)blockIdx.x + i;
-    pg[i].p = lp * 16 + w;                              // position of this warp's token
-    const int64_t j = pg[i].p - start;
-    pg[i].valid = j >= 0 && j < n_b;
-    const bool page_ok = lp < kv.bt_stride;
-    int64_t page = page_ok ? kv.block_table[b * kv.bt_stride + lp] : -1;
-    pg[i].store = page >= 0 && page < kv.num_pages;
-    if (!pg[i].store) page = 0;
-    // the page is covered completely when its first and last positions are both appended
-    pg[i].full = lp * 16 >= start && lp * 16 + 15 < start + n_b;
-    pg[i].krec = kv.k_pool + (page * kv.hkv + h) * rec_bytes;
-    pg[i].vrec = kv.v_pool + (page * kv.hkv + h) * rec_bytes;
-    if (pg[i].valid && pg[i].store) {
-      const int64_t bt = b * Tn + j;
-      load_raw<T, D>(k + bt * ks + (int64_t)h * D, lane, x[i]);
-      load_raw<T, D>(v + bt * vs_ + (int64_t)h * D, lane, xv[i]);
+      for (int i = 0; i < 4; ++i) u[i] = (unsigned)__bfloat16_as_ushort(p[2 * i]) | ((unsigned)__bfloat16_as_ushort(p[2 * i + 1]) << 16);
     }
   }
+  __device__ __forceinline__ void load_shared(const __nv_bfloat16* p) { load(p, true); }
+  __device__ __forceinline__ void store(__nv_bfloat16* p, bool vec) const {
+    if (vec) {
+      *reinterpret_cast<uint4*>(p) = make_uint4(u[0], u[1], u[2], u[3]);
+    } else {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint8_t* const krec = pg[i].krec;
-    uint8_t* const vrec = pg[i].vrec;
-    if (pg[i].valid && pg[i].store) {
-      const int64_t rp = pg[i].p >= rope_rows ? rope_rows - 1 : pg[i].p;
-      rope_vec<T, D>(lane, x[i], rope, rope ? rope_cos + rp * (D / 2) : nullptr, rope ? rope_sin + rp * (D / 2) : nullptr);
-      quant_store<D, FMT, false>(x[i], lane, krec, w, kscale);
-      quant_store<D, FMT, false>(xv[i], lane, stage, w, vscale);        // token-major, into shared memory
-    }
-    __syncthreads();
-    if (pg[i].store && pg[i].full) {
-      // transposed record: row e (16 bytes) = the codes of element (pair) e for tokens 0..15
-      for (int e = threadIdx.x; e < VB; e += blockDim.x) {
-        unsigned wds[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          wds[c] = (unsigned)stage[(4 * c) * VB + e] | ((unsigned)stage[(4 * c + 1) * VB + e] << 8) |
-                   ((unsigned)stage[(4 * c + 2) * VB + e] << 16) | ((unsigned)stage[(4 * c + 3) * VB + e] << 24);
-        *reinterpret_cast<uint4*>(vrec + (int64_t)e * 16) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
-      }
-      if constexpr (FMT == TSB200_KV_INT8) {              // fp32 scale per token: same place in both forms
-        if (threadIdx.x < 16) reinterpret_cast<float*>(vrec + 16 * D)[threadIdx.x] = reinterpret_cast<const float*>(stage + 16 * D)[threadIdx.x];
-      } else if constexpr (FMT == TSB200_KV_NVFP4) {      // block scales: [16 tokens][D/16] -> [D/16][16 tokens]
-        if (threadIdx.x < D) {
-          const int blk = threadIdx.x >> 4, t = threadIdx.x & 15;
-          vrec[16 * (D / 2) + blk * 16 + t] = stage[16 * (D / 2) + t * (D / 16) + blk];
-        }
-      }
-    } else if (pg[i].store && pg[i].valid) {
-      // partly covered page: only this warp's slot is written
-      for (int e = lane; e < VB; e += 32) vrec[(int64_t)e * 16 + w] = stage[w * VB + e];
-      if constexpr (FMT == TSB200_KV_INT8) {
-        if (lane == 0) reinterpret_cast<float*>(vrec + 16 * D)[w] = reinterpret_cast<const float*>(stage + 16 * D)[w];
-      } else if constexpr (FMT == TSB200_KV_NVFP4) {
-        if (lane < D / 16) vrec[16 * (D / 2) + lane * 16 + w] = stage[16 * (D / 2) + w * (D / 16) + lane];
+      for (int i = 0; i < 4; ++i) {
+        p[2 * i] = __ushort_as_bfloat16((unsigned short)(u[i] & 0xffffu));
+        p[2 * i + 1] = __ushort_as_bfloat16((unsigned short)(u[i] >> 16));
       }
     }
-    if (i == 0) __syncthreads();                           // the staging buffer is reused by the second page
+  }
+  __device__ __forceinline__ void unpack(float (&v)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+  }
+  // largest magnitude, as the bits of a positive bf16
+  __device__ __forceinline__ float amax(float m) const {
+    float v[8];
+    unpack(v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+    return m;
+  }
+};
+template <> struct Raw8<float> {
+  float f[8];
+  __device__ __forceinline__ void load(const float* p, bool vec) {
+    if (vec) {
+      const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = p[i];
+    }
+  }
+  __device__ __forceinline__ void load_shared(const float* p) { load(p, true); }
+  __device__ __forceinline__ void store(float* p, bool vec) const {
+    if (vec) {
+      *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(p + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) p[i] = f[i];
+    }
+  }
+  __device__ __forceinline__ void unpack(float (&v)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = f[i];
+  }
+  __device__ __forceinline__ float amax(float m) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(f[i]));
+    return m;
+  }
+};
+// Half-split rotation of elements (a[i], b[i]), i and i + d/2 of one vector: every product and sum rounded to the act dtype
+// (blocks/rope.py:140-173).  bf16: packed arithmetic - one rounding per operation; the fp32 detour rounds the sum twice, which is
+// the same, since two bf16 numbers whose sum has more than 24 bits are too far apart for it to lie near a midpoint.
+__device__ __forceinline__ void rope8(Raw8<__nv_bfloat16>& a, Raw8<__nv_bfloat16>& b, const Raw8<__nv_bfloat16>& c, const Raw8<__nv_bfloat16>& s) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    __nv_bfloat162 x = *reinterpret_cast<__nv_bfloat162*>(&a.u[i]), y = *reinterpret_cast<__nv_bfloat162*>(&b.u[i]);
+    const __nv_bfloat162 cc = *reinterpret_cast<const __nv_bfloat162*>(&c.u[i]), ss = *reinterpret_cast<const __nv_bfloat162*>(&s.u[i]);
+    const __nv_bfloat162 r = __hsub2_rn(__hmul2_rn(x, cc), __hmul2_rn(y, ss)), q = __hadd2_rn(__hmul2_rn(x, ss), __hmul2_rn(y, cc));
+    a.u[i] = *reinterpret_cast<const unsigned*>(&r);
+    b.u[i] = *reinterpret_cast<const unsigned*>(&q);
+  }
+}
+__device__ __forceinline__ void rope8(Raw8<float>& a, Raw8<float>& b, const Raw8<float>& c, const Raw8<float>& s) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float x = a.f[i], y = b.f[i];
+    a.f[i] = __fsub_rn(__fmul_rn(x, c.f[i]), __fmul_rn(y, s.f[i]));
+    b.f[i] = __fadd_rn(__fmul_rn(x, s.f[i]), __fmul_rn(y, c.f[i]));
   }
 }
 
-// One CTA per (b, h): amax over the T tokens of the prompt -> scale = amax/448 (1 if 0).
+// x / d for a divisor that many elements share: correctly rounded from the correctly rounded reciprocal (Markstein's theorem,
+// Computation of elementary functions on the IBM RISC System/6000 processor, 1990: q' = q + (x - d q) y is the rounded quotient when
+// q is within an ulp of it, which one correction of x y is).  Divisors near the ends of the exponent range divide.
+struct Divisor {
+  float d, y;
+  bool slow;
+  template <bool SLOW> __device__ __forceinline__ float of(float x) const {
+    if (SLOW) return __fdiv_rn(x, d);
+    float q = x * y;
+    q = fmaf(fmaf(-q, d, x), y, q);
+    return fmaf(fmaf(-q, d, x), y, q);
+  }
+};
+__device__ __forceinline__ Divisor divisor(float v) { return Divisor{v, __frcp_rn(v), !(v >= 1e-18f && v <= 1e18f)}; }
+
+// Codes of one token's eight elements (half a lane's share): two words (8-bit formats) or one (NVFP4).
+template <int FMT, bool SLOW> __device__ __forceinline__ void encode8_by(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
+  float q[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i] = d.of<SLOW>(x[i]);
+  if (FMT == TSB200_KV_FP8) {
+    unsigned h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = __nv_cvt_float2_to_fp8x2(make_float2(q[2 * i], q[2 * i + 1]), __NV_SATFINITE, __NV_E4M3);
+    w0 = __byte_perm(h[0], h[1], 0x5410);
+    w1 = __byte_perm(h[2], h[3], 0x5410);
+  } else if (FMT == TSB200_KV_INT8) {
+    unsigned c[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = __float_as_uint(fminf(fmaxf(q[i], -127.f), 127.f) + 12582912.0f);   // 1.5 * 2^23: half-to-even, in the low bits
+    w0 = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
+    w1 = __byte_perm(__byte_perm(c[4], c[5], 0x0040), __byte_perm(c[6], c[7], 0x0040), 0x5410);
+  } else {
+    w0 = w1 = 0;
+    if (d.d > 0.f) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w0 |= (unsigned)__nv_cvt_float2_to_fp4x2(make_float2(q[2 * i], q[2 * i + 1]), __NV_E2M1, cudaRoundNearest) << (8 * i);
+    }
+  }
+}
+template <int FMT> __device__ __forceinline__ void encode8(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
+  if (d.slow) encode8_by<FMT, true>(x, d, w0, w1);
+  else encode8_by<FMT, false>(x, d, w0, w1);
+}
+// 4 x 4 byte transpose: out[j] = byte j of in[0..3]
+__device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&out)[4]) {
+  const unsigned a = __byte_perm(in[0], in[1], 0x5140), b = __byte_perm(in[2], in[3], 0x5140);
+  const unsigned c = __byte_perm(in[0], in[1], 0x7362), d = __byte_perm(in[2], in[3], 0x7362);
+  out[0] = __byte_perm(a, b, 0x5410); out[1] = __byte_perm(a, b, 0x7632);
+  out[2] = __byte_perm(c, d, 0x5410); out[3] = __byte_perm(c, d, 0x7632);
+}
+
+// Bulk append (T >= 16 tokens per sequence, quantized formats): a CTA owns the pages of 2048 / d consecutive slots of one sequence
+// (d 128: one page, d 64: two), its 8 warps take the heads.  A lane holds four tokens x (8 + 8) elements, e and e + d/2, so that
+//   * the rotation needs no other lane; cos and sin of the CTA's positions are rounded to the act dtype once, in shared memory, and
+//     serve every key and query head;
+//   * quantization shares one reciprocal per scale (the quotients the rules prescribe are IEEE divisions, ~10 instructions each
+//     otherwise);
+//   * V, stored token-minor, is transposed four bytes at a time in registers and leaves through a swizzled tile of shared memory as
+//     16-byte rows, 512 contiguous bytes per warp.
+// Pages that the range covers in part keep their other slots: those go out token by token.  A task is K or V of one head: both at once
+// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions bound it (about 2.5 an element): 32 x 2048
+// tokens, 8 heads, d 128, FP8, 402 MB: 97 us, 242 us with one warp per token vector and a byte-wise transpose.
+template <typename T, int D, int FMT>
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 1)
+kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,
+                       const T* __restrict__ v, int64_t ks, int64_t vs_, int64_t Tn, const int32_t* __restrict__ new_lens,
+                       const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int64_t rope_rows,
+                       int64_t rec_bytes) {
+  constexpr bool FP4 = FMT == TSB200_KV_NVFP4;
+  constexpr int HALF = D / 2, PAGES = 128 / D, TOK = 16 * PAGES;          // tokens of the CTA
+  constexpr int EG = HALF / 8;                                            // lanes side by side on a vector
+  constexpr int ROWS = FP4 ? D / 2 : D;                                   // 16-byte rows of a V record
+  __shared__ __align__(16) T s_cos[TOK][HALF], s_sin[TOK][HALF];
+  __shared__ __align__(16) unsigned s_v[8][PAGES][ROWS * 4];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int eg = lane % EG, tq = lane / EG;                               // elements 8 eg .., tokens 4 tq .. of the CTA's
+  const int64_t b = blockIdx.y;
+  const int64_t n_b = new_lens ? min((int64_t)new_lens[b], Tn) : Tn;
+  const int64_t start = kv.seq_lens[b];
+  const int64_t lp0 = (start >> 4) + (int64_t)blockIdx.x * PAGES;         // first logical page of the CTA
+  const int64_t p0 = lp0 * 16;
+  if (p0 >= start + n_b) return;
+  if (rope_cos) {
+    for (int i = threadIdx.x; i < TOK * HALF; i += 256) {
+      int64_t p = p0 + i / HALF;
+      p = p < 0 ? 0 : (p >= rope_rows ? rope_rows - 1 : p);
+      s_cos[i / HALF][i % HALF] = from_f32<T>(rope_cos[p * HALF + i % HALF]);
+      s_sin[i / HALF][i % HALF] = from_f32<T>(rope_sin[p * HALF + i % HALF]);
+    }
+    __syncthreads();
+  }
+  const int page_of_lane = tq >> 2;                                       // of the CTA's PAGES
+  const int slot0 = (tq & 3) * 4;                                         // first of the lane's four slots in that page
+  const int64_t lp = lp0 + page_of_lane;
+  int64_t page = lp >= 0 && lp < kv.bt_stride ? (int64_t)kv.block_table[b * kv.bt_stride + lp] : -1;
+  const bool page_ok = page >= 0 && page < kv.num_pages;
+  const bool full = lp * 16 >= start && lp * 16 + 16 <= start + n_b;      // every slot of the page is appended
+  const int64_t j0 = lp * 16 + slot0 - start;                             // index of the lane's first token in the chunk
+  bool tok[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) tok[i] = j0 + i >= 0 && j0 + i < n_b;
+  const bool kvec = (reinterpret_cast<uintptr_t>(k) & 15) == 0 && ks * sizeof(T) % 16 == 0;
+  const bool vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0 && vs_ * sizeof(T) % 16 == 0;
+  const int lt = page_of_lane * 16 + slot0;                               // the lane's first token in the tables
+
+  for (int task = w; task < 2 * kv.hkv; task += 8) {                      // head, K or V: half the registers of both at once
+    const int h = task >> 1;
+    const bool is_v = task & 1;
+    uint8_t* rec = (is_v ? kv.v_pool : kv.k_pool) + ((page_ok ? page : 0) * kv.hkv + h) * rec_bytes;
+    const T* src = (is_v ? v : k) + (int64_t)h * D + eg * 8;
+    const int64_t stride = is_v ? vs_ : ks;
+    const bool vec = is_v ? vvec : kvec;
+    Raw8<T> x[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (tok[i] && page_ok) {
+        const T* p = src + (b * Tn + j0 + i) * stride;
+        x[i][0].load(p, vec); x[i][1].load(p + HALF, vec);
+      } else {
+        x[i][0] = x[i][1] = Raw8<T>{};
+      }
+    }
+    const Divisor shared = divisor(FMT == TSB200_KV_FP8 ? (is_v ? kv.v_scale : kv.k_scale)[b * kv.hkv + h] : 1.f);
+    // one vector's codes: per token two words per half (8-bit formats) or one, and its scale(s)
+    auto encode = [&](Raw8<T> (&a)[2], unsigned (&c)[4], float& s8, unsigned (&sb)[2]) {
+      float f[2][8];
+      a[0].unpack(f[0]);
+      a[1].unpack(f[1]);
+      if (FMT == TSB200_KV_FP8) {
+        encode8<FMT>(f[0], shared, c[0], c[1]);
+        encode8<FMT>(f[1], shared, c[2], c[3]);
+      } else if (FMT == TSB200_KV_INT8) {
+        float m = a[1].amax(a[0].amax(0.f));
+#pragma unroll
+        for (int o = 1; o < EG; o *= 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        s8 = __fdiv_rn(m, 127.0f);
+        const Divisor d = divisor(__fadd_rn(s8, 1e-6f));
+        encode8<FMT>(f[0], d, c[0], c[1]);
+        encode8<FMT>(f[1], d, c[2], c[3]);
+      } else {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          float m = a[g].amax(0.f);
+          m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));              // a block of 16 is two lanes' eights
+          sb[g] = (unsigned)__nv_cvt_float_to_fp8(__fdiv_rn(m, 6.0f), __NV_SATFINITE, __NV_E4M3);
+          const Divisor d = divisor(e4m3_to_f32((unsigned char)sb[g]));
+          encode8<FMT>(f[g], d, c[2 * g], c[2 * g + 1]);
+        }
+      }
+    };
+    if (!is_v) {                             // K, token-major
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (rope_cos) {
+          Raw8<T> cc, ss;
+          cc.load_shared(&s_cos[lt + i][eg * 8]);
+          ss.load_shared(&s_sin[lt + i][eg * 8]);
+          rope8(x[i][0], x[i][1], cc, ss);
+        }
+        unsigned c[4], sb[2];
+        float s8 = 0.f;
+        encode(x[i], c, s8, sb);
+        if (tok[i] && page_ok) {
+          const int slot = slot0 + i;
+          if (FP4) {
+            *reinterpret_cast<unsigned*>(rec + slot * (D / 2) + eg * 4) = c[0];
+            *reinterpret_cast<unsigned*>(rec + slot * (D / 2) + HALF / 2 + eg * 4) = c[2];
+            if ((eg & 1) == 0) {
+              rec[16 * (D / 2) + slot * (D / 16) + (eg >> 1)] = (uint8_t)sb[0];
+              rec[16 * (D / 2) + slot * (D / 16) + HALF / 16 + (eg >> 1)] = (uint8_t)sb[1];
+            }
+          } else {
+            *reinterpret_cast<uint2*>(rec + slot * D + eg * 8) = make_uint2(c[0], c[1]);
+            *reinterpret_cast<uint2*>(rec + slot * D + HALF + eg * 8) = make_uint2(c[2], c[3]);
+            if (FMT == TSB200_KV_INT8 && eg == 0) reinterpret_cast<float*>(rec + 16 * D)[slot] = s8;
+          }
+        }
+      }
+      continue;
+    }
+    // ---- V, token-minor
+    unsigned vc[4][4], vsb[4][2];
+    float vs8[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) encode(x[i], vc[i], vs8[i], vsb[i]);
+    constexpr int GROUPS = FP4 ? 2 : 4;                                   // groups of four rows per lane
+    unsigned t[GROUPS][4];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      const int src = FP4 ? 2 * g : g;
+      const unsigned in[4] = {vc[0][src], vc[1][src], vc[2][src], vc[3][src]};
+      transpose4(in, t[g]);
+    }
+    // row of word (g, j): 8-bit: element g / 2 * HALF + 8 eg + 4 (g & 1) + j; NVFP4: pair g * HALF / 2 + 4 eg + j
+    auto row_of = [&](int g, int j) { return FP4 ? g * (HALF / 2) + eg * 4 + j : (g >> 1) * HALF + eg * 8 + (g & 1) * 4 + j; };
+    auto swz = [](int r) { return (r & ~7) | ((r ^ (r >> 3)) & 7); };     // rows that a store meets fall into different banks
+    if (__any_sync(0xffffffffu, full && page_ok)) {
+      unsigned* sv = s_v[w][page_of_lane];
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sv[swz(row_of(g, j)) * 4 + (slot0 >> 2)] = t[g][j];
+      __syncwarp();
+#pragma unroll
+      for (int pg = 0; pg < PAGES; ++pg) {
+        // the whole warp writes page pg: its address and state come from a lane of that page
+        const int from = pg * 4 * EG;
+        const bool go = __shfl_sync(0xffffffffu, (int)(full && page_ok), from);
+        const unsigned long long dst = __shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)rec, from);
+        if (go) {
+#pragma unroll
+          for (int r = lane; r < ROWS; r += 32)
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>((uintptr_t)dst) + r * 16) = *reinterpret_cast<const uint4*>(&s_v[w][pg][swz(r) * 4]);
+        }
+      }
+    }
+    if (page_ok && !full) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (tok[i]) {
+#pragma unroll
+          for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) rec[row_of(g, j) * 16 + slot0 + i] = (uint8_t)(t[g][j] >> (8 * i));
+        }
+    }
+    if (page_ok) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (tok[i]) {
+          if (FMT == TSB200_KV_INT8 && eg == 0) reinterpret_cast<float*>(rec + 16 * D)[slot0 + i] = vs8[i];
+          if (FP4 && (eg & 1) == 0) {
+            rec[16 * (D / 2) + (eg >> 1) * 16 + slot0 + i] = (uint8_t)vsb[i][0];
+            rec[16 * (D / 2) + (HALF / 16 + (eg >> 1)) * 16 + slot0 + i] = (uint8_t)vsb[i][1];
+          }
+        }
+    }
+  }
+  // ---- query heads of the same positions, in place
+  if (q == nullptr || rope_cos == nullptr) return;
+  const bool qvec = (reinterpret_cast<uintptr_t>(q) & 15) == 0 && qs * sizeof(T) % 16 == 0;
+  for (int h = w; h < qheads; h += 8) {
+    Raw8<T> x[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (tok[i]) {
+        const T* qp = q + (b * Tn + j0 + i) * qs + (int64_t)h * D + eg * 8;
+        x[i][0].load(qp, qvec); x[i][1].load(qp + HALF, qvec);
+      }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (tok[i]) {
+        T* qp = q + (b * Tn + j0 + i) * qs + (int64_t)h * D + eg * 8;
+        Raw8<T> cc, ss;
+        cc.load_shared(&s_cos[lt + i][eg * 8]);
+        ss.load_shared(&s_sin[lt + i][eg * 8]);
+        rope8(x[i][0], x[i][1], cc, ss);
+        x[i][0].store(qp, qvec); x[i][1].store(qp + HALF, qvec);
+      }
+  }
+}
+
+// FP8 scales of a prompt: amax over the T tokens of a (sequence, kv head) -> amax / 448 (1 if 0).  A cluster of eight CTAs shares the
+// tokens, D / 16 lanes a vector ((8 + 8) elements each, so the rotation needs no other lane), the maxima meet in distributed shared
+// memory.  Bound by the one trip of K and V from memory: 32 x 2048 tokens, 8 heads, d 128: 268 MB, 56 us (41 at the copy rate); the
+// version with one CTA per (sequence, head), a warp per vector and five shuffles per rotation took 343 us.
+constexpr int kScaleRanks = 8;
 template <typename T, int D>
-__global__ void kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t Tn, int hkv,
-                                     const int32_t* __restrict__ pos0, const float* __restrict__ rope_cos,
-                                     const float* __restrict__ rope_sin, int64_t rope_rows, float* __restrict__ k_scale,
-                                     float* __restrict__ v_scale) {
-  __shared__ float shk[32], shv[32];
-  const int64_t b = blockIdx.x / hkv;
-  const int h = blockIdx.x % hkv;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const bool rope = rope_cos != nullptr;
+__global__ void __launch_bounds__(256)
+kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t Tn, int hkv,
+                     const int32_t* __restrict__ pos0, const float* __restrict__ rope_cos,
+                     const float* __restrict__ rope_sin, int64_t rope_rows, float* __restrict__ k_scale,
+                     float* __restrict__ v_scale) {
+  constexpr int HALF = D / 2, EG = HALF / 8, PER = 256 / EG;              // vectors of a CTA side by side
+  __shared__ float sh[2][8], srank[2][kScaleRanks];
+  const int rank = blockIdx.x % kScaleRanks;
+  const int64_t pair = blockIdx.x / kScaleRanks, b = pair / hkv;
+  const int h = (int)(pair % hkv);
+  const int eg = threadIdx.x % EG, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t start = pos0 ? (int64_t)pos0[b] : 0;
+  const bool kvec = (reinterpret_cast<uintptr_t>(k) & 15) == 0, vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0;
+  const bool rvec = ((reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin)) & 15) == 0;
   float mk = 0.f, mv = 0.f;
-#pragma unroll 4                         // several tokens' vectors in flight per warp: the loop is latency-bound otherwise
-  for (int64_t t = w; t < Tn; t += nw) {
-    const int64_t vec = (b * Tn + t) * hkv + h;
-    int64_t p = (pos0 ? (int64_t)pos0[b] : 0) + t;
-    p = p >= rope_rows ? rope_rows - 1 : p;
-    float x[D / 32];
-    load_vec<T, D>(k + vec * D, lane, x, rope, rope ? rope_cos + p * (D / 2) : nullptr, rope ? rope_sin + p * (D / 2) : nullptr);
+#pragma unroll 2
+  for (int64_t t = (int64_t)rank * PER + threadIdx.x / EG; t < Tn; t += kScaleRanks * PER) {
+    const int64_t at = ((b * Tn + t) * hkv + h) * D + eg * 8;
+    Raw8<T> x0, x1, y0, y1;
+    x0.load(k + at, kvec); x1.load(k + at + HALF, kvec);
+    y0.load(v + at, vvec); y1.load(v + at + HALF, vvec);
+    if (rope_cos) {
+      int64_t p = start + t;
+      p = p >= rope_rows ? rope_rows - 1 : p;
+      Raw8<T> cc, ss;
+      Raw8<float> c, s;
+      c.load(rope_cos + p * HALF + eg * 8, rvec);
+      s.load(rope_sin + p * HALF + eg * 8, rvec);
+      if constexpr (sizeof(T) == 2) {
 #pragma unroll
-    for (int i = 0; i < D / 32; ++i) mk = fmaxf(mk, fabsf(x[i]));
-    load_vec<T, D>(v + vec * D, lane, x, false, nullptr, nullptr);
-#pragma unroll
-    for (int i = 0; i < D / 32; ++i) mv = fmaxf(mv, fabsf(x[i]));
+        for (int i = 0; i < 4; ++i) {
+          const __nv_bfloat162 c2 = __floats2bfloat162_rn(c.f[2 * i], c.f[2 * i + 1]), s2 = __floats2bfloat162_rn(s.f[2 * i], s.f[2 * i + 1]);
+          cc.u[i] = *reinterpret_cast<const unsigned*>(&c2);
+          ss.u[i] = *reinterpret_cast<const unsigned*>(&s2);
+        }
+      } else {
+        cc = *reinterpret_cast<Raw8<T>*>(&c);
+        ss = *reinterpret_cast<Raw8<T>*>(&s);
+      }
+      rope8(x0, x1, cc, ss);
+    }
+    mk = x1.amax(x0.amax(mk));
+    mv = y1.amax(y0.amax(mv));
   }
   mk = warp_max(mk);
   mv = warp_max(mv);
-  if (lane == 0) { shk[w] = mk; shv[w] = mv; }
+  if (lane == 0) { sh[0][w] = mk; sh[1][w] = mv; }
   __syncthreads();
-  if (w == 0) {
-    mk = warp_max(lane < nw ? shk[lane] : 0.f);
-    mv = warp_max(lane < nw ? shv[lane] : 0.f);
-    if (lane == 0) {
-      k_scale[blockIdx.x] = mk > 0.f ? __fdiv_rn(mk, 448.0f) : 1.0f;
-      v_scale[blockIdx.x] = mv > 0.f ? __fdiv_rn(mv, 448.0f) : 1.0f;
-    }
+  if (threadIdx.x < 2) {
+    float m = sh[threadIdx.x][0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, sh[threadIdx.x][i]);
+    unsigned dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"((unsigned)__cvta_generic_to_shared(&srank[threadIdx.x][rank])));
+    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(dst), "f"(m) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (rank == 0 && threadIdx.x < 2) {
+    float m = srank[threadIdx.x][0];
+#pragma unroll
+    for (int i = 1; i < kScaleRanks; ++i) m = fmaxf(m, srank[threadIdx.x][i]);
+    (threadIdx.x ? v_scale : k_scale)[pair] = m > 0.f ? __fdiv_rn(m, 448.0f) : 1.0f;
   }
 }
 
@@ -363,20 +635,19 @@ template <typename T, int D>
 int launch_append(const tsb200_kv_desc& kv, void* q, int64_t qs, int qheads, const void* k, const void* v, int64_t ks, int64_t vs, int64_t B, int64_t Tn, const int32_t* new_lens,
                   const float* rc, const float* rs, int64_t rr, cudaStream_t s) {
   const int64_t rec = (int64_t)tsb200_kv_record_bytes(kv.format, D);
-  if (Tn >= 16 && kv.format <= TSB200_KV_NVFP4 && B <= 65535 && kv.hkv <= 65535) {
-    // bulk: one CTA per (sequence, kv head, page touched) + CTAs that rotate the query heads
-    const int page_blocks = (int)(((Tn + 15) / 16 + 1 + 1) / 2);  // two pages per CTA; the range may straddle one more page than it fills
-    const int64_t q_blocks = q ? (Tn * qheads + 16 * kv.hkv - 1) / (16 * (int64_t)kv.hkv) : 0;
-    const dim3 grid((unsigned)(page_blocks + q_blocks), (unsigned)kv.hkv, (unsigned)B);
+  if (Tn >= 16 && kv.format <= TSB200_KV_NVFP4 && B <= 65535) {
+    // bulk: one CTA per (sequence, page group touched); the range may straddle one more page than it fills
+    constexpr int PAGES = 128 / D;
+    const dim3 grid((unsigned)(((Tn + 15) / 16 + 1 + PAGES - 1) / PAGES), (unsigned)B);
     switch (kv.format) {
       case TSB200_KV_INT8:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_INT8>, grid, dim3(512), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec, page_blocks));
+        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_INT8>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
         break;
       case TSB200_KV_FP8:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_FP8>, grid, dim3(512), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec, page_blocks));
+        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_FP8>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
         break;
       default:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_NVFP4>, grid, dim3(512), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec, page_blocks));
+        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_NVFP4>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
     }
     TSB_LAUNCH_CHECK();
     return TSB200_OK;
@@ -440,14 +711,23 @@ int tsb200_kv_fp8_scales(const void* k, const void* v, int dtype, int64_t B, int
   if (B == 0) return TSB200_OK;
   if (!k_scale || !v_scale || (T > 0 && (!k || !v))) return TSB200_ERR_ARG;
   if ((rope_cos != nullptr) != (rope_sin != nullptr) || (rope_cos && rope_rows <= 0)) return TSB200_ERR_ARG;
-  if (B * hkv > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
+  if (B * hkv * kScaleRanks > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   cudaStream_t s = as_stream(stream);
-  const unsigned g = (unsigned)(B * hkv);
-#define TSB_SC(TT, DD) kv_fp8_scales_kernel<TT, DD><<<g, 256, 0, s>>>((const TT*)k, (const TT*)v, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(B * hkv * kScaleRanks));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kScaleRanks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+#define TSB_SC(TT, DD) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD>, (const TT*)k, (const TT*)v, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
   if (dtype == TSB200_F32) { if (head_dim == 64) TSB_SC(float, 64); else TSB_SC(float, 128); }
   else { if (head_dim == 64) TSB_SC(__nv_bfloat16, 64); else TSB_SC(__nv_bfloat16, 128); }
 #undef TSB_SC
-  TSB_LAUNCH_CHECK();
   return TSB200_OK;
 }
 
