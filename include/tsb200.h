@@ -226,6 +226,12 @@ int tsb200_kv_fp8_scales(const void* k, const void* v, int dtype, int64_t B, int
                          int hkv, int head_dim, const int32_t* pos0,
                          const float* rope_cos, const float* rope_sin, int64_t rope_rows,
                          float* k_scale, float* v_scale, void* stream);
+/* The same for token vectors that lie k_token_stride / v_token_stride elements apart (column slices
+ * of a fused projection output; 0 = hkv * head_dim). */
+int tsb200_kv_fp8_scales_strided(const void* k, const void* v, int dtype, int64_t k_token_stride,
+                                 int64_t v_token_stride, int64_t B, int64_t T, int hkv, int head_dim,
+                                 const int32_t* pos0, const float* rope_cos, const float* rope_sin,
+                                 int64_t rope_rows, float* k_scale, float* v_scale, void* stream);
 
 /* Fused (RoPE on k +) quantize-and-append of T new tokens per sequence.
  * k, v [B, T, hkv, d]; token j of sequence b goes to position seq_lens[b] + j.

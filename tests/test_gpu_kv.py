@@ -349,6 +349,10 @@ def test_bulk_append_of_strided_prompts(cuda, fmt, name, H, Hkv, d, pad):
     k4 = buf[..., H * d + pad:(H + Hkv) * d + pad].unflatten(2, (Hkv, d))
     v4 = buf[..., (H + Hkv) * d + pad:(H + 2 * Hkv) * d + pad].unflatten(2, (Hkv, d))
     q4.copy_(q); k4.copy_(k); v4.copy_(v)
+    if fmt == "fp8":                              # the scales of the same slices
+        dense = g.k_scale.clone(), g.v_scale.clone()
+        g.set_fp8_scales(k4, v4, rope=rope, pos0=g.seq_lens)
+        assert torch.equal(g.k_scale, dense[0]) and torch.equal(g.v_scale, dense[1])
     g.rope_append(q4, k4, v4, rope, new_lens=torch.from_numpy(new_lens).to(cuda))
     pos = torch.from_numpy(start.astype(np.int64))[:, None] + torch.arange(T)[None, :]
     kr, qr = (torch.stack([oatt.apply_rope(x[b], cos[pos[b]], sin[pos[b]]) for b in range(B)]) for x in (k, q))

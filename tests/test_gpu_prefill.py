@@ -93,3 +93,25 @@ def test_prefill_attention_strided_q_and_argument_errors(cuda):
     assert torch.equal(out, ops.prefill_attention(kv, q.contiguous(), L))
     with pytest.raises(Tsb200Error):
         ops.prefill_attention(kv, q.contiguous(), L - 1)         # fewer cached positions than query tokens
+
+
+@pytest.mark.parametrize("fmt", ["int8", "fp8", "nvfp4", "bf16", "fp32"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("L", [1, 63, 64, 130])
+def test_head_major_gather_equals_token_major_gather(cuda, fmt, d, L):
+    """K [B, hkv, L, d] and V^T [B, hkv, d, Lp] hold what the token-major gather returns; zeros beyond a sequence's length and up to the pitch."""
+    import ctypes as C
+    from transformer_surgeon_b200 import _lib
+    B, Hkv = 3, 2
+    ops, kv, g = setup(cuda, fmt, B, L, 2, Hkv, d, torch.float32 if fmt == "fp32" else torch.bfloat16, 90 + L)
+    kv.seq_lens.copy_(torch.tensor([L, L // 2, 0], dtype=torch.int32))
+    Lp = (L + 7) // 8 * 8
+    kd = torch.full((B, Hkv, L, d), 7.0, dtype=torch.bfloat16, device=cuda)
+    vt = torch.full((B, Hkv, d, Lp), 7.0, dtype=torch.bfloat16, device=cuda)
+    desc = kv.desc(None)
+    st = _lib.load().tsb200_kv_gather_heads(C.byref(desc), kd.data_ptr(), vt.data_ptr(), B, L, Lp, ops._stream())
+    assert st == 0
+    k, v = ops.kv_gather(kv, L, dtype=torch.bfloat16)
+    assert torch.equal(kd, k.transpose(1, 2))
+    assert torch.equal(vt[..., :L], v.permute(0, 2, 3, 1))
+    assert not vt[..., L:].any()

@@ -567,7 +567,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
 constexpr int kScaleRanks = 8;
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
-kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t Tn, int hkv,
+kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t ks, int64_t vs, int64_t Tn, int hkv,
                      const int32_t* __restrict__ pos0, const float* __restrict__ rope_cos,
                      const float* __restrict__ rope_sin, int64_t rope_rows, float* __restrict__ k_scale,
                      float* __restrict__ v_scale) {
@@ -578,15 +578,17 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t T
   const int h = (int)(pair % hkv);
   const int eg = threadIdx.x % EG, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t start = pos0 ? (int64_t)pos0[b] : 0;
-  const bool kvec = (reinterpret_cast<uintptr_t>(k) & 15) == 0, vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0;
+  const bool kvec = (reinterpret_cast<uintptr_t>(k) & 15) == 0 && ks * sizeof(T) % 16 == 0;
+  const bool vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0 && vs * sizeof(T) % 16 == 0;
   const bool rvec = ((reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin)) & 15) == 0;
   float mk = 0.f, mv = 0.f;
 #pragma unroll 2
   for (int64_t t = (int64_t)rank * PER + threadIdx.x / EG; t < Tn; t += kScaleRanks * PER) {
-    const int64_t at = ((b * Tn + t) * hkv + h) * D + eg * 8;
+    const T* kp = k + (b * Tn + t) * ks + h * D + eg * 8;
+    const T* vp = v + (b * Tn + t) * vs + h * D + eg * 8;
     Raw8<T> x0, x1, y0, y1;
-    x0.load(k + at, kvec); x1.load(k + at + HALF, kvec);
-    y0.load(v + at, vvec); y1.load(v + at + HALF, vvec);
+    x0.load(kp, kvec); x1.load(kp + HALF, kvec);
+    y0.load(vp, vvec); y1.load(vp + HALF, vvec);
     if (rope_cos) {
       int64_t p = start + t;
       p = p >= rope_rows ? rope_rows - 1 : p;
@@ -704,6 +706,12 @@ size_t tsb200_kv_record_bytes(int format, int head_dim) {
 int tsb200_kv_fp8_scales(const void* k, const void* v, int dtype, int64_t B, int64_t T, int hkv, int head_dim,
                          const int32_t* pos0, const float* rope_cos, const float* rope_sin, int64_t rope_rows,
                          float* k_scale, float* v_scale, void* stream) {
+  return tsb200_kv_fp8_scales_strided(k, v, dtype, 0, 0, B, T, hkv, head_dim, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale, stream);
+}
+
+int tsb200_kv_fp8_scales_strided(const void* k, const void* v, int dtype, int64_t k_token_stride, int64_t v_token_stride, int64_t B,
+                                 int64_t T, int hkv, int head_dim, const int32_t* pos0, const float* rope_cos, const float* rope_sin,
+                                 int64_t rope_rows, float* k_scale, float* v_scale, void* stream) {
   TSB_REQUIRE_DEVICE();
   if (B < 0 || T < 0 || hkv <= 0) return TSB200_ERR_ARG;
   if (head_dim != 64 && head_dim != 128) return TSB200_ERR_UNSUPPORTED;
@@ -711,6 +719,9 @@ int tsb200_kv_fp8_scales(const void* k, const void* v, int dtype, int64_t B, int
   if (B == 0) return TSB200_OK;
   if (!k_scale || !v_scale || (T > 0 && (!k || !v))) return TSB200_ERR_ARG;
   if ((rope_cos != nullptr) != (rope_sin != nullptr) || (rope_cos && rope_rows <= 0)) return TSB200_ERR_ARG;
+  const int64_t dense = (int64_t)hkv * head_dim;
+  const int64_t ks = k_token_stride ? k_token_stride : dense, vs = v_token_stride ? v_token_stride : dense;
+  if (ks < dense || vs < dense) return TSB200_ERR_ARG;
   if (B * hkv * kScaleRanks > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   cudaStream_t s = as_stream(stream);
   cudaLaunchConfig_t cfg = {};
@@ -724,7 +735,7 @@ int tsb200_kv_fp8_scales(const void* k, const void* v, int dtype, int64_t B, int
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-#define TSB_SC(TT, DD) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD>, (const TT*)k, (const TT*)v, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
+#define TSB_SC(TT, DD) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD>, (const TT*)k, (const TT*)v, ks, vs, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
   if (dtype == TSB200_F32) { if (head_dim == 64) TSB_SC(float, 64); else TSB_SC(float, 128); }
   else { if (head_dim == 64) TSB_SC(__nv_bfloat16, 64); else TSB_SC(__nv_bfloat16, 128); }
 #undef TSB_SC

@@ -327,7 +327,6 @@ class CompressedDecoder:
             else:
                 q, k, v = L.qkv_group(xn)
                 q4, k4, v4 = q.view(B, T, H, d), k.view(B, T, Hkv, d), v.view(B, T, Hkv, d)
-            q4, k4, v4 = q4.contiguous(), k4.contiguous(), v4.contiguous()
             kv = self.kv[li]
             if kv.k_scale is not None:
                 kv.set_fp8_scales(k4, v4, rope=rope, pos0=zeros)

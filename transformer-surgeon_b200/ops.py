@@ -429,13 +429,14 @@ class PagedKV:
                       0 if self.v_scale is None else self.v_scale.data_ptr())
 
     def set_fp8_scales(self, k, v, rope=None, pos0=None):
-        """scale = amax/448 over the prompt k, v [B, T, hkv, d] (k after RoPE when given)."""
+        """scale = amax/448 over the prompt k, v [B, T, hkv, d] (k after RoPE when given); tokens may be evenly strided."""
         lib = _lib.load()
         B, T = k.shape[:2]
         cos, sin = (None, None) if rope is None else rope
-        check(lib.tsb200_kv_fp8_scales(_p(_cuda(k, "k")), _p(_cuda(v, "v")), _dt(k), B, T, self.hkv, self.head_dim,
-                                       _p(pos0), _p(cos), _p(sin), 0 if cos is None else cos.shape[0],
-                                       _p(self.k_scale), _p(self.v_scale), _stream()), "tsb200_kv_fp8_scales")
+        ks, vs = _token_strided(k, "k"), _token_strided(v, "v")
+        check(lib.tsb200_kv_fp8_scales_strided(_p(k), _p(v), _dt(k), ks, vs, B, T, self.hkv, self.head_dim, _p(pos0), _p(cos), _p(sin),
+                                               0 if cos is None else cos.shape[0], _p(self.k_scale), _p(self.v_scale), _stream()),
+              "tsb200_kv_fp8_scales_strided")
         self.fp8_scales_set = True
 
     def rope_append(self, q, k, v, rope, new_lens=None, seq_lens=None):
