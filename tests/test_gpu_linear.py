@@ -230,6 +230,49 @@ def test_gated_mlp_block(cuda, name, p, M, K, I, r, N):
     assert ops.PackedLinear.device_status(ws=ops.workspace(cuda, 1, "mlp")) == 0
 
 
+@pytest.mark.parametrize("p", [8, 4, 2, "binary"])
+@pytest.mark.parametrize("M,K,I,r", [(129, 512, 14336, 256), (257, 256, 14344, 0), (300, 512, 7304, 136), (2048, 512, 2048, 128), (2500, 1024, 4104, 0), (200, 512, 640, 64)])
+def test_gated_mlp_prompt(cuda, p, M, K, I, r):
+    """More than 128 tokens: gate's tiles read by up's outputs (one to several items per CTA, ragged tokens and rows, K splits in the
+    V phase, items shorter than the ring of stages), or the composed path where up's tiles split K; same as composing the pieces up
+    to the rounding of SiLU."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(11)
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+
+    def layer(out, inn, rank, bias):
+        U = (torch.randn(out, rank or inn, generator=g, device=cuda) * (rank or inn) ** -0.5).bfloat16()
+        V = (torch.randn(rank, inn, generator=g, device=cuda) * inn ** -0.5).bfloat16() if rank else None
+        return ops.PackedLinear(ops.Factor.quantize(U, p), ops.Factor.quantize(V, p) if rank else None,
+                                torch.randn(out, generator=g, device=cuda).bfloat16() if bias else None, torch.bfloat16)
+
+    gate, up, down = layer(I, K, r, True), layer(I, K, r, True), layer(256, I, r, False)
+    mlp = ops.GatedMLP(gate, up, down)
+    y, y2 = mlp(x), mlp(x)
+    assert torch.equal(y, y2)
+    a = ops.swiglu(gate(x), up(x))
+    assert rel_err(y, down(a)) < 4e-3
+    assert ops.PackedLinear.device_status(ws=ops.workspace(cuda, 1, "mlp")) == 0
+
+
+@pytest.mark.parametrize("p", [8, 4, 2, "binary"])
+@pytest.mark.parametrize("M,K,N", [(129, 128, 40000), (256, 64, 19072), (600, 192, 12928), (1000, 320, 9004), (4100, 256, 2560), (777, 1280, 6150)])
+def test_many_short_items_per_cta(cuda, p, M, K, N):
+    """256-token tiles: items of one to a few stages, widened ahead of the previous item's outputs; ragged tokens, rows and row pitches."""
+    from transformer_surgeon_b200 import ops
+    if p == "binary":
+        K = (K + 127) // 128 * 128
+    g = torch.Generator(device=cuda).manual_seed(12)
+    f = ops.Factor.quantize((torch.randn(N, K, generator=g, device=cuda) * K ** -0.5).bfloat16(), p)
+    b = torch.randn(N, generator=g, device=cuda).bfloat16()
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+    lin = ops.PackedLinear(f, None, b, torch.bfloat16)
+    y = lin(x)
+    ref = x.float() @ f.reconstruct(torch.float32).T + b.float()
+    assert (y.float() - ref).abs().max() <= 2 ** -8 * ref.abs().max()
+    assert torch.equal(y, lin(x))
+
+
 @pytest.mark.parametrize("p", [4, 8, 2, "binary"])
 @pytest.mark.parametrize("M,K,N,r", [(32, 4096, 4096, 0),        # o_proj
                                      (32, 4096, 6144, 0),        # q|k|v

@@ -4,24 +4,24 @@
 //
 // Decode-time GEMMs stream a few MB of packed weights per call, so the kernel is built around
 // keeping many weight bytes in flight per SM, paying the set-up cost once per SM, and
-// synchronising once per 16 KB of weights rather than once per k-block.  Warp roles (12 warps):
-//   * warps 0 and 11, one lane each: PRODUCERS.  grid = min(#work items, #SMs); a work item = (128-row
+// synchronising once per 16 KB of weights rather than once per k-block.  Warp roles (12 warps, 20 at 256 tokens):
+//   * warps 0 and 11 (19), one lane each: PRODUCERS.  grid = min(#work items, #SMs); a work item = (128-row
 //     weight tile, token tile, K split); each lane walks the CTA's items and keeps issuing TMA loads across
 //     item and phase boundaries into a ring of STAGES.  A stage = KBS consecutive k-blocks: one
 //     weight box of 128 rows x up to 128 bytes of codes (swizzled, warp 0) + the activation tiles of those
-//     k-blocks (one 3-D box, warp 11).  Issuing one copy costs its lane several hundred cycles, hence a
+//     k-blocks (one 3-D box, the last warp).  Issuing one copy costs its lane several hundred cycles, hence a
 //     lane per operand; the weight lane runs ahead of the grid barrier that the activation lane must
 //     respect (weights are constants), so a phase's first weight boxes land before its activations exist;
-//   * warps 2-9: DEQUANT, two groups of 4 sharing every stage (even / odd k-blocks).  A thread owns
+//   * warps 2-9 (256-token tile: 2-17): DEQUANT, two groups of 4 sharing every stage (even / odd k-blocks).  A thread owns
 //     one weight row: it reads the row's codes from shared memory, widens them to bf16 pairs in
 //     registers (exact integers) and stores them with tcgen05.st straight into TENSOR MEMORY, where
 //     they are the A operand of the MMA (M = 128 weight rows; K-major, two bf16 per 32-bit column)
 //     - no shared-memory A tile, no generic->async proxy fence;
-//   * warps 1 and 10, one lane each: MMA ISSUERS (A from TMEM, B = activation tile from shared
+//   * warps 1 and 10 (18), one lane each: MMA ISSUERS (A from TMEM, B = activation tile from shared
 //     memory through a 128-byte-swizzle descriptor, N = token tile), each into its own accumulator
 //     chain (see QLayout); one barrier per stage tells them that both operands are in place, one
 //     commit per stage frees the stage's shared memory and A buffer;
-//   * the 8 dequant warps run the epilogue from TMEM (one lane = one weight row): chains added,
+//   * the dequant warps run the epilogue from TMEM (one lane = one weight row): chains added,
 //     scale, bias, store;
 //   * split-K: every item stores its fp32 partial tile in a private slice of the workspace (plain
 //     stores, no zero-fill needed).  When each CTA holds one item of the phase, the CTAs of a tile
@@ -43,14 +43,20 @@ namespace tsb {
 using namespace tc;
 namespace {
 
-constexpr int kDqWarps = 8;                 // two groups of four
-constexpr int kThreadsQ = 64 + kDqWarps * 32 + 64;   // weight producer, MMA issuer 0, 8 dequant warps, MMA issuer 1, activation producer
-constexpr int kIssuer1Warp = 2 + kDqWarps;
-constexpr int kXWarp = 3 + kDqWarps;
 constexpr int kSmemBudget = 216 * 1024;     // three 72 KB stages of the 256-token tile (int4), six 32 KB stages of the decode tiles
 constexpr unsigned kTmemCols = 512;
 
 template <int TN, int BITS> struct QLayout {
+  // Widening warps, in groups of four (one per TMEM lane quarter).  Two groups share every stage (its even and odd k-blocks); a stage
+  // takes a warp ~750 cycles, almost all of it latency, against 1024 cycles of MMAs at 256 tokens, and the epilogue comes on top:
+  // there two more groups take every other stage and half of each warp's outputs.
+  static constexpr int kGroups = TN == 256 ? 4 : 2;
+  static constexpr int kDqWarps = 4 * kGroups;
+  static constexpr int kStageWarps = 8;                    // warps that widen one stage
+  // weight producer, MMA issuer 0, widening warps, MMA issuer 1, activation producer
+  static constexpr int kThreads = (4 + kDqWarps) * 32;
+  static constexpr int kIssuer1Warp = 2 + kDqWarps;
+  static constexpr int kXWarp = 3 + kDqWarps;
   static constexpr int kKbsFull = 1024 / BITS / BK;        // k-blocks in a 128-byte row of codes
   // A buffer = KBS * 32 TMEM columns <= 128; 64- and 256-token tiles keep two k-blocks per stage (16 / 64 KB of activations)
   static constexpr int kKbsCap = (TN <= 32 || TN == 128) ? 4 : 2;
@@ -77,9 +83,10 @@ template <int TN, int BITS> struct QLayout {
   static constexpr int NBUF = kNBufFit < NR ? (kNBufFit < 4 ? kNBufFit : 4) : (NR < 4 ? NR : 4);
   static_assert(NBUF >= 2 && kACol0 + NBUF * kABufCols <= 512, "tensor memory columns");
   static constexpr int kBarBytes = 1024;
-  // Token tiles of 128 and more transpose their outputs through shared memory (16 tokens x 32 rows of bf16 per warp),
+  // Token tiles of 128 and more transpose their outputs through shared memory (kOutTokens tokens x 32 rows of bf16 per warp),
   // so that they leave as 16-byte stores instead of 2-byte stores
-  static constexpr int kOutStage = TN >= 128 ? kDqWarps * 16 * 32 * 2 : 0;
+  static constexpr int kOutTokens = TN == 256 ? 8 : 16;
+  static constexpr int kOutStage = TN >= 128 ? kDqWarps * kOutTokens * 32 * 2 : 0;
   static constexpr int kBytes = NR * kStage + kBarBytes + kOutStage + 1024;
   static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
   // The tensor pipe needs ~55 + N/2 cycles per tcgen05.mma (the A operand is read from tensor memory), and
@@ -98,6 +105,14 @@ template <int TN, int BITS> struct QLayout {
   // issues every stage's MMAs for ITS 128 tokens (N = 128: the lane's ~114 cycles per MMA cover 64 cycles of the pipe,
   // two lanes keep it busy; one lane issuing N = 256 needs 141-171 cycles per 128 cycles of the pipe)
   static constexpr bool kSplitTokens = TN == 256;
+  // An item's epilogue (read the sums, scale, round, transpose, store: ~4600 cycles a CTA) used to stand between two items' MMAs,
+  // against 512 cycles of MMAs per k-block: a third of the time at 16 k-blocks an item.  The 256-token tile therefore widens the
+  // next item's first stages before it waits for the sums, moves the sums into registers as bf16 pairs (32 a thread), gives
+  // the accumulator back and stores while the next item's MMAs run: 16384 tokens, 1024 -> 14336, int4: 448 us (535 with eight
+  // warps and all of a warp's outputs in one go).  (Smaller tiles have at most a few items per CTA and phase.)
+  static constexpr bool kAhead = kSplitTokens;
+  static constexpr int kAheadStages = NBUF < 3 ? NBUF - 1 : 2;   // before the sums: A buffers that earlier stages have left
+  static constexpr int kMaxRegs = TN == 256 ? 96 : 128;
 };
 
 __device__ __forceinline__ uint4 lds128(unsigned addr) {
@@ -191,6 +206,24 @@ __device__ __forceinline__ void tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
                : "r"(taddr)
                : "memory");
 }
+// 16 TMEM lanes x 64 columns as 8 x 8 fragments: registers 4 i .. 4 i + 3 of a lane = columns 8 i + 2 (lane % 4) and one further of
+// TMEM lane lane / 4, then of TMEM lane 8 + lane / 4.
+__device__ __forceinline__ void tmem_ld_frag(unsigned taddr, unsigned (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values, transposed: lane 8 m + i gives the address of column i of matrix m.
+__device__ __forceinline__ void stmatrix4_trans(unsigned saddr, const unsigned (&r)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(saddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
 template <int W> __device__ __forceinline__ void tmem_ldw(unsigned taddr, unsigned (&r)[W]) {
   if constexpr (W == 16) tmem_ld16(taddr, r);
   else tmem_ld8(taddr, r);
@@ -245,6 +278,7 @@ struct SubGemm {                 // one packed weight matrix and its operands
   const float* scale;            // [N]
   const __nv_bfloat16* bias;     // [N] or null
   __nv_bfloat16* y;              // [M, N]
+  const __nv_bfloat16* gate;     // [M, N] or null: y = silu(gate) * (the product), rounded as the separate kernels round
 };
 struct Phase {
   SubGemm sub[2];
@@ -281,11 +315,25 @@ __device__ __forceinline__ bool grid_wait(const int* ctr, int target, volatile i
   return false;
 }
 
+// SiLU(gate) * up of eight outputs: the rounding points of separate gate / up / SiLU * up kernels (blocks/mlp.py:181-183).
+__device__ __forceinline__ uint4 gate_eight(uint4 gv, uint4 uv) {
+  const unsigned g[4] = {gv.x, gv.y, gv.z, gv.w}, u[4] = {uv.x, uv.y, uv.z, uv.w};
+  unsigned o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float g0 = __uint_as_float(g[i] << 16), g1 = __uint_as_float(g[i] & 0xffff0000u);
+    const __nv_bfloat162 a = __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)), __fdividef(g1, 1.0f + __expf(-g1)));
+    const __nv_bfloat162 r = __hmul2_rn(a, *reinterpret_cast<const __nv_bfloat162*>(&u[i]));
+    o[i] = *reinterpret_cast<const unsigned*>(&r);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 template <int TN, int BITS>
 // 128 registers (not the 168 a 384-thread CTA could have): the CTA of a launch then fits beside the CTAs of the small
 // kernel before it, so its set-up and first weight copies run under programmatic dependent launch while that kernel
 // still executes.  With 168 registers the decode step was 4 % slower although this kernel alone was faster.
-__global__ void __maxnreg__(128)
+__global__ void __maxnreg__((QLayout<TN, BITS>::kMaxRegs))
 linear_tcq_kernel(const __grid_constant__ Program prog) {
   using L = QLayout<TN, BITS>;
   constexpr int NR = L::NR;
@@ -302,7 +350,8 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
                                                             //      weight box, activation tiles and A buffer are free
   unsigned long long* acc_full = bars + 3 * NR;             // [1]  MMA commit: accumulator(s) of the item complete
   unsigned long long* ep_bar = acc_full + 1;                // [1]  rendezvous of the 8 warps
-  unsigned* tmem_slot = reinterpret_cast<unsigned*>(ep_bar + 1);
+  unsigned long long* acc_free = ep_bar + 1;                // [2]  256-token tile: a token half's accumulator has been read
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* last_flag = abort_flag + 1;
 
@@ -329,9 +378,11 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
 
   int pre_w = 0;                                            // weight boxes issued during the set-up (thread 0)
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NR; ++i) { mbar_init(&w_full[i], 1); mbar_init(&x_full[i], 1 + kDqWarps); mbar_init(&stage_done[i], (L::kSplitStage || L::kSplitTokens) ? 2 : 1); }
+    for (int i = 0; i < NR; ++i) { mbar_init(&w_full[i], 1); mbar_init(&x_full[i], 1 + L::kStageWarps); mbar_init(&stage_done[i], (L::kSplitStage || L::kSplitTokens) ? 2 : 1); }
     mbar_init(acc_full, 2);                                 // both issuers commit, with or without MMAs of their own
-    mbar_init(ep_bar, kDqWarps);
+    mbar_init(ep_bar, L::kDqWarps);
+    mbar_init(&acc_free[0], L::kDqWarps / 2);
+    mbar_init(&acc_free[1], L::kDqWarps / 2);
     *abort_flag = 0;
     *last_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -386,7 +437,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
         }
       }
     }
-  } else if (warp == kXWarp) {
+  } else if (warp == L::kXWarp) {
     // ---------------------------------------------------------------- TMA producer: activations
     // Same stage sequence; a phase's activations exist once the preceding kernel (phase 0) or the previous phase
     // (grid barrier) has produced them.
@@ -484,19 +535,25 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
         }
       }
     }
-  } else if (warp == 1 || warp == kIssuer1Warp) {
+  } else if (warp == 1 || warp == L::kIssuer1Warp) {
     // ---------------------------------------------------------------- MMA issuers
     if (lane == 0) {
       const int me = warp == 1 ? 0 : 1;                       // issuer 0: even stages / chain 0; issuer 1: odd stages / chain 1
       constexpr unsigned idesc = idesc_bf16(L::kSplitTokens ? TN / 2 : TN);
-      int gs = 0;
+      int gs = 0, it_count = 0;
       bool ok = true;
       for (int p = 0; p < prog.n_phases && ok; ++p) {
         const Phase& ph = prog.ph[p];
         const bool two = ph.gated ? L::kTwoChainsGated : L::kTwoChains;
-        for (int item = blockIdx.x; item < ph.items && ok; item += gridDim.x) {
+        for (int item = blockIdx.x; item < ph.items && ok; item += gridDim.x, ++it_count) {
           const Item it = decode(ph, item);
           const int passes = ph.gated ? 2 : 1;
+          // 256-token tile: A operands of this item may be in place while the previous item's sums are still being read
+          if (L::kAhead && it_count > 0) {
+            ok = mbar_wait(&acc_free[me], (it_count - 1) & 1, abort_flag, 8);
+            if (!ok) break;
+            tc_fence_after();
+          }
           for (int ps = 0; ps < passes && ok; ++ps) {
             const unsigned d_tmem = L::kSplitTokens ? tmem_base + (unsigned)(me * (TN / 2))
                                                     : tmem_base + (unsigned)((ph.gated ? 2 * (two ? me : 0) + ps : (two ? me : 0)) * TN);
@@ -535,14 +592,36 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
     }
   } else {
     // ---------------------------------------------------------------- dequant + epilogue
-    const int grp = (warp - 2) >> 2;                         // dequant group 0 / 1: k-blocks of that parity in every stage
+    const int grp = (warp - 2) >> 2;                         // group; widens the k-blocks of parity grp & 1 in every (four groups: every other) stage
     const int q = warp & 3;                                  // TMEM lane quarter this warp may access
     const int row = q * 32 + lane;                           // weight row within the tile = TMEM lane
     const unsigned lane_addr = tmem_base + ((unsigned)(q * 32) << 16);
     int gs = 0, it_count = 0, ep_uses = 0;
-    __nv_bfloat16* out_stage = reinterpret_cast<__nv_bfloat16*>(r_ring + NR * L::kStage + L::kBarBytes) + (warp - 2) * (16 * 32);   // this warp's
+    __nv_bfloat16* out_stage = reinterpret_cast<__nv_bfloat16*>(r_ring + NR * L::kStage + L::kBarBytes) + (warp - 2) * (L::kOutTokens * 32);   // this warp's
     bool ok = true;
     bool waited = false;
+    int ahead = 0;                                           // stages of the coming item that are widened already
+    // Widens this warp's share of stage jj of an item (absolute stage g) into its A buffer.
+    auto fill = [&](const Item& it, int jj, int g) -> bool {
+      if (L::kGroups == 4 && (g & 1) != (grp >> 1)) return true;
+      const int s = g % NR, buf = g % L::NBUF;
+      if (!mbar_wait_relaxed(&w_full[s], (g / NR) & 1, abort_flag, 4)) return false;
+      // the A buffer is free once the MMAs of the stage NBUF back are complete
+      if (g >= L::NBUF && !mbar_wait_relaxed(&stage_done[(g - L::NBUF) % NR], ((g - L::NBUF) / NR) & 1, abort_flag, 5)) return false;
+      tc_fence_after();
+      const unsigned raw = smem_u32(r_ring + s * L::kStage + L::kX);
+      const int nsub = min(KBS, it.nkb - jj * KBS);
+      for (int j = grp & 1; j < nsub; j += 2) {                // two groups work on the stage: half the latency
+        unsigned regs[32];
+        dequant_row_regs<BITS, L::kRawStageRow>(raw, row, j, regs);
+        tmem_st32(lane_addr + L::kACol0 + buf * L::kABufCols + j * 32, regs);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&x_full[s]);
+      return true;
+    };
     for (int p = 0; p < prog.n_phases && ok; ++p) {
       const Phase& ph = prog.ph[p];
       for (int item = blockIdx.x; item < ph.items && ok; item += gridDim.x, ++it_count) {
@@ -559,26 +638,26 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
           bv1 = (ph.sub[1].bias && n < ph.N) ? __bfloat162float(ph.sub[1].bias[n]) : 0.f;
         }
         for (int ps = 0; ps < passes && ok; ++ps) {
-          for (int jj = 0; jj < it.ns; ++jj, ++gs) {
-            const int i = jj * KBS;
-            const int s = gs % NR, buf = gs % L::NBUF;
-            ok = mbar_wait_relaxed(&w_full[s], (gs / NR) & 1, abort_flag, 4);
-            // the A buffer is free once the MMAs of the stage NBUF back are complete
-            if (ok && gs >= L::NBUF) ok = mbar_wait_relaxed(&stage_done[(gs - L::NBUF) % NR], ((gs - L::NBUF) / NR) & 1, abort_flag, 5);
+          gs += ahead;
+          for (int jj = ahead; jj < it.ns; ++jj, ++gs) {
+            ok = fill(it, jj, gs);
             if (!ok) break;
-            tc_fence_after();
-            const unsigned raw = smem_u32(r_ring + s * L::kStage + L::kX);
-            const int nsub = min(KBS, it.nkb - i);
-            for (int j = grp; j < nsub; j += 2) {              // both groups work on the stage: half the latency
-              unsigned regs[32];
-              dequant_row_regs<BITS, L::kRawStageRow>(raw, row, j, regs);
-              tmem_st32(lane_addr + L::kACol0 + buf * L::kABufCols + j * 32, regs);
-            }
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&x_full[s]);
           }
+          ahead = 0;
+        }
+        if (!ok) break;
+        // 256-token tile: stages of the next item, while this one's last MMAs run
+        Item nx{};
+        auto fill_next = [&]() {
+          if (L::kAhead && ok && ahead < nx.ns) {
+            ok = fill(nx, ahead, gs + ahead);
+            ++ahead;
+          }
+        };
+        if constexpr (L::kAhead) {
+          if (item + (int)gridDim.x < ph.items) nx = decode(ph, item + gridDim.x);
+#pragma unroll 1
+          for (int i = 0; i < L::kAheadStages; ++i) fill_next();
         }
         if (!ok) break;
         ok = mbar_wait_relaxed(acc_full, it_count & 1, abort_flag, 6);
@@ -587,7 +666,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
         if (!waited) { pdl_wait(); waited = true; }          // outputs / scratch may still be in use upstream
         const int64_t m0 = (int64_t)it.mt * TN;
         const bool split = ph.splits > 1;
-        constexpr int CH = TN / 2;                           // token columns handled by this warp
+        constexpr int CH = TN / L::kGroups;                  // token columns handled by this warp
         // accumulator chains: with two issuers chain c holds the stages of parity c; a pass of a single stage
         // leaves the other chain unwritten.  g0 = first stage of the (gate) pass, g0u = of the up pass.
         const bool two = ph.gated ? L::kTwoChainsGated : L::kTwoChains;
@@ -605,6 +684,89 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
         // warp ~115 cycles to issue whatever its width, so few wide loads, not many narrow ones); a gated item first
         // turns the gate columns into SiLU(g), then fetches the up columns into the freed registers
         constexpr int W = CH >= 16 ? 16 : 8;
+        if constexpr (L::kAhead) {
+          if (!split) {
+            const int nw0 = it.nt * BM + q * 32;                   // first weight row of the warp
+            const int64_t mh = m0 + grp * CH;                      // first token of the warp
+            // The 16-byte piece that this lane moves per eight tokens: token lane / 4, rows 8 (lane % 4) ..  All that the loop below needs
+            // is in registers before it (program fields in constant memory cost it a serial load each).
+            const int64_t at = ((mh + (lane >> 2)) * ph.N + nw0 + (lane & 3) * 8) * 2;
+            char* yp = reinterpret_cast<char*>(y) + at;
+            const char* gp = sg0.gate ? reinterpret_cast<const char*>(sg0.gate) + at : nullptr;
+            unsigned step8 = (unsigned)ph.N * 16u;                 // bytes from a token to the eighth after it
+            int left = (int)min(prog.M - mh - (lane >> 2), (int64_t)CH);                       // tokens: piece j of the lane is token 8 j
+            int rows = (int)min(ph.N - nw0 - (lane & 3) * 8, (int64_t)8);                      // valid rows of the pieces
+            if (rows <= 0) left = 0;
+            bool whole = vec;
+            asm volatile("" : "+r"(step8), "+r"(left), "+r"(rows), "+l"(yp), "+l"(gp));
+            uint4 gt = {};
+            auto gates = [&]() {
+              if (gp && left > 0) gt = __ldcg(reinterpret_cast<const uint4*>(gp));
+              if (gp) gp += step8;
+            };
+            gates();
+            // The sums come as 8 x 8 fragments (lane: row lane / 4, tokens 2 (lane % 4) and one further), so that one stmatrix turns
+            // eight tokens of the warp's 32 rows around.
+            static_assert(CH == 64, "one fragment load covers the warp's tokens");
+            unsigned pk[CH / 8][4];                                // [eight tokens][eight rows]: two tokens of a row
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {                       // rows 16 hf .. of the warp
+              float sc[2], bv[2];
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                sc[k] = __shfl_sync(0xffffffffu, sc0, hf * 16 + k * 8 + (lane >> 2));
+                bv[k] = __shfl_sync(0xffffffffu, bv0, hf * 16 + k * 8 + (lane >> 2));
+              }
+              unsigned r[32];
+              tmem_ld_frag(lane_addr + ((unsigned)(hf * 16) << 16) + (unsigned)(grp * CH), r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < CH / 8; ++i)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[4 * i + 2 * k]) * sc[k] + bv[k], __uint_as_float(r[4 * i + 2 * k + 1]) * sc[k] + bv[k]);
+                  pk[i][hf * 2 + k] = *reinterpret_cast<const unsigned*>(&v);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_free[grp >> 1]);
+            // staging: eight tokens x 64 bytes; 16-byte pieces swizzled so that eight rows of a matrix, and two tokens of a read, cover
+            // all banks
+            const unsigned sb = smem_u32(out_stage);
+            const unsigned st_at = sb + (unsigned)((lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4));
+            const unsigned ld_at = sb + (unsigned)((lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4));
+            // eight tokens, a stage of the next item, eight tokens, ...: outputs that follow one another hold the warps while the MMAs
+            // run out of stages
+#pragma unroll 1
+            for (int h = 0; h < CH / 8; ++h) {
+              stmatrix4_trans(st_at, pk[0]);
+#pragma unroll
+              for (int i = 0; i + 1 < CH / 8; ++i)                 // the next eight tokens move up
+#pragma unroll
+                for (int k = 0; k < 4; ++k) pk[i][k] = pk[i + 1][k];
+              __syncwarp();
+              uint4 o = lds128(ld_at);
+              if (gp) o = gate_eight(gt, o);
+              const bool live = left > 0;
+              left -= 8;
+              gates();                                             // of the next eight tokens
+              if (whole) {
+                if (live) *reinterpret_cast<uint4*>(yp) = o;
+              } else if (live) {
+                const unsigned w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  if (i < rows) reinterpret_cast<unsigned short*>(yp)[i] = (unsigned short)((i & 1) ? w[i / 2] >> 16 : w[i / 2] & 0xffffu);
+              }
+              yp += step8;
+              __syncwarp();
+              fill_next();
+            }
+            if (!ok) break;
+            continue;
+          }
+        }
 #pragma unroll 1
         for (int c0 = grp * CH; c0 < (grp + 1) * CH; c0 += W) {
           unsigned r[W], t[W];
@@ -644,7 +806,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
 #pragma unroll
             for (int j = 0; j < W; ++j) __stcg(&slice[(c0 + j) * BM + row], __uint_as_float(r[j]));
           } else {
-            if constexpr (TN >= 128) {
+            if constexpr (TN == 128) {
               if (vec) {
                 float v[W];
 #pragma unroll
@@ -663,6 +825,10 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
           }
         }
         tc_fence_before();
+        if constexpr (L::kAhead) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_free[grp >> 1]);
+        }
         // every warp is done reading the accumulator before any warp stores the next item's A operand
         if (!(ok = warps_rendezvous(ep_bar, ep_uses, lane, abort_flag))) break;
         if (split && ph.scatter) {
@@ -692,7 +858,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
               // per thread spill under the 128-register cap): one round
               // trip to the L2 instead of one per column.  A column's slices are added in split order.  (Rows beyond N exist in
               // the slices and are summed like the others; they are never stored.)
-              const int cstep = 2 * ph.splits;
+              const int cstep = L::kGroups * ph.splits;
               auto batch = [&](auto cb_c, auto sb_c) -> bool {
                 constexpr int CB = decltype(cb_c)::value, SB = decltype(sb_c)::value;
                 for (int cb = sp + grp * ph.splits; cb < TN; cb += CB * cstep) {
@@ -717,7 +883,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
                     if (vec) {
 #pragma unroll
                       for (int u = 0; u < CB; ++u) v[u] = v[u] * sc0 + bv0;
-                      constexpr int CS = CB < 16 ? CB : 16;      // the staging tile holds 16 token columns
+                      constexpr int CS = CB < L::kOutTokens ? CB : L::kOutTokens;   // the staging tile's token columns
 #pragma unroll
                       for (int h = 0; h < CB / CS; ++h)
                         store_transposed<CS, TN>(*reinterpret_cast<const float(*)[CS]>(&v[h * CS]), out_stage, lane, y, ph.N, prog.M,
@@ -747,7 +913,7 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
               const float* tile0 = ph.partial + (size_t)(item - sp) * (TN * BM) + row;
               // all of this thread's columns and slices in flight at once (up to 8 x 4, 4 x 8 or 2 x 16 loads): one round trip
               // to the L2 instead of one per column.  A column's slices are added in split order.
-              const int cstep = 2 * ph.splits;
+              const int cstep = L::kGroups * ph.splits;
               auto batch = [&](auto cb_c, auto sb_c) {
                 constexpr int CB = decltype(cb_c)::value, SB = decltype(sb_c)::value;
                 for (int cb = sp + grp * ph.splits; cb < TN; cb += CB * cstep) {
@@ -886,7 +1052,7 @@ int launch_q(const Program& prog, int grid, bool coresident, cudaStream_t s) {
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kThreadsQ);
+  cfg.blockDim = dim3(L::kThreads);
   cfg.dynamicSmemBytes = (size_t)L::kBytes;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
@@ -966,6 +1132,7 @@ bool fill_sub(SubGemm& sg, const GemmSpec& g, int64_t M, int tn, int bits, bool 
   sg.scale = g.scale;
   sg.bias = (const __nv_bfloat16*)g.bias;
   sg.y = (__nv_bfloat16*)g.y;
+  sg.gate = (const __nv_bfloat16*)g.gate;
   return true;
 }
 
@@ -994,6 +1161,9 @@ int run_program_tcq(const PhaseSpec* specs, int n_phases, int bits, int64_t M, u
     const GemmPlan g = plan_gemm(M, ps.g[0].N, ps.g[0].K, ps.gated ? 1 : ps.nsub, ps.gated != 0, bits == 1 ? 2 : 1);
     if (p == 0) tn = g.tn;
     if (ps.gated && (g.tn > 64 || ps.nsub != 2)) return TSB200_ERR_UNSUPPORTED;
+    for (int j = 0; j < ps.nsub; ++j)                        // gate tiles are read by the lanes that move the 256-token tile's outputs
+      if (ps.g[j].gate && (g.tn != 256 || g.splits != 1 || ps.gated || ps.g[j].N % 8 || !aligned(ps.g[j].gate, 16) || !aligned(ps.g[j].y, 16)))
+        return TSB200_ERR_UNSUPPORTED;
     ph.nsub = ps.nsub;
     ph.gated = ps.gated;
     ph.N = ps.g[0].N;

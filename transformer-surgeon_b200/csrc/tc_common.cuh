@@ -228,6 +228,7 @@ struct GemmSpec {
   const void* x;
   void* y;
   int64_t N, K;
+  const void* gate = nullptr;    // [M, N]: y = silu(gate) * (the product); 256-token tiles only
 };
 // One phase of a multi-phase launch: 1 matrix, 2 independent matrices of the same shape, or
 // (gated) a gate / up pair whose epilogue stores silu(gate) * up into g[0].y.
