@@ -256,9 +256,11 @@ def test_gated_mlp_prompt(cuda, p, M, K, I, r):
 
 
 @pytest.mark.parametrize("p", [8, 4, 2, "binary"])
-@pytest.mark.parametrize("M,K,N", [(129, 128, 40000), (256, 64, 19072), (600, 192, 12928), (1000, 320, 9004), (4100, 256, 2560), (777, 1280, 6150)])
+@pytest.mark.parametrize("M,K,N", [(129, 128, 40000), (256, 64, 19072), (600, 192, 12928), (1000, 320, 9004), (4100, 256, 2560), (777, 1280, 6150),
+                                   (300, 1024, 3600), (250, 1024, 4104), (131, 2048, 2200), (1000, 1024, 640)])
 def test_many_short_items_per_cta(cuda, p, M, K, N):
-    """256-token tiles: items of one to a few stages, widened ahead of the previous item's outputs; ragged tokens, rows and row pitches."""
+    """256-token tiles: items of one to a few stages, widened ahead of the previous item's outputs; ragged tokens, rows and row pitches;
+    K ranges shared by two, four, eight and seven CTAs."""
     from transformer_surgeon_b200 import ops
     if p == "binary":
         K = (K + 127) // 128 * 128

@@ -219,6 +219,20 @@ __device__ __forceinline__ void tmem_ld_frag(unsigned taddr, unsigned (&r)[32]) 
       : "r"(taddr)
       : "memory");
 }
+// The same for U units of eight columns.
+template <int U> __device__ __forceinline__ void tmem_ld_units(unsigned taddr, unsigned (&r)[4 * U]) {
+  if constexpr (U == 4)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+  else if constexpr (U == 2)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
 // Four 8 x 8 matrices of 16-bit values, transposed: lane 8 m + i gives the address of column i of matrix m.
 __device__ __forceinline__ void stmatrix4_trans(unsigned saddr, const unsigned (&r)[4]) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(saddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
@@ -685,19 +699,42 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
         // turns the gate columns into SiLU(g), then fetches the up columns into the freed registers
         constexpr int W = CH >= 16 ? 16 : 8;
         if constexpr (L::kAhead) {
-          if (!split) {
-            const int nw0 = it.nt * BM + q * 32;                   // first weight row of the warp
-            const int64_t mh = m0 + grp * CH;                      // first token of the warp
+          static_assert(CH == 64, "one fragment load covers the warp's tokens");
+          const int nw0 = it.nt * BM + q * 32;                     // first weight row of the warp
+          // The sums come as 8 x 8 fragments (lane: row lane / 4, tokens 2 (lane % 4) and one further), so that one stmatrix turns
+          // eight tokens of the warp's 32 rows around.
+          auto frag = [&](int hf, unsigned (&r)[32]) {             // rows 16 hf .. of the warp
+            tmem_ld_frag(lane_addr + ((unsigned)(hf * 16) << 16) + (unsigned)(grp * CH), r);
+            tmem_ld_wait();
+          };
+          auto release = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_free[grp >> 1]);
+          };
+          float sc[2][2], bv[2][2];                                // of the lane's rows in the fragments
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            sc[k >> 1][k & 1] = __shfl_sync(0xffffffffu, sc0, k * 8 + (lane >> 2));
+            bv[k >> 1][k & 1] = __shfl_sync(0xffffffffu, bv0, k * 8 + (lane >> 2));
+          }
+          auto pair = [&](int hf, int k, unsigned a, unsigned b) {
+            const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(a) * sc[hf][k] + bv[hf][k], __uint_as_float(b) * sc[hf][k] + bv[hf][k]);
+            return *reinterpret_cast<const unsigned*>(&v);
+          };
+          // NU units of eight tokens from token mh on, read by `get` as [unit][rows 8 k ..]: two tokens of a row each
+          auto emit = [&](auto nu_c, int64_t mh, auto&& get) {
+            constexpr int NU = decltype(nu_c)::value;
             // The 16-byte piece that this lane moves per eight tokens: token lane / 4, rows 8 (lane % 4) ..  All that the loop below needs
             // is in registers before it (program fields in constant memory cost it a serial load each).
             const int64_t at = ((mh + (lane >> 2)) * ph.N + nw0 + (lane & 3) * 8) * 2;
             char* yp = reinterpret_cast<char*>(y) + at;
             const char* gp = sg0.gate ? reinterpret_cast<const char*>(sg0.gate) + at : nullptr;
             unsigned step8 = (unsigned)ph.N * 16u;                 // bytes from a token to the eighth after it
-            int left = (int)min(prog.M - mh - (lane >> 2), (int64_t)CH);                       // tokens: piece j of the lane is token 8 j
+            int left = (int)min(prog.M - mh - (lane >> 2), (int64_t)(8 * NU));                 // tokens: piece j of the lane is token 8 j
             int rows = (int)min(ph.N - nw0 - (lane & 3) * 8, (int64_t)8);                      // valid rows of the pieces
             if (rows <= 0) left = 0;
-            bool whole = vec;
+            const bool whole = vec;
             asm volatile("" : "+r"(step8), "+r"(left), "+r"(rows), "+l"(yp), "+l"(gp));
             uint4 gt = {};
             auto gates = [&]() {
@@ -705,32 +742,8 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
               if (gp) gp += step8;
             };
             gates();
-            // The sums come as 8 x 8 fragments (lane: row lane / 4, tokens 2 (lane % 4) and one further), so that one stmatrix turns
-            // eight tokens of the warp's 32 rows around.
-            static_assert(CH == 64, "one fragment load covers the warp's tokens");
-            unsigned pk[CH / 8][4];                                // [eight tokens][eight rows]: two tokens of a row
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {                       // rows 16 hf .. of the warp
-              float sc[2], bv[2];
-#pragma unroll
-              for (int k = 0; k < 2; ++k) {
-                sc[k] = __shfl_sync(0xffffffffu, sc0, hf * 16 + k * 8 + (lane >> 2));
-                bv[k] = __shfl_sync(0xffffffffu, bv0, hf * 16 + k * 8 + (lane >> 2));
-              }
-              unsigned r[32];
-              tmem_ld_frag(lane_addr + ((unsigned)(hf * 16) << 16) + (unsigned)(grp * CH), r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < CH / 8; ++i)
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                  const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[4 * i + 2 * k]) * sc[k] + bv[k], __uint_as_float(r[4 * i + 2 * k + 1]) * sc[k] + bv[k]);
-                  pk[i][hf * 2 + k] = *reinterpret_cast<const unsigned*>(&v);
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_free[grp >> 1]);
+            unsigned pk[NU][4];
+            get(pk);
             // staging: eight tokens x 64 bytes; 16-byte pieces swizzled so that eight rows of a matrix, and two tokens of a read, cover
             // all banks
             const unsigned sb = smem_u32(out_stage);
@@ -739,10 +752,10 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
             // eight tokens, a stage of the next item, eight tokens, ...: outputs that follow one another hold the warps while the MMAs
             // run out of stages
 #pragma unroll 1
-            for (int h = 0; h < CH / 8; ++h) {
+            for (int h = 0; h < NU; ++h) {
               stmatrix4_trans(st_at, pk[0]);
 #pragma unroll
-              for (int i = 0; i + 1 < CH / 8; ++i)                 // the next eight tokens move up
+              for (int i = 0; i + 1 < NU; ++i)                     // the next eight tokens move up
 #pragma unroll
                 for (int k = 0; k < 4; ++k) pk[i][k] = pk[i + 1][k];
               __syncwarp();
@@ -761,8 +774,90 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
               }
               yp += step8;
               __syncwarp();
-              fill_next();
+              if constexpr (NU == CH / 8) fill_next();             // (a CTA with a share of a split tile has one item in the phase)
             }
+          };
+          if (!split) {
+            emit(std::integral_constant<int, CH / 8>{}, m0 + grp * CH, [&](unsigned (&pk)[CH / 8][4]) {
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {
+                unsigned r[32];
+                frag(hf, r);
+#pragma unroll
+                for (int i = 0; i < CH / 8; ++i)
+#pragma unroll
+                  for (int k = 0; k < 2; ++k) pk[i][hf * 2 + k] = pair(hf, k, r[4 * i + 2 * k], r[4 * i + 2 * k + 1]);
+              }
+              release();
+            });
+            if (!ok) break;
+            continue;
+          }
+          if (ph.scatter && (ph.splits == 2 || ph.splits == 4 || ph.splits == 8)) {
+            // Two, four or eight CTAs share a tile's K range; CTA sp finishes units [sp U, sp U + U) of eight tokens of every warp's
+            // eight.  The other units go to the slice as fragments (16 bytes a lane, in lane order), its own stay in tensor memory, and
+            // every warp has eight reads of slices in flight.  10.2 k cycles of a 2048-token, 4096 -> 1024, two-split phase; whole slices as
+            // rows, summed from memory, took 15.7 k.
+            int* ctr = &ph.counters[(it.sub * ph.m_tiles + it.mt) * ph.n_tiles + it.nt];
+            const int sp = item % ph.splits;
+            // this lane's 16 bytes of slice 0, unit 0, rows 0 ..; a slice is 128 KB on, a unit 1024 bytes, the upper rows 512
+            char* mine = reinterpret_cast<char*>(ph.partial) + (size_t)(item - sp) * (TN * BM * 4) + (warp - 2) * 8192 + lane * 16;
+            asm volatile("" : "+l"(mine));
+            auto exchange = [&](auto s_c) {
+              constexpr int S = decltype(s_c)::value, U = 8 / S;
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {
+                unsigned r[32];
+                frag(hf, r);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  if (i / U != sp) __stcg(reinterpret_cast<uint4*>(mine + sp * (TN * BM * 4) + i * 1024 + hf * 512), make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]));
+              }
+              ok = warps_rendezvous(ep_bar, ep_uses, lane, abort_flag);
+              if (!ok) return;
+              if (threadIdx.x == 64) {
+                // fence, arrival, acquire polling and departure as below
+                __threadfence();
+                atomicAdd(ctr, 1);
+                grid_wait(ctr, S, abort_flag);
+                atomicInc(reinterpret_cast<unsigned*>(ctr), 2u * (unsigned)S - 1u);
+              }
+              ok = warps_rendezvous(ep_bar, ep_uses, lane, abort_flag) && !*abort_flag;
+              if (!ok) return;
+              emit(std::integral_constant<int, U>{}, m0 + grp * CH + sp * U * 8, [&](unsigned (&pk)[U][4]) {
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                  uint4 a[U][S];                                   // 8 loads of 16 bytes (in place of the own slice, its neighbour again)
+#pragma unroll
+                  for (int t = 0; t < S; ++t) {
+                    const char* from = mine + (sp * (U * 1024) + (t == sp ? t ^ 1 : t) * (TN * BM * 4) + hf * 512);
+#pragma unroll
+                    for (int i = 0; i < U; ++i) a[i][t] = __ldcg(reinterpret_cast<const uint4*>(from + i * 1024));
+                  }
+                  unsigned own[4 * U];
+                  tmem_ld_units<U>(lane_addr + ((unsigned)(hf * 16) << 16) + (unsigned)(grp * CH + sp * U * 8), own);
+                  tmem_ld_wait();
+#pragma unroll
+                  for (int i = 0; i < U; ++i) {
+                    float v[4] = {0.f, 0.f, 0.f, 0.f};             // splits in order: the order of arrival does not matter
+#pragma unroll
+                    for (int t = 0; t < S; ++t) {
+                      const bool own_t = t == sp;
+                      v[0] += own_t ? __uint_as_float(own[4 * i]) : __uint_as_float(a[i][t].x);
+                      v[1] += own_t ? __uint_as_float(own[4 * i + 1]) : __uint_as_float(a[i][t].y);
+                      v[2] += own_t ? __uint_as_float(own[4 * i + 2]) : __uint_as_float(a[i][t].z);
+                      v[3] += own_t ? __uint_as_float(own[4 * i + 3]) : __uint_as_float(a[i][t].w);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) pk[i][hf * 2 + k] = pair(hf, k, __float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
+                  }
+                }
+                release();
+              });
+            };
+            if (ph.splits == 2) exchange(std::integral_constant<int, 2>{});
+            else if (ph.splits == 4) exchange(std::integral_constant<int, 4>{});
+            else exchange(std::integral_constant<int, 8>{});
             if (!ok) break;
             continue;
           }
