@@ -7,15 +7,19 @@
 // (tokens contiguous, zero beyond L), both bf16, so that every MMA operand tile is K-major and one TMA box:
 //     S[128 q, 128 keys]  = Q[128, d] . K_tile[128, d]^T          (tcgen05.mma kind::f16, fp32 in TMEM)
 //     O[128 q, d]        += P[128, 128] . Vt_tile[d, 128]^T
-// One CTA = one (sequence, query head, 128-query tile); tiles are issued longest first.  Warp roles (6 warps):
-//   warp 0      TMA: the Q tile once, then K / Vt tiles into a 2-stage ring
-//   warp 1      TMEM allocation (S double-buffered, O); one lane issues the MMAs: S(j+1) is issued before it
-//               waits for P(j), so the score MMAs of the next tile overlap the softmax of this one
-//   warps 2..5  softmax: one thread = one query row (its TMEM lane): tcgen05.ld the 128 scores, mask the
+// A persistent CTA works on TWO query tiles of one kv head at a time (their K / Vt tiles are shared), so that the tensor pipe multiplies
+// for one while the other's softmax runs; the tiles of a kv head's query group are enumerated query-tile-major and paired in that
+// order (two heads of one tile, now and then the last head of a tile with the first of the next), pairs go longest first.  11 warps:
+//   warp 0      TMA: the pair's Q tiles, then K0, K1, V0, K2, V1, ... into a ring of three 128-key tiles, across pairs
+//   warps 1, 2  one lane each: MMA issuer of a query tile (one lane needs ~114 cycles per MMA of 64 cycles of the pipe): S(j+1) as soon
+//               as the softmax has moved S(j) to registers, then O += P(j) . V(j); warp 1 allocates the tensor memory (S, S', O, O')
+//   warps 3..6, 7..10  softmax of a query tile: one thread = one query row (its TMEM lane): tcgen05.ld the 128 scores, mask the
 //               diagonal tile, running maximum with LAZY rescaling (O and the row sum are rescaled only when the
 //               maximum grew by more than 2^8; the final division uses the same reference maximum, so the result is
 //               exact), exp2, row sum in fp32, P rounded to bf16 into shared memory in the swizzled K-major layout
-//               the MMA descriptor expects; at the end O / l, rounded, 16-byte stores
+//               the MMA descriptor expects; at the end O / l, rounded, while the next pair's scores are computed
+// Bounds at 128 x 128 scores of a tile: 1024 cycles of the tensor pipe, 1024 of the exponential unit, ~1500 of shared memory.
+// 8 x 2048 tokens, 32 / 8 heads of 128: 570 us with one query tile per CTA (4300 cycles a tile).
 // Every mbarrier wait is bounded; on expiry the CTA records a code in the status word, frees its TMEM and returns.
 #include "tc_common.cuh"
 #include "decode_attn_common.cuh"
@@ -24,8 +28,8 @@ namespace tsb {
 using namespace tc;
 namespace {
 
-constexpr int kPfThreads = 192;
-constexpr int BQ = 128, BKEY = 128;
+constexpr int kPfThreads = 352;
+constexpr int BQ = 128, BKEY = 128, kRing = 3;
 
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
   asm volatile(
@@ -53,6 +57,7 @@ __device__ __forceinline__ void tmem_st_wait_pf() { asm volatile("tcgen05.wait::
 struct PfParams {
   int64_t B, T, L;
   int H, hkv;
+  int nq, pairs, items;      // query tiles per head, pairs per (sequence, kv head), pairs in all
   float scale_log2;          // sm_scale * log2(e)
   __nv_bfloat16* out;        // [B, T, H, D]
   int* status;
@@ -61,14 +66,19 @@ struct PfParams {
 template <int D> struct PfLayout {
   static constexpr int KB = D / 64;                    // 64-column blocks of the head dimension
   static constexpr int kQ = KB * BQ * 128;             // Q tile
-  static constexpr int kK = KB * BKEY * 128;           // K tile: KB blocks of [128 keys x 128 B]
-  static constexpr int kV = 2 * D * 128;               // Vt tile: 2 blocks (64 keys each) of [D rows x 128 B]
+  static constexpr int kTile = D * 256;                // K tile: KB blocks of [128 keys x 128 B]; Vt tile: 2 blocks (64 keys each) of [D rows x 128 B]
   static constexpr int kP = 2 * BQ * 128;              // P tile: 2 blocks (64 keys each) of [128 rows x 128 B]
-  static constexpr int kStage = kK + kV;
-  static constexpr int kBytes = kQ + 2 * kStage + kP + 1024 /*barriers*/ + 1024 /*alignment*/;
-  static constexpr unsigned kSCol = 0;                 // S buffers at columns 0 and 128
-  static constexpr unsigned kOCol = 256;               // O accumulator: D columns
+  static constexpr int kBytes = 2 * kQ + kRing * kTile + 2 * kP + 1024 /*barriers*/ + 1024 /*alignment*/;
+  static constexpr unsigned kSCol = 0;                 // S of tile i at columns 128 i
+  static constexpr unsigned kOCol = 256;               // O of tile i at 256 + 128 i
+  static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
 };
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));   // below 2^-126: 0, which adds as little to a row's sum (at least 2^-8)
+  return y;
+}
 
 template <int D>
 __global__ void __launch_bounds__(kPfThreads, 1)
@@ -77,33 +87,43 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   using Lt = PfLayout<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + Lt::kQ;                          // 2 stages of {K, Vt}
-  uint8_t* sP = sKV + 2 * Lt::kStage;
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(sP + Lt::kP);
-  unsigned long long* q_full = bars;                   // [1]
-  unsigned long long* kv_full = bars + 1;              // [2] K and Vt tile landed
-  unsigned long long* kv_empty = bars + 3;             // [2] the tile's second MMA group (P.V) is complete
-  unsigned long long* s_full = bars + 5;               // [2] scores of a tile are in TMEM buffer (tile & 1)
-  unsigned long long* p_full = bars + 7;               // [1] the four softmax warps wrote P (and are done with S)
-  unsigned long long* o_done = bars + 8;               // [1] P.V of a tile is complete: P and O may be touched
-  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 9);
+  uint8_t* sQ = smem;                                  // two tiles
+  uint8_t* sKV = sQ + 2 * Lt::kQ;                      // ring
+  uint8_t* sP = sKV + kRing * Lt::kTile;               // two tiles
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(sP + 2 * Lt::kP);
+  unsigned long long* q_full = bars;                   // [1] the pair's Q tiles landed
+  unsigned long long* q_empty = bars + 1;              // [1] both issuers: the pair's last score MMAs are complete
+  unsigned long long* kv_full = bars + 2;              // [kRing] a K or Vt tile landed
+  unsigned long long* kv_empty = kv_full + kRing;      // [kRing] both issuers: MMAs that read it are complete
+  unsigned long long* s_full = kv_empty + kRing;       // [2] scores of query tile i are in TMEM
+  unsigned long long* s_free = s_full + 2;             // [2] its four softmax warps have them in registers
+  unsigned long long* p_full = s_free + 2;             // [2] ... have written P
+  unsigned long long* o_done = p_full + 2;             // [2] P.V is complete: P and O may be touched
+  unsigned long long* o_free = o_done + 2;             // [2] the four warps have read the finished O
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;            // longest tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hk = h / (p.H / p.hkv);
   const int64_t off = p.L - p.T;                                   // position of query 0
-  const int64_t q0 = (int64_t)qt * BQ;
-  const int64_t max_pos = off + min(p.T - 1, q0 + BQ - 1);
-  const int n_tiles = (int)(max_pos / BKEY) + 1;
+  const int G = p.H / p.hkv;
+  // Work item w: sequence, kv head and, for query tile i of the pair, its head, first query and number of key tiles (0: no tile).
+  struct Work { int b, hk, pair; };
+  struct Tile { int h, n; int64_t q0; };
+  auto work = [&](int w) {
+    const int per = p.hkv * (int)p.B, rest = w % per;
+    return Work{rest / p.hkv, rest % p.hkv, p.pairs - 1 - w / per};   // longest first
+  };
+  auto tile = [&](const Work& k, int i) {
+    const int u = 2 * k.pair + i, qt = u / G;
+    const int64_t q0 = (int64_t)qt * BQ;
+    return Tile{k.hk * G + u % G, qt < p.nq ? (int)((off + min(p.T - 1, q0 + BQ - 1)) / BKEY) + 1 : 0, q0};
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); mbar_init(&s_full[i], 1); }
-    mbar_init(p_full, 4);
-    mbar_init(o_done, 1);
+    mbar_init(q_empty, 2);
+    for (int i = 0; i < kRing; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4); mbar_init(&o_done[i], 1); mbar_init(&o_free[i], 4); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -118,167 +138,232 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      mbar_expect_tx(q_full, (unsigned)Lt::kQ);
-      for (int kb = 0; kb < Lt::KB; ++kb)
-        tma_load_3d(sQ + kb * BQ * 128, &map_q, kb * 64, h, (int)(b * p.T + q0), q_full);
-      const int64_t krow0 = ((int64_t)b * p.hkv + hk) * p.L;
-      const int64_t vrow0 = ((int64_t)b * p.hkv + hk) * D;
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j & 1;
-        if (j >= 2 && !mbar_wait(&kv_empty[s], ((j >> 1) - 1) & 1, abort_flag, 1)) break;
-        uint8_t* st = sKV + s * Lt::kStage;
-        mbar_expect_tx(&kv_full[s], (unsigned)Lt::kStage);
-        for (int kb = 0; kb < Lt::KB; ++kb)
-          tma_load_2d(st + kb * BKEY * 128, &map_k, kb * 64, (int)(krow0 + (int64_t)j * BKEY), &kv_full[s]);
-        for (int kb = 0; kb < 2; ++kb)
-          tma_load_2d(st + Lt::kK + kb * D * 128, &map_vt, j * BKEY + kb * 64, (int)vrow0, &kv_full[s]);
+      int c = 0, it = 0;                                // tiles of the ring, work items so far
+      bool ok = true;
+      for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x, ++it) {
+        const Work k = work(w);
+        const Tile x = tile(k, 0), y = tile(k, 1);
+        const int most = max(x.n, y.n);
+        if (it > 0 && !mbar_wait(q_empty, (it - 1) & 1, abort_flag, 1)) break;
+        mbar_expect_tx(q_full, (unsigned)((x.n > 0) + (y.n > 0)) * Lt::kQ);
+        for (int kb = 0; kb < Lt::KB; ++kb) {
+          if (x.n > 0) tma_load_3d(sQ + kb * BQ * 128, &map_q, kb * 64, x.h, (int)(k.b * p.T + x.q0), q_full);
+          if (y.n > 0) tma_load_3d(sQ + Lt::kQ + kb * BQ * 128, &map_q, kb * 64, y.h, (int)(k.b * p.T + y.q0), q_full);
+        }
+        const int64_t krow0 = ((int64_t)k.b * p.hkv + k.hk) * p.L;
+        const int64_t vrow0 = ((int64_t)k.b * p.hkv + k.hk) * D;
+        auto slot = [&]() -> uint8_t* {
+          const int s = c % kRing;
+          if (c >= kRing && !mbar_wait(&kv_empty[s], (c / kRing - 1) & 1, abort_flag, 2)) { ok = false; return nullptr; }
+          mbar_expect_tx(&kv_full[s], (unsigned)Lt::kTile);
+          return sKV + s * Lt::kTile;
+        };
+        for (int j = 0; j <= most && ok; ++j) {         // K(j), V(j - 1)
+          if (j < most) {
+            uint8_t* st = slot();
+            if (!ok) break;
+            for (int kb = 0; kb < Lt::KB; ++kb)
+              tma_load_2d(st + kb * BKEY * 128, &map_k, kb * 64, (int)(krow0 + (int64_t)j * BKEY), &kv_full[c % kRing]);
+            ++c;
+          }
+          if (j > 0) {
+            uint8_t* st = slot();
+            if (!ok) break;
+            for (int kb = 0; kb < 2; ++kb)
+              tma_load_2d(st + kb * D * 128, &map_vt, (j - 1) * BKEY + kb * 64, (int)vrow0, &kv_full[c % kRing]);
+            ++c;
+          }
+        }
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+  } else if (warp <= 2) {
+    // ------------------------------------------------------------------ MMA issuer of query tile i
     if (lane == 0) {
+      const int i = warp - 1;
       constexpr unsigned idesc_s = idesc_bf16(BKEY);
       constexpr unsigned idesc_o = idesc_bf16(D);
-      bool ok = mbar_wait(q_full, 0, abort_flag, 2);
-      auto issue_s = [&](int j) {                      // scores of tile j into S buffer j & 1
-        const int s = j & 1;
-        if (!mbar_wait(&kv_full[s], (j >> 1) & 1, abort_flag, 3)) return false;
-        tc_fence_after();
-        const unsigned d_tmem = tmem_base + Lt::kSCol + (unsigned)s * 128;
-        const uint8_t* st = sKV + s * Lt::kStage;
+      const unsigned s_tmem = tmem_base + Lt::kSCol + 128 * i, o_tmem = tmem_base + Lt::kOCol + 128 * i;
+      const unsigned q_addr = smem_u32(sQ + i * Lt::kQ), p_addr = smem_u32(sP + i * Lt::kP);
+      int c = 0, it = 0;                                // tiles of the ring, work items so far
+      int ts = 0, tp = 0, outs = 0;                     // scores issued, P.V issued, finished O tiles so far
+      bool ok = true;
+      for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x, ++it) {
+        const Work k = work(w);
+        const int n = tile(k, i).n, most = max(n, tile(k, 1 - i).n);
+        ok = mbar_wait(q_full, it & 1, abort_flag, 3);
+        for (int j = 0; j <= most && ok; ++j) {         // S(j), then P(j - 1) . V(j - 1)
+          if (j < most) {
+            const int s = c % kRing;
+            ok = mbar_wait(&kv_full[s], (c / kRing) & 1, abort_flag, 4);
+            if (ok && j < n && ts > 0) ok = mbar_wait(&s_free[i], (ts - 1) & 1, abort_flag, 5);
+            if (!ok) break;
+            if (j < n) {
+              tc_fence_after();
+              const unsigned k_addr = smem_u32(sKV + s * Lt::kTile);
 #pragma unroll
-        for (int kb = 0; kb < Lt::KB; ++kb) {
-          const unsigned long long ad = smem_desc_sw128(smem_u32(sQ + kb * BQ * 128));
-          const unsigned long long bd = smem_desc_sw128(smem_u32(st + kb * BKEY * 128));
+              for (int kb = 0; kb < Lt::KB; ++kb) {
+                const unsigned long long ad = smem_desc_sw128(q_addr + kb * BQ * 128);
+                const unsigned long long bd = smem_desc_sw128(k_addr + kb * BKEY * 128);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16(d_tmem, ad + 2 * k, bd + 2 * k, idesc_s, (kb | k) ? 1u : 0u);
+                for (int kk = 0; kk < 4; ++kk) umma_bf16(s_tmem, ad + 2 * kk, bd + 2 * kk, idesc_s, (kb | kk) ? 1u : 0u);
+              }
+              umma_commit(&s_full[i]);
+              umma_commit(&kv_empty[s]);
+              ++ts;
+            } else {
+              mbar_arrive(&kv_empty[s]);
+            }
+            if (j == most - 1) umma_commit(q_empty);
+            ++c;
+          }
+          if (j > 0) {
+            const int s = c % kRing;
+            ok = mbar_wait(&kv_full[s], (c / kRing) & 1, abort_flag, 6);
+            if (ok && j - 1 < n) {
+              ok = mbar_wait(&p_full[i], tp & 1, abort_flag, 7);
+              if (ok && j == 1 && outs > 0) ok = mbar_wait(&o_free[i], (outs - 1) & 1, abort_flag, 8);
+            }
+            if (!ok) break;
+            if (j - 1 < n) {
+              tc_fence_after();
+              const unsigned v_addr = smem_u32(sKV + s * Lt::kTile);
+#pragma unroll
+              for (int kb = 0; kb < 2; ++kb) {
+                const unsigned long long ad = smem_desc_sw128(p_addr + kb * BQ * 128);
+                const unsigned long long bd = smem_desc_sw128(v_addr + kb * D * 128);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) umma_bf16(o_tmem, ad + 2 * kk, bd + 2 * kk, idesc_o, (j > 1 || (kb | kk)) ? 1u : 0u);
+              }
+              umma_commit(&o_done[i]);
+              umma_commit(&kv_empty[s]);
+              ++tp;
+            } else {
+              mbar_arrive(&kv_empty[s]);
+            }
+            ++c;
+          }
         }
-        umma_commit(&s_full[s]);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        // S buffer (j + 1) & 1 was read by the softmax of tile j - 1, which p_full(j - 1) reported
-        if (j + 1 < n_tiles) ok = issue_s(j + 1);
-        if (!ok) break;
-        ok = mbar_wait(p_full, j & 1, abort_flag, 4);
-        if (!ok) break;
-        tc_fence_after();
-        const int s = j & 1;
-        const uint8_t* st = sKV + s * Lt::kStage + Lt::kK;
-        const unsigned o_tmem = tmem_base + Lt::kOCol;
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-          const unsigned long long ad = smem_desc_sw128(smem_u32(sP + kb * BQ * 128));
-          const unsigned long long bd = smem_desc_sw128(smem_u32(st + kb * D * 128));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16(o_tmem, ad + 2 * k, bd + 2 * k, idesc_o, (j | kb | k) ? 1u : 0u);
-        }
-        umma_commit(&kv_empty[s]);
-        umma_commit(o_done);
+        if (n > 0) ++outs;
       }
     }
   } else {
-    // ------------------------------------------------------------------ softmax + epilogue
+    // ------------------------------------------------------------------ softmax + epilogue of query tile i
+    const int i = (warp - 3) >> 2;
     const int quarter = warp & 3;                      // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;               // query row of the tile
     const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
-    const int64_t qpos = off + q0 + row;               // position of this row's query
-    float m_ref = -INFINITY, l_sum = 0.f;
+    const unsigned s_tmem = lane_addr + Lt::kSCol + 128 * i, o_tmem = lane_addr + Lt::kOCol + 128 * i;
+    uint8_t* my_p = sP + i * Lt::kP;
+    int t = 0;                                         // tiles so far
     bool ok = true;
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int s = j & 1;
-      ok = mbar_wait(&s_full[s], (j >> 1) & 1, abort_flag, 5);
-      if (!ok) break;
-      tc_fence_after();
-      float sc[128];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        unsigned r[32];
-        tmem_ld32(lane_addr + Lt::kSCol + (unsigned)s * 128 + c * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sc[c * 32 + i] = __uint_as_float(r[i]) * p.scale_log2;
-      }
-      const int64_t key0 = (int64_t)j * BKEY;
-      if (key0 + BKEY - 1 > off + q0) {                // a tile that reaches past the tile's first query: mask
-#pragma unroll
-        for (int i = 0; i < 128; ++i)
-          if (key0 + i > qpos) sc[i] = -INFINITY;
-      }
-      float m_tile = sc[0];
-#pragma unroll
-      for (int i = 1; i < 128; ++i) m_tile = fmaxf(m_tile, sc[i]);
-      // lazy rescaling: keep the reference maximum until the true maximum has outgrown it by 2^8
-      float alpha = 1.0f;
-      const bool grow = m_tile > m_ref + 8.0f || m_ref == -INFINITY;
-      if (grow && m_tile > -INFINITY) {
-        alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_tile);
-        m_ref = m_tile;
-        l_sum *= alpha;
-      }
-      const float mr = m_ref == -INFINITY ? 0.f : m_ref;
-      float psum = 0.f;
-      unsigned pk[64];
-#pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        const float p0 = exp2f(sc[2 * i] - mr), p1 = exp2f(sc[2 * i + 1] - mr);
-        psum += p0 + p1;
-        __nv_bfloat162 q2 = __floats2bfloat162_rn(p0, p1);
-        pk[i] = *reinterpret_cast<unsigned*>(&q2);
-      }
-      l_sum += psum;
-      // P(j - 1) . V must be complete before P is overwritten and before O is rescaled
-      if (j > 0) {
-        ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, 6);
+    for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x) {
+      const Work k = work(w);
+      const Tile mine = tile(k, i);
+      const int n = mine.n;
+      const int64_t q0 = mine.q0, qpos = off + q0 + row;           // position of this row's query
+      float m_ref = -INFINITY, l_sum = 0.f;
+      for (int j = 0; j < n && ok; ++j, ++t) {
+        ok = mbar_wait(&s_full[i], t & 1, abort_flag, 9);
         if (!ok) break;
         tc_fence_after();
-        if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+        float sc[128];
+        {
+          unsigned (&r)[4][32] = reinterpret_cast<unsigned (&)[4][32]>(sc);
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            unsigned r[32];
-            tmem_ld32(lane_addr + Lt::kOCol + c * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-            tmem_st32f(lane_addr + Lt::kOCol + c * 32, r);
-          }
-          tmem_st_wait_pf();
+          for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + c * 32, r[c]);
+          tmem_ld_wait();
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[i]);
+#pragma unroll
+        for (int e = 0; e < 128; ++e) sc[e] *= p.scale_log2;
+        const int64_t key0 = (int64_t)j * BKEY;
+        if (key0 + BKEY - 1 > off + q0) {                // a tile that reaches past the tile's first query: mask
+          const int last = (int)min(qpos - key0, (int64_t)BKEY);   // last visible key of the tile
+#pragma unroll
+          for (int e = 0; e < 128; ++e)
+            if (e > last) sc[e] = -INFINITY;
+        }
+        float m_tile = sc[0];
+#pragma unroll
+        for (int e = 1; e < 128; ++e) m_tile = fmaxf(m_tile, sc[e]);
+        // lazy rescaling: keep the reference maximum until the true maximum has outgrown it by 2^8
+        float alpha = 1.0f;
+        const bool grow = m_tile > m_ref + 8.0f || m_ref == -INFINITY;
+        if (grow && m_tile > -INFINITY) {
+          alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_tile);
+          m_ref = m_tile;
+          l_sum *= alpha;
+        }
+        const float mr = m_ref == -INFINITY ? 0.f : m_ref;
+        float psum = 0.f;
+        unsigned pk[64];
+#pragma unroll
+        for (int e = 0; e < 64; ++e) {
+          const float p0 = ex2(sc[2 * e] - mr), p1 = ex2(sc[2 * e + 1] - mr);
+          psum += p0 + p1;
+          __nv_bfloat162 q2 = __floats2bfloat162_rn(p0, p1);
+          pk[e] = *reinterpret_cast<unsigned*>(&q2);
+        }
+        l_sum += psum;
+        // P(j - 1) . V must be complete before P is overwritten and before O is rescaled
+        if (j > 0) {
+          ok = mbar_wait(&o_done[i], (t - 1) & 1, abort_flag, 10);
+          if (!ok) break;
+          tc_fence_after();
+          if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+              unsigned r[32];
+              tmem_ld32(o_tmem + c * 32, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+              tmem_st32f(o_tmem + c * 32, r);
+            }
+            tmem_st_wait_pf();
+          }
+        }
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            store_chunk(my_p + kb * BQ * 128, row, c, make_uint4(pk[kb * 32 + c * 4], pk[kb * 32 + c * 4 + 1], pk[kb * 32 + c * 4 + 2], pk[kb * 32 + c * 4 + 3]));
+        fence_async_proxy();                             // generic-proxy writes -> visible to the MMA (async proxy)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[i]);
       }
+      if (!ok || n == 0) continue;
+      // ---- epilogue: O / l
+      ok = mbar_wait(&o_done[i], (t - 1) & 1, abort_flag, 11);
+      if (!ok) break;
+      tc_fence_after();
+      float o[D];
+      {
+        unsigned (&r)[D / 32][32] = reinterpret_cast<unsigned (&)[D / 32][32]>(o);
 #pragma unroll
-      for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          store_chunk(sP + kb * BQ * 128, row, c, make_uint4(pk[kb * 32 + c * 4], pk[kb * 32 + c * 4 + 1], pk[kb * 32 + c * 4 + 2], pk[kb * 32 + c * 4 + 3]));
-      fence_async_proxy();                             // generic-proxy writes -> visible to the MMA (async proxy)
+        for (int c = 0; c < D / 32; ++c) tmem_ld32(o_tmem + c * 32, r[c]);
+        tmem_ld_wait();
+      }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-    }
-    // ---- epilogue: O / l
-    if (ok && n_tiles > 0) ok = mbar_wait(o_done, (n_tiles - 1) & 1, abort_flag, 7);
-    if (ok) {
-      tc_fence_after();
+      if (lane == 0) mbar_arrive(&o_free[i]);
       const float inv = l_sum > 0.f ? 1.0f / l_sum : 0.f;
       const int64_t tok = q0 + row;
-      __nv_bfloat16* o = p.out + (((int64_t)b * p.T + tok) * p.H + h) * D;
+      if (tok < p.T) {
+        __nv_bfloat16* dst = p.out + (((int64_t)k.b * p.T + tok) * p.H + mine.h) * D;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        unsigned r[32];
-        tmem_ld32(lane_addr + Lt::kOCol + c * 32, r);
-        tmem_ld_wait();
-        if (tok < p.T) {
+        for (int c = 0; c < D / 16; ++c) {
+          unsigned v[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint4 v;
-            __nv_bfloat162 q2;
-            q2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i]) * inv, __uint_as_float(r[8 * i + 1]) * inv); v.x = *reinterpret_cast<unsigned*>(&q2);
-            q2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i + 2]) * inv, __uint_as_float(r[8 * i + 3]) * inv); v.y = *reinterpret_cast<unsigned*>(&q2);
-            q2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i + 4]) * inv, __uint_as_float(r[8 * i + 5]) * inv); v.z = *reinterpret_cast<unsigned*>(&q2);
-            q2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i + 6]) * inv, __uint_as_float(r[8 * i + 7]) * inv); v.w = *reinterpret_cast<unsigned*>(&q2);
-            *reinterpret_cast<uint4*>(o + c * 32 + i * 8) = v;
+          for (int e = 0; e < 8; ++e) {
+            __nv_bfloat162 q2 = __floats2bfloat162_rn(o[c * 16 + 2 * e] * inv, o[c * 16 + 2 * e + 1] * inv);
+            v[e] = *reinterpret_cast<unsigned*>(&q2);
           }
+          *reinterpret_cast<uint4*>(dst + c * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+          *reinterpret_cast<uint4*>(dst + c * 16 + 8) = make_uint4(v[4], v[5], v[6], v[7]);
         }
       }
     }
@@ -446,7 +531,12 @@ int launch_prefill(const void* q, int64_t q_token_stride, const void* k, const v
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   p.out = (__nv_bfloat16*)out;
   p.status = status;
-  dim3 grid((unsigned)((T + BQ - 1) / BQ), (unsigned)H, (unsigned)B);
+  p.nq = (int)((T + BQ - 1) / BQ);
+  const int64_t pairs = ((int64_t)p.nq * (H / hkv) + 1) / 2, items = pairs * hkv * B;
+  if (items > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
+  p.pairs = (int)pairs;
+  p.items = (int)items;
+  const dim3 grid((unsigned)(items < kPlanSMs ? items : kPlanSMs));        // one CTA per SM
   TSB_CUDA(launch_kernel(prefill_attn_kernel<D>, grid, dim3(kPfThreads), (size_t)Lt::kBytes, s, mq, mk, mv, p));
   return TSB200_OK;
 }
