@@ -56,6 +56,11 @@ inline int choose_splits_fp8(int64_t B, int hkv, int64_t max_seq_len) {
   return (int)s;
 }
 
+// Whether the last CTA of a (sequence, kv head, head chunk) merges its splits.  That takes ~80 cycles per (head, split) row - 35 k
+// cycles, 20 us, at 7 heads and 63 splits -, a reduction launch that is resident before the partials are complete ~3 us whatever the
+// shape: the launch from 64 rows on.
+inline bool last_cta_merges(int splits, int H, int hkv) { return splits == 1 || splits * (H / hkv < 8 ? H / hkv : 8) < 64; }
+
 // Pages [begin, end) of sequence with `len` tokens handled by split s of S.
 __device__ __forceinline__ void split_range(int len, int s, int S, int& begin, int& end) {
   const int pages = (len + 15) >> 4;

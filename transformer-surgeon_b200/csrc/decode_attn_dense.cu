@@ -215,6 +215,7 @@ int attn_dense(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, in
   int S = choose_splits(B, kv->hkv, max_seq_len);
   const int64_t cap = (max_seq_len + 255) / 256;
   if (S > cap) S = (int)(cap < 1 ? 1 : cap);
+  if (!last_cta_merges(S, H, kv->hkv)) counters = nullptr;
 #define TSB_GO(TT, PP)                                                                                                       \
   return kv->head_dim == 64 ? launch_dense<TT, PP, 64>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, counters, out, s)    \
                             : launch_dense<TT, PP, 128>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, counters, out, s)

@@ -13,7 +13,7 @@
 // an e2m1 code times its e4m3 block scale is exact in f16 (2 x 4 significant bits), so K goes to
 // the MMA as code * scale; for V the block scale of a token is folded into that token's softmax
 // weight (one product per 16-dim block and token instead of one per element).
-// Partials (m, l, acc) go to the workspace; decode_attn_reduce_kernel merges splits.
+// Partials (m, l, acc) go to the workspace; the last CTA of a (sequence, kv head) or decode_attn_reduce_kernel merges them.
 #include "decode_attn_common.cuh"
 
 namespace tsb {
@@ -145,22 +145,32 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   int pb, pe;
   split_range(len, s, S, pb, pe);
 
-  // Q^T fragments (B operand): this lane holds head g0+gid at the dims of its k-slots.
+  // Q^T fragments (B operand): this lane holds head g0+gid at the dims of its k-slots: 16 consecutive ones per four steps, fetched as
+  // 16-byte pieces where q allows it (element by element: 32 loads, 2500 cycles before the first page of a short split).
   unsigned qf[NC][2];
   {
     const bool valid = gid < gn;
-    const T* qp = q + (int64_t)b * qs + (int64_t)(hk * g + g0 + (valid ? gid : 0)) * D;
+    const T* qp = q + (int64_t)b * qs + (int64_t)(hk * g + g0 + (valid ? gid : 0)) * D + 16 * tid;
+    const bool vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0 && qs * sizeof(T) % 16 == 0;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      // int8 / fp8: the step's k-slots are 4 consecutive dims; NVFP4: dims (x, x + 4) and (x + 1, x + 5),
-      // the pairs that e2m1_pair_alu extracts from a word of 8 codes
-      const int base = FMT == TSB200_KV_NVFP4 ? 16 * (tid + 4 * (c >> 2)) + 8 * ((c & 3) >> 1) + 2 * (c & 1)
-                                              : 16 * (tid + 4 * (c >> 2)) + 4 * (c & 3);
-      constexpr int o1 = FMT == TSB200_KV_NVFP4 ? 4 : 1, o2 = FMT == TSB200_KV_NVFP4 ? 1 : 2, o3 = FMT == TSB200_KV_NVFP4 ? 5 : 3;
-      float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
-      if (valid) { f0 = to_f32<T>(qp[base]); f1 = to_f32<T>(qp[base + o1]); f2 = to_f32<T>(qp[base + o2]); f3 = to_f32<T>(qp[base + o3]); }
-      qf[c][0] = pack_h2(f0, f1);
-      qf[c][1] = pack_h2(f2, f3);
+    for (int hh = 0; hh < NC / 4; ++hh) {
+      __align__(16) T x[16];
+      if (vec) {
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T); ++i) reinterpret_cast<uint4*>(x)[i] = reinterpret_cast<const uint4*>(qp + 64 * hh)[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = qp[64 * hh + i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // int8 / fp8: the step's k-slots are 4 consecutive dims; NVFP4: dims (x, x + 4) and (x + 1, x + 5),
+        // the pairs that e2m1_pair_alu extracts from a word of 8 codes
+        const int base = FP4 ? 8 * (i >> 1) + 2 * (i & 1) : 4 * i;
+        constexpr int o1 = FP4 ? 4 : 1, o2 = FP4 ? 1 : 2, o3 = FP4 ? 5 : 3;
+        qf[4 * hh + i][0] = valid ? pack_h2(to_f32<T>(x[base]), to_f32<T>(x[base + o1])) : 0u;
+        qf[4 * hh + i][1] = valid ? pack_h2(to_f32<T>(x[base + o2]), to_f32<T>(x[base + o3])) : 0u;
+      }
     }
   }
   float kscale = 1.f, vscale = 1.f;
@@ -326,45 +336,60 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
     l1 += __shfl_xor_sync(0xffffffffu, l1, o);
   }
   __syncthreads();   // every warp is done with its ring; reuse shared memory for the merge
+  constexpr int AR = D + 4;                                  // row pitch: the fragments' four head rows fall into different banks
   float* sm_m = reinterpret_cast<float*>(smem);              // [warps][8]
   float* sm_l = sm_m + kWarps * 8;                           // [warps][8]
-  float* sm_acc = sm_l + kWarps * 8;                         // [warps][8][D]
+  float* sm_c = sm_l + kWarps * 8;                           // [warps][8]
+  float* sm_acc = sm_c + kWarps * 8;                         // [warps][8][AR]
   if (gid == 0) {
     sm_m[w * 8 + 2 * tid] = m0; sm_m[w * 8 + 2 * tid + 1] = m1;
     sm_l[w * 8 + 2 * tid] = l0; sm_l[w * 8 + 2 * tid + 1] = l1;
   }
 #pragma unroll
   for (int mt = 0; mt < NC; ++mt) {
-    float* a = sm_acc + (size_t)w * 8 * D;
+    float* a = sm_acc + (size_t)w * 8 * AR;
     const int da = FP4 ? 16 * mt + 2 * gid : 16 * mt + gid;         // dims of MMA rows gid and gid + 8
     const int db = FP4 ? da + 1 : da + 8;
-    a[(2 * tid) * D + da] = oacc[mt][0];
-    a[(2 * tid + 1) * D + da] = oacc[mt][1];
-    a[(2 * tid) * D + db] = oacc[mt][2];
-    a[(2 * tid + 1) * D + db] = oacc[mt][3];
+    a[(2 * tid) * AR + da] = oacc[mt][0];
+    a[(2 * tid + 1) * AR + da] = oacc[mt][1];
+    a[(2 * tid) * AR + db] = oacc[mt][2];
+    a[(2 * tid + 1) * AR + db] = oacc[mt][3];
   }
   __syncthreads();
-  // merge the 4 warps; with one split the result is final, otherwise it is this split's partial
-  for (int idx = threadIdx.x; idx < gn * D; idx += blockDim.x) {
-    const int i = idx / D, e = idx % D;
+  // merge the warps; with one split the result is final, otherwise it is this split's partial.  Coefficients once per (warp, head).
+  if (threadIdx.x < kWarps * 8) {
+    const int i = threadIdx.x & 7;
     float mm = -INFINITY;
 #pragma unroll
     for (int ww = 0; ww < kWarps; ++ww) mm = fmaxf(mm, sm_m[ww * 8 + i]);
-    float ll = 0.f, a = 0.f;
+    const float mw = sm_m[threadIdx.x];
+    sm_c[threadIdx.x] = mw == -INFINITY ? 0.f : exp2f(mw - mm);
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < gn * (D / 2); idx += blockDim.x) {
+    const int i = idx / (D / 2), e = idx % (D / 2) * 2;
+    float ll = 0.f, a0 = 0.f, a1 = 0.f;
 #pragma unroll
     for (int ww = 0; ww < kWarps; ++ww) {
-      const float mw = sm_m[ww * 8 + i];
-      const float c = mw == -INFINITY ? 0.f : exp2f(mw - mm);
+      const float c = sm_c[ww * 8 + i];
+      const float2 x = *reinterpret_cast<const float2*>(&sm_acc[((size_t)ww * 8 + i) * AR + e]);
       ll += sm_l[ww * 8 + i] * c;
-      a += sm_acc[((size_t)ww * 8 + i) * D + e] * c;
+      a0 += x.x * c;
+      a1 += x.y * c;
     }
     const int64_t bh = (int64_t)b * H + hk * g + g0 + i;
     if (S == 1 && fuse_reduce) {
-      out[bh * D + e] = from_f32<T>(ll > 0.f ? a * vscale / ll : 0.f);
+      out[bh * D + e] = from_f32<T>(ll > 0.f ? a0 * vscale / ll : 0.f);
+      out[bh * D + e + 1] = from_f32<T>(ll > 0.f ? a1 * vscale / ll : 0.f);
     } else {
       float* o = ws + (bh * S + s) * (2 + D);
-      if (e == 0) { o[0] = mm * 0.6931471805599453f; o[1] = ll; }   // natural-log domain (shared with the reducer kernel)
-      o[2 + e] = a * vscale;
+      if (e == 0) {                                          // natural-log domain (shared with the reducer kernel)
+        float mm = -INFINITY;
+#pragma unroll
+        for (int ww = 0; ww < kWarps; ++ww) mm = fmaxf(mm, sm_m[ww * 8 + i]);
+        *reinterpret_cast<float2*>(o) = make_float2(mm * 0.6931471805599453f, ll);
+      }
+      *reinterpret_cast<float2*>(o + 2 + e) = make_float2(a0 * vscale, a1 * vscale);
     }
   }
   if (S == 1 || !fuse_reduce) return;
@@ -389,7 +414,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   constexpr int REC = RecBytes<FMT, D>::value;
   constexpr int kWarps = AttnCfg<FMT>::kWarps, kStages = AttnCfg<FMT>::kStages;
   constexpr size_t pipe = (size_t)kWarps * kStages * 2 * REC;
-  constexpr size_t merge = (size_t)(kWarps * 16 + kWarps * 8 * D) * sizeof(float);
+  constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4)) * sizeof(float);
   constexpr size_t smem = pipe > merge ? pipe : merge;
   static bool configured[64] = {false};   // per device: the attribute lives in the device's context
   int dev = 0;
@@ -400,7 +425,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
     configured[dev] = true;
   }
   const int g = H / kv.hkv;
-  dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((g + 7) / 8));
+  dim3 grid((unsigned)(B * kv.hkv), (unsigned)(S < 0 ? -S : S), (unsigned)((g + 7) / 8));   // S < 0: partials only
   TSB_CUDA(launch_kernel(decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, counters, (T*)out));
   return TSB200_OK;
@@ -434,18 +459,20 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   const int D = kv->head_dim;
   const int64_t n_ctr = B * kv->hkv * ((H / kv->hkv + 7) / 8);
   // the last int of the counter block is the status word of the bounded waits, so one counter fewer is usable
-  const bool fused = n_ctr < (int64_t)(kAttnCounterBytes / sizeof(int));           // else: separate reduction launch
+  const bool room = n_ctr < (int64_t)(kAttnCounterBytes / sizeof(int));
+  const bool fused = room && last_cta_merges(S, H, kv->hkv);      // else: separate reduction launch
   int* status = counters + kAttnStatusIndex;
   int r;
   if (kv->format > TSB200_KV_NVFP4)    // unquantized pages: fp32 math (decode_attn_dense.cu)
-    return attn_dense(kv, q, out, dtype, qs, B, H, sm_scale, max_seq_len, ws, fused ? counters : nullptr, s);
+    return attn_dense(kv, q, out, dtype, qs, B, H, sm_scale, max_seq_len, ws, room ? counters : nullptr, s);
   if (kv->format == TSB200_KV_FP8 && D == 128 && H / kv->hkv <= 4) {
     // e4m3 pages go to the tensor cores as FP8 (decode_attn_fp8.cu)
-    int* ctr = fused ? counters : nullptr;
     const int S8 = choose_splits_fp8(B, kv->hkv, max_seq_len);   // never more than choose_splits(): the workspace fits
+    const bool fused8 = room && last_cta_merges(S8, H, kv->hkv);
+    int* ctr = fused8 ? counters : nullptr;
     if (dtype == TSB200_F32) r = launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, ctr, out, status, s);
     else r = launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, ctr, out, status, s);
-    if (r != TSB200_OK || fused) return r;
+    if (r != TSB200_OK || fused8) return r;
     return dtype == TSB200_F32 ? launch_reduce<float, 128>(ws, B * H, S8, out, s) : launch_reduce<__nv_bfloat16, 128>(ws, B * H, S8, out, s);
   }
 #define TSB_GO(TT, DD, FF)                                                                                              \

@@ -83,37 +83,63 @@ __global__ void decode_attn_simt_kernel(tsb200_kv_desc kv, const T* __restrict__
   }
 }
 
-// One warp per (b, h): combine S partials -> out.
+// One CTA per (b, h), one thread per dim: combine S partials -> out, in split order (the sums of merge_splits).  Bound by one round trip:
+// all of a thread's partials and the splits' (m, l) are in flight together, while the coefficients wait for the latter only.
 template <typename T, int D>
-__global__ void decode_attn_reduce_kernel(const float* __restrict__ ws, int64_t BH, int S, T* __restrict__ out) {
-  constexpr int EPL = D / 32;
+__global__ void __launch_bounds__(D)
+decode_attn_reduce_kernel(const float* __restrict__ ws, int S, T* __restrict__ out) {
+  constexpr int kMax = 64;                                // splits (<= D)
+  __shared__ float sm[kMax], sl[kMax], sc[kMax], s_sum;
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int64_t bh = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (bh >= BH) return;
-  const float* p = ws + bh * S * (2 + D);
-  float mm = -INFINITY;
-  for (int s = 0; s < S; ++s) mm = fmaxf(mm, p[s * (2 + D)]);
-  float ll = 0.f, a[EPL];
+  const int t = threadIdx.x;
+  const float* p = ws + (int64_t)blockIdx.x * S * (2 + D);
+  float v[kMax];
 #pragma unroll
-  for (int e = 0; e < EPL; ++e) a[e] = 0.f;
-  for (int s = 0; s < S; ++s) {
-    const float ms = p[s * (2 + D)];
-    const float c = ms == -INFINITY ? 0.f : __expf(ms - mm);
-    ll += p[s * (2 + D) + 1] * c;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) a[e] += p[s * (2 + D) + 2 + lane * EPL + e] * c;
+  for (int u = 0; u < kMax; ++u)
+    if (u < S) v[u] = __ldcg(p + (size_t)u * (2 + D) + 2 + t);
+  if (t < S) {
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(p + (size_t)t * (2 + D)));
+    sm[t] = ml.x;
+    sl[t] = ml.y;
   }
-  const float inv = ll > 0.f ? 1.0f / ll : 0.f;
+  __syncthreads();
+  if (t < kMax) {
+    const int lane = t & 31;
+    const float mm = warp_max(fmaxf(lane < S ? sm[lane] : -INFINITY, lane + 32 < S ? sm[lane + 32] : -INFINITY));
+    if (t < S) sc[t] = sm[t] == -INFINITY ? 0.f : __expf(sm[t] - mm);
+  }
+  __syncthreads();
+  if (t == 0) {
+    float ll = 0.f;
 #pragma unroll
-  for (int e = 0; e < EPL; ++e) out[bh * D + lane * EPL + e] = from_f32<T>(a[e] * inv);
+    for (int u = 0; u < kMax; ++u)
+      if (u < S) ll += sl[u] * sc[u];
+    s_sum = ll;
+  }
+  float a = 0.f;
+#pragma unroll
+  for (int u = 0; u < kMax; ++u)
+    if (u < S) a += v[u] * sc[u];
+  __syncthreads();
+  const float ll = s_sum;
+  out[(int64_t)blockIdx.x * D + t] = from_f32<T>(ll > 0.f ? a / ll : 0.f);
 }
 
+// Chained to the attention launch whether or not the caller's launches are: that one waits for what precedes it.
 template <typename T, int D>
 int launch_reduce(const float* ws, int64_t BH, int S, void* out, cudaStream_t st) {
-  const int64_t blocks = (BH + 3) / 4;
-  TSB_CUDA(launch_kernel(decode_attn_reduce_kernel<T, D>, dim3((unsigned)blocks), dim3(128), 0, st, ws, BH, S, (T*)out));
+  if (BH > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)BH);
+  cfg.blockDim = dim3(D);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, decode_attn_reduce_kernel<T, D>, ws, S, (T*)out));
   return TSB200_OK;
 }
 template int launch_reduce<float, 64>(const float*, int64_t, int, void*, cudaStream_t);
