@@ -363,6 +363,24 @@ def test_bulk_append_of_strided_prompts(cuda, fmt, name, H, Hkv, d, pad):
         assert torch.equal(q4[b, :new_lens[b]].cpu(), qr[b, :new_lens[b]])
 
 
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("B,Hkv,d", [(40, 3, 128), (20, 3, 64), (2, 3, 128)])
+@pytest.mark.parametrize("T", [1, 37, 300])
+def test_fp8_scales_of_head_groups(cuda, name, B, Hkv, d, T):
+    """Four, two and one heads per CTA (the last group short): amax / 448 of the rotated keys and of the values."""
+    from transformer_surgeon_b200 import ops
+    rng = np.random.default_rng(23)
+    o, g = make_pair("fp8", B, 1, Hkv, d, cuda, rng)
+    k, v = outlier_kv(rng, B, T, Hkv, d, DT[name])
+    cos, sin = oatt.rope_tables(d, 5e5, torch.arange(T + 8))
+    start = torch.arange(B, dtype=torch.int32) % 8
+    g.set_fp8_scales(k.to(cuda), v.to(cuda), rope=(cos.to(cuda), sin.to(cuda)), pos0=start.to(cuda))
+    pos = start.long()[:, None] + torch.arange(T)[None, :]
+    kr = torch.stack([oatt.apply_rope(k[b], cos[pos[b]], sin[pos[b]]) for b in range(B)])
+    assert np.array_equal(g.k_scale.cpu().numpy(), kc.fp8_scale_from_amax(kr.float().abs().amax(dim=(1, 3)).numpy()))
+    assert np.array_equal(g.v_scale.cpu().numpy(), kc.fp8_scale_from_amax(v.float().abs().amax(dim=(1, 3)).numpy()))
+
+
 def test_fp8_attention_after_append_under_dependent_launch(cuda):
     """One decode step's append -> attention pair with programmatic dependent launch on: the attention may fetch pages
     older than the newest token before the append has finished.  Lengths sit on, before and after page boundaries and

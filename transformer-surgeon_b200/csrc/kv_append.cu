@@ -561,34 +561,44 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
 }
 
 // FP8 scales of a prompt: amax over the T tokens of a (sequence, kv head) -> amax / 448 (1 if 0).  A cluster of eight CTAs shares the
-// tokens, D / 16 lanes a vector ((8 + 8) elements each, so the rotation needs no other lane), the maxima meet in distributed shared
-// memory.  Bound by the one trip of K and V from memory: 32 x 2048 tokens, 8 heads, d 128: 268 MB, 56 us (41 at the copy rate); the
-// version with one CTA per (sequence, head), a warp per vector and five shuffles per rotation took 343 us.
+// tokens of G heads, D / 16 lanes a vector ((8 + 8) elements each, so the rotation needs no other lane; its cos and sin, as many bytes
+// as K and V, are fetched and rounded once for the G heads), the maxima meet in distributed shared memory.  Bound by the one trip of
+// K and V from memory: 32 x 2048 tokens, 8 heads, d 128: 268 MB, 41 us at the copy rate; 50 us with four heads, 71 with one; one CTA per
+// (sequence, head), a warp per vector and five shuffles per rotation took 343 us.
 constexpr int kScaleRanks = 8;
-template <typename T, int D>
+template <typename T, int D, int G>
 __global__ void __launch_bounds__(256)
 kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t ks, int64_t vs, int64_t Tn, int hkv,
                      const int32_t* __restrict__ pos0, const float* __restrict__ rope_cos,
                      const float* __restrict__ rope_sin, int64_t rope_rows, float* __restrict__ k_scale,
                      float* __restrict__ v_scale) {
   constexpr int HALF = D / 2, EG = HALF / 8, PER = 256 / EG;              // vectors of a CTA side by side
-  __shared__ float sh[2][8], srank[2][kScaleRanks];
-  const int rank = blockIdx.x % kScaleRanks;
-  const int64_t pair = blockIdx.x / kScaleRanks, b = pair / hkv;
-  const int h = (int)(pair % hkv);
+  __shared__ float sh[2 * G][8], srank[2 * G][kScaleRanks];
+  const int rank = blockIdx.x % kScaleRanks, groups = (hkv + G - 1) / G;
+  const int64_t item = blockIdx.x / kScaleRanks, b = item / groups;
+  const int h0 = (int)(item % groups) * G;
   const int eg = threadIdx.x % EG, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t start = pos0 ? (int64_t)pos0[b] : 0;
   const bool kvec = (reinterpret_cast<uintptr_t>(k) & 15) == 0 && ks * sizeof(T) % 16 == 0;
   const bool vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0 && vs * sizeof(T) % 16 == 0;
   const bool rvec = ((reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin)) & 15) == 0;
-  float mk = 0.f, mv = 0.f;
-#pragma unroll 2
-  for (int64_t t = (int64_t)rank * PER + threadIdx.x / EG; t < Tn; t += kScaleRanks * PER) {
-    const T* kp = k + (b * Tn + t) * ks + h * D + eg * 8;
-    const T* vp = v + (b * Tn + t) * vs + h * D + eg * 8;
-    Raw8<T> x0, x1, y0, y1;
-    x0.load(kp, kvec); x1.load(kp + HALF, kvec);
-    y0.load(vp, vvec); y1.load(vp + HALF, vvec);
+  float mk[G], mv[G];
+#pragma unroll
+  for (int h = 0; h < G; ++h) mk[h] = mv[h] = 0.f;
+  const int64_t t_first = (int64_t)rank * PER + threadIdx.x / EG, t_step = kScaleRanks * PER;
+  const T* kp = k + (b * Tn + t_first) * ks + h0 * D + eg * 8;
+  const T* vp = v + (b * Tn + t_first) * vs + h0 * D + eg * 8;
+#pragma unroll (G == 1 ? 4 : (G == 2 ? 2 : 1))
+  for (int64_t t = t_first; t < Tn; t += t_step, kp += t_step * ks, vp += t_step * vs) {
+    Raw8<T> x[G][2], y[G][2];
+#pragma unroll
+    for (int h = 0; h < G; ++h)
+      if (G == 1 || h0 + h < hkv) {
+        x[h][0].load(kp + h * D, kvec); x[h][1].load(kp + h * D + HALF, kvec);
+        y[h][0].load(vp + h * D, vvec); y[h][1].load(vp + h * D + HALF, vvec);
+      } else {
+        x[h][0] = x[h][1] = y[h][0] = y[h][1] = Raw8<T>{};
+      }
     if (rope_cos) {
       int64_t p = start + t;
       p = p >= rope_rows ? rope_rows - 1 : p;
@@ -607,16 +617,22 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
         cc = *reinterpret_cast<Raw8<T>*>(&c);
         ss = *reinterpret_cast<Raw8<T>*>(&s);
       }
-      rope8(x0, x1, cc, ss);
+#pragma unroll
+      for (int h = 0; h < G; ++h) rope8(x[h][0], x[h][1], cc, ss);
     }
-    mk = x1.amax(x0.amax(mk));
-    mv = y1.amax(y0.amax(mv));
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      mk[h] = x[h][1].amax(x[h][0].amax(mk[h]));
+      mv[h] = y[h][1].amax(y[h][0].amax(mv[h]));
+    }
   }
-  mk = warp_max(mk);
-  mv = warp_max(mv);
-  if (lane == 0) { sh[0][w] = mk; sh[1][w] = mv; }
+#pragma unroll
+  for (int h = 0; h < G; ++h) {
+    const float a = warp_max(mk[h]), c = warp_max(mv[h]);
+    if (lane == 0) { sh[2 * h][w] = a; sh[2 * h + 1][w] = c; }
+  }
   __syncthreads();
-  if (threadIdx.x < 2) {
+  if (threadIdx.x < 2 * G) {
     float m = sh[threadIdx.x][0];
 #pragma unroll
     for (int i = 1; i < 8; ++i) m = fmaxf(m, sh[threadIdx.x][i]);
@@ -625,11 +641,11 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(dst), "f"(m) : "memory");
   }
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-  if (rank == 0 && threadIdx.x < 2) {
+  if (rank == 0 && threadIdx.x < 2 * G && h0 + (int)threadIdx.x / 2 < hkv) {
     float m = srank[threadIdx.x][0];
 #pragma unroll
     for (int i = 1; i < kScaleRanks; ++i) m = fmaxf(m, srank[threadIdx.x][i]);
-    (threadIdx.x ? v_scale : k_scale)[pair] = m > 0.f ? __fdiv_rn(m, 448.0f) : 1.0f;
+    ((threadIdx.x & 1) ? v_scale : k_scale)[b * hkv + h0 + threadIdx.x / 2] = m > 0.f ? __fdiv_rn(m, 448.0f) : 1.0f;
   }
 }
 
@@ -724,8 +740,11 @@ int tsb200_kv_fp8_scales_strided(const void* k, const void* v, int dtype, int64_
   if (ks < dense || vs < dense) return TSB200_ERR_ARG;
   if (B * hkv * kScaleRanks > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   cudaStream_t s = as_stream(stream);
+  // heads per CTA: as many as leave every SM two CTAs
+  int g = 4;
+  while (g > 1 && B * ((hkv + g - 1) / g) * kScaleRanks < 296) g /= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(B * hkv * kScaleRanks));
+  cfg.gridDim = dim3((unsigned)(B * ((hkv + g - 1) / g) * kScaleRanks));
   cfg.blockDim = dim3(256);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -735,9 +754,11 @@ int tsb200_kv_fp8_scales_strided(const void* k, const void* v, int dtype, int64_
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-#define TSB_SC(TT, DD) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD>, (const TT*)k, (const TT*)v, ks, vs, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
+#define TSB_SG(TT, DD, GG) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD, GG>, (const TT*)k, (const TT*)v, ks, vs, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
+#define TSB_SC(TT, DD) do { if (g == 4) TSB_SG(TT, DD, 4); else if (g == 2) TSB_SG(TT, DD, 2); else TSB_SG(TT, DD, 1); } while (0)
   if (dtype == TSB200_F32) { if (head_dim == 64) TSB_SC(float, 64); else TSB_SC(float, 128); }
   else { if (head_dim == 64) TSB_SC(__nv_bfloat16, 64); else TSB_SC(__nv_bfloat16, 128); }
+#undef TSB_SG
 #undef TSB_SC
   return TSB200_OK;
 }
