@@ -181,6 +181,37 @@ def test_decode_attention_against_oracle(cuda, fmt, name, H, Hkv, d, simt):
     assert np.all(np.abs(out - ref) <= tol), (np.abs(out - ref) / tol).max()
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("H,Hkv,d,cap,qpad", [(7, 1, 128, 576, 0), (7, 1, 128, 640, 3), (14, 2, 64, 3968, 8), (4, 1, 128, 4400, 0), (9, 1, 128, 520, 0)])
+def test_decode_attention_split_merges(cuda, fmt, name, H, Hkv, d, cap, qpad):
+    """Splits merged by the last CTA (63 rows) and by the chained reduction (70 rows, 62 splits, short and empty sequences, two head
+    chunks); queries off a 16-byte boundary and strided."""
+    from transformer_surgeon_b200 import ops
+    rng = np.random.default_rng(29)
+    B = 3
+    lens = np.array([cap, 17, 0], dtype=np.int32)
+    o, g = make_pair(fmt, B, (cap + 15) // 16, Hkv, d, cuda, rng)
+    k, v = outlier_kv(rng, B, cap, Hkv, d, DT[name])
+    sync_scales(o, g, k, v)
+    nl = torch.from_numpy(lens).to(cuda)
+    g.append(k.to(cuda), v.to(cuda), new_lens=nl)
+    g.seq_lens.copy_(nl)
+    kc.append_vectorized(o, k.float().numpy(), v.float().numpy())      # tokens beyond a length are never read
+    o.seq_lens[:] = lens
+    q = torch.from_numpy(rng.standard_normal((B, H, d)).astype(np.float32)).to(DT[name])
+    buf = torch.zeros((B, H * d + qpad), dtype=DT[name], device=cuda)
+    qv = buf[:, qpad:].unflatten(1, (H, d))
+    qv.copy_(q)
+    ref, ref_abs = oatt.paged_decode_attention(o, q.float().numpy(), with_abs=True)
+    out = ops.paged_decode_attention(g, qv, max_seq_len=cap)
+    assert torch.equal(out, ops.paged_decode_attention(g, qv, max_seq_len=cap))
+    out = out.float().cpu().numpy()
+    assert np.all(out[2] == 0)
+    tol = attn_tol(ref, ref_abs, name, False)
+    assert np.all(np.abs(out - ref) <= tol), (np.abs(out - ref) / tol).max()
+
+
 @pytest.mark.parametrize("fmt", ["fp32", "bf16"])
 @pytest.mark.parametrize("H,Hkv,d", [(14, 2, 64), (9, 1, 128), (4, 4, 128)])
 @pytest.mark.parametrize("lens", [(1, 16, 17), (0, 129, 150), (700, 2049, 33)])
