@@ -231,11 +231,11 @@ def test_gated_mlp_block(cuda, name, p, M, K, I, r, N):
 
 
 @pytest.mark.parametrize("p", [8, 4, 2, "binary"])
-@pytest.mark.parametrize("M,K,I,r", [(129, 512, 14336, 256), (257, 256, 14344, 0), (300, 512, 7304, 136), (2048, 512, 2048, 128), (2500, 1024, 4104, 0), (200, 512, 640, 64)])
+@pytest.mark.parametrize("M,K,I,r", [(129, 512, 14336, 256), (257, 256, 14344, 0), (300, 512, 7304, 136), (2048, 512, 2048, 128), (2500, 1024, 4104, 0), (200, 512, 640, 64), (350, 4096, 7296, 576)])
 def test_gated_mlp_prompt(cuda, p, M, K, I, r):
     """More than 128 tokens: gate's tiles read by up's outputs (one to several items per CTA, ragged tokens and rows, K splits in the
-    V phase, items shorter than the ring of stages), or the composed path where up's tiles split K; same as composing the pieces up
-    to the rounding of SiLU."""
+    V phase, items shorter than the ring of stages), or the composed path where up's tiles split K; the same bits as composing the
+    pieces."""
     from transformer_surgeon_b200 import ops
     g = torch.Generator(device=cuda).manual_seed(11)
     x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
@@ -251,7 +251,7 @@ def test_gated_mlp_prompt(cuda, p, M, K, I, r):
     y, y2 = mlp(x), mlp(x)
     assert torch.equal(y, y2)
     a = ops.swiglu(gate(x), up(x))
-    assert rel_err(y, down(a)) < 4e-3
+    assert torch.equal(y, down(a))
     assert ops.PackedLinear.device_status(ws=ops.workspace(cuda, 1, "mlp")) == 0
 
 

@@ -329,14 +329,21 @@ __device__ __forceinline__ bool grid_wait(const int* ctr, int target, volatile i
   return false;
 }
 
-// SiLU(gate) * up of eight outputs: the rounding points of separate gate / up / SiLU * up kernels (blocks/mlp.py:181-183).
+// SiLU(gate) * up of eight outputs, bit for bit that of separate gate / up / SiLU * up kernels (blocks/mlp.py:181-183): SiLU is rounded
+// to bf16, and over all bf16 gates the fast exponential and division round to what expf and an IEEE division round to, but for
+// -88.5 .. -87.5, whose denominators are beyond the fast division's range.
 __device__ __forceinline__ uint4 gate_eight(uint4 gv, uint4 uv) {
   const unsigned g[4] = {gv.x, gv.y, gv.z, gv.w}, u[4] = {uv.x, uv.y, uv.z, uv.w};
   unsigned o[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float g0 = __uint_as_float(g[i] << 16), g1 = __uint_as_float(g[i] & 0xffff0000u);
-    const __nv_bfloat162 a = __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)), __fdividef(g1, 1.0f + __expf(-g1)));
+    float s0 = __fdividef(g0, 1.0f + __expf(-g0)), s1 = __fdividef(g1, 1.0f + __expf(-g1));
+    if (fminf(g0, g1) < -87.0f) {
+      s0 = g0 / (1.0f + expf(-g0));
+      s1 = g1 / (1.0f + expf(-g1));
+    }
+    const __nv_bfloat162 a = __floats2bfloat162_rn(s0, s1);
     const __nv_bfloat162 r = __hmul2_rn(a, *reinterpret_cast<const __nv_bfloat162*>(&u[i]));
     o[i] = *reinterpret_cast<const unsigned*>(&r);
   }

@@ -73,7 +73,10 @@ bool f32_chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, con
 static size_t region0_bytes(const tsb200_linear_desc* gate, const tsb200_linear_desc* up, const tsb200_linear_desc* down,
                             int64_t M) {
   size_t scratch = 0;
-  if (gate->rank > 0) scratch += phase_scratch_bytes(M, gate->rank, gate->in_features, 2, false);
+  if (gate->rank > 0) {                        // V factors as one phase, or as two
+    const size_t one = phase_scratch_bytes(M, gate->rank, gate->in_features, 2, false), two = 2 * phase_scratch_bytes(M, gate->rank, gate->in_features, 1, false);
+    scratch += one > two ? one : two;
+  }
   if (down->rank > 0) {
     scratch += phase_scratch_bytes(M, down->rank, down->in_features, 1, false);
     scratch += phase_scratch_bytes(M, down->out_features, down->rank, 1, false);
@@ -232,15 +235,23 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
       validate_linear(up, x, buf_a, M, noop_u) == TSB200_OK && !noop_g && !noop_u) {
     // Prompts: [gate V | up V] -> gate U -> up U with SiLU(gate) * up as its outputs leave -> down.  The separate SwiGLU pass over
     // [M, intermediate] (read twice, written once) and up's own round trip go away: 16384 tokens, 14336 features, 325 us of a
-    // 1.97 ms block; the two V factors in one phase end in a fuller last wave (1024 tiles on 148 SMs, not twice 512).
-    PhaseSpec ps[3];
+    // 1.97 ms block; the two V factors in one phase end in a fuller last wave (1024 tiles on 148 SMs, not twice 512).  Where a V
+    // factor splits its K range the two stay apart: side by side they would split it differently and sum in another order than the
+    // layers do by themselves.
+    PhaseSpec ps[4];
     int n = 0;
     const bool low = gate->rank > 0;
     const int64_t kgu = low ? gate->rank : gate->in_features;
     if (low) {
-      ps[n].nsub = 2; ps[n].gated = 0;
-      ps[n].g[0] = GemmSpec{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features};
-      ps[n++].g[1] = GemmSpec{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features};
+      const bool together = tc::plan_gemm(M, gate->rank, gate->in_features, 1, false, gate->u_bits == 1 ? 2 : 1).splits == 1;
+      const GemmSpec gv{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features}, uv{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features};
+      ps[n].nsub = together ? 2 : 1; ps[n].gated = 0;
+      ps[n].g[0] = gv;
+      ps[n++].g[1] = uv;
+      if (!together) {
+        ps[n].nsub = 1; ps[n].gated = 0;
+        ps[n++].g[0] = uv;
+      }
     }
     ps[n].nsub = 1; ps[n].gated = 0;
     ps[n++].g[0] = GemmSpec{gate->u, gate->u_scale, gate->bias, low ? h0 : x, buf_g, gate->out_features, kgu};
