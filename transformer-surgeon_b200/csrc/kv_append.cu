@@ -574,6 +574,8 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
                      float* __restrict__ v_scale) {
   constexpr int HALF = D / 2, EG = HALF / 8, PER = 256 / EG;              // vectors of a CTA side by side
   __shared__ float sh[2 * G][8], srank[2 * G][kScaleRanks];
+  // "has started": a rank's shared memory may be written by another only once its CTA runs; awaited before the remote store below
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
   const int rank = blockIdx.x % kScaleRanks, groups = (hkv + G - 1) / G;
   const int64_t item = blockIdx.x / kScaleRanks, b = item / groups;
   const int h0 = (int)(item % groups) * G;
@@ -632,6 +634,7 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
     if (lane == 0) { sh[2 * h][w] = a; sh[2 * h + 1][w] = c; }
   }
   __syncthreads();
+  asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
   if (threadIdx.x < 2 * G) {
     float m = sh[threadIdx.x][0];
 #pragma unroll
@@ -640,6 +643,7 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"((unsigned)__cvta_generic_to_shared(&srank[threadIdx.x][rank])));
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(dst), "f"(m) : "memory");
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   if (rank == 0 && threadIdx.x < 2 * G && h0 + (int)threadIdx.x / 2 < hkv) {
     float m = srank[threadIdx.x][0];

@@ -238,6 +238,8 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, unsigned col) 
 template <typename T>
 __global__ void __launch_bounds__(kArgThreads) argmax_rows_kernel(const T* __restrict__ y, int64_t N, int64_t* __restrict__ out) {
   __shared__ unsigned long long sw[kArgThreads / 32], srank[kArgRanks];
+  // "has started": a rank's shared memory may be written by another only once its CTA runs; awaited before the remote store below
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
   pdl_launch_dependents();
   pdl_wait();
   constexpr int E = 16 / sizeof(T);
@@ -265,12 +267,14 @@ __global__ void __launch_bounds__(kArgThreads) argmax_rows_kernel(const T* __res
   for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
   if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = best;
   __syncthreads();
+  asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
   if (threadIdx.x == 0) {
     for (int i = 1; i < kArgThreads / 32; ++i) best = max(best, sw[i]);
     unsigned dst;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(dst) : "r"(smem_u32(&srank[rank])));
     asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(dst), "l"(best) : "memory");
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   if (rank == 0 && threadIdx.x == 0) {
     best = srank[0];
