@@ -307,6 +307,27 @@ def test_few_tokens_at_model_widths(cuda, p, M, K, N, r):
     assert ops.PackedLinear.device_status(device=cuda) == 0
 
 
+@pytest.mark.parametrize("M,K,N,r,shift", [(16, 7232, 14336, 0, 0), (8, 14144, 14336, 0, 0), (16, 1024, 14336, 7232, 0), (16, 7232, 14336, 192, 0),
+                                           (1, 192, 72, 0, 1), (16, 320, 64, 192, 3), (17, 192, 72, 0, 1)])
+def test_binary_rows_of_an_odd_number_of_blocks(cuda, M, K, N, r, shift):
+    """1-bit rows that the copy engine does not take (an odd number of 64-column blocks): where the decode-sized kernel has no plan (its
+    activations do not fit an SM) or x lies at any alignment (`shift` elements into a buffer), the call runs all the same."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(33)
+    rnd = lambda a, b, s: (torch.randn((a, b), generator=g, device=cuda) * s).bfloat16()
+    signs = lambda a, b: rnd(a, b, 0.05).abs().clamp_min(1e-4) * (torch.randint(0, 2, (a, b), generator=g, device=cuda) * 2 - 1).bfloat16()   # no zeros
+    fu = ops.Factor.quantize(signs(N, r or K), "binary")
+    fv = ops.Factor.quantize(signs(r, K), "binary") if r else None
+    assert fu.bits == 1
+    bias = rnd(1, N, 0.1)[0].contiguous()
+    buf = torch.empty(M * K + shift, dtype=torch.bfloat16, device=cuda)
+    x = buf[shift:].view(M, K).copy_(rnd(M, K, 1.0))
+    h = (x.float() @ fv.reconstruct(torch.bfloat16).float().T).bfloat16().float() if r else x.float()
+    ref = h @ fu.reconstruct(torch.bfloat16).float().T + bias.float()
+    y = ops.PackedLinear(fu, fv, bias, torch.bfloat16)(x)
+    assert rel_err(y, ref) < 1e-2
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 512, 1000), (32, 1024, 50257), (100, 256, 4099)])
 def test_greedy_head_equals_argmax_of_logits(cuda, M, K, N):
     """tsb200_linear_argmax on a dense bf16 head (reduction in the GEMM epilogue, logits never stored) picks the token

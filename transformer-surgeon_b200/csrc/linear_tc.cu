@@ -368,10 +368,12 @@ int gemm_tc(const void* W, int bits, const float* scale, const void* bias, const
   return TSB200_OK;
 }
 
-// 1-bit rows are 8 bytes per 64 columns: the copy engine wants a 16-byte row pitch
+// 1-bit rows are 8 bytes per 64 columns, and the copy engine wants a 16-byte row pitch: with an odd number of 64-column blocks only
+// the decode-sized kernel takes them, where it has a plan.
+bool odd_binary(int bits, int64_t K) { return bits == 1 && K % 128 != 0; }
 bool tc_supported_factor(int bits, int64_t K, int64_t M) {
-  if (bits == 1) return K % 128 == 0 || (M <= kGvTokens && K % 8 == 0);
-  return (bits == 2 || bits == 4 || bits == 8 || bits == 16) && (K % 8) == 0;
+  if (odd_binary(bits, K)) return M <= kGvTokens && K % 8 == 0;
+  return bits == 1 || ((bits == 2 || bits == 4 || bits == 8 || bits == 16) && (K % 8) == 0);
 }
 
 }  // namespace
@@ -413,6 +415,9 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
   const int64_t ku = d->rank > 0 ? d->rank : d->in_features;
   if (!tc_supported_factor(d->u_bits, ku, M)) return TSB200_ERR_UNSUPPORTED;
   if (d->rank > 0 && !tc_supported_factor(d->v_bits, d->in_features, M)) return TSB200_ERR_UNSUPPORTED;
+  // what the CUDA-core kernel takes instead, it takes at any alignment and, at full rank, without a workspace
+  const bool odd = odd_binary(d->u_bits, ku) || (d->rank > 0 && odd_binary(d->v_bits, d->in_features));
+  if (odd && (!aligned(x, 16) || !workspace || !aligned(workspace, 256) || workspace_bytes < tsb200_linear_workspace_bytes(d, M))) return TSB200_ERR_UNSUPPORTED;
   if (!aligned(x, 16) || !aligned(y, 2)) return TSB200_ERR_ARG;
   if (!workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
   if (workspace_bytes < tsb200_linear_workspace_bytes(d, M)) return TSB200_ERR_WORKSPACE;
@@ -435,7 +440,7 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
                   int64_t N) {
     if (bits == 16) return gemm_tc(W, bits, scale, bias, in, out, M, K, N, partial, status, s);
     const int st = small(W, bits, scale, bias, in, out, K, N, g_pdl != 0, nullptr);
-    if (st != TSB200_ERR_UNSUPPORTED) return st;
+    if (st != TSB200_ERR_UNSUPPORTED || odd_binary(bits, K)) return st;
     return gemm_tcq(W, bits, scale, bias, in, out, M, K, N, partial, counters, status, s);
   };
   if (d->rank > 0 && d->u_bits <= 8 && d->v_bits <= 8 && M <= kGvTokens && gv_supported(d->u_bits, M, d->out_features, ku)) {
@@ -444,7 +449,7 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
     if (st == TSB200_OK) st = small(d->u, d->u_bits, d->u_scale, d->bias, h, y, ku, d->out_features, true, nullptr);
     if (st != TSB200_ERR_UNSUPPORTED) return st;
   }
-  if (d->rank > 0 && d->u_bits == d->v_bits && d->u_bits <= 8) {
+  if (d->rank > 0 && d->u_bits == d->v_bits && d->u_bits <= 8 && !odd) {
     // both factors packed alike: V then U as two phases of ONE launch (grid barrier in between);
     // the rank-r intermediate is produced and consumed through L2
     PhaseSpec ps[2];
