@@ -412,6 +412,43 @@ def test_fp8_scales_of_head_groups(cuda, name, B, Hkv, d, T):
     assert np.array_equal(g.v_scale.cpu().numpy(), kc.fp8_scale_from_amax(v.float().abs().amax(dim=(1, 3)).numpy()))
 
 
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("d", [64, 128])
+def test_append_of_infinities_and_of_quotients_beyond_the_type(cuda, fmt, name, d):
+    """Infinities, NaN, the largest finite values and tiny ones, over FP8 scales fixed beforehand (quotients that overflow fp32): a token's
+    codes do not depend on whether it came in a chunk or by itself, and FP8 codes saturate."""
+    from transformer_surgeon_b200 import ops
+    rng = np.random.default_rng(37)
+    B, T, Hkv = 2, 35, 2
+    _, bulk = make_pair(fmt, B, 3, Hkv, d, cuda, rng)
+    single = ops.PagedKV(fmt, bulk.k_pool.shape[0], Hkv, d, bulk.block_table, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+    k, v = (x.float() for x in outlier_kv(rng, B, T, Hkv, d, DT[name]))
+    big, inf = torch.finfo(DT[name]).max, float("inf")
+    for x in (k, v):
+        for i, val in enumerate((inf, -inf, big, -big, float("nan"), 1e-30, -1e-30)):
+            x[:, 3 * i + 1, :, 5 * i + 2] = val
+            x[:, 22 + i, :, (17 * i + 3) % d] = val
+    k, v = k.to(DT[name]).to(cuda), v.to(DT[name]).to(cuda)
+    for scales in (((1e-6, 0.25), (3e-18, 1e17), (0.0, inf), (-0.5, float("nan")), (1e-30, 1e30)) if fmt == "fp8" else ((1.0, 1.0),)):
+        if fmt == "fp8":
+            bulk.fill_fp8_scales(*scales)
+            single.fill_fp8_scales(*scales)
+        bulk.append(k, v)
+        single.seq_lens.zero_()
+        for t in range(T):
+            single.append(k[:, t:t + 1].contiguous(), v[:, t:t + 1].contiguous())
+            single.seq_lens += 1
+        assert torch.equal(bulk.k_pool, single.k_pool)
+        assert torch.equal(bulk.v_pool, single.v_pool)
+    if fmt == "fp8":
+        bulk.fill_fp8_scales(1e-6, 0.25)
+        bulk.append(k, v)
+        rec = bulk.k_pool[bulk.block_table[0, 0].long(), 0].cpu()          # head 0 of the first page: codes [16][d]
+        codes = rec[:16 * d].view(16, d)
+        assert [int(codes[3 * i + 1, 5 * i + 2]) for i in range(4)] == [0x7e, 0xfe, 0x7e, 0xfe]
+
+
 def test_fp8_attention_after_append_under_dependent_launch(cuda):
     """One decode step's append -> attention pair with programmatic dependent launch on: the attention may fetch pages
     older than the newest token before the append has finished.  Lengths sit on, before and after page boundaries and

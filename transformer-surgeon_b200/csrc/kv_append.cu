@@ -294,17 +294,28 @@ __device__ __forceinline__ void rope8(Raw8<float>& a, Raw8<float>& b, const Raw8
   }
 }
 
-// x / d for a divisor that many elements share: correctly rounded from the correctly rounded reciprocal (Markstein's theorem,
+// Quotients by a divisor that many elements share: correctly rounded from the correctly rounded reciprocal (Markstein's theorem,
 // Computation of elementary functions on the IBM RISC System/6000 processor, 1990: q' = q + (x - d q) y is the rounded quotient when
-// q is within an ulp of it, which one correction of x y is).  Divisors near the ends of the exponent range divide.
+// q is within an ulp of it, which one correction of x y is), two at a time.  Divisors near the ends of the exponent range divide.  An
+// infinite product (of an infinite x, or a quotient beyond the type) stands as it is where MAY_OVERFLOW: it saturates, and its
+// corrections are NaN.
 struct Divisor {
   float d, y;
   bool slow;
-  template <bool SLOW> __device__ __forceinline__ float of(float x) const {
-    if (SLOW) return __fdiv_rn(x, d);
-    float q = x * y;
-    q = fmaf(fmaf(-q, d, x), y, q);
-    return fmaf(fmaf(-q, d, x), y, q);
+  template <bool MAY_OVERFLOW> __device__ __forceinline__ void of(float x0, float x1, float& q0, float& q1) const {
+    float p0, p1;
+    asm("{\n.reg .b64 x, y, n, p, q, e;\n"
+        "mov.b64 x, {%4, %5};\nmov.b64 y, {%6, %6};\nmov.b64 n, {%7, %7};\n"
+        "mul.rn.f32x2 p, x, y;\n"
+        "fma.rn.f32x2 e, p, n, x;\nfma.rn.f32x2 q, e, y, p;\n"
+        "fma.rn.f32x2 e, q, n, x;\nfma.rn.f32x2 q, e, y, q;\n"
+        "mov.b64 {%0, %1}, q;\nmov.b64 {%2, %3}, p;\n}\n"
+        : "=f"(q0), "=f"(q1), "=f"(p0), "=f"(p1)
+        : "f"(x0), "f"(x1), "f"(y), "f"(-d));
+    if (MAY_OVERFLOW) {
+      q0 = fabsf(p0) <= 3.4028235e38f ? q0 : p0;
+      q1 = fabsf(p1) <= 3.4028235e38f ? q1 : p1;
+    }
   }
 };
 __device__ __forceinline__ Divisor divisor(float v) { return Divisor{v, __frcp_rn(v), !(v >= 1e-18f && v <= 1e18f)}; }
@@ -313,7 +324,11 @@ __device__ __forceinline__ Divisor divisor(float v) { return Divisor{v, __frcp_r
 template <int FMT, bool SLOW> __device__ __forceinline__ void encode8_by(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
   float q[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] = d.of<SLOW>(x[i]);
+  for (int i = 0; i < 8; i += 2) {
+    // FP8: a scale from elsewhere; the other formats' divisors come from the elements' own maximum
+    if (SLOW) { q[i] = __fdiv_rn(x[i], d.d); q[i + 1] = __fdiv_rn(x[i + 1], d.d); }
+    else d.of<FMT == TSB200_KV_FP8>(x[i], x[i + 1], q[i], q[i + 1]);
+  }
   if (FMT == TSB200_KV_FP8) {
     unsigned h[4];
 #pragma unroll
@@ -442,7 +457,8 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
           float m = a[g].amax(0.f);
           m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));              // a block of 16 is two lanes' eights
           sb[g] = (unsigned)__nv_cvt_float_to_fp8(__fdiv_rn(m, 6.0f), __NV_SATFINITE, __NV_E4M3);
-          const Divisor d = divisor(e4m3_to_f32((unsigned char)sb[g]));
+          Divisor d = divisor(e4m3_to_f32((unsigned char)sb[g]));
+          d.slow = m > 3.4028235e38f;                                    // the scale is one of e4m3's, or 0 and not divided by
           encode8<FMT>(f[g], d, c[2 * g], c[2 * g + 1]);
         }
       }
