@@ -412,15 +412,51 @@ def test_fp8_scales_of_head_groups(cuda, name, B, Hkv, d, T):
     assert np.array_equal(g.v_scale.cpu().numpy(), kc.fp8_scale_from_amax(v.float().abs().amax(dim=(1, 3)).numpy()))
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("H,Hkv,d", [(14, 2, 64), (9, 9, 128), (0, 1, 128)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_large_chunks_equal_small_ones(cuda, fmt, name, H, Hkv, d, pad):
+    """Four ragged sequences appended by themselves (small chunks: a warp per vector) and repeated until the chunk goes by page, its heads
+    over one or several CTAs per page: the same records and rotated queries."""
+    from transformer_surgeon_b200 import ops
+    T, copies = 53, 12 if Hkv * d < 1000 else 2
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    cos, sin = (x.to(cuda) for x in oatt.rope_tables(d, 5e5, torch.arange(96)))
+    small = (torch.randn((4, T, (H + 2 * Hkv) * d + 2 * pad), generator=gen, device=cuda) * 3).to(DT[name])
+    start = torch.tensor([0, 5, 16, 27], dtype=torch.int32, device=cuda)
+    new_lens = torch.tensor([53, 32, 16, 0], dtype=torch.int32, device=cuda)
+    runs = []
+    for n in (1, copies, 8 * copies):
+        B = 4 * n
+        assert n == 1 or B * T * Hkv * d >= 1 << 18 or Hkv == 1
+        buf = small.repeat(n, 1, 1)
+        table = torch.arange(B * 5, dtype=torch.int32, device=cuda).reshape(B, 5)
+        kv = ops.PagedKV(fmt, B * 5, Hkv, d, table, start.repeat(n), cuda)
+        if fmt == "fp8":
+            kv.fill_fp8_scales(torch.full((1,), 0.03, device=cuda), torch.full((1,), 0.02, device=cuda))
+        q4 = buf[..., :H * d].unflatten(2, (H, d)) if H else None
+        k4 = buf[..., H * d + pad:(H + Hkv) * d + pad].unflatten(2, (Hkv, d))
+        v4 = buf[..., (H + Hkv) * d + pad:(H + 2 * Hkv) * d + pad].unflatten(2, (Hkv, d))
+        if H:
+            kv.rope_append(q4, k4, v4, (cos, sin), new_lens=new_lens.repeat(n))
+        else:
+            kv.append(k4, v4, new_lens=new_lens.repeat(n))
+        runs.append((kv.k_pool.view(n, -1), kv.v_pool.view(n, -1), buf.view(n, -1)))
+    for big in runs[1:]:
+        for a, b in zip(big, runs[0]):
+            assert torch.equal(a, b.expand_as(a))
+
+
 @pytest.mark.parametrize("name", ["fp32", "bf16"])
 @pytest.mark.parametrize("fmt", FMTS)
 @pytest.mark.parametrize("d", [64, 128])
 def test_append_of_infinities_and_of_quotients_beyond_the_type(cuda, fmt, name, d):
     """Infinities, NaN, the largest finite values and tiny ones, over FP8 scales fixed beforehand (quotients that overflow fp32): a token's
-    codes do not depend on whether it came in a chunk or by itself, and FP8 codes saturate."""
+    codes do not depend on whether it came in a chunk (large enough for the kernel by page) or by itself, and FP8 codes saturate."""
     from transformer_surgeon_b200 import ops
     rng = np.random.default_rng(37)
-    B, T, Hkv = 2, 35, 2
+    B, T, Hkv = 4096 // d, 35, 2
     _, bulk = make_pair(fmt, B, 3, Hkv, d, cuda, rng)
     single = ops.PagedKV(fmt, bulk.k_pool.shape[0], Hkv, d, bulk.block_table, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
     k, v = (x.float() for x in outlier_kv(rng, B, T, Hkv, d, DT[name]))

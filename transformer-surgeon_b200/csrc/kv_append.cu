@@ -1,8 +1,8 @@
 // Fused (RoPE on K +) quantize-and-append into the paged KV pools, and the FP8 scale
 // reduction over a prompt.  One warp owns one (token, kv head) vector of d elements:
 // lane l holds elements [l*d/32, (l+1)*d/32).  HBM-bound: reads 2*d*sizeof(act) bytes
-// and writes 2*d*b_elem (+ scales) per vector.  Decode steps (one token per sequence) use
-// kv_append_kernel; prompt chunks of 16 tokens or more use kv_append_pages_kernel, in which
+// and writes 2*d*b_elem (+ scales) per vector.  Decode steps (one token per sequence) and small
+// chunks use kv_append_kernel; larger prompt chunks use kv_append_pages_kernel, in which
 // a CTA owns a whole page and writes the token-minor V record with 16-byte vectors.
 //
 // Quantization arithmetic (IEEE fp32, round-to-nearest-even) per format:
@@ -361,7 +361,7 @@ __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&o
   out[2] = __byte_perm(c, d, 0x5410); out[3] = __byte_perm(c, d, 0x7632);
 }
 
-// Bulk append (T >= 16 tokens per sequence, quantized formats): a CTA owns the pages of 2048 / d consecutive slots of one sequence
+// Bulk append (quantized formats; launch_append says from which size on): a CTA owns the pages of 2048 / d consecutive slots of one sequence
 // (d 128: one page, d 64: two), its 8 warps take the heads.  A lane holds four tokens x (8 + 8) elements, e and e + d/2, so that
 //   * the rotation needs no other lane; cos and sin of the CTA's positions are rounded to the act dtype once, in shared memory, and
 //     serve every key and query head;
@@ -370,8 +370,9 @@ __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&o
 //   * V, stored token-minor, is transposed four bytes at a time in registers and leaves through a swizzled tile of shared memory as
 //     16-byte rows, 512 contiguous bytes per warp.
 // Pages that the range covers in part keep their other slots: those go out token by token.  A task is K or V of one head: both at once
-// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions bound it (about 2.5 an element): 32 x 2048
-// tokens, 8 heads, d 128, FP8, 402 MB: 97 us, 242 us with one warp per token vector and a byte-wise transpose.
+// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions bound it, about 26 an element (an instruction
+// more per element is 3.7 us): 32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB: 94 us, 242 us with one warp per token vector and a
+// byte-wise transpose.
 template <typename T, int D, int FMT>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 1)
 kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,
@@ -395,6 +396,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   const int64_t p0 = lp0 * 16;
   if (p0 >= start + n_b) return;
   if (rope_cos) {
+#pragma unroll
     for (int i = threadIdx.x; i < TOK * HALF; i += 256) {
       int64_t p = p0 + i / HALF;
       p = p < 0 ? 0 : (p >= rope_rows ? rope_rows - 1 : p);
@@ -417,7 +419,10 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   const bool vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0 && vs_ * sizeof(T) % 16 == 0;
   const int lt = page_of_lane * 16 + slot0;                               // the lane's first token in the tables
 
-  for (int task = w; task < 2 * kv.hkv; task += 8) {                      // head, K or V: half the registers of both at once
+  // tasks: K or V of a head (half the registers of both at once), then query heads; dealt out over the grid's CTAs of these pages
+  const int tasks = 2 * kv.hkv + (q && rope_cos ? qheads : 0), task_step = 8 * (int)gridDim.z;
+  int task = w + 8 * (int)blockIdx.z;
+  for (; task < 2 * kv.hkv; task += task_step) {
     const int h = task >> 1;
     const bool is_v = task & 1;
     uint8_t* rec = (is_v ? kv.v_pool : kv.k_pool) + ((page_ok ? page : 0) * kv.hkv + h) * rec_bytes;
@@ -447,7 +452,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
         float m = a[1].amax(a[0].amax(0.f));
 #pragma unroll
         for (int o = 1; o < EG; o *= 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        s8 = __fdiv_rn(m, 127.0f);
+        s8 = m > 0.f ? __fdiv_rn(m, 127.0f) : 0.f;         // 0 (slots outside the chunk) takes the division's slow path
         const Divisor d = divisor(__fadd_rn(s8, 1e-6f));
         encode8<FMT>(f[0], d, c[0], c[1]);
         encode8<FMT>(f[1], d, c[2], c[3]);
@@ -456,7 +461,8 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
         for (int g = 0; g < 2; ++g) {
           float m = a[g].amax(0.f);
           m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));              // a block of 16 is two lanes' eights
-          sb[g] = (unsigned)__nv_cvt_float_to_fp8(__fdiv_rn(m, 6.0f), __NV_SATFINITE, __NV_E4M3);
+          // 0 (slots outside the chunk) takes the division's slow path
+          sb[g] = m > 0.f ? (unsigned)__nv_cvt_float_to_fp8(__fdiv_rn(m, 6.0f), __NV_SATFINITE, __NV_E4M3) : 0u;
           Divisor d = divisor(e4m3_to_f32((unsigned char)sb[g]));
           d.slow = m > 3.4028235e38f;                                    // the scale is one of e4m3's, or 0 and not divided by
           encode8<FMT>(f[g], d, c[2 * g], c[2 * g + 1]);
@@ -553,9 +559,9 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
     }
   }
   // ---- query heads of the same positions, in place
-  if (q == nullptr || rope_cos == nullptr) return;
   const bool qvec = (reinterpret_cast<uintptr_t>(q) & 15) == 0 && qs * sizeof(T) % 16 == 0;
-  for (int h = w; h < qheads; h += 8) {
+  for (; task < tasks; task += task_step) {
+    const int h = task - 2 * kv.hkv;
     Raw8<T> x[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -673,10 +679,19 @@ template <typename T, int D>
 int launch_append(const tsb200_kv_desc& kv, void* q, int64_t qs, int qheads, const void* k, const void* v, int64_t ks, int64_t vs, int64_t B, int64_t Tn, const int32_t* new_lens,
                   const float* rc, const float* rs, int64_t rr, cudaStream_t s) {
   const int64_t rec = (int64_t)tsb200_kv_record_bytes(kv.format, D);
-  if (Tn >= 16 && kv.format <= TSB200_KV_NVFP4 && B <= 65535) {
-    // bulk: one CTA per (sequence, page group touched); the range may straddle one more page than it fills
+  // By page from 2^17 K elements on (NVFP4, whose V is half as many scattered bytes: 2^18); below that the chain of a page's CTA (tables,
+  // vectors, codes, staged V) is longer than that of a warp per vector, whose byte stores are still few.  8 heads, d 128, both kernels:
+  // 64 tokens int8 5.5 us by page, 4.9 by vector; 192 tokens 5.6 / 6.3 (NVFP4 6.0 / 4.9); 512 tokens 6.1 / 10.2 (NVFP4 6.1 / 5.9).
+  const int64_t elements = B * Tn * kv.hkv * D;
+  if (Tn >= 16 && kv.format <= TSB200_KV_NVFP4 && B <= 65535 && elements >= (kv.format == TSB200_KV_NVFP4 ? 1 << 18 : 1 << 17)) {
+    // one CTA per (sequence, page group touched); the range may straddle one more page than it fills
     constexpr int PAGES = 128 / D;
-    const dim3 grid((unsigned)(((Tn + 15) / 16 + 1 + PAGES - 1) / PAGES), (unsigned)B);
+    const int64_t groups = ((Tn + 15) / 16 + 1 + PAGES - 1) / PAGES, tasks = 2 * (int64_t)kv.hkv + (q ? qheads : 0);
+    // A short chunk leaves most SMs without a page: its heads are dealt out over as many CTAs per page as three an SM leave room for,
+    // at most until a warp has one task.
+    int64_t z = 444 / (groups * B);
+    if (z > (tasks + 7) / 8) z = (tasks + 7) / 8;
+    const dim3 grid((unsigned)groups, (unsigned)B, (unsigned)(z < 1 ? 1 : z));
     switch (kv.format) {
       case TSB200_KV_INT8:
         TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_INT8>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
