@@ -307,6 +307,39 @@ def test_few_tokens_at_model_widths(cuda, p, M, K, N, r):
     assert ops.PackedLinear.device_status(device=cuda) == 0
 
 
+@pytest.mark.parametrize("p", [4, 8, 2, "binary"])
+@pytest.mark.parametrize("K,N,r", [(4096, 4096, 0), (896, 4864, 0), (3584, 1024, 0), (14336, 4096, 1024), (11008, 6144, 0), (8192, 14336, 0), (640, 200, 0)])
+def test_few_tokens_have_the_bits_of_more(cuda, p, K, N, r):
+    """Up to 16 tokens run on warp-level MMAs or on the tcgen05 kernel, whichever is modelled to be faster, more always on the latter: the
+    same bits, token by token."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(32)
+    def factor(a, b):
+        w = (torch.randn((a, b), generator=g, device=cuda) * 0.05).bfloat16()
+        return ops.Factor.quantize(torch.where(w == 0, torch.full_like(w, 0.01), w), p)
+    lin = ops.PackedLinear(factor(N, r or K), factor(r, K) if r else None, torch.randn(N, generator=g, device=cuda).bfloat16(), torch.bfloat16)
+    x = torch.randn((32, K), generator=g, device=cuda).bfloat16()
+    y = lin(x)
+    for m in (1, 2, 6, 8, 9, 12, 16):
+        assert torch.equal(lin(x[:m]), y[:m]), m
+
+
+@pytest.mark.parametrize("p", [4, 8, 2])
+@pytest.mark.parametrize("K,I,r", [(896, 7296, 0), (3584, 18944, 0), (4096, 14336, 1024), (512, 7168, 64)])
+def test_few_tokens_of_an_mlp_have_the_bits_of_more(cuda, p, K, I, r):
+    """The same for the gated block: chained launches or phases of one, silu(gate) * up rounded alike."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(34)
+    def layer(o, i):
+        f = lambda a, b: ops.Factor.quantize((torch.randn((a, b), generator=g, device=cuda) * b ** -0.5).bfloat16(), p)
+        return ops.PackedLinear(f(o, r or i), f(r, i) if r else None, torch.randn(o, generator=g, device=cuda).bfloat16(), torch.bfloat16)
+    mlp = ops.GatedMLP(layer(I, K), layer(I, K), layer(K, I))
+    x = torch.randn((32, K), generator=g, device=cuda).bfloat16()
+    y = mlp(x)
+    for m in (1, 6, 8, 9, 12, 16):
+        assert torch.equal(mlp(x[:m]), y[:m]), m
+
+
 @pytest.mark.parametrize("M,K,N,r,shift", [(16, 7232, 14336, 0, 0), (8, 14144, 14336, 0, 0), (16, 1024, 14336, 7232, 0), (16, 7232, 14336, 192, 0),
                                            (1, 192, 72, 0, 1), (16, 320, 64, 192, 3), (17, 192, 72, 0, 1)])
 def test_binary_rows_of_an_odd_number_of_blocks(cuda, M, K, N, r, shift):

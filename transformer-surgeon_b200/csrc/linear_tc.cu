@@ -428,44 +428,41 @@ int linear_tc(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, vo
   const size_t hbytes = ((size_t)M * (size_t)(d->rank > 0 ? d->rank : 0) * 2 + 255) / 256 * 256;
   float* partial = (float*)(ws + kWsHeader + hbytes);
   // decode-sized token counts on packed factors: one launch per factor, the second chained to the first
-  auto small = [&](const void* W, int bits, const float* scale, const void* bias, const void* in, void* out, int64_t K, int64_t N,
-                   bool pdl, const GvSpan* ahead) {
-    if (bits > 8 || M > kGvTokens) return (int)TSB200_ERR_UNSUPPORTED;
-    PhaseSpec ps;
-    ps.nsub = 1; ps.gated = 0;
-    ps.g[0] = GemmSpec{W, scale, bias, in, out, N, K};
-    return gv_gemm(ps, bits, M, pdl, ahead, ahead ? 1 : 0, s);
+  PhaseSpec pv, pu;
+  pv.nsub = pu.nsub = 1;
+  pv.gated = pu.gated = 0;
+  pv.g[0] = GemmSpec{d->v, d->v_scale, nullptr, x, h, d->rank, d->in_features};
+  pu.g[0] = GemmSpec{d->u, d->u_scale, d->bias, d->rank > 0 ? (const void*)h : x, y, d->out_features, ku};
+  auto gemm = [&](const PhaseSpec& ps, int bits) {
+    const GemmSpec& g = ps.g[0];
+    if (bits == 16) return gemm_tc(g.W, bits, g.scale, g.bias, g.x, g.y, M, g.K, g.N, partial, status, s);
+    if (odd_binary(bits, g.K) || gv_faster(&ps, &bits, 1, M)) {
+      const int st = gv_gemm(ps, bits, M, g_pdl != 0, nullptr, 0, s);
+      if (st != TSB200_ERR_UNSUPPORTED || odd_binary(bits, g.K)) return st;
+    }
+    return gemm_tcq(g.W, bits, g.scale, g.bias, g.x, g.y, M, g.K, g.N, partial, counters, status, s);
   };
-  auto gemm = [&](const void* W, int bits, const float* scale, const void* bias, const void* in, void* out, int64_t K,
-                  int64_t N) {
-    if (bits == 16) return gemm_tc(W, bits, scale, bias, in, out, M, K, N, partial, status, s);
-    const int st = small(W, bits, scale, bias, in, out, K, N, g_pdl != 0, nullptr);
-    if (st != TSB200_ERR_UNSUPPORTED || odd_binary(bits, K)) return st;
-    return gemm_tcq(W, bits, scale, bias, in, out, M, K, N, partial, counters, status, s);
-  };
-  if (d->rank > 0 && d->u_bits <= 8 && d->v_bits <= 8 && M <= kGvTokens && gv_supported(d->u_bits, M, d->out_features, ku)) {
-    const GvSpan u{d->u, (size_t)d->out_features * tsb200_packed_row_bytes(ku, d->u_bits)};
-    int st = small(d->v, d->v_bits, d->v_scale, nullptr, x, h, d->in_features, d->rank, g_pdl != 0, &u);
-    if (st == TSB200_OK) st = small(d->u, d->u_bits, d->u_scale, d->bias, h, y, ku, d->out_features, true, nullptr);
-    if (st != TSB200_ERR_UNSUPPORTED) return st;
+  if (d->rank > 0 && d->u_bits <= 8 && d->v_bits <= 8 && M <= kGvTokens) {
+    const PhaseSpec both[2] = {pv, pu};
+    const int bits[2] = {d->v_bits, d->u_bits};
+    if (odd || gv_faster(both, bits, 2, M)) {
+      const GvSpan u{d->u, (size_t)d->out_features * tsb200_packed_row_bytes(ku, d->u_bits)};
+      int st = gv_gemm(pv, d->v_bits, M, g_pdl != 0, &u, 1, s);
+      if (st == TSB200_OK) st = gv_gemm(pu, d->u_bits, M, true, nullptr, 0, s);
+      if (st != TSB200_ERR_UNSUPPORTED) return st;
+    }
   }
   if (d->rank > 0 && d->u_bits == d->v_bits && d->u_bits <= 8 && !odd) {
     // both factors packed alike: V then U as two phases of ONE launch (grid barrier in between);
     // the rank-r intermediate is produced and consumed through L2
-    PhaseSpec ps[2];
-    ps[0].nsub = 1; ps[0].gated = 0;
-    ps[0].g[0] = GemmSpec{d->v, d->v_scale, nullptr, x, h, d->rank, d->in_features};
-    ps[1].nsub = 1; ps[1].gated = 0;
-    ps[1].g[0] = GemmSpec{d->u, d->u_scale, d->bias, h, y, d->out_features, d->rank};
+    const PhaseSpec ps[2] = {pv, pu};
     return run_program_tcq(ps, 2, d->u_bits, M, (uint8_t*)partial, counters, (int*)(ws + kWsGridBar), status, s);
   }
-  const void* in = x;
   if (d->rank > 0) {
-    int st = gemm(d->v, d->v_bits, d->v_scale, nullptr, x, h, d->in_features, d->rank);
+    const int st = gemm(pv, d->v_bits);
     if (st != TSB200_OK) return st;
-    in = h;
   }
-  return gemm(d->u, d->u_bits, d->u_scale, d->bias, in, y, ku, d->out_features);
+  return gemm(pu, d->u_bits);
 }
 
 }  // namespace tsb

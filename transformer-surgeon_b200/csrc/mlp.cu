@@ -1,10 +1,11 @@
 // Gated MLP block: y = down(silu(gate(x)) * up(x)), the whole of
 // transformersurgeon/blocks/mlp.py:171-185 (MLPGated.forward) behind one entry point.
 //
-// When the three layers are packed alike (same container bits, bf16, 9 <= M <= 64) the block runs as
-// ONE persistent tcgen05 launch of up to four phases (linear_tcq.cu): [gate V | up V] -> [gate U,
-// up U with SiLU(g) * u in the epilogue] -> [down V] -> [down U].  Otherwise it is composed from
-// tsb200_linear and tsb200_swiglu calls.
+// Up to 64 tokens through three layers packed alike (2, 4 or 8 bits, bf16) the block is [gate V | up V] -> [gate U, up U with
+// SiLU(g) * u in the epilogue] -> [down V] -> [down U]: phases of ONE persistent tcgen05 launch (linear_tcq.cu) or, up to 16
+// tokens and where that is faster, a chain of decode-sized launches (linear_gv.cu).  More than 128 tokens through gate and up packed
+// alike take SiLU(g) * u into up's outputs; fp32 layers run as a chain on the FMA kernel (linear_f32.cu).  Otherwise the block is
+// composed from tsb200_linear and tsb200_swiglu calls.
 #include "tc_common.cuh"
 
 namespace tsb {
@@ -43,7 +44,8 @@ bool promptable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, int64_
   const int64_t step = bits == 1 ? 128 : 8;                  // columns of a row pitch that the copy engine takes
   return g->in_features % step == 0 && g->rank % step == 0;
 }
-// Few enough tokens for the chain of decode-sized launches (linear_gv.cu); its results are those of the one-launch block.
+// Few enough tokens for the chain of decode-sized launches (linear_gv.cu); its results are those of the one-launch block, and
+// gv_faster() chooses between the two.
 bool chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, const tsb200_linear_desc* d, int64_t M) {
   const int b = g->u_bits;
   return M <= kGvTokens && (g->rank == 0 || gv_supported(b, M, g->rank, g->in_features)) &&
@@ -128,53 +130,7 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
   uint8_t* h1 = h0 + r_b;
   uint8_t* h2 = h1 + r_b;
 
-  const bool fused = fusable(gate, up, down, M);
-  if (fused && chainable(gate, up, down, M)) {
-    // [gate V | up V] -> [gate U, up U with SiLU(g) * u] -> [down V] -> [down U]: chained launches, the first one also requests
-    // the codes of the others into the L2
-    GvSpan ahead[3];
-    int na = 0;
-    const int64_t kgu = gate->rank > 0 ? gate->rank : gate->in_features, kd = down->rank > 0 ? down->rank : down->in_features;
-    auto span = [&](const void* p, int bits, int64_t rows, int64_t cols) { ahead[na++] = GvSpan{p, (size_t)rows * tsb200_packed_row_bytes(cols, bits)}; };
-    PhaseSpec ps;
-    int st = TSB200_OK;
-    bool pdl = g_pdl != 0;
-    ps.g[1] = GemmSpec{};
-    const void* gx = x;
-    const void* ux = x;
-    if (gate->rank > 0) {
-      span(gate->u, gate->u_bits, gate->out_features, kgu);
-      span(up->u, up->u_bits, up->out_features, kgu);
-      span(down->rank > 0 ? down->v : down->u, down->rank > 0 ? down->v_bits : down->u_bits, down->rank > 0 ? down->rank : down->out_features, down->in_features);
-      ps.nsub = 2; ps.gated = 0;
-      ps.g[0] = GemmSpec{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features};
-      ps.g[1] = GemmSpec{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features};
-      st = gv_gemm(ps, gate->v_bits, M, pdl, ahead, na, s);
-      gx = h0; ux = h1;
-      pdl = true;
-    }
-    if (st == TSB200_OK) {
-      na = 0;
-      span(down->u, down->u_bits, down->out_features, kd);
-      ps.nsub = 2; ps.gated = 1;
-      ps.g[0] = GemmSpec{gate->u, gate->u_scale, gate->bias, gx, buf_g, gate->out_features, kgu};
-      ps.g[1] = GemmSpec{up->u, up->u_scale, up->bias, ux, buf_g, up->out_features, kgu};
-      st = gv_gemm(ps, gate->u_bits, M, pdl, ahead, na, s);
-    }
-    ps.nsub = 1; ps.gated = 0;
-    const void* dx = buf_g;
-    if (st == TSB200_OK && down->rank > 0) {
-      ps.g[0] = GemmSpec{down->v, down->v_scale, nullptr, buf_g, h2, down->rank, down->in_features};
-      st = gv_gemm(ps, down->v_bits, M, true, nullptr, 0, s);
-      dx = h2;
-    }
-    if (st == TSB200_OK) {
-      ps.g[0] = GemmSpec{down->u, down->u_scale, down->bias, dx, y, down->out_features, kd};
-      st = gv_gemm(ps, down->u_bits, M, true, nullptr, 0, s);
-    }
-    if (st != TSB200_ERR_UNSUPPORTED) return st;
-  }
-  if (fused) {
+  if (fusable(gate, up, down, M)) {
     PhaseSpec ps[4];
     int n = 0;
     const void* gx = x;
@@ -204,8 +160,23 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
       ps[n].g[0] = GemmSpec{down->u, down->u_scale, down->bias, buf_g, y, down->out_features, down->in_features};
       ++n;
     }
-    const int st = run_program_tcq(ps, n, gate->u_bits, M, ws + tc::kWsHeader, (int*)(ws + tc::kWsCounters),
-                                   (int*)(ws + tc::kWsGridBar), (int*)ws, s);
+    const int bits[4] = {gate->u_bits, gate->u_bits, gate->u_bits, gate->u_bits};
+    int st = TSB200_ERR_UNSUPPORTED;
+    if (chainable(gate, up, down, M) && gv_faster(ps, bits, n, M)) {
+      // [gate V | up V] -> [gate U, up U with SiLU(g) * u] -> [down V] -> [down U]: chained launches, the first two also request
+      // codes of later ones into the L2
+      auto span = [](const void* p, int bits, int64_t rows, int64_t cols) { return GvSpan{p, (size_t)rows * tsb200_packed_row_bytes(cols, bits)}; };
+      const GvSpan down_u = span(down->u, down->u_bits, down->out_features, down->rank > 0 ? down->rank : down->in_features);
+      const GvSpan first[3] = {span(gate->u, gate->u_bits, gate->out_features, kgu), span(up->u, up->u_bits, up->out_features, kgu),
+                               down->rank > 0 ? span(down->v, down->v_bits, down->rank, down->in_features) : down_u};
+      st = TSB200_OK;
+      for (int p = 0; p < n && st == TSB200_OK; ++p) {
+        const bool before_gated = !ps[p].gated && ps[p].nsub == 2;
+        st = gv_gemm(ps[p], gate->u_bits, M, p > 0 || g_pdl != 0, before_gated ? first : &down_u, before_gated ? 3 : (ps[p].gated ? 1 : 0), s);
+      }
+      if (st != TSB200_ERR_UNSUPPORTED) return st;
+    }
+    st = run_program_tcq(ps, n, gate->u_bits, M, ws + tc::kWsHeader, (int*)(ws + tc::kWsCounters), (int*)(ws + tc::kWsGridBar), (int*)ws, s);
     if (st != TSB200_ERR_UNSUPPORTED) return st;
   }
   if (f32_chainable(gate, up, down)) {

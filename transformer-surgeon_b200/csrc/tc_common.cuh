@@ -243,14 +243,17 @@ size_t phase_scratch_bytes(int64_t M, int64_t N, int64_t K, int nsub, bool gated
 
 // Decode-sized packed GEMM (linear_gv.cu): one phase, one launch, no workspace.  `ahead`: constants of the launches that follow,
 // requested into the L2 while this one runs.
-// Token counts it serves.  Above 16 tokens the tcgen05 kernel is as fast: 32 tokens through 4096 x 4096 take 9.8 us there and
-// 10.1 here, through 4096 x 6144 11.7 and 20.5 (its MMAs take 32 tokens at the price of 16; these pay per 8).
+// Token counts it serves, where its activations fit an SM.  Above 16 tokens the tcgen05 kernel is as fast on most factors: 32 tokens
+// through 4096 x 4096 take 9.8 us there and 10.1 here, through 4096 x 6144 11.7 and 20.5 (its MMAs take 32 tokens at the price of 16;
+// these pay per 8).  Up to 16 gv_faster() says which of the two a chain of phases takes.
 constexpr int64_t kGvTokens = 16;
 struct GvSpan {
   const void* p;
   size_t bytes;
 };
 bool gv_supported(int bits, int64_t M, int64_t N, int64_t K);
+// Whether n phases, one launch each, are modelled to take less time here than in linear_tcq.cu (they are the same bits).
+bool gv_faster(const PhaseSpec* ps, const int* bits, int n, int64_t M);
 // fp32 activations (linear_f32.cu): n <= 4 matrices of one container and reduction length in one launch; a gate / up pair.
 int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s);
 int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s);
