@@ -582,24 +582,24 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   }
 }
 
-// FP8 scales of a prompt: amax over the T tokens of a (sequence, kv head) -> amax / 448 (1 if 0).  A cluster of eight CTAs shares the
-// tokens of G heads, D / 16 lanes a vector ((8 + 8) elements each, so the rotation needs no other lane; its cos and sin, as many bytes
-// as K and V, are fetched and rounded once for the G heads), the maxima meet in distributed shared memory.  Bound by the one trip of
-// K and V from memory: 32 x 2048 tokens, 8 heads, d 128: 268 MB, 41 us at the copy rate; 50 us with four heads, 71 with one; one CTA per
-// (sequence, head), a warp per vector and five shuffles per rotation took 343 us.
+// FP8 scales of a prompt: amax over the T tokens of a (sequence, kv head) -> amax / 448 (1 if 0).  A cluster of eight CTAs (for few
+// tokens a single one) shares the tokens of G heads, D / 16 lanes a vector ((8 + 8) elements each, so the rotation needs no other lane;
+// its cos and sin, as many bytes as K and V, are fetched and rounded once for the G heads), the maxima meet in distributed shared memory.
+// Bound by the one trip of K and V from memory: 32 x 2048 tokens, 8 heads, d 128: 268 MB, 41 us at the copy rate; 50 us with four heads,
+// 71 with one; one CTA per (sequence, head), a warp per vector and five shuffles per rotation took 343 us.
 constexpr int kScaleRanks = 8;
-template <typename T, int D, int G>
+template <typename T, int D, int G, int RANKS>
 __global__ void __launch_bounds__(256)
 kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t ks, int64_t vs, int64_t Tn, int hkv,
                      const int32_t* __restrict__ pos0, const float* __restrict__ rope_cos,
                      const float* __restrict__ rope_sin, int64_t rope_rows, float* __restrict__ k_scale,
                      float* __restrict__ v_scale) {
   constexpr int HALF = D / 2, EG = HALF / 8, PER = 256 / EG;              // vectors of a CTA side by side
-  __shared__ float sh[2 * G][8], srank[2 * G][kScaleRanks];
+  __shared__ float sh[2 * G][8], srank[2 * G][RANKS];
   // "has started": a rank's shared memory may be written by another only once its CTA runs; awaited before the remote store below
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
-  const int rank = blockIdx.x % kScaleRanks, groups = (hkv + G - 1) / G;
-  const int64_t item = blockIdx.x / kScaleRanks, b = item / groups;
+  const int rank = blockIdx.x % RANKS, groups = (hkv + G - 1) / G;
+  const int64_t item = blockIdx.x / RANKS, b = item / groups;
   const int h0 = (int)(item % groups) * G;
   const int eg = threadIdx.x % EG, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t start = pos0 ? (int64_t)pos0[b] : 0;
@@ -609,7 +609,7 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
   float mk[G], mv[G];
 #pragma unroll
   for (int h = 0; h < G; ++h) mk[h] = mv[h] = 0.f;
-  const int64_t t_first = (int64_t)rank * PER + threadIdx.x / EG, t_step = kScaleRanks * PER;
+  const int64_t t_first = (int64_t)rank * PER + threadIdx.x / EG, t_step = RANKS * PER;
   const T* kp = k + (b * Tn + t_first) * ks + h0 * D + eg * 8;
   const T* vp = v + (b * Tn + t_first) * vs + h0 * D + eg * 8;
 #pragma unroll (G == 1 ? 4 : (G == 2 ? 2 : 1))
@@ -670,7 +670,7 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
   if (rank == 0 && threadIdx.x < 2 * G && h0 + (int)threadIdx.x / 2 < hkv) {
     float m = srank[threadIdx.x][0];
 #pragma unroll
-    for (int i = 1; i < kScaleRanks; ++i) m = fmaxf(m, srank[threadIdx.x][i]);
+    for (int i = 1; i < RANKS; ++i) m = fmaxf(m, srank[threadIdx.x][i]);
     ((threadIdx.x & 1) ? v_scale : k_scale)[b * hkv + h0 + threadIdx.x / 2] = m > 0.f ? __fdiv_rn(m, 448.0f) : 1.0f;
   }
 }
@@ -775,24 +775,28 @@ int tsb200_kv_fp8_scales_strided(const void* k, const void* v, int dtype, int64_
   if (ks < dense || vs < dense) return TSB200_ERR_ARG;
   if (B * hkv * kScaleRanks > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   cudaStream_t s = as_stream(stream);
-  // heads per CTA: as many as leave every SM two CTAs
+  // A single CTA where it takes all tokens at once (4096 / head_dim; 32 sequences x 17 tokens, 8 heads: 4.1 us, 6.6 with a cluster), and
+  // heads per CTA: as many as leave every SM two CTAs.
+  const int ranks = T <= 4096 / head_dim ? 1 : kScaleRanks;
   int g = 4;
-  while (g > 1 && B * ((hkv + g - 1) / g) * kScaleRanks < 296) g /= 2;
+  while (g > 1 && B * ((hkv + g - 1) / g) * ranks < 296) g /= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(B * ((hkv + g - 1) / g) * kScaleRanks));
+  cfg.gridDim = dim3((unsigned)(B * ((hkv + g - 1) / g) * ranks));
   cfg.blockDim = dim3(256);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kScaleRanks;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-#define TSB_SG(TT, DD, GG) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD, GG>, (const TT*)k, (const TT*)v, ks, vs, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
+#define TSB_SR(TT, DD, GG, RR) TSB_CUDA(cudaLaunchKernelEx(&cfg, kv_fp8_scales_kernel<TT, DD, GG, RR>, (const TT*)k, (const TT*)v, ks, vs, T, hkv, pos0, rope_cos, rope_sin, rope_rows, k_scale, v_scale))
+#define TSB_SG(TT, DD, GG) do { if (ranks == 1) TSB_SR(TT, DD, GG, 1); else TSB_SR(TT, DD, GG, kScaleRanks); } while (0)
 #define TSB_SC(TT, DD) do { if (g == 4) TSB_SG(TT, DD, 4); else if (g == 2) TSB_SG(TT, DD, 2); else TSB_SG(TT, DD, 1); } while (0)
   if (dtype == TSB200_F32) { if (head_dim == 64) TSB_SC(float, 64); else TSB_SC(float, 128); }
   else { if (head_dim == 64) TSB_SC(__nv_bfloat16, 64); else TSB_SC(__nv_bfloat16, 128); }
+#undef TSB_SR
 #undef TSB_SG
 #undef TSB_SC
   return TSB200_OK;
