@@ -228,24 +228,25 @@ __global__ void argmax_finalize_kernel(const float* __restrict__ val, const int*
 
 // Argmax over stored logits y [M, N]: the first maximum of a row, NaN counting as largest (torch.argmax).  A cluster of eight
 // CTAs shares a row, 16-byte loads, one 64-bit key per candidate (order-preserving value bits, then the complement of the column),
-// exchanged through distributed shared memory.  [32, 128256] bf16: 42 us with the library reduction, about 5 here.
+// exchanged through distributed shared memory.  [32, 128256] bf16: 42 us with the library reduction, about 5 here.  Rows that one CTA
+// reads in two trips or so have no cluster (32 rows of 1000: the launch of eight times the CTAs took 3 us).
 constexpr int kArgRanks = 8, kArgThreads = 1024;
 __device__ __forceinline__ unsigned long long argmax_key(float v, unsigned col) {
   const unsigned b = __float_as_uint(v + 0.f);                       // -0 counts as +0
   const unsigned o = v != v ? 0xffffffffu : ((b >> 31) ? ~b : (b | 0x80000000u));
   return ((unsigned long long)o << 32) | (unsigned)~col;
 }
-template <typename T>
+template <typename T, int RANKS>
 __global__ void __launch_bounds__(kArgThreads) argmax_rows_kernel(const T* __restrict__ y, int64_t N, int64_t* __restrict__ out) {
-  __shared__ unsigned long long sw[kArgThreads / 32], srank[kArgRanks];
+  __shared__ unsigned long long sw[kArgThreads / 32], srank[RANKS];
   // "has started": a rank's shared memory may be written by another only once its CTA runs; awaited before the remote store below
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
   pdl_launch_dependents();
   pdl_wait();
   constexpr int E = 16 / sizeof(T);
-  const unsigned rank = blockIdx.x % kArgRanks;
-  const T* row = y + (int64_t)(blockIdx.x / kArgRanks) * N;
-  const int64_t len = ((N + kArgRanks - 1) / kArgRanks + E - 1) / E * E;
+  const unsigned rank = blockIdx.x % RANKS;
+  const T* row = y + (int64_t)(blockIdx.x / RANKS) * N;
+  const int64_t len = ((N + RANKS - 1) / RANKS + E - 1) / E * E;
   const int64_t c0 = rank * len, c1 = min(N, c0 + len);
   unsigned long long best = 0;                                       // below every key of a column
   if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
@@ -278,8 +279,8 @@ __global__ void __launch_bounds__(kArgThreads) argmax_rows_kernel(const T* __res
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   if (rank == 0 && threadIdx.x == 0) {
     best = srank[0];
-    for (int i = 1; i < kArgRanks; ++i) best = max(best, srank[i]);
-    out[blockIdx.x / kArgRanks] = (int64_t)(unsigned)~(unsigned)best;
+    for (int i = 1; i < RANKS; ++i) best = max(best, srank[i]);
+    out[blockIdx.x / RANKS] = (int64_t)(unsigned)~(unsigned)best;
   }
 }
 
@@ -392,20 +393,22 @@ int linear_argmax_tc(const tsb200_linear_desc* d, const void* x, int64_t* tokens
 int argmax_rows(const void* y, int dtype, int64_t M, int64_t N, int64_t* tokens, cudaStream_t s) {
   if (N > 0xfffffffell || M * kArgRanks > 0x7fffffffll) return TSB200_ERR_UNSUPPORTED;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(M * kArgRanks));
+  const int ranks = N <= 2 * 8 * kArgThreads ? 1 : kArgRanks;
+  cfg.gridDim = dim3((unsigned)(M * ranks));
   cfg.blockDim = dim3(kArgThreads);
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kArgRanks;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_pdl ? 2 : 1;
-  if (dtype == TSB200_F32) TSB_CUDA(cudaLaunchKernelEx(&cfg, argmax_rows_kernel<float>, (const float*)y, N, tokens));
-  else TSB_CUDA(cudaLaunchKernelEx(&cfg, argmax_rows_kernel<__nv_bfloat16>, (const __nv_bfloat16*)y, N, tokens));
+  auto go = [&](auto* kernel, auto* rows) { return cudaLaunchKernelEx(&cfg, kernel, rows, N, tokens); };
+  if (dtype == TSB200_F32) TSB_CUDA(ranks == 1 ? go(argmax_rows_kernel<float, 1>, (const float*)y) : go(argmax_rows_kernel<float, kArgRanks>, (const float*)y));
+  else TSB_CUDA(ranks == 1 ? go(argmax_rows_kernel<__nv_bfloat16, 1>, (const __nv_bfloat16*)y) : go(argmax_rows_kernel<__nv_bfloat16, kArgRanks>, (const __nv_bfloat16*)y));
   return TSB200_OK;
 }
 
