@@ -57,6 +57,19 @@ def test_prefill_attention_bf16_against_oracle(cuda, T, L, H, Hkv, d):
         assert torch.all((out[b] - ref).abs() <= tol), ((out[b] - ref).abs() / tol).max()
 
 
+@pytest.mark.parametrize("B,T,L,H,Hkv,d", [(8, 300, 300, 7, 1, 128), (6, 257, 700, 9, 1, 64), (5, 129, 129, 32, 8, 128)])
+def test_paired_query_tiles_equal_single_ones(cuda, B, T, L, H, Hkv, d):
+    """A batch with more query tiles than SMs (two tiles to a CTA; an odd number of them per kv head, heads of different tiles together)
+    against its sequences one by one (a tile to a CTA): the same bits."""
+    ops, kv, g = setup(cuda, "bf16", B, L, H, Hkv, d, torch.bfloat16, 6)
+    q = torch.randn((B, T, H, d), generator=g, device=cuda).bfloat16()
+    out = ops.prefill_attention(kv, q, L)
+    for b in range(B):
+        one = ops.PagedKV.__new__(ops.PagedKV)
+        one.__dict__.update(kv.__dict__, block_table=kv.block_table[b:b + 1].contiguous(), seq_lens=kv.seq_lens[b:b + 1].contiguous(), _desc=None)
+        assert torch.equal(ops.prefill_attention(one, q[b:b + 1], L), out[b:b + 1])
+
+
 @pytest.mark.parametrize("fmt", ["int8", "fp8", "nvfp4"])
 def test_prefill_attention_reads_dequantized_pages(cuda, fmt):
     """Quantized pages: the kernel attends over exactly the values the dequantizing gather returns."""

@@ -58,6 +58,7 @@ struct PfParams {
   int64_t B, T, L;
   int H, hkv;
   int nq, pairs, items;      // query tiles per head, pairs per (sequence, kv head), pairs in all
+  int per;                   // tiles of a pair: 2, or 1 where the tiles are fewer than the SMs
   float scale_log2;          // sm_scale * log2(e)
   __nv_bfloat16* out;        // [B, T, H, D]
   int* status;
@@ -122,9 +123,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     return Work{rest / p.hkv, rest % p.hkv, p.pairs - 1 - w / per};   // longest first
   };
   auto tile = [&](const Work& k, int i) {
-    const int u = 2 * k.pair + i, qt = u / G;
+    const int u = p.per * k.pair + i, qt = u / G;
     const int64_t q0 = (int64_t)qt * BQ;
-    return Tile{k.hk * G + u % G, qt < p.nq ? (int)((off + min(p.T - 1, q0 + BQ - 1)) / BKEY) + 1 : 0, q0};
+    return Tile{k.hk * G + u % G, i < p.per && qt < p.nq ? (int)((off + min(p.T - 1, q0 + BQ - 1)) / BKEY) + 1 : 0, q0};
   };
 
   if (threadIdx.x == 0) {
@@ -549,7 +550,11 @@ int launch_prefill(const void* q, int64_t q_token_stride, const void* k, const v
   p.out = (__nv_bfloat16*)out;
   p.status = status;
   p.nq = (int)((T + BQ - 1) / BQ);
-  const int64_t pairs = ((int64_t)p.nq * (H / hkv) + 1) / 2, items = pairs * hkv * B;
+  // Two tiles to a CTA take up to 1.5 times the time of one: with a tile for at most every SM each gets its own (1 x 64 tokens at the end
+  // of 4096, 32 / 8 heads: 92 us in pairs, 63 here).
+  const int64_t tiles = (int64_t)p.nq * (H / hkv);
+  p.per = tiles * hkv * B <= kPlanSMs ? 1 : 2;
+  const int64_t pairs = (tiles + p.per - 1) / p.per, items = pairs * hkv * B;
   if (items > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   p.pairs = (int)pairs;
   p.items = (int)items;
