@@ -33,12 +33,16 @@ struct F32Params {
   int64_t row_bytes;
 };
 
-// CNT consecutive weights of a lane: a 16-byte piece of a dense row (4) or one 32-bit word of codes (4 / 8 / 16 / 32).
-template <int BITS> struct Piece {
-  static constexpr int kCnt = BITS == 32 ? 4 : 32 / BITS;
-  static constexpr int kBytes = BITS == 32 ? 16 : 4;
+// Consecutive weights of a lane: a 16-byte piece of a dense row (4) or one 32-bit word of codes (4 / 8 / 16 / 32).  Bits are shared out
+// eight to a lane where the products of four tokens or more outweigh the loads (a row of 896 bits is 28 words: 8 tokens, 896 rows:
+// 12.9 us by words, 10.3 by halves, 7.5 by bytes).
+template <int BITS, int MT> struct Piece {
+  static constexpr int kCnt = BITS == 32 ? 4 : (BITS == 1 && MT >= 4 ? 8 : 32 / BITS);
+  static constexpr int kPerWord = BITS == 32 ? 1 : 32 / BITS / kCnt;
+  static __device__ __forceinline__ int64_t at(int i) { return (int64_t)(i / kPerWord) * (BITS == 32 ? 16 : 4); }
 };
-template <int BITS> __device__ __forceinline__ void load_piece(const uint8_t* p, float (&v)[Piece<BITS>::kCnt]) {
+// p: the 16 bytes or the word that piece i of a row lies in.
+template <int BITS, int CNT> __device__ __forceinline__ void load_piece(const uint8_t* p, int i, float (&v)[CNT]) {
   if constexpr (BITS == 32) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(p));
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
@@ -46,19 +50,20 @@ template <int BITS> __device__ __forceinline__ void load_piece(const uint8_t* p,
     const unsigned w = __ldg(reinterpret_cast<const unsigned*>(p));
     if constexpr (BITS == 8) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = (float)(int8_t)(w >> (8 * i));
+      for (int j = 0; j < 4; ++j) v[j] = (float)(int8_t)(w >> (8 * j));
     } else if constexpr (BITS == 1) {
+      const unsigned x = w >> (i % (32 / CNT) * (CNT / 2));
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        v[2 * i] = (float)(int)(((w >> i) & 1u) * 2u) - 1.0f;
-        v[2 * i + 1] = (float)(int)(((w >> (i + 16)) & 1u) * 2u) - 1.0f;
+      for (int j = 0; j < CNT / 2; ++j) {
+        v[2 * j] = (float)(int)(((x >> j) & 1u) * 2u) - 1.0f;
+        v[2 * j + 1] = (float)(int)(((x >> (j + 16)) & 1u) * 2u) - 1.0f;
       }
     } else {
-      constexpr int half = 16 / BITS;          // pair-interleaved: field i = column 2 i, field i + half = column 2 i + 1
+      constexpr int half = 16 / BITS;          // pair-interleaved: field j = column 2 j, field j + half = column 2 j + 1
 #pragma unroll
-      for (int i = 0; i < half; ++i) {
-        v[2 * i] = (float)sext((int)(w >> (BITS * i)), BITS);
-        v[2 * i + 1] = (float)sext((int)(w >> (BITS * i + 16)), BITS);
+      for (int j = 0; j < half; ++j) {
+        v[2 * j] = (float)sext((int)(w >> (BITS * j)), BITS);
+        v[2 * j + 1] = (float)sext((int)(w >> (BITS * j + 16)), BITS);
       }
     }
   }
@@ -85,7 +90,7 @@ template <int V> __device__ __forceinline__ float reduce_scatter(float (&v)[V]) 
 template <int BITS, int MT, int R, bool GATED>
 __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_constant__ F32Params p) {
   constexpr int MATS = GATED ? 2 : 1;
-  constexpr int CNT = Piece<BITS>::kCnt;
+  constexpr int CNT = Piece<BITS, MT>::kCnt;
   constexpr int V = MATS * R * MT;
   constexpr int kKT = kXFloats / (MATS * MT);
   static_assert(V <= 32 && (V & (V - 1)) == 0, "one sum per lane");
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
     for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (i < pre_end) load_piece<BITS>(rows[mat][r] + (int64_t)i * Piece<BITS>::kBytes, pre[q][mat][r]);
+        if (i < pre_end) load_piece<BITS>(rows[mat][r] + Piece<BITS, MT>::at(i), i, pre[q][mat][r]);
   }
   if (lane < MATS * R && ks == 0 && row0 < sg.n) {
     const uint8_t* q = rows[0][0];
@@ -159,7 +164,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
     __syncthreads();
     // pieces of this warp: lane + 32 ks, then every 32 * ks_n; beyond the row's end the activations are zero, and no piece is read
     const int pieces = (kt + CNT - 1) / CNT;
-    const int64_t b0 = (int64_t)k0 * Piece<BITS>::kBytes / CNT;
+    const int64_t b0 = Piece<BITS, MT>::at(k0 / CNT);
     auto use = [&](int i, const float (&w)[MATS][R][CNT]) {
 #pragma unroll
       for (int mat = 0; mat < MATS; ++mat)
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
 #pragma unroll
       for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
-        for (int r = 0; r < R; ++r) load_piece<BITS>(rows[mat][r] + b0 + (int64_t)i * Piece<BITS>::kBytes, w[mat][r]);
+        for (int r = 0; r < R; ++r) load_piece<BITS>(rows[mat][r] + b0 + Piece<BITS, MT>::at(i), i, w[mat][r]);
       use(i, w);
     }
   }
@@ -307,7 +312,7 @@ int launch_cfg(F32Params& p, bool pdl, cudaStream_t s) {
   const int groups = (p.M + MT - 1) / MT;
   int ks = 0;
   while (ks < 3 && (int64_t)((rows + (kWarps >> ks) * R - 1) / ((kWarps >> ks) * R)) * groups < 296 &&
-         p.K >= (64 << ks) * Piece<BITS>::kCnt)
+         p.K >= (64 << ks) * Piece<BITS, MT>::kCnt)
     ++ks;
   p.ks_log2 = ks;
   const int per = (kWarps >> ks) * R;
