@@ -485,6 +485,25 @@ def test_append_of_infinities_and_of_quotients_beyond_the_type(cuda, fmt, name, 
         assert [int(codes[3 * i + 1, 5 * i + 2]) for i in range(4)] == [0x7e, 0xfe, 0x7e, 0xfe]
 
 
+@pytest.mark.parametrize("fmt", ["fp32", "bf16"])
+@pytest.mark.parametrize("H,Hkv,d", [(4, 4, 128), (32, 8, 128), (6, 2, 64), (28, 4, 128)])
+def test_unquantized_pages_of_many_sequences(cuda, fmt, H, Hkv, d):
+    """Enough sequences to fill the machine, up to four query heads to a kv head and more: against the CUDA-core kernel (both in fp32)."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(41)
+    B, L = 60, 77
+    table = torch.randperm(B * 5, generator=g, device=cuda).to(torch.int32).reshape(B, 5)
+    seq = torch.zeros(B, dtype=torch.int32, device=cuda)
+    kv = ops.PagedKV(fmt, B * 5, Hkv, d, table, seq, cuda)
+    k, v = (torch.randn((B, L, Hkv, d), generator=g, device=cuda).to(DT[fmt]) for _ in range(2))
+    kv.append(k, v)
+    seq.copy_(torch.arange(B) % (L + 1))
+    q = torch.randn((B, H, d), generator=g, device=cuda)
+    out, ref = ops.paged_decode_attention(kv, q, L), ops.paged_decode_attention(kv, q, L, simt=True)
+    # sums of 77 products of unit size in two orders, __expf against expf: 2e-4 of the values' scale, as for that kernel against the oracle
+    assert (out - ref).abs().max() <= C_P_SIMT * v.float().abs().max()
+
+
 def test_fp8_attention_after_append_under_dependent_launch(cuda):
     """One decode step's append -> attention pair with programmatic dependent launch on: the attention may fetch pages
     older than the newest token before the append has finished.  Lengths sit on, before and after page boundaries and
