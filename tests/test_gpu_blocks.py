@@ -82,3 +82,18 @@ def test_rmsnorm_row_lengths(cuda, name, hidden):
     tol = dict(rtol=1e-5, atol=1e-5) if name == "fp32" else dict(rtol=1e-2, atol=1e-2)
     assert torch.equal(res.cpu(), s)
     torch.testing.assert_close(y.cpu(), oatt.rmsnorm_hf(s, w, 1e-6), **tol)
+
+
+@pytest.mark.parametrize("name,hidden", [("bf16", 8192), ("bf16", 5000), ("fp32", 4096), ("fp32", 2052)])
+def test_rmsnorm_of_many_wide_rows(cuda, name, hidden):
+    """More rows than eight an SM: the weights come behind the sum; the same bits as a few rows at a time."""
+    from transformer_surgeon_b200 import ops
+    dt = torch.float32 if name == "fp32" else torch.bfloat16
+    g = torch.Generator(device=cuda).manual_seed(8)
+    r, d, w = (torch.randn(s, generator=g, device=cuda).to(dt) for s in ((1300, hidden), (1300, hidden), (hidden,)))
+    r1, r2 = r.clone(), r.clone()
+    y = ops.add_rmsnorm(r1, d, w, 1e-5)
+    for i in range(0, 1300, 650):
+        part = r2[i:i + 650]
+        assert torch.equal(ops.add_rmsnorm(part, d[i:i + 650], w, 1e-5), y[i:i + 650])
+    assert torch.equal(r1, r2)

@@ -134,8 +134,10 @@ template <> struct Vec16<__nv_bfloat16> {
 
 // Hugging Face variant, rows of whole 16-byte pieces, at most IT * 256 of them: one pass over global memory; the row stays in
 // registers between the statistic and the scaling.  With a decode batch the launch is a chain of latencies (launch, row, sum, row
-// out): the weights, constants, are requested ahead of the dependency wait so that they are no link of it.
-template <typename T, int IT>
+// out): the weights, constants, are requested ahead of the dependency wait so that they are no link of it (AHEAD).  Many rows of the
+// widest kind want the registers for more CTAs instead (x 8192 bf16: 1000 rows 10.0 us, 10.4 with the weights behind the sum; 2500: 32.4 /
+// 30.7; 16384: 183 / 172).
+template <typename T, int IT, bool AHEAD>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_hf_kernel(T* __restrict__ residual, const T* __restrict__ delta, const T* __restrict__ w, T* __restrict__ y, int hidden, float eps) {
   using V = Vec16<T>;
@@ -148,7 +150,7 @@ add_rmsnorm_hf_kernel(T* __restrict__ residual, const T* __restrict__ delta, con
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int i = threadIdx.x + it * 256;
-    if (i < nvec) ww[it] = __ldg(wv + i);
+    if (AHEAD && i < nvec) ww[it] = __ldg(wv + i);
   }
   pdl_wait();
   uint4* r = reinterpret_cast<uint4*>(residual + row * hidden);
@@ -179,7 +181,7 @@ add_rmsnorm_hf_kernel(T* __restrict__ residual, const T* __restrict__ delta, con
     const int i = threadIdx.x + it * 256;
     if (i < nvec) {
       float f[V::N], o[V::N];
-      V::unpack(ww[it], f);
+      V::unpack(AHEAD ? ww[it] : __ldg(wv + i), f);
 #pragma unroll
       for (int j = 0; j < V::N; ++j) o[j] = __fmul_rn(f[j], rnd<T>(__fmul_rn(v[it][j], inv)));
       yo[i] = V::pack(o);
@@ -193,7 +195,10 @@ int launch_rmsnorm_hf(void* residual, const void* delta, const void* w, void* y,
     return launch_kernel(kernel, dim3((unsigned)M), dim3(256), 0, s, (T*)residual, (const T*)delta, (const T*)w, (T*)y, (int)hidden, eps);
   };
   const int64_t pieces = hidden / Vec16<T>::N;
-  TSB_CUDA(pieces <= 256 ? go(add_rmsnorm_hf_kernel<T, 1>) : (pieces <= 512 ? go(add_rmsnorm_hf_kernel<T, 2>) : go(add_rmsnorm_hf_kernel<T, 4>)));
+  if (pieces <= 256) TSB_CUDA(go(add_rmsnorm_hf_kernel<T, 1, true>));
+  else if (pieces <= 512) TSB_CUDA(go(add_rmsnorm_hf_kernel<T, 2, true>));
+  else if (M <= 8 * 148) TSB_CUDA(go(add_rmsnorm_hf_kernel<T, 4, true>));
+  else TSB_CUDA(go(add_rmsnorm_hf_kernel<T, 4, false>));
   return TSB200_OK;
 }
 
