@@ -166,6 +166,8 @@ class Factor:
         w = _cuda(w, "w")
         rows, cols = w.shape
         code, bits = precision_code(precision), container_bits(precision)
+        if cols > 32768:                 # rows too long for one pass
+            return Factor.from_codes(*quantize_weight(w, precision, granularity, eps), precision)
         per_channel = granularity == "per_channel"
         scales = torch.empty(rows, dtype=torch.float32, device=w.device)
         ws = None if per_channel else torch.empty(16, dtype=torch.uint8, device=w.device)
@@ -174,8 +176,6 @@ class Factor:
             flag = torch.zeros(1, dtype=torch.int32, device=w.device) if bits == 1 else None
             st = _lib.load().tsb200_quantize_pack(w.data_ptr(), _dt(w), rows, cols, code, int(per_channel), float(eps), bits, packed.data_ptr(),
                                                   scales.data_ptr(), _p(flag), _p(ws), 16, _stream())
-            if st == _lib.ERR_UNSUPPORTED and rows and cols:         # rows too long for one pass
-                return Factor.from_codes(*quantize_weight(w, precision, granularity, eps), precision)
             check(st, "tsb200_quantize_pack")
             if flag is None or not bool(flag.item()):
                 return Factor(packed, scales, bits, rows, cols)
