@@ -66,7 +66,8 @@ int tsb200_check_device(void);
  * in the FP8 decode attention with one split, pages of the cache STRICTLY OLDER than the one that holds a sequence's
  * newest token.  With this setting on, the launch that directly precedes an append or a decode attention on its stream
  * must therefore not be the one that writes those: advance lengths, remap pages and refresh scales at least two launches
- * ahead (the engine of this package does so at the start of a step), or turn the setting off around such a pair. */
+ * ahead (the engine of this package does so at the start of a step), or turn the setting off around such a pair, or (decode attention)
+ * say so in the cache's flags. */
 int tsb200_set_pdl(int enabled);
 
 /* ------------------------------------------------------------------------------------
@@ -203,11 +204,15 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
  * ---------------------------------------------------------------------------------- */
 size_t tsb200_kv_record_bytes(int format, int head_dim);
 
+/* seq_lens, block_table or the scales may come from the launch that directly precedes a decode attention on its stream: that attention
+ * then starts after it even where tsb200_set_pdl lets launches overlap. */
+#define TSB200_KV_FRESH 1
+
 typedef struct {
   int32_t format;        /* tsb200_kv_format                                            */
   int32_t hkv;           /* number of kv heads                                           */
   int32_t head_dim;      /* 64 or 128                                                    */
-  int32_t reserved;
+  int32_t flags;         /* 0, or TSB200_KV_FRESH                                        */
   int64_t num_pages;
   uint8_t* k_pool;       /* 16-byte aligned                                              */
   uint8_t* v_pool;

@@ -96,6 +96,32 @@ def test_prefill_attention_fp32_route(cuda):
         assert torch.all((out[b] - ref).abs() <= 2e-4 * ref_abs + 1e-5 * ref.abs() + 1e-6)
 
 
+@pytest.mark.parametrize("fmt", ["fp32", "int8", "fp8"])
+def test_fp32_prompt_under_dependent_launch(cuda, fmt, monkeypatch):
+    """Lengths, block-table rows and scales of the one-token sequences are made by the launches right before the attention, which must
+    not look at them early: the call says so in the cache's flags (not where the caller made the sequences), and the result does not
+    depend on the setting."""
+    from transformer_surgeon_b200 import _lib
+    B, H, Hkv, d = 2, 4, 2, 128
+    ops, kv, g = setup(cuda, fmt, B, 90, H, Hkv, d, torch.float32, 5)
+    flags = []
+    attention = ops.paged_decode_attention
+    monkeypatch.setattr(ops, "paged_decode_attention", lambda c, *a, **k: (flags.append(c.desc().flags), attention(c, *a, **k))[1])
+    for T, L in ((33, 90), (90, 90), (5, 17), (64, 80)):
+        q = torch.randn((B, T, H, d), generator=g, device=cuda)
+        off = ops.prefill_attention(kv, q, L)
+        old = ops.set_pdl(True)
+        try:
+            on = ops.prefill_attention(kv, q, L)
+            torch.cuda.synchronize()
+        finally:
+            ops.set_pdl(old)
+        assert torch.equal(on, off)
+        assert torch.equal(ops.prefill_attention(kv, q, L, sequences=ops.query_sequences(kv, B, T, L)), off)
+    assert flags == [_lib.KV_FRESH, _lib.KV_FRESH, _lib.KV_FRESH if fmt == "fp8" else 0] * 4
+    assert kv.flags == 0
+
+
 def test_prefill_attention_strided_q_and_argument_errors(cuda):
     from transformer_surgeon_b200 import Tsb200Error
     B, T, L, H, Hkv, d = 1, 64, 64, 4, 2, 128

@@ -12,6 +12,7 @@ LIB_PATH = os.path.join(_HERE, "libtsb200.so")
 OK, ERR_ARG, ERR_UNSUPPORTED, ERR_CUDA, ERR_WORKSPACE, ERR_DEVICE, ERR_TIMEOUT = 0, -1, -2, -3, -4, -5, -6
 F32, BF16 = 0, 1
 KV_INT8, KV_FP8, KV_NVFP4, KV_F32, KV_BF16 = 0, 1, 2, 3, 4
+KV_FRESH = 1
 
 
 class Tsb200Error(RuntimeError):
@@ -28,7 +29,7 @@ class LinearDesc(C.Structure):
 
 
 class KVDesc(C.Structure):
-    _fields_ = [("format", C.c_int32), ("hkv", C.c_int32), ("head_dim", C.c_int32), ("reserved", C.c_int32),
+    _fields_ = [("format", C.c_int32), ("hkv", C.c_int32), ("head_dim", C.c_int32), ("flags", C.c_int32),
                 ("num_pages", C.c_int64), ("k_pool", C.c_void_p), ("v_pool", C.c_void_p),
                 ("block_table", C.c_void_p), ("bt_stride", C.c_int64), ("seq_lens", C.c_void_p),
                 ("k_scale", C.c_void_p), ("v_scale", C.c_void_p)]

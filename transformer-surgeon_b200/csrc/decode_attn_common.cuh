@@ -12,9 +12,8 @@ constexpr size_t kAttnCounterBytes = 16384;
 // The last int32 of the counter block is a status word: a kernel that gave up on a bounded wait for its own
 // copies records a non-zero code there (the result of that call is then not to be trusted).
 constexpr int kAttnStatusIndex = (int)(kAttnCounterBytes / sizeof(int)) - 1;
-struct AttnSplit {
-  int splits;
-};
+// Whether an attention may start while the launch before it drains: it looks up lengths, block table and scales ahead of its wait.
+inline bool attn_overlaps(const tsb200_kv_desc& kv) { return g_pdl != 0 && !(kv.flags & TSB200_KV_FRESH); }
 
 inline int choose_splits(int64_t B, int hkv, int64_t max_seq_len) {
   const int64_t base = B * hkv;

@@ -192,7 +192,7 @@ template <typename T, typename PT, int D, int W, int HC>
 int launch_cfg(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S, int64_t B, float* ws,
                int* counters, void* out, cudaStream_t st) {
   const dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((H / kv.hkv + HC - 1) / HC));
-  TSB_CUDA(launch_kernel(decode_attn_dense_kernel<T, PT, D, W, HC>, grid, dim3(W * 32), 0, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
+  TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_dense_kernel<T, PT, D, W, HC>, grid, dim3(W * 32), 0, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
                          counters ? S : -S, ws, counters, (T*)out));
   return counters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }

@@ -447,7 +447,7 @@ int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, 
     configured[dev] = true;
   }
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, 1);
-  TSB_CUDA(launch_kernel(decode_attn_fp8_kernel<T>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
+  TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_fp8_kernel<T>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
                          S, ws, counters, (T*)out, status));
   return TSB200_OK;
 }

@@ -426,7 +426,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   }
   const int g = H / kv.hkv;
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)(S < 0 ? -S : S), (unsigned)((g + 7) / 8));   // S < 0: partials only
-  TSB_CUDA(launch_kernel(decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
+  TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, counters, (T*)out));
   return TSB200_OK;
 }

@@ -389,6 +389,8 @@ def kv_record_bytes(fmt, head_dim):
 class PagedKV:
     """Pools + block table + lengths of ONE layer's quantized paged KV cache."""
 
+    flags = 0          # _lib.KV_FRESH: see the header
+
     def __init__(self, fmt, num_pages, hkv, head_dim, block_table, seq_lens, device, k_scale=None, v_scale=None):
         self.fmt = KV_FORMATS[fmt] if isinstance(fmt, str) else fmt
         self.hkv, self.head_dim, self.num_pages = hkv, head_dim, num_pages
@@ -423,7 +425,7 @@ class PagedKV:
     def desc(self, seq_lens=None):
         # rebuilt on every call: block_table / seq_lens tensors may have been swapped
         seq = self.seq_lens if seq_lens is None else seq_lens
-        return KVDesc(self.fmt, self.hkv, self.head_dim, 0, self.num_pages, self.k_pool.data_ptr(),
+        return KVDesc(self.fmt, self.hkv, self.head_dim, self.flags, self.num_pages, self.k_pool.data_ptr(),
                       self.v_pool.data_ptr(), self.block_table.data_ptr(), self.block_table.shape[1],
                       seq.data_ptr(), 0 if self.k_scale is None else self.k_scale.data_ptr(),
                       0 if self.v_scale is None else self.v_scale.data_ptr())
@@ -502,6 +504,8 @@ def prefill_attention(kv, q, L, sm_scale=None, out=None, status=None, seq_lens=N
         view = PagedKV.__new__(PagedKV)
         view.__dict__.update(kv.__dict__)
         view.block_table, view.seq_lens = table, lens
+        if sequences is None or kv.k_scale is not None:
+            view.flags = _lib.KV_FRESH       # tables or scales were made just now
         if kv.k_scale is not None:
             view.k_scale, view.v_scale = kv.k_scale.repeat_interleave(T, dim=0).contiguous(), kv.v_scale.repeat_interleave(T, dim=0).contiguous()
         qq = q.reshape(B * T, H, d) if q.is_contiguous() else q.contiguous().reshape(B * T, H, d)
