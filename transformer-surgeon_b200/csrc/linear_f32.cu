@@ -38,8 +38,8 @@ struct F32Params {
 // 12.9 us by words, 10.3 by halves, 7.5 by bytes).
 template <int BITS, int MT> struct Piece {
   static constexpr int kCnt = BITS == 32 ? 4 : (BITS == 1 && MT >= 4 ? 8 : 32 / BITS);
-  static constexpr int kPerWord = BITS == 32 ? 1 : 32 / BITS / kCnt;
-  static __device__ __forceinline__ int64_t at(int i) { return (int64_t)(i / kPerWord) * (BITS == 32 ? 16 : 4); }
+  static constexpr int kBytes = BITS == 32 ? 16 : kCnt * BITS / 8;
+  static constexpr int kWord = kBytes < 4 ? 4 : 1;              // pieces of less than a word: the word's address
 };
 // p: the 16 bytes or the word that piece i of a row lies in.
 template <int BITS, int CNT> __device__ __forceinline__ void load_piece(const uint8_t* p, int i, float (&v)[CNT]) {
@@ -90,7 +90,8 @@ template <int V> __device__ __forceinline__ float reduce_scatter(float (&v)[V]) 
 template <int BITS, int MT, int R, bool GATED>
 __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_constant__ F32Params p) {
   constexpr int MATS = GATED ? 2 : 1;
-  constexpr int CNT = Piece<BITS, MT>::kCnt;
+  using P = Piece<BITS, MT>;
+  constexpr int CNT = P::kCnt;
   constexpr int V = MATS * R * MT;
   constexpr int kKT = kXFloats / (MATS * MT);
   static_assert(V <= 32 && (V & (V - 1)) == 0, "one sum per lane");
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
     for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (i < pre_end) load_piece<BITS>(rows[mat][r] + Piece<BITS, MT>::at(i), i, pre[q][mat][r]);
+        if (i < pre_end) load_piece<BITS>(rows[mat][r] + (int64_t)(i / P::kWord * P::kWord) * P::kBytes, i, pre[q][mat][r]);
   }
   if (lane < MATS * R && ks == 0 && row0 < sg.n) {
     const uint8_t* q = rows[0][0];
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
     __syncthreads();
     // pieces of this warp: lane + 32 ks, then every 32 * ks_n; beyond the row's end the activations are zero, and no piece is read
     const int pieces = (kt + CNT - 1) / CNT;
-    const int64_t b0 = Piece<BITS, MT>::at(k0 / CNT);
+    const int64_t b0 = (int64_t)k0 * P::kBytes / CNT;
     auto use = [&](int i, const float (&w)[MATS][R][CNT]) {
 #pragma unroll
       for (int mat = 0; mat < MATS; ++mat)
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
 #pragma unroll
       for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
-        for (int r = 0; r < R; ++r) load_piece<BITS>(rows[mat][r] + b0 + Piece<BITS, MT>::at(i), i, w[mat][r]);
+        for (int r = 0; r < R; ++r) load_piece<BITS>(rows[mat][r] + b0 + (int64_t)(i / P::kWord * P::kWord) * P::kBytes, i, w[mat][r]);
       use(i, w);
     }
   }
