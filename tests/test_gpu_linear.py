@@ -324,6 +324,22 @@ def test_few_tokens_have_the_bits_of_more(cuda, p, K, N, r):
         assert torch.equal(lin(x[:m]), y[:m]), m
 
 
+@pytest.mark.parametrize("M", [1, 5, 16])
+@pytest.mark.parametrize("N", [1, 33, 100, 4099])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_few_tokens_with_a_bias_of_any_length_and_place(cuda, M, N, shift):
+    """A bias of odd length, or that starts within a 32-bit word: its first and last elements share their words with what is not bias."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(35)
+    buf = torch.randn(N + 2, generator=g, device=cuda).bfloat16()
+    f = ops.Factor.quantize((torch.randn((N, 512), generator=g, device=cuda) * 0.05).bfloat16(), 4)
+    x = torch.randn((M, 512), generator=g, device=cuda).bfloat16()
+    bias = buf[shift:shift + N]
+    y = ops.PackedLinear(f, None, bias, torch.bfloat16)(x)
+    plain = x.float() @ f.reconstruct(torch.float32).T + bias.float()
+    assert (y.float() - plain).abs().max() <= 2 ** -8 * plain.abs().max()
+
+
 @pytest.mark.parametrize("p", [4, 8, 2])
 @pytest.mark.parametrize("K,I,r", [(896, 7296, 0), (3584, 18944, 0), (4096, 14336, 1024), (512, 7168, 64)])
 def test_few_tokens_of_an_mlp_have_the_bits_of_more(cuda, p, K, I, r):

@@ -231,14 +231,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, NT == 1 && R == 1 ? 2 : 1) lin
     cp_commit();
   };
   // Scales and biases of the CTA's rows (constants): asynchronous copies that join the first step's group.  A bias is copied as
-  // the aligned word that holds it (copies are 4 bytes at least); the epilogue picks the half.
+  // the aligned word that holds it (copies are 4 bytes at least) where all of that word belongs to the bias; the epilogue picks the half.
   for (int i = tid; i < MATS * crows; i += threads) {
     const int lr = GATED && i >= crows ? i - crows : i;
     int tile = tile0 + lr / 16, sub = GATED && i >= crows ? 1 : 0;
     if (!GATED && tile >= p.tiles) { sub = 1; tile -= p.tiles; }
     const int n = min(tile * 16 + lr % 16, p.N - 1);
     cp_async4(smem_addr(consts + i), p.sub[sub].scale + n);
-    if (p.sub[sub].bias) cp_async4(smem_addr(consts + crows * MATS + i), reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(p.sub[sub].bias + n) & ~(uintptr_t)3));
+    if (const __nv_bfloat16* bias = p.sub[sub].bias) {
+      const uintptr_t at = reinterpret_cast<uintptr_t>(bias + n), word = at & ~(uintptr_t)3;
+      if (word >= reinterpret_cast<uintptr_t>(bias) && word + 4 <= reinterpret_cast<uintptr_t>(bias + p.N)) cp_async4(smem_addr(consts + crows * MATS + i), reinterpret_cast<const void*>(word));
+      else reinterpret_cast<unsigned*>(consts)[crows * MATS + i] = (unsigned)__bfloat16_as_ushort(bias[n]) << ((at & 2) ? 16 : 0);
+    }
   }
 #pragma unroll
   for (int u = 0; u < kRing; ++u) issue();
