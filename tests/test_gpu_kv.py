@@ -504,6 +504,21 @@ def test_unquantized_pages_of_many_sequences(cuda, fmt, H, Hkv, d):
     assert (out - ref).abs().max() <= C_P_SIMT * v.float().abs().max()
 
 
+def test_fp8_scales_of_flat_vectors(cuda):
+    """Contiguous prompts may come with a token's heads as one vector; what is neither that nor evenly strided is refused."""
+    rng = np.random.default_rng(43)
+    _, g = make_pair("fp8", 3, 1, 2, 64, cuda, rng)
+    k, v = (x.to(cuda) for x in outlier_kv(rng, 3, 7, 2, 64, torch.bfloat16))
+    g.set_fp8_scales(k, v)
+    ks, vs = g.k_scale.clone(), g.v_scale.clone()
+    g.fill_fp8_scales(1.0, 1.0)
+    g.set_fp8_scales(k.flatten(2), v.flatten(2))
+    assert torch.equal(g.k_scale, ks) and torch.equal(g.v_scale, vs)
+    for bad in (k.transpose(2, 3).contiguous().transpose(2, 3), k.cpu()):
+        with pytest.raises(ValueError):
+            g.set_fp8_scales(bad, v)
+
+
 def test_fp8_attention_after_append_under_dependent_launch(cuda):
     """One decode step's append -> attention pair with programmatic dependent launch on: the attention may fetch pages
     older than the newest token before the append has finished.  Lengths sit on, before and after page boundaries and

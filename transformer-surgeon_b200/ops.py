@@ -435,7 +435,7 @@ class PagedKV:
         lib = _lib.load()
         B, T = k.shape[:2]
         cos, sin = (None, None) if rope is None else rope
-        ks, vs = _token_strided(k, "k"), _token_strided(v, "v")
+        ks, vs = (0 if t.is_cuda and t.is_contiguous() else _token_strided(t, name) for t, name in ((k, "k"), (v, "v")))   # [B, T, hkv * d] too
         check(lib.tsb200_kv_fp8_scales_strided(_p(k), _p(v), _dt(k), ks, vs, B, T, self.hkv, self.head_dim, _p(pos0), _p(cos), _p(sin),
                                                0 if cos is None else cos.shape[0], _p(self.k_scale), _p(self.v_scale), _stream()),
               "tsb200_kv_fp8_scales_strided")
