@@ -152,8 +152,9 @@ int tsb200_linear(const tsb200_linear_desc* d, const void* x, void* y, int64_t M
 int tsb200_linear_simt(const tsb200_linear_desc* d, const void* x, void* y, int64_t M,
                        void* workspace, size_t workspace_bytes, void* stream);
 
-/* n layers that read the same x (q, k and v of a decoder layer): y[i] [M, out_i], equal to n calls of tsb200_linear in order.
- * fp32 layers with alike factors (same rank and containers; n <= 4) run as one launch per factor.  `d` and `y` are host
+/* n layers that read the same x (q, k and v of a decoder layer): y[i] [M, out_i], the bits of n calls of tsb200_linear in order.
+ * fp32 layers with alike factors (same rank and containers; n <= 4) run as one launch per factor; their K split, and with it the
+ * order of their sums, is chosen for all rows together, so they equal the single calls up to that order.  `d` and `y` are host
  * arrays.  The workspace follows the rules of tsb200_linear's. */
 size_t tsb200_linear_group_workspace_bytes(const tsb200_linear_desc* const* d, int n, int64_t M);
 int tsb200_linear_group(const tsb200_linear_desc* const* d, int n, const void* x, void* const* y, int64_t M,

@@ -135,7 +135,7 @@ def test_decode_sized_token_counts(cuda, p, M, K, N, r):
                                      (16, 40, 65, 8), (67, 264, 1000, 136), (130, 512, 4100, 0)])   # 64 x 64 tiles (dense), ragged in both directions
 def test_fp32_layers(cuda, p, M, K, N, r):
     """fp32 activations: every token group (1, 2, 4, 8 tokens), ragged rows, pieces that end inside a word of codes; a group of
-    layers equals the layers one by one."""
+    layers equals the layers one by one up to the order of summation."""
     from transformer_surgeon_b200 import ops
     x, U, V, b = _case(M, K, N, r, p, "fp32", seed=4)
     mk = (lambda w: ops.Factor.dense(w.to(cuda))) if p is None else (lambda w: ops.Factor.quantize(w.to(cuda), p))
@@ -148,6 +148,29 @@ def test_fp32_layers(cuda, p, M, K, N, r):
     ya, yb = ops.LinearGroup([lin, small])(x.to(cuda))
     torch.testing.assert_close(ya, y, rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(yb, small(x.to(cuda)), rtol=1e-5, atol=1e-5)
+
+
+def test_group_follows_its_layers(cuda):
+    """A group of layers marked for the CUDA-core kernel runs on it; a decoder layer's group has the layers it has now."""
+    from transformer_surgeon_b200 import ops
+    from transformer_surgeon_b200.decoder import LayerWeights
+    g = torch.Generator(device=cuda).manual_seed(36)
+    mk = lambda n: ops.PackedLinear(ops.Factor.dense(torch.randn((n, 512), generator=g, device=cuda)), None, None, torch.float32)
+    x = torch.randn((5, 512), generator=g, device=cuda)
+    q, k, v = mk(64), mk(32), mk(32)
+    L = LayerWeights(None, None, mk(64), mk(64), mk(64), mk(64), q=q, k=k, v=v)
+    first = L.qkv_group(x)
+    assert L.qkv_group is L.qkv_group
+    for l in (q, k, v):
+        l.force_simt = True
+    for y, l in zip(L.qkv_group(x), (q, k, v)):
+        assert torch.equal(y, l(x))
+    for l in (q, k, v):
+        l.force_simt = False
+    L.k = mk(32)
+    again = L.qkv_group(x)
+    assert torch.equal(again[0], first[0]) and not torch.equal(again[1], first[1])
+    torch.testing.assert_close(again[1], L.k(x), rtol=1e-5, atol=1e-4)
 
 
 def test_config2_shape_sweep(cuda):

@@ -48,7 +48,16 @@ class LayerWeights:
         self.ln1, self.ln2, self.o, self.gate, self.up, self.down = ln1, ln2, o, gate, up, down
         self.qkv, self.q, self.k, self.v = qkv, q, k, v
         self.mlp = ops.GatedMLP(gate, up, down)
-        self.qkv_group = None if qkv is not None else ops.LinearGroup([q, k, v])
+        self._group = None
+
+    @property
+    def qkv_group(self):
+        """q, k and v behind one call (None where they are packed as one layer)."""
+        if self.qkv is not None:
+            return None
+        if self._group is None or self._group.layers != [self.q, self.k, self.v]:      # a layer may have been replaced
+            self._group = ops.LinearGroup([self.q, self.k, self.v])
+        return self._group
 
 
 def fuse_rows(factors, biases, act_dtype):

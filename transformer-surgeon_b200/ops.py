@@ -329,7 +329,8 @@ class PackedLinear:
 
 
 class LinearGroup:
-    """PackedLinear layers that read the same x (q, k, v of a decoder layer) behind one call; equal to calling them in turn."""
+    """PackedLinear layers that read the same x (q, k, v of a decoder layer) behind one call: the bits of calling them in turn, for fp32
+    layers up to the order of summation."""
 
     def __init__(self, layers):
         self.layers = list(layers)
@@ -350,6 +351,10 @@ class LinearGroup:
             outs = [x.new_empty((*lead, l.out_features)) for l in self.layers]
         if ws is None:
             ws = workspace(x.device, self.workspace_bytes(M))
+        if any(l.force_simt for l in self.layers):
+            for l, o in zip(self.layers, outs):
+                l(x, out=o, ws=ws)
+            return outs
         ptrs = self._ptrs(*(o.data_ptr() for o in outs))
         check(_lib.load().tsb200_linear_group(self._descs, len(self.layers), x.data_ptr(), ptrs, M, ws.data_ptr(), ws.numel(), _stream()),
               "tsb200_linear_group")
