@@ -278,6 +278,33 @@ def test_gated_mlp_prompt(cuda, p, M, K, I, r):
     assert ops.PackedLinear.device_status(ws=ops.workspace(cuda, 1, "mlp")) == 0
 
 
+def test_every_gate_of_a_prompt(cuda):
+    """All finite bf16 gates through the block whose up outputs take SiLU(gate) along: the bits of the separate kernels."""
+    from transformer_surgeon_b200 import ops
+    bits = torch.arange(65536, dtype=torch.int32)
+    gates = bits[(bits & 0x7f80) != 0x7f80].to(torch.int16).view(torch.bfloat16).to(cuda)
+    g = torch.Generator(device=cuda).manual_seed(37)
+    x = torch.zeros((gates.numel(), 64), dtype=torch.bfloat16, device=cuda)
+    # up within +-1: a product beyond the type would be infinite, and infinity times the zeros of `down` NaN
+    x[:, 0], x[:, 1] = gates, torch.randn(gates.numel(), generator=g, device=cuda).clamp(-1, 1).bfloat16()
+
+    def copies(n, k, column):                                     # n outputs that are column `column` of the input (None: one each)
+        codes = torch.zeros((n, k), dtype=torch.int8, device=cuda)
+        codes[torch.arange(n), torch.arange(n) if column is None else column] = 1
+        return ops.PackedLinear(ops.Factor.from_codes(codes, torch.ones(n, device=cuda), 8), None, None, torch.bfloat16)
+
+    gate, up, down = copies(64, 64, 0), copies(64, 64, 1), copies(64, 64, None)
+    y = ops.GatedMLP(gate, up, down)(x)
+    assert torch.equal(gate(x)[:, 0], x[:, 0])
+    ref = down(ops.swiglu(gate(x), up(x)))
+    off = (y != ref).any(1)
+    assert not off.any(), (int(off.sum()), gates[off][:8], y[off][:8, 0], ref[off][:8, 0])
+    want = torch.nn.functional.silu(gates.double()).bfloat16().double()
+    got = ops.swiglu(gates[:, None].expand(-1, 8).contiguous(), torch.ones((gates.numel(), 8), dtype=torch.bfloat16, device=cuda))[:, 0].double()
+    assert got.isfinite().all()
+    assert ((got - want).abs() <= 2 ** -7 * want.abs() + 2e-36).all()      # one rounding apart at most; exp(-gate) overflows fp32 below -88.7
+
+
 @pytest.mark.parametrize("p", [8, 4, 2, "binary"])
 @pytest.mark.parametrize("M,K,N", [(129, 128, 40000), (256, 64, 19072), (600, 192, 12928), (1000, 320, 9004), (4100, 256, 2560), (777, 1280, 6150),
                                    (300, 1024, 3600), (250, 1024, 4104), (131, 2048, 2200), (1000, 1024, 640)])
