@@ -370,9 +370,9 @@ __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&o
 //   * V, stored token-minor, is transposed four bytes at a time in registers and leaves through a swizzled tile of shared memory as
 //     16-byte rows, 512 contiguous bytes per warp.
 // Pages that the range covers in part keep their other slots: those go out token by token.  A task is K or V of one head: both at once
-// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions bound it, about 26 an element (an instruction
-// more per element is 3.7 us): 32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB: 94 us, 242 us with one warp per token vector and a
-// byte-wise transpose.
+// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions and their latencies bound it: 14 an element, the
+// issue slots 58 % busy with the 22 warps that 80 registers a thread leave an SM, memory at 47 %; a further instruction an element costs 2
+// to 4 us.  32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB: 94 us, 242 us with one warp per token vector and a byte-wise transpose.
 template <typename T, int D, int FMT>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 1)
 kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,

@@ -252,7 +252,7 @@ __device__ __forceinline__ void umma_bf16_ts(unsigned d_tmem, unsigned a_tmem, u
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Rendezvous of the 8 dequant/epilogue warps on an mbarrier (count 8) with a bounded wait, so a
+// Rendezvous of the dequant/epilogue warps (QLayout::kDqWarps) on an mbarrier with a bounded wait, so a
 // warp that gave up elsewhere can never leave the others blocked.
 __device__ __forceinline__ bool warps_rendezvous(unsigned long long* bar, int& uses, int lane, volatile int* abort_flag) {
   __syncwarp();
@@ -353,7 +353,8 @@ __device__ __forceinline__ uint4 gate_eight(uint4 gv, uint4 uv) {
 template <int TN, int BITS>
 // 128 registers (not the 168 a 384-thread CTA could have): the CTA of a launch then fits beside the CTAs of the small
 // kernel before it, so its set-up and first weight copies run under programmatic dependent launch while that kernel
-// still executes.  With 168 registers the decode step was 4 % slower although this kernel alone was faster.
+// still executes.  With 168 registers the decode step was 4 % slower although this kernel alone was faster.  (256-token tile: 96 for its
+// 640 threads; 88 bytes a thread spill, 8 with 8-bit codes.)
 __global__ void __maxnreg__((QLayout<TN, BITS>::kMaxRegs))
 linear_tcq_kernel(const __grid_constant__ Program prog) {
   using L = QLayout<TN, BITS>;
@@ -365,12 +366,12 @@ linear_tcq_kernel(const __grid_constant__ Program prog) {
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(r_ring + NR * L::kStage);
   unsigned long long* w_full = bars;                        // [NR] weight box landed (the dequant warps wait on it)
   unsigned long long* x_full = bars + NR;                   // [NR] stage ready for the MMA lanes: activation tiles landed
-                                                            //      (one arrival + bytes) AND the 8 dequant warps stored
+                                                            //      (one arrival + bytes) AND the 8 warps of the stage stored
                                                             //      its A operand - one wait per stage for the issuers
   unsigned long long* stage_done = bars + 2 * NR;           // [NR] MMA commit: the stage's MMAs are complete, so its
                                                             //      weight box, activation tiles and A buffer are free
   unsigned long long* acc_full = bars + 3 * NR;             // [1]  MMA commit: accumulator(s) of the item complete
-  unsigned long long* ep_bar = acc_full + 1;                // [1]  rendezvous of the 8 warps
+  unsigned long long* ep_bar = acc_full + 1;                // [1]  rendezvous of the dequant warps
   unsigned long long* acc_free = ep_bar + 1;                // [2]  256-token tile: a token half's accumulator has been read
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);

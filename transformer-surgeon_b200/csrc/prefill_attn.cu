@@ -19,7 +19,8 @@
 //               exact), exp2, row sum in fp32, P rounded to bf16 into shared memory in the swizzled K-major layout
 //               the MMA descriptor expects; at the end O / l, rounded, while the next pair's scores are computed
 // Bounds at 128 x 128 scores of a tile: 1024 cycles of the tensor pipe, 1024 of the exponential unit, ~1500 of shared memory.
-// 8 x 2048 tokens, 32 / 8 heads of 128: 383 us (570 with one query tile per CTA, 4300 cycles a tile).
+// 8 x 2048 tokens, 32 / 8 heads of 128: 383 us (570 with one query tile per CTA, 4300 cycles a tile).  The softmax warps hold a row of 128
+// scores: 168 registers a thread are all that 352 threads can have, and 128 bytes (head dimension 64: 108) spill.
 // Every mbarrier wait is bounded; on expiry the CTA records a code in the status word, frees its TMEM and returns.
 #include "tc_common.cuh"
 #include "decode_attn_common.cuh"

@@ -163,7 +163,8 @@ __global__ void dequantize_kernel(const uint8_t* __restrict__ packed, const floa
 // whole row shares comes from its correctly rounded reciprocal y: q = w y, r = w - d q (exact), q + r y - correctly rounded by
 // Markstein's theorem (Computation of elementary functions on the IBM RISC System/6000 processor, 1990) as long as nothing leaves
 // the normal range, which the divisor's range guarantees for every quotient that does not round to zero; other divisors divide.
-// Together with its packing launch the two-pass form took 177 us on that matrix; this one takes 36 us.  The row stays in the weights'
+// Together with its packing launch the two-pass form took 177 us on that matrix; this one takes 37 us (14 instructions a
+// column, the issue slots 73 % busy, memory 42 %).  The row stays in the weights'
 // own type (as floats: 88 registers a thread, too few warps in flight, 108 us), and bf16 codes of up to four bits are rounded and
 // clamped in pairs.
 //
