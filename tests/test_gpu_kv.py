@@ -558,3 +558,32 @@ def test_fp8_attention_after_append_under_dependent_launch(cuda):
     ref, ref_abs = oatt.paged_decode_attention(o, q.float().cpu().numpy(), with_abs=True)
     tol = attn_tol(ref, ref_abs, "bf16", False)
     assert np.all(np.abs(outs[1].float().cpu().numpy() - ref) <= tol)
+
+
+@pytest.mark.parametrize("fmt,H,Hkv,d", [("int8", 16, 8, 128), ("int8", 28, 4, 64), ("nvfp4", 28, 4, 128), ("nvfp4", 16, 8, 64), ("fp8", 28, 4, 128), ("fp8", 16, 8, 64),
+                                          ("fp8", 32, 8, 128)])
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+@pytest.mark.parametrize("B", [304, 40])
+def test_decode_attention_of_every_length(cuda, fmt, H, Hkv, d, B, name):
+    """Every length from 0 to 303: pairs of pages to a warp's round, a single one at the end, warps without pages, splits too short for pairs; many
+    sequences (one split, more CTAs than the GPU holds at a time) and few (several), against the one-lane-per-element kernel.  The bound is attn_tol's: keys without outlier channels
+    and V's magnitudes through the same weights."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(51)
+    pages = 19
+    bt = torch.randperm(B * pages, generator=g, device=cuda).to(torch.int32).reshape(B, pages)
+    k, v = (torch.randn((B, pages * 16, Hkv, d), generator=g, device=cuda).to(DT[name]) for _ in range(2))
+    q = torch.randn((B, H, d), generator=g, device=cuda).to(DT[name])
+    lens = (torch.arange(B, device=cuda) * (304 // B) + (0 if B == 304 else 3)).to(torch.int32)
+    refs = []
+    for vals in (v.abs(), v):
+        kv = ops.PagedKV(fmt, B * pages, Hkv, d, bt, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+        if fmt == "fp8":
+            kv.fill_fp8_scales(6.0 / 448, 6.0 / 448)
+        kv.append(k, vals)
+        kv.seq_lens = lens
+        refs.append(ops.paged_decode_attention(kv, q, pages * 16, simt=True).float())
+    out = ops.paged_decode_attention(kv, q, pages * 16)
+    assert torch.equal(out, ops.paged_decode_attention(kv, q, pages * 16))
+    assert torch.all(out[lens == 0] == 0)
+    assert torch.all((out.float() - refs[1]).abs() <= C_P_TC * refs[0] + 2 * C_OUT[name] * refs[1].abs() + 1e-6)

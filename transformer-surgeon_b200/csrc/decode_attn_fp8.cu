@@ -40,7 +40,8 @@ constexpr int D = 128;
 constexpr int REC = 16 * D;                 // bytes of one K or V record
 constexpr int STAGE = 4 * REC;              // K_A, V_A, K_B, V_B
 constexpr int PBUF = 2 * 4 * 16 * 4;        // softmax weights of a stage: [page][head][token] words
-constexpr int WARP_SMEM = kStages * STAGE + PBUF + 64;
+constexpr int WARP_SMEM = kStages * STAGE + PBUF;
+constexpr int QEXP = 4 * D * 4 + 64;        // expanded query and its magnitudes
 constexpr unsigned kWaitLimit = 1u << 22;
 
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
@@ -93,7 +94,9 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
 
   uint8_t* ring = smem + (size_t)w * WARP_SMEM;
   unsigned* pbuf = reinterpret_cast<unsigned*>(ring + kStages * STAGE);
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(ring + kStages * STAGE + PBUF);
+  // Behind everything else, not with the warp's ring: the merge at the end writes over the rings, and the words of an mbarrier may not be
+  // reused (they lay there once: with more CTAs than an SM holds at a time, some of their sums were overwritten).
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + (size_t)kWarps * WARP_SMEM + QEXP) + w * kStages;
   if (lane == 0) {
     for (int i = 0; i < kStages; ++i) mbar_init(&bars[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -435,9 +438,9 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
 template <typename T>
 int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
                     int64_t B, float* ws, int* counters, void* out, int* status, cudaStream_t st) {
-  constexpr size_t pipe = (size_t)kWarps * WARP_SMEM + 4 * D * 4 + 64;   // rings + expanded q
-  constexpr size_t merge = (size_t)(kWarps * 16 + kWarps * 8 * D) * sizeof(float);
-  constexpr size_t smem = pipe > merge ? pipe : merge;
+  constexpr size_t pipe = (size_t)kWarps * WARP_SMEM + QEXP + kWarps * kStages * 8;   // rings, expanded q, barriers
+  static_assert((kWarps * 16 + kWarps * 8 * D) * sizeof(float) <= (size_t)kWarps * WARP_SMEM, "the merge stays clear of the barriers");
+  constexpr size_t smem = pipe;
   static bool configured[64] = {false};
   int dev = 0;
   TSB_CUDA(cudaGetDevice(&dev));
