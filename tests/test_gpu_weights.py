@@ -102,3 +102,18 @@ def test_bad_arguments_are_rejected(cuda):
         ops.quantize_weight(w.cpu(), 8)
     with pytest.raises(Tsb200Error):
         ops.pack_codes(torch.zeros((4, 64), dtype=torch.int8, device=cuda), 3)
+
+
+@pytest.mark.parametrize("p", [8, 4, 3, 2])
+def test_quotients_of_all_bf16_significands(cuda, p):
+    """bf16 weights of every significand over row maxima of every significand: the one-pass kernel's quotients (a product with the
+    reciprocal) round to the codes that dividing gives."""
+    from transformer_surgeon_b200 import ops
+    sig = torch.arange(128, 256, dtype=torch.float32)
+    cols = torch.cat([sig * 2.0 ** -e * s for e in range(1, 9) for s in (1, -1)])           # below the row's maximum
+    w = torch.cat([cols.expand(128, -1), (sig * 1.0)[:, None]], dim=1) * 2.0 ** -7
+    w = (w * 2.0 ** torch.arange(-3, 5).repeat(16)[:, None]).bfloat16().contiguous()
+    for eps in (0.0, 1e-6):
+        codes, scales = ops.quantize_weight(w.to(cuda), p, "per_channel", eps)
+        f = ops.Factor.quantize(w.to(cuda), p, "per_channel", eps)
+        assert torch.equal(f.codes(), codes) and torch.equal(f.scales, scales)

@@ -160,13 +160,15 @@ __global__ void dequantize_kernel(const uint8_t* __restrict__ packed, const floa
 // Bound by the weights' one trip from memory (a 14336 x 4096 bf16 matrix: 147 MB, 22 us) and, next to it, by the arithmetic: the
 // quotient that vanilla.py prescribes is an IEEE division per element.  TPR threads own a row and keep it in registers between the
 // statistic and the codes (IT units of 8 columns each), the codes never exist as bytes, and the quotient by a divisor that the
-// whole row shares comes from its correctly rounded reciprocal y: q = w y, r = w - d q (exact), q + r y - correctly rounded by
+// whole row shares comes from its correctly rounded reciprocal y: for bf16 weights the product w y (unit_quotients), for fp32 ones
+// q = w y, r = w - d q (exact), q + r y - correctly rounded by
 // Markstein's theorem (Computation of elementary functions on the IBM RISC System/6000 processor, 1990) as long as nothing leaves
 // the normal range, which the divisor's range guarantees for every quotient that does not round to zero; other divisors divide.
-// Together with its packing launch the two-pass form took 177 us on that matrix; this one takes 37 us (14 instructions a
-// column, the issue slots 73 % busy, memory 42 %).  The row stays in the weights'
-// own type (as floats: 88 registers a thread, too few warps in flight, 108 us), and bf16 codes of up to four bits are rounded and
-// clamped in pairs.
+// Together with its packing launch the two-pass form took 177 us on that matrix; this one takes 33 us (36.9 with a correction of the
+// quotients and codes placed one by one instead of in pairs).  The row stays in the weights'
+// own type (as floats: 88 registers a thread, too few warps in flight, 108 us), and bf16 codes of up to four bits are rounded,
+// clamped and placed in pairs.  CTAs that walk their rows and fetch the next one under the codes of this one were no faster (37.5 us: their warps
+// keep step, and loads and arithmetic overlap less than those of independent CTAs do); 128 threads a row: 34.8, 256: 40.9.
 //
 // Eight columns in the weights' own type (bf16: as four packed pairs).
 template <typename T> struct Unit;
@@ -211,10 +213,10 @@ template <> struct Unit<float> {
   }
 };
 
-// The unit's codes in the low BITS bits of q[0..7] (the other bits are anything).  y: correctly rounded 1 / denom.
-template <typename T, int BITS, bool DIVIDE>
-__device__ __forceinline__ void unit_codes(const Unit<T>& v, float denom, float y, float qmax, unsigned (&q)[8]) {
-  float p[8];
+// The unit's quotients.  y: correctly rounded 1 / denom.  bf16: the quotient is rounded to bf16 next, whose midpoints no quotient of two
+// 8-bit numbers hits (9 significant bits times the divisor's are more than 8) or comes closer to than 2^-17, so that the product,
+// within 2^-23, rounds alike; fp32: corrected twice.
+template <typename T, bool DIVIDE> __device__ __forceinline__ void unit_quotients(const Unit<T>& v, float denom, float y, float (&p)[8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float x = v.at(j);
@@ -222,26 +224,34 @@ __device__ __forceinline__ void unit_codes(const Unit<T>& v, float denom, float 
       p[j] = __fdiv_rn(x, denom);
     } else {
       p[j] = x * y;
-      p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);                        // bf16: enough (exact where the quotient is; no other quotient of
-      if (sizeof(T) == 4) p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);    // two 8-bit numbers is within 2^-17 of a rounding boundary)
+      if (sizeof(T) == 4) {
+        p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);
+        p[j] = fmaf(fmaf(-p[j], denom, x), y, p[j]);
+      }
     }
   }
-  if constexpr (sizeof(T) == 2 && BITS < 8) {
-    // packed: round to bf16, clamp, and add 192: bf16 numbers of [128, 256) are whole, so the sum is rounded half-to-even to a whole
-    // number that stands in its low bits (|code| <= 7)
-    const __nv_bfloat162 hi = __float2bfloat162_rn(qmax), lo = __float2bfloat162_rn(-qmax), magic = __float2bfloat162_rn(192.f);
+}
+// The unit's codes in the low BITS bits of q[0..7] (the other bits are anything).
+template <typename T, bool DIVIDE> __device__ __forceinline__ void unit_codes(const Unit<T>& v, float denom, float y, float qmax, unsigned (&q)[8]) {
+  float p[8];
+  unit_quotients<T, DIVIDE>(v, denom, y, p);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __nv_bfloat162 h = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
-      h = __hadd2_rn(__hmin2(__hmax2(h, lo), hi), magic);
-      const unsigned b = *reinterpret_cast<unsigned*>(&h);
-      q[2 * i] = b;
-      q[2 * i + 1] = b >> 16;
-    }
-  } else {
+  for (int j = 0; j < 8; ++j)       // the bounds are whole numbers: clamping before or after rounding is the same; 1.5 * 2^23: half-to-even
+    q[j] = __float_as_uint(fminf(fmaxf(rnd<T>(p[j]), -qmax), qmax) + 12582912.0f);
+}
+// bf16 weights, codes of up to four bits: the codes of columns 2 i and 2 i + 1 in the low bits of the halves of h[i] (the other bits are
+// anything).  Rounded to bf16, clamped and added to 192 in pairs: bf16 numbers of [128, 256) are whole, so the sum is rounded
+// half-to-even to a whole number that stands in its low bits (|code| <= 7).
+template <bool DIVIDE>
+__device__ __forceinline__ void unit_code_pairs(const Unit<__nv_bfloat16>& v, float denom, float y, float qmax, unsigned (&h)[4]) {
+  float p[8];
+  unit_quotients<__nv_bfloat16, DIVIDE>(v, denom, y, p);
+  const __nv_bfloat162 hi = __float2bfloat162_rn(qmax), lo = __float2bfloat162_rn(-qmax), magic = __float2bfloat162_rn(192.f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j)     // the bounds are whole numbers: clamping before or after rounding is the same; 1.5 * 2^23: half-to-even
-      q[j] = __float_as_uint(fminf(fmaxf(rnd<T>(p[j]), -qmax), qmax) + 12582912.0f);
+  for (int i = 0; i < 4; ++i) {
+    __nv_bfloat162 r = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+    r = __hadd2_rn(__hmin2(__hmax2(r, lo), hi), magic);
+    h[i] = *reinterpret_cast<const unsigned*>(&r);
   }
 }
 
@@ -281,6 +291,15 @@ template <int BITS> __device__ __forceinline__ unsigned place(const unsigned (&q
 #pragma unroll
   for (int i = 0; i < 4; ++i) w |= ((q[2 * i] & mask) << (BITS * i)) | ((q[2 * i + 1] & mask) << (BITS * (i + per / 2)));
   return BITS == 4 ? w : w << (BITS * f0);
+}
+
+// The same from pairs: the container word interleaves its columns in pairs too, field i and field i + per / 2, 16 bits apart.
+template <int BITS> __device__ __forceinline__ unsigned place_pairs(const unsigned (&h)[4], int64_t c) {
+  constexpr unsigned mask = ((1u << BITS) - 1u) * 0x10001u;
+  unsigned w = h[0] & mask;
+#pragma unroll
+  for (int i = 1; i < 4; ++i) w |= (h[i] << (BITS * i)) & (mask << (BITS * i));
+  return BITS == 4 ? w : w << (BITS * ((int)(c % (32 / BITS)) >> 1));
 }
 
 template <typename T, int TPR, int IT, int BITS>
@@ -339,6 +358,17 @@ quantize_pack_kernel(const T* __restrict__ w, int64_t rows, int64_t cols, int pr
 #pragma unroll
   for (int i = 0; i < IT; ++i) {
     const int64_t u = t + (int64_t)i * TPR;
+    if constexpr (sizeof(T) == 2 && BITS > 1 && BITS < 8) {
+      if (precision != 0) {
+        unsigned h[4];
+        if (divide) unit_code_pairs<true>(v[i], denom, y, qmax, h);
+        else unit_code_pairs<false>(v[i], denom, y, qmax, h);
+        unsigned word = u < units ? place_pairs<BITS>(h, u * 8) : 0u;
+        if (BITS == 2) word |= __shfl_xor_sync(0xffffffffu, word, 1);      // a word is two units
+        if (u < units && u % (4 / BITS) == 0) *reinterpret_cast<unsigned*>(out + u * BITS) = word;
+        continue;
+      }
+    }
     unsigned q[8];
     if (precision == 0) {
 #pragma unroll
@@ -349,9 +379,9 @@ quantize_pack_kernel(const T* __restrict__ w, int64_t rows, int64_t cols, int pr
         q[j] = BITS == 1 ? (unsigned)(sgn > 0) : (unsigned)sgn;
       }
     } else if (divide) {
-      unit_codes<T, BITS, true>(v[i], denom, y, qmax, q);
+      unit_codes<T, true>(v[i], denom, y, qmax, q);
     } else {
-      unit_codes<T, BITS, false>(v[i], denom, y, qmax, q);
+      unit_codes<T, false>(v[i], denom, y, qmax, q);
     }
     if constexpr (BITS == 8) {
       if (u < units) {
