@@ -6,7 +6,7 @@
 namespace tsb {
 
 // Workspace: kAttnCounterBytes of int32 counters (zero between calls; one per (sequence, kv head,
-// head chunk), used by the tensor-core kernel to let the last split merge the partials), then
+// head chunk), used by the kernel of unquantized pages to let the last split merge the partials), then
 // float [B][H][S][2 + d]  ->  m, l, acc[d] per (sequence, q head, split).
 constexpr size_t kAttnCounterBytes = 16384;
 // The last int32 of the counter block is a status word: a kernel that gave up on a bounded wait for its own
@@ -55,7 +55,8 @@ inline int choose_splits_fp8(int64_t B, int hkv, int64_t max_seq_len) {
   return (int)s;
 }
 
-// Whether the last CTA of a (sequence, kv head, head chunk) merges its splits.  That takes ~80 cycles per (head, split) row - 35 k
+// Whether the last CTA of a (sequence, kv head, head chunk) of unquantized pages merges its splits (the quantized formats always launch the
+// reduction).  That takes ~80 cycles per (head, split) row - 35 k
 // cycles, 20 us, at 7 heads and 63 splits -, a reduction launch that is resident before the partials are complete ~3 us whatever the
 // shape: the launch from 64 rows on.
 inline bool last_cta_merges(int splits, int H, int hkv) { return splits == 1 || splits * (H / hkv < 8 ? H / hkv : 8) < 64; }

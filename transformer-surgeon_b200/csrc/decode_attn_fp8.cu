@@ -83,7 +83,7 @@ __device__ __forceinline__ void split3x2(float x0, float x1, unsigned& w0, unsig
 template <typename T>
 __global__ void __launch_bounds__(kWarps * 32)
 decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
-                       float* __restrict__ ws, int* __restrict__ counters, T* __restrict__ out, int* __restrict__ status) {
+                       float* __restrict__ ws, T* __restrict__ out, int* __restrict__ status) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -366,7 +366,6 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
     }
   __syncthreads();
   const float oscale = vscale * (1.0f / 256.0f);
-  const bool fuse_reduce = counters != nullptr;
   for (int idx = threadIdx.x; idx < g * D; idx += blockDim.x) {
     const int i = idx / D, e = idx % D;
     float mm = -INFINITY;
@@ -381,7 +380,7 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       a += sm_acc[((size_t)ww * 8 + i) * D + e] * c;
     }
     const int64_t bh = (int64_t)b * H + hk * g + i;
-    if (S == 1 && fuse_reduce) {
+    if (S == 1) {
       out[bh * D + e] = from_f32<T>(ll > 0.f ? a * oscale / ll : 0.f);
     } else {
       float* o = ws + (bh * S + s) * (2 + D);
@@ -389,27 +388,15 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       o[2 + e] = a * oscale;
     }
   }
-  if (S == 1 || !fuse_reduce) return;
-  __shared__ int s_last;
-  __threadfence();
-  __syncthreads();
-  int* ctr = counters + blockIdx.x;
-  if (threadIdx.x == 0) s_last = (atomicAdd(ctr, 1) == S - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const int64_t bh0 = (int64_t)b * H + hk * g;
-  merge_splits<T, D>(ws + bh0 * S * (2 + D), g, S, reinterpret_cast<float*>(smem), out + bh0 * D);
-  if (threadIdx.x == 0) *ctr = 0;
 }
 
 }  // namespace
 
 // FP8 pages, head_dim 128, group <= 4: returns TSB200_ERR_UNSUPPORTED otherwise (the caller then
-// uses the f16 tensor-core kernel).  `counters` may be null: partials only, a reducer launch follows.
+// uses the f16 tensor-core kernel).  With several splits the partials are left to a reduction launch.
 template <typename T>
 int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
-                    int64_t B, float* ws, int* counters, void* out, int* status, cudaStream_t st) {
+                    int64_t B, float* ws, void* out, int* status, cudaStream_t st) {
   constexpr size_t pipe = (size_t)kWarps * WARP_SMEM + QEXP + kWarps * kStages * 8;   // rings, expanded q, barriers
   static_assert((kWarps * 16 + kWarps * 8 * D) * sizeof(float) <= (size_t)kWarps * WARP_SMEM, "the merge stays clear of the barriers");
   constexpr size_t smem = pipe;
@@ -423,12 +410,11 @@ int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, 
   }
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, 1);
   TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_fp8_kernel<T>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
-                         S, ws, counters, (T*)out, status));
+                         S, ws, (T*)out, status));
   return TSB200_OK;
 }
-template int launch_attn_fp8<float>(const tsb200_kv_desc&, const void*, int64_t, int, float, int64_t, int, int64_t, float*, int*,
-                                    void*, int*, cudaStream_t);
-template int launch_attn_fp8<__nv_bfloat16>(const tsb200_kv_desc&, const void*, int64_t, int, float, int64_t, int, int64_t, float*,
-                                            int*, void*, int*, cudaStream_t);
+template int launch_attn_fp8<float>(const tsb200_kv_desc&, const void*, int64_t, int, float, int64_t, int, int64_t, float*, void*, int*,
+                                    cudaStream_t);
+template int launch_attn_fp8<__nv_bfloat16>(const tsb200_kv_desc&, const void*, int64_t, int, float, int64_t, int, int64_t, float*, void*, int*, cudaStream_t);
 
 }  // namespace tsb

@@ -3,8 +3,8 @@
 // Replaces transformersurgeon/blocks/mha.py:9-103 (attention(): GQA, softmax, @V) for the
 // decode step.  One CTA = one (sequence, kv head, split); its warps (4, or 6 for int8 pages) take pages
 // round-robin.  Each warp streams its pages through a private ring of shared-memory
-// stages with 16-byte cp.async copies (K record placed with an XOR swizzle so the
-// fragment reads are bank-conflict free), and computes, per 16-token page,
+// stages (two lanes, one cp.async.bulk per record, on an mbarrier; a page's number is looked up a
+// page before its copy leaves), and computes, per 16-token page,
 //     S^T[token, head] = K_page . Q^T          (8 x mma.m16n8k16, f16 in / f32 acc)
 //     online softmax over tokens per head       (warp shuffles over the token lanes)
 //     O^T[dim, head]  += V^T_page . P^T         (8 x mma.m16n8k16)
@@ -13,7 +13,14 @@
 // an e2m1 code times its e4m3 block scale is exact in f16 (2 x 4 significant bits), so K goes to
 // the MMA as code * scale; for V the block scale of a token is folded into that token's softmax
 // weight (one product per 16-dim block and token instead of one per element).
-// Partials (m, l, acc) go to the workspace; the last CTA of a (sequence, kv head) or decode_attn_reduce_kernel merges them.
+// Several splits leave partials (m, l, acc) in the workspace for decode_attn_reduce_kernel: that launch is resident before the last
+// partial is there, and 3-5 us faster than a merge by the last CTA of a pair, whatever the number of splits (int8, 2 sequences x 32 / 8
+// heads x 500 tokens 8.2 -> 5.5 us, NVFP4, 1 x 32 / 8 x 1000 9.6 -> 6.2).
+//
+// Bound by the page loop's instructions.  Against copies by all 32 lanes (cp.async, 4 to 9 a lane and page), block scales widened by every
+// lane and a rescale of the accumulators on every page, half to all of the stated tokens: int8, 64 x 8 kv heads x 4096 95.1 -> 89.6 us, 16 x 4 x
+// 8192 35.7 -> 33.6; NVFP4, 64 x 8 x 4096 96.9 -> 90.8, 30 x 4 x 3000 31.3 -> 26.6, 8 x 4 x 32768 58.8 -> 57.3.
+#include "tc_common.cuh"
 #include "decode_attn_common.cuh"
 
 namespace tsb {
@@ -21,7 +28,7 @@ namespace tsb {
 template <typename T, int D> int launch_reduce(const float* ws, int64_t BH, int S, void* out, cudaStream_t st);
 template <typename T>
 int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
-                    int64_t B, float* ws, int* counters, void* out, int* status, cudaStream_t st);
+                    int64_t B, float* ws, void* out, int* status, cudaStream_t st);
 int validate_attn_args(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, int64_t B, int H,
                        int64_t max_seq_len, void* workspace, size_t workspace_bytes, bool& noop, size_t need_bytes);
 int attn_dense(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, int64_t qs, int64_t B, int H, float sm_scale,
@@ -29,19 +36,32 @@ int attn_dense(const tsb200_kv_desc* kv, const void* q, void* out, int dtype, in
 
 namespace {
 
-// Warps per CTA and ring stages per warp, by page format (measured at batch 32-64, context 2k-4k): int8 pages
-// run 8 % faster with 6 warps x 3 stages (two CTAs = 12 warps per SM); NVFP4 and FP8 keep 4 x 4 (three CTAs).
-template <int FMT> struct AttnCfg {
+using tc::mbar_expect_tx;
+using tc::mbar_init;
+using tc::mbar_try_wait;
+using tc::smem_u32;
+
+constexpr unsigned kWaitLimit = 1u << 22;
+// Warps per CTA, ring stages (pages) per warp, CTAs per SM that registers are to allow.  What counts is how many CTAs an SM holds: the page
+// loop is bound by the instructions that widen codes and by the chain of a page's softmax, and the warps of other CTAs fill its gaps.  int8,
+// head_dim 64: 30 sequences x 2 kv heads x 1.5k-3k tokens 12.4 us at 5 CTAs, 13.5 at 4; head_dim 128 is limited by registers (3).  NVFP4, 128:
+// 5 CTAs of 3 stages against 4 of 4: 16 x 4 x 1k-2k tokens 14.2 us to 15.1, 16 x 8 x 1k-2k 19.2 to 21.4; 8 x 4 x 16k-32k 57.3 to 54.0.
+template <int FMT, int D> struct AttnCfg {
   static constexpr int kWarps = FMT == TSB200_KV_INT8 ? 6 : 4;
-  static constexpr int kStages = FMT == TSB200_KV_INT8 ? 3 : 4;
+  static constexpr int kStages = FMT == TSB200_KV_INT8 && D == 128 ? 2 : 3;
+  static constexpr int kCtas = FMT == TSB200_KV_INT8 ? (D == 128 ? 3 : 5) : (FMT == TSB200_KV_NVFP4 && D == 128 ? 5 : 4);
 };
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float ex2(float x) {                       // (weights below 2^-126 are 0)
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+  return y;
+}
 
 __device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
   asm volatile(
@@ -87,25 +107,13 @@ template <int FMT> __device__ __forceinline__ unsigned widen2_k(unsigned w16) {
   return (FMT == TSB200_KV_FP8 && TSB_ATTN_ALU_WIDEN) ? widen2_e4m3_alu(w16) : widen2<FMT>(w16);
 }
 
-// Row swizzle of the K record (rows of 128 bytes = 8 chunks): adjacent token rows land in
-// different halves of the bank space, rows two apart in different chunks.
-__device__ __forceinline__ int kswz(int row) { return ((row & 1) << 2) | ((row >> 1) & 3); }
-
-template <int D> __device__ __forceinline__ int k_phys_chunk(int row, int j) {
-  return row * (D / 16) + (D == 128 ? (j ^ kswz(row)) : j);
-}
-// NVFP4 K rows are D/2 bytes (D/32 chunks): rows four apart would meet in the same banks, so the
-// 32-byte half of the row is flipped for every other group of four rows.
-template <int D> __device__ __forceinline__ int k4_phys_chunk(int row, int j) {
-  return row * (D / 32) + (D == 128 ? (j ^ (((row >> 2) & 1) << 1)) : j);
-}
 // e2m1 codes n_A and n_{A+4} of the 8 in a 32-bit word (16 bits apart, so one shift serves both) ->
 // f16x2 holding value * 2^-14, with integer instructions only: the sign goes to bit 15 and the
 // three magnitude bits (2 exponent, 1 mantissa; bias 1 against f16's 15) to f16 bits 11..9; code
 // 0.5 lands on an f16 subnormal, also exactly.  The conversion instructions are far slower.
 template <int A> __device__ __forceinline__ unsigned e2m1_pair_alu(unsigned w) {
-  const unsigned x = w << (12 - 4 * A);
-  return (x & 0x80008000u) | ((x >> 3) & 0x0E000E00u);
+  const unsigned m = A < 3 ? w << (9 - 4 * (A < 3 ? A : 0)) : w >> 3;
+  return ((w << (12 - 4 * A)) & 0x80008000u) | (m & 0x0E000E00u);
 }
 // e4m3 codes in bytes 1 and 3 of t -> f16x2 of value * 2^-8 (see widen2_e4m3_alu)
 __device__ __forceinline__ unsigned e4m3_hi_bytes_alu(unsigned t) { return (t & 0x80008000u) | ((t >> 1) & 0x3f803f80u); }
@@ -113,37 +121,65 @@ __device__ __forceinline__ unsigned hmul2_u(unsigned a, unsigned b) {
   __half2 h = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
   return *reinterpret_cast<unsigned*>(&h);
 }
+constexpr int kBarBytes = 256;                 // barriers of all warps, ahead of the rings; never anything else (an mbarrier's words may not be reused)
 template <int FMT, int D> struct RecBytes {
   static constexpr int value = FMT == TSB200_KV_INT8 ? 16 * D + 64 : (FMT == TSB200_KV_NVFP4 ? 9 * D : 16 * D);
 };
 
 template <typename T, int D, int FMT>
-__global__ void __launch_bounds__(AttnCfg<FMT>::kWarps * 32)
+__global__ void __launch_bounds__(AttnCfg<FMT, D>::kWarps * 32, AttnCfg<FMT, D>::kCtas)
 decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
-                       float* __restrict__ ws, int* __restrict__ counters, T* __restrict__ out) {
+                       float* __restrict__ ws, T* __restrict__ out, int* __restrict__ status) {
   constexpr bool FP4 = FMT == TSB200_KV_NVFP4;
-  constexpr int kWarps = AttnCfg<FMT>::kWarps, kStages = AttnCfg<FMT>::kStages;
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int CODE_CHUNKS = FP4 ? D / 2 : D; // 16-byte chunks of K codes (placed with the row swizzle)
-  constexpr int ROW_CHUNKS = FP4 ? D / 32 : D / 16;
-  constexpr int REC_CHUNKS = REC / 16;
-  constexpr int STAGE = 2 * REC;
+  constexpr int kWarps = AttnCfg<FMT, D>::kWarps, kStages = AttnCfg<FMT, D>::kStages;
+  constexpr int STAGE = 2 * REC;                // K and V of a page
   constexpr int NC = D / 16;                    // k-steps of QK, m-tiles of PV
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_launch_dependents();
-  pdl_wait();     // q, the page just appended and seq_lens come from the preceding kernels
 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int gid = lane >> 2, tid = lane & 3;
   const int b = blockIdx.x / kv.hkv, hk = blockIdx.x % kv.hkv, s = blockIdx.y;
   const int g = H / kv.hkv;
   const int g0 = blockIdx.z * 8, gn = min(8, g - g0);
+  uint8_t* ring = smem + kBarBytes + (size_t)w * kStages * STAGE;
+  uint2* vscales = reinterpret_cast<uint2*>(smem + kBarBytes + (size_t)kWarps * kStages * STAGE) + w * (D / 4);    // NVFP4
+  const unsigned ring_a = smem_u32(ring), bar_a = smem_u32(smem) + w * kStages * 8;
+  if (lane == 0) {
+    for (int i = 0; i < kStages; ++i) mbar_init(reinterpret_cast<unsigned long long*>(smem) + w * kStages + i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncwarp();
+  // lengths and block table do not come from the preceding launch (see tsb200_set_pdl): looked up ahead of the dependency wait
   int len = kv.seq_lens[b];
   len = len < 0 ? 0 : (len > max_seq_len ? (int)max_seq_len : len);
-  const bool fuse_reduce = S > 0;      // S < 0: |S| splits, partials only (a reducer kernel follows)
-  S = S < 0 ? -S : S;
   int pb, pe;
   split_range(len, s, S, pb, pe);
+
+  // ---- this warp's pages: pb + w, pb + w + kWarps, ...  Lane 0 copies K, lane 1 V; a page's number is looked up a page before its copy leaves.
+  const int n_my = pe - pb > w ? (pe - pb - w + kWarps - 1) / kWarps : 0;
+  const int64_t rec_stride = (int64_t)kv.hkv * REC;
+  const uint8_t* pool = ((lane & 1) ? kv.v_pool : kv.k_pool) + (int64_t)hk * REC;
+  const int* table = kv.block_table + (int64_t)b * kv.bt_stride + pb + w;
+  auto look_up = [&](int it) { return lane < 2 && it < n_my ? table[it * kWarps] : 0; };
+  auto issue = [&](int it, int page) {
+    if (it < n_my) {
+      if (lane == 0) mbar_expect_tx(reinterpret_cast<unsigned long long*>(smem) + w * kStages + it % kStages, 2u * REC);
+      __syncwarp();
+      if (lane < 2) {
+        const int64_t at = page < 0 ? 0 : (page >= kv.num_pages ? kv.num_pages - 1 : page);
+        bulk_g2s(ring_a + (it % kStages) * STAGE + lane * REC, pool + at * rec_stride, REC, bar_a + (it % kStages) * 8);
+      }
+    }
+  };
+  int ahead[kStages];
+#pragma unroll
+  for (int i = 0; i < kStages; ++i) ahead[i] = look_up(i);
+  pdl_wait();     // q and the page just appended come from the preceding kernels
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) issue(i, ahead[i]);
+  int next_page = ahead[kStages - 1];
 
   // Q^T fragments (B operand): this lane holds head g0+gid at the dims of its k-slots: 16 consecutive ones per four steps, fetched as
   // 16-byte pieces where q allows it (element by element: 32 loads, 2500 cycles before the first page of a short split).
@@ -186,41 +222,22 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   for (int i = 0; i < NC; ++i) { oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f; }
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // heads 2*tid, 2*tid+1 (log2 domain)
 
-  uint8_t* ring = smem + (size_t)w * kStages * STAGE;
-  const int n_my = (pe - pb - w + kWarps - 1) / kWarps > 0 ? (pe - pb - w + kWarps - 1) / kWarps : 0;
-  const int64_t rec_stride = (int64_t)kv.hkv * REC;
-
-  auto issue = [&](int it) {
-    if (it < n_my) {
-      const int pg = pb + w + it * kWarps;
-      int64_t page = kv.block_table[(int64_t)b * kv.bt_stride + pg];
-      page = page < 0 ? 0 : (page >= kv.num_pages ? kv.num_pages - 1 : page);
-      const uint8_t* kr = kv.k_pool + page * rec_stride + (int64_t)hk * REC;
-      const uint8_t* vr = kv.v_pool + page * rec_stride + (int64_t)hk * REC;
-      uint8_t* sK = ring + (it % kStages) * STAGE;
-      uint8_t* sV = sK + REC;
-#pragma unroll
-      for (int ci = lane; ci < REC_CHUNKS; ci += 32) {
-        int phys = ci;
-        if (ci < CODE_CHUNKS)
-          phys = FP4 ? k4_phys_chunk<D>(ci / ROW_CHUNKS, ci % ROW_CHUNKS) : k_phys_chunk<D>(ci / ROW_CHUNKS, ci % ROW_CHUNKS);
-        cp_async16(sK + phys * 16, kr + ci * 16);
-        cp_async16(sV + ci * 16, vr + ci * 16);
-      }
-    }
-    cp_async_commit();
-  };
-
-#pragma unroll
-  for (int i = 0; i < kStages - 1; ++i) issue(i);
-
   const int r1 = 4 * (gid >> 1) + (gid & 1), r2 = r1 + 2;   // token rows of this lane in S^T
+  bool ok = true;
   for (int it = 0; it < n_my; ++it) {
-    issue(it + kStages - 1);
-    cp_async_wait<kStages - 1>();
-    __syncwarp();
-    const int pg = pb + w + it * kWarps;
-    const int nt = min(16, len - pg * 16);
+    issue(it + kStages - 1, next_page);
+    next_page = look_up(it + kStages);
+    {
+      unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem) + w * kStages + it % kStages;
+      const unsigned parity = (it / kStages) & 1;
+      unsigned spins = 0;
+      while (!mbar_try_wait(bar, parity)) {
+        if (++spins > kWaitLimit) { ok = false; break; }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+    }
+    const int nt = min(16, len - (pb + w + it * kWarps) * 16);
     const uint8_t* sK = ring + (it % kStages) * STAGE;
     const uint8_t* sV = sK + REC;
 
@@ -228,17 +245,18 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
     float sacc[4] = {0.f, 0.f, 0.f, 0.f};
     if (FP4) {
       // the lane's 16 dims of a row = 8 bytes of codes = exactly one scale block
-      const uint8_t* ksc = sK + 16 * (D / 2);
+      // block scale * 2^-8 (integer widening) * 2^15 -> scale * 2^7 <= 57344; code * 2^-14 times that is
+      // code * scale * 2^-7, exact in f16 (6 significant bits, >= 2^-17)
+      const unsigned k215 = 0x78007800u, sel = tid * 0x1010u + 0x0404u;
+      const unsigned* s1 = reinterpret_cast<const unsigned*>(sK + 16 * (D / 2) + r1 * (D / 16));
+      const unsigned* s2 = reinterpret_cast<const unsigned*>(sK + 16 * (D / 2) + r2 * (D / 16));
 #pragma unroll
       for (int hh = 0; hh < D / 64; ++hh) {
         const int j = tid + 4 * hh;
-        const uint2 ka = *reinterpret_cast<const uint2*>(sK + k4_phys_chunk<D>(r1, j >> 1) * 16 + 8 * (j & 1));
-        const uint2 kb = *reinterpret_cast<const uint2*>(sK + k4_phys_chunk<D>(r2, j >> 1) * 16 + 8 * (j & 1));
-        // block scale * 2^-8 (integer widening) * 2^15 -> scale * 2^7 <= 57344; code * 2^-14 times that is
-        // code * scale * 2^-7, exact in f16 (6 significant bits, >= 2^-17)
-        const unsigned k215 = 0x78007800u;
-        const unsigned sa = hmul2_u(e4m3_hi_bytes_alu((unsigned)ksc[r1 * (D / 16) + j] * 0x01000100u), k215);
-        const unsigned sb = hmul2_u(e4m3_hi_bytes_alu((unsigned)ksc[r2 * (D / 16) + j] * 0x01000100u), k215);
+        const uint2 ka = *reinterpret_cast<const uint2*>(sK + r1 * (D / 2) + 8 * j);
+        const uint2 kb = *reinterpret_cast<const uint2*>(sK + r2 * (D / 2) + 8 * j);
+        const unsigned sa = hmul2_u(e4m3_hi_bytes_alu(__byte_perm(s1[hh], 0u, sel)), k215);
+        const unsigned sb = hmul2_u(e4m3_hi_bytes_alu(__byte_perm(s2[hh], 0u, sel)), k215);
         mma16816(sacc, hmul2_u(e2m1_pair_alu<0>(ka.x), sa), hmul2_u(e2m1_pair_alu<0>(kb.x), sb), hmul2_u(e2m1_pair_alu<1>(ka.x), sa),
                  hmul2_u(e2m1_pair_alu<1>(kb.x), sb), qf[4 * hh][0], qf[4 * hh][1]);
         mma16816(sacc, hmul2_u(e2m1_pair_alu<2>(ka.x), sa), hmul2_u(e2m1_pair_alu<2>(kb.x), sb), hmul2_u(e2m1_pair_alu<3>(ka.x), sa),
@@ -248,19 +266,20 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
         mma16816(sacc, hmul2_u(e2m1_pair_alu<2>(ka.y), sa), hmul2_u(e2m1_pair_alu<2>(kb.y), sb), hmul2_u(e2m1_pair_alu<3>(ka.y), sa),
                  hmul2_u(e2m1_pair_alu<3>(kb.y), sb), qf[4 * hh + 3][0], qf[4 * hh + 3][1]);
       }
-    }
+    } else {
 #pragma unroll
-    for (int hh = 0; hh < (FP4 ? 0 : D / 64); ++hh) {
-      const int j = tid + 4 * hh;
-      const uint4 ka = *reinterpret_cast<const uint4*>(sK + k_phys_chunk<D>(r1, j) * 16);
-      const uint4 kb = *reinterpret_cast<const uint4*>(sK + k_phys_chunk<D>(r2, j) * 16);
-      const unsigned wa[4] = {ka.x, ka.y, ka.z, ka.w};
-      const unsigned wb[4] = {kb.x, kb.y, kb.z, kb.w};
+      for (int hh = 0; hh < D / 64; ++hh) {
+        const int j = tid + 4 * hh;
+        const uint4 ka = *reinterpret_cast<const uint4*>(sK + r1 * D + 16 * j);
+        const uint4 kb = *reinterpret_cast<const uint4*>(sK + r2 * D + 16 * j);
+        const unsigned wa[4] = {ka.x, ka.y, ka.z, ka.w};
+        const unsigned wb[4] = {kb.x, kb.y, kb.z, kb.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = 4 * hh + i;
-        mma16816(sacc, widen2_k<FMT>(wa[i]), widen2_k<FMT>(wb[i]), widen2_k<FMT>(wa[i] >> 16), widen2_k<FMT>(wb[i] >> 16),
-                 qf[c][0], qf[c][1]);
+        for (int i = 0; i < 4; ++i) {
+          const int c = 4 * hh + i;
+          mma16816(sacc, widen2_k<FMT>(wa[i]), widen2_k<FMT>(wb[i]), widen2_k<FMT>(wa[i] >> 16), widen2_k<FMT>(wb[i] >> 16),
+                   qf[c][0], qf[c][1]);
+        }
       }
     }
     // ---- online softmax over the page's tokens (rows) per head (column) -------------
@@ -282,53 +301,74 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
     }
     const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);   // finite: token 0 of a page is always valid
-    const float c0 = exp2f(m0 - mn0), c1 = exp2f(m1 - mn1);
-    const float p0 = exp2f(s0 - mn0), p1 = exp2f(s1 - mn1), p2 = exp2f(s2 - mn0), p3 = exp2f(s3 - mn1);
-    l0 = l0 * c0 + (p0 + p2);
-    l1 = l1 * c1 + (p1 + p3);
+    const float c0 = ex2(m0 - mn0), c1 = ex2(m1 - mn1);
+    const float p0 = ex2(s0 - mn0), p1 = ex2(s1 - mn1), p2 = ex2(s2 - mn0), p3 = ex2(s3 - mn1);
+    l0 = __fmaf_rn(l0, c0, p0 + p2);
+    l1 = __fmaf_rn(l1, c1, p1 + p3);
     m0 = mn0; m1 = mn1;
-    if (FP4) vs1 = vs2 = 256.0f;                // NVFP4: the block scales multiply P as scale * 2^-8
-    const unsigned P1 = pack_h2(ok1 ? p0 * vs1 : 0.f, ok1 ? p1 * vs1 : 0.f);
-    const unsigned P2 = pack_h2(ok2 ? p2 * vs2 : 0.f, ok2 ? p3 * vs2 : 0.f);
-    unsigned pb0 = movmatrix_trans(P1);         // tokens 4*tid, 4*tid+1 of head gid
-    unsigned pb1 = movmatrix_trans(P2);         // tokens 4*tid+2, 4*tid+3
-    if (FP4) {                                  // NVFP4 pairs tokens (4*tid, 4*tid+2) and (4*tid+1, 4*tid+3)
-      const unsigned t0 = __byte_perm(pb0, pb1, 0x5410), t1 = __byte_perm(pb0, pb1, 0x7632);
-      pb0 = t0; pb1 = t1;
-    }
-    // bytes of this lane's 4 tokens that are inside the sequence (stale slots -> +0)
-    unsigned vmask = 0xffffffffu;
-    if (nt < 16) {
-      const int left = nt - 4 * tid;
-      vmask = left >= 4 ? 0xffffffffu : (left <= 0 ? 0u : (0xffffffffu >> (8 * (4 - left))));
+    if (__any_sync(0xffffffffu, c0 != 1.0f || c1 != 1.0f)) {  // (a product by 1 changes nothing)
+#pragma unroll
+      for (int mt = 0; mt < NC; ++mt) { oacc[mt][0] *= c0; oacc[mt][1] *= c1; oacc[mt][2] *= c0; oacc[mt][3] *= c1; }
     }
     // ---- O^T += V^T . P^T -----------------------------------------------------------
-    if (FP4) {
-      const uint8_t* vsc = sV + 16 * (D / 2);
+    {
+      if (FP4) vs1 = vs2 = 256.0f;               // NVFP4: the block scales multiply P as scale * 2^-8
+      const unsigned P1 = pack_h2(ok1 ? p0 * vs1 : 0.f, ok1 ? p1 * vs1 : 0.f);        // (a stale slot may hold any scale)
+      const unsigned P2 = pack_h2(ok2 ? p2 * vs2 : 0.f, ok2 ? p3 * vs2 : 0.f);
+      unsigned pb0 = movmatrix_trans(P1);         // tokens 4*tid, 4*tid+1 of head gid
+      unsigned pb1 = movmatrix_trans(P2);         // tokens 4*tid+2, 4*tid+3
+      if (FP4) {                                  // NVFP4 pairs tokens (4*tid, 4*tid+2) and (4*tid+1, 4*tid+3)
+        const unsigned t0 = __byte_perm(pb0, pb1, 0x5410), t1 = __byte_perm(pb0, pb1, 0x7632);
+        pb0 = t0; pb1 = t1;
+      }
+      if (FP4) {
+        // the page's block scales, widened once for the warp (every lane for itself they were a seventh of the kernel's instructions: 8 sequences x
+        // half to all of 32k tokens, 28 / 4 heads: 59 us against 52): f16 pairs of tokens (0, 2) and (1, 3) of four, value * 2^-8, stale slots +0
+        if (lane < D / 4) {
+          unsigned sw = *reinterpret_cast<const unsigned*>(sV + 16 * (D / 2) + lane * 4);
+          if (nt < 16) {
+            const int rest = nt - 4 * (lane & 3);
+            sw &= rest >= 4 ? 0xffffffffu : (rest <= 0 ? 0u : (0xffffffffu >> (8 * (4 - rest))));
+          }
+          vscales[lane] = make_uint2(e4m3_hi_bytes_alu(__byte_perm(sw, 0u, 0x2404)), e4m3_hi_bytes_alu(__byte_perm(sw, 0u, 0x3414)));
+        }
+        __syncwarp();
 #pragma unroll
-      for (int mt = 0; mt < NC; ++mt) {
-        // one word = tokens 4*tid..4*tid+3 of dims 16*mt + 2*gid (low nibbles) and + 1 (high nibbles):
-        // MMA rows gid / gid + 8 are those two dims
-        const unsigned wv = *reinterpret_cast<const unsigned*>(sV + (8 * mt + gid) * 16 + 4 * tid);
-        const unsigned sw = *reinterpret_cast<const unsigned*>(vsc + mt * 16 + 4 * tid) & vmask;   // stale slots: scale +0
-        // code pairs 16 bits apart = tokens (0, 2) and (1, 3) of the lane's four; values enter as code * 2^-14
-        // (2^14 is restored with the split scale), weights as p * 2^8 * (block scale * 2^-8)
-        const unsigned b0 = hmul2_u(pb0, e4m3_hi_bytes_alu(__byte_perm(sw, 0u, 0x2404)));
-        const unsigned b1 = hmul2_u(pb1, e4m3_hi_bytes_alu(__byte_perm(sw, 0u, 0x3414)));
-        oacc[mt][0] *= c0; oacc[mt][1] *= c1; oacc[mt][2] *= c0; oacc[mt][3] *= c1;
-        mma16816(oacc[mt], e2m1_pair_alu<0>(wv), e2m1_pair_alu<1>(wv), e2m1_pair_alu<2>(wv), e2m1_pair_alu<3>(wv), b0, b1);
+        for (int mt = 0; mt < NC; ++mt) {
+          // one word = tokens 4*tid..4*tid+3 of dims 16*mt + 2*gid (low nibbles) and + 1 (high nibbles):
+          // MMA rows gid / gid + 8 are those two dims
+          const unsigned wv = *reinterpret_cast<const unsigned*>(sV + (8 * mt + gid) * 16 + 4 * tid);
+          const uint2 sc2 = vscales[mt * 4 + tid];
+          // code pairs 16 bits apart = tokens (0, 2) and (1, 3) of the lane's four; values enter as code * 2^-14
+          // (2^14 is restored with the split scale), weights as p * 2^8 * (block scale * 2^-8)
+          mma16816(oacc[mt], e2m1_pair_alu<0>(wv), e2m1_pair_alu<1>(wv), e2m1_pair_alu<2>(wv), e2m1_pair_alu<3>(wv),
+                   hmul2_u(pb0, sc2.x), hmul2_u(pb1, sc2.y));
+        }
+        __syncwarp();                            // the next page's take their place
+      } else {
+        // bytes of this lane's 4 tokens that are inside the sequence (stale slots -> +0)
+        unsigned vmask = 0xffffffffu;
+        if (nt < 16) {
+          const int rest = nt - 4 * tid;
+          vmask = rest >= 4 ? 0xffffffffu : (rest <= 0 ? 0u : (0xffffffffu >> (8 * (4 - rest))));
+        }
+#pragma unroll
+        for (int mt = 0; mt < NC; ++mt) {
+          unsigned w1 = *reinterpret_cast<const unsigned*>(sV + (16 * mt + gid) * 16 + 4 * tid);
+          unsigned w2 = *reinterpret_cast<const unsigned*>(sV + (16 * mt + gid + 8) * 16 + 4 * tid);
+          if (FMT == TSB200_KV_FP8) { w1 &= vmask; w2 &= vmask; }     // (an int8 code is finite whatever it is)
+          mma16816(oacc[mt], widen2<FMT>(w1), widen2<FMT>(w2), widen2<FMT>(w1 >> 16), widen2<FMT>(w2 >> 16), pb0, pb1);
+        }
       }
     }
-#pragma unroll
-    for (int mt = 0; mt < (FP4 ? 0 : NC); ++mt) {
-      const unsigned w1 = *reinterpret_cast<const unsigned*>(sV + (16 * mt + gid) * 16 + 4 * tid) & vmask;
-      const unsigned w2 = *reinterpret_cast<const unsigned*>(sV + (16 * mt + gid + 8) * 16 + 4 * tid) & vmask;
-      oacc[mt][0] *= c0; oacc[mt][1] *= c1; oacc[mt][2] *= c0; oacc[mt][3] *= c1;
-      mma16816(oacc[mt], widen2<FMT>(w1), widen2<FMT>(w2), widen2<FMT>(w1 >> 16), widen2<FMT>(w2 >> 16), pb0, pb1);
-    }
-    __syncwarp();
+    __syncwarp();                                // every lane has read the stage: the next round's copies may take it
   }
-  cp_async_wait<0>();
+  if (!ok) {
+    // error path only: a wait ran out.  Give the copies still in flight a bounded time to land before
+    // shared memory is reused, and record the event.
+    if (lane == 0 && status) atomicMax(status, 8);
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+  }
   // row sums: add the partial sums of the 8 token lanes
 #pragma unroll
   for (int o = 4; o < 32; o <<= 1) {
@@ -337,7 +377,7 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   }
   __syncthreads();   // every warp is done with its ring; reuse shared memory for the merge
   constexpr int AR = D + 4;                                  // row pitch: the fragments' four head rows fall into different banks
-  float* sm_m = reinterpret_cast<float*>(smem);              // [warps][8]
+  float* sm_m = reinterpret_cast<float*>(smem + kBarBytes);  // [warps][8]
   float* sm_l = sm_m + kWarps * 8;                           // [warps][8]
   float* sm_c = sm_l + kWarps * 8;                           // [warps][8]
   float* sm_acc = sm_c + kWarps * 8;                         // [warps][8][AR]
@@ -378,7 +418,7 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       a1 += x.y * c;
     }
     const int64_t bh = (int64_t)b * H + hk * g + g0 + i;
-    if (S == 1 && fuse_reduce) {
+    if (S == 1) {
       out[bh * D + e] = from_f32<T>(ll > 0.f ? a0 * vscale / ll : 0.f);
       out[bh * D + e + 1] = from_f32<T>(ll > 0.f ? a1 * vscale / ll : 0.f);
     } else {
@@ -392,30 +432,17 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       *reinterpret_cast<float2*>(o + 2 + e) = make_float2(a0 * vscale, a1 * vscale);
     }
   }
-  if (S == 1 || !fuse_reduce) return;
-  // The last CTA of this (sequence, kv head, head chunk) to finish merges the S partials in split
-  // order and resets the counter, so no separate reduction launch is needed.
-  __shared__ int s_last;
-  __threadfence();
-  __syncthreads();
-  int* ctr = counters + ((int64_t)blockIdx.x * gridDim.z + blockIdx.z);
-  if (threadIdx.x == 0) s_last = (atomicAdd(ctr, 1) == S - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const int64_t bh0 = (int64_t)b * H + hk * g + g0;
-  merge_splits<T, D>(ws + bh0 * S * (2 + D), gn, S, reinterpret_cast<float*>(smem), out + bh0 * D);
-  if (threadIdx.x == 0) *ctr = 0;
 }
 
 template <typename T, int D, int FMT>
-int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S, int64_t B,
-               float* ws, int* counters, void* out, cudaStream_t st) {
+int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int64_t B, float* ws, void* out,
+               int* status, cudaStream_t st) {
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int kWarps = AttnCfg<FMT>::kWarps, kStages = AttnCfg<FMT>::kStages;
-  constexpr size_t pipe = (size_t)kWarps * kStages * 2 * REC;
+  constexpr int kWarps = AttnCfg<FMT, D>::kWarps, kStages = AttnCfg<FMT, D>::kStages;
+  static_assert(kWarps * kStages * 8 <= kBarBytes, "barriers");
+  constexpr size_t pipe = (size_t)kWarps * (kStages * 2 * REC + (FMT == TSB200_KV_NVFP4 ? D * 2 : 0));
   constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4)) * sizeof(float);
-  constexpr size_t smem = pipe > merge ? pipe : merge;
+  constexpr size_t smem = kBarBytes + (pipe > merge ? pipe : merge);
   static bool configured[64] = {false};   // per device: the attribute lives in the device's context
   int dev = 0;
   TSB_CUDA(cudaGetDevice(&dev));
@@ -424,11 +451,11 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
     TSB_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<T, D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev] = true;
   }
-  const int g = H / kv.hkv;
-  dim3 grid((unsigned)(B * kv.hkv), (unsigned)(S < 0 ? -S : S), (unsigned)((g + 7) / 8));   // S < 0: partials only
+  const int g = H / kv.hkv, S = choose_splits(B, kv.hkv, max_seq_len);
+  dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((g + 7) / 8));
   TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
-                         max_seq_len, S, ws, counters, (T*)out));
-  return TSB200_OK;
+                         max_seq_len, S, ws, (T*)out, status));
+  return S == 1 ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }
 
 }  // namespace
@@ -436,7 +463,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
 
 using namespace tsb;
 
-// Bytes the dispatch below really uses for a problem: counters + partials of the split count it will pick
+// Bytes that serve a problem: counters + partials of choose_splits() splits, which no format's own split count exceeds
 // (tsb200_paged_decode_attn_workspace_bytes is the hkv-independent upper bound of this).
 static size_t attn_exact_workspace_bytes(const tsb200_kv_desc* kv, int64_t B, int H, int64_t max_seq_len) {
   const int S = choose_splits(B, kv->hkv, max_seq_len);
@@ -453,44 +480,32 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   const int64_t qs = q_batch_stride ? q_batch_stride : (int64_t)H * kv->head_dim;
   if (qs < (int64_t)H * kv->head_dim) return TSB200_ERR_ARG;
   cudaStream_t s = as_stream(stream);
-  const int S = choose_splits(B, kv->hkv, max_seq_len);
   int* counters = (int*)workspace;                               // zero between calls
   float* ws = (float*)((char*)workspace + kAttnCounterBytes);
   const int D = kv->head_dim;
   const int64_t n_ctr = B * kv->hkv * ((H / kv->hkv + 7) / 8);
   // the last int of the counter block is the status word of the bounded waits, so one counter fewer is usable
   const bool room = n_ctr < (int64_t)(kAttnCounterBytes / sizeof(int));
-  const bool fused = room && last_cta_merges(S, H, kv->hkv);      // else: separate reduction launch
   int* status = counters + kAttnStatusIndex;
-  int r;
   if (kv->format > TSB200_KV_NVFP4)    // unquantized pages: fp32 math (decode_attn_dense.cu)
     return attn_dense(kv, q, out, dtype, qs, B, H, sm_scale, max_seq_len, ws, room ? counters : nullptr, s);
   if (kv->format == TSB200_KV_FP8 && D == 128 && H / kv->hkv <= 4) {
     // e4m3 pages go to the tensor cores as FP8 (decode_attn_fp8.cu)
     const int S8 = choose_splits_fp8(B, kv->hkv, max_seq_len);   // never more than choose_splits(): the workspace fits
-    const bool fused8 = room && last_cta_merges(S8, H, kv->hkv);
-    int* ctr = fused8 ? counters : nullptr;
-    if (dtype == TSB200_F32) r = launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, ctr, out, status, s);
-    else r = launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, ctr, out, status, s);
-    if (r != TSB200_OK || fused8) return r;
+    const int r = dtype == TSB200_F32 ? launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s)
+                                      : launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s);
+    if (r != TSB200_OK || S8 == 1) return r;
     return dtype == TSB200_F32 ? launch_reduce<float, 128>(ws, B * H, S8, out, s) : launch_reduce<__nv_bfloat16, 128>(ws, B * H, S8, out, s);
   }
-#define TSB_GO(TT, DD, FF)                                                                                              \
-  if (fused) return launch_mma<TT, DD, FF>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, counters, out, s);        \
-  r = launch_mma<TT, DD, FF>(*kv, q, qs, H, sm_scale, max_seq_len, -S, B, ws, counters, out, s);                      \
-  if (r != TSB200_OK) return r;                                                                                         \
-  return launch_reduce<TT, DD>(ws, B * H, S, out, s)
-  if (kv->format == TSB200_KV_NVFP4) {
-    if (dtype == TSB200_F32) { if (D == 64) { TSB_GO(float, 64, TSB200_KV_NVFP4); } else { TSB_GO(float, 128, TSB200_KV_NVFP4); } }
-    else { if (D == 64) { TSB_GO(__nv_bfloat16, 64, TSB200_KV_NVFP4); } else { TSB_GO(__nv_bfloat16, 128, TSB200_KV_NVFP4); } }
-  }
-  if (dtype == TSB200_F32) {
-    if (D == 64) { if (kv->format == TSB200_KV_INT8) { TSB_GO(float, 64, TSB200_KV_INT8); } else { TSB_GO(float, 64, TSB200_KV_FP8); } }
-    else { if (kv->format == TSB200_KV_INT8) { TSB_GO(float, 128, TSB200_KV_INT8); } else { TSB_GO(float, 128, TSB200_KV_FP8); } }
-  } else {
-    if (D == 64) { if (kv->format == TSB200_KV_INT8) { TSB_GO(__nv_bfloat16, 64, TSB200_KV_INT8); } else { TSB_GO(__nv_bfloat16, 64, TSB200_KV_FP8); } }
-    else { if (kv->format == TSB200_KV_INT8) { TSB_GO(__nv_bfloat16, 128, TSB200_KV_INT8); } else { TSB_GO(__nv_bfloat16, 128, TSB200_KV_FP8); } }
-  }
+#define TSB_GO(TT, DD, FF) return launch_mma<TT, DD, FF>(*kv, q, qs, H, sm_scale, max_seq_len, B, ws, out, status, s)
+#define TSB_FMT(FF)                                                                                                       \
+  if (dtype == TSB200_F32) { if (D == 64) TSB_GO(float, 64, FF); TSB_GO(float, 128, FF); }                               \
+  if (D == 64) TSB_GO(__nv_bfloat16, 64, FF);                                                                             \
+  TSB_GO(__nv_bfloat16, 128, FF)
+  if (kv->format == TSB200_KV_NVFP4) { TSB_FMT(TSB200_KV_NVFP4); }
+  if (kv->format == TSB200_KV_INT8) { TSB_FMT(TSB200_KV_INT8); }
+  TSB_FMT(TSB200_KV_FP8);
+#undef TSB_FMT
 #undef TSB_GO
 }
 
