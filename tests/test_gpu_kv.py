@@ -587,3 +587,33 @@ def test_decode_attention_of_every_length(cuda, fmt, H, Hkv, d, B, name):
     assert torch.equal(out, ops.paged_decode_attention(kv, q, pages * 16))
     assert torch.all(out[lens == 0] == 0)
     assert torch.all((out.float() - refs[1]).abs() <= C_P_TC * refs[0] + 2 * C_OUT[name] * refs[1].abs() + 1e-6)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+def test_append_of_quotients_at_the_midpoints_of_codes(cuda, fmt, name):
+    """bf16 elements of every significand over FP8 scales within a few ulps of the divisors that put one of them on the midpoint of two
+    codes (and scales of all ones): by page as by vector, which divides."""
+    from transformer_surgeon_b200 import ops
+    rng = np.random.default_rng(53)
+    B, T, Hkv, d = 64, 16, 2, 128
+    _, bulk = make_pair(fmt, B, 1, Hkv, d, cuda, rng)
+    single = ops.PagedKV(fmt, bulk.k_pool.shape[0], Hkv, d, bulk.block_table, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+    k, v = (torch.from_numpy((rng.integers(128, 256, (B, T, Hkv, d)) * 2.0 ** rng.integers(-17, 3, (B, T, Hkv, d)) * rng.choice([-1, 1], (B, T, Hkv, d))).astype(np.float32))
+            .to(DT[name]).to(cuda) for _ in range(2))
+    if fmt == "fp8":
+        scales = []
+        for _ in range(2):
+            near = (rng.integers(128, 256, (B, Hkv)) / (2 * rng.integers(0, 16, (B, Hkv)) + 1)).astype(np.float32)
+            s = (near.view(np.int32) + rng.integers(-4, 5, (B, Hkv))).astype(np.int32).view(np.float32)
+            s[::8] = np.nextafter(np.float32(2.0), np.float32(0))
+            scales.append(torch.from_numpy(s * np.float32(2.0 ** -6)).to(cuda))
+        bulk.fill_fp8_scales(*scales)
+        single.fill_fp8_scales(*scales)
+    assert B * T * Hkv * d >= 1 << 18
+    bulk.append(k, v)
+    for t in range(T):
+        single.append(k[:, t:t + 1].contiguous(), v[:, t:t + 1].contiguous())
+        single.seq_lens += 1
+    assert torch.equal(bulk.k_pool, single.k_pool)
+    assert torch.equal(bulk.v_pool, single.v_pool)

@@ -10,6 +10,7 @@
 //           rule, compression/quantization_methods/vanilla.py:16-24, applied per vector)
 //   fp8   : code = e4m3_satfinite(x / S[b, h])
 //   nvfp4 : per 16 elements sb = e4m3_satfinite(amax/6), code = e2m1_satfinite(x/decode(sb))
+#include <type_traits>
 #include "common.cuh"
 
 namespace tsb {
@@ -217,6 +218,9 @@ template <> struct Raw8<__nv_bfloat16> {
     }
   }
   __device__ __forceinline__ void load_shared(const __nv_bfloat16* p) { load(p, true); }
+  // 16-byte pieces 32 apart in shared memory
+  __device__ __forceinline__ void load_strided(const uint4* p) { load(reinterpret_cast<const __nv_bfloat16*>(p), true); }
+  __device__ __forceinline__ void store_strided(uint4* p) const { store(reinterpret_cast<__nv_bfloat16*>(p), true); }
   __device__ __forceinline__ void store(__nv_bfloat16* p, bool vec) const {
     if (vec) {
       *reinterpret_cast<uint4*>(p) = make_uint4(u[0], u[1], u[2], u[3]);
@@ -231,6 +235,15 @@ template <> struct Raw8<__nv_bfloat16> {
   __device__ __forceinline__ void unpack(float (&v)[8]) const {
 #pragma unroll
     for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+  }
+  // into [-c, c], both halves of c2 holding c (NaN stays)
+  __device__ __forceinline__ void clamp(unsigned c2) {
+    const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&c2), lo = __hneg2(hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 r = __hmin2_nan(__hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&u[i]), lo), hi);
+      u[i] = *reinterpret_cast<const unsigned*>(&r);
+    }
   }
   // largest magnitude, as the bits of a positive bf16
   __device__ __forceinline__ float amax(float m) const {
@@ -253,6 +266,14 @@ template <> struct Raw8<float> {
     }
   }
   __device__ __forceinline__ void load_shared(const float* p) { load(p, true); }
+  __device__ __forceinline__ void load_strided(const uint4* p) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 32);
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+  }
+  __device__ __forceinline__ void store_strided(uint4* p) const {
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+    *reinterpret_cast<float4*>(p + 32) = make_float4(f[4], f[5], f[6], f[7]);
+  }
   __device__ __forceinline__ void store(float* p, bool vec) const {
     if (vec) {
       *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
@@ -272,6 +293,15 @@ template <> struct Raw8<float> {
     return m;
   }
 };
+// fp32 elements rounded to the act dtype
+__device__ __forceinline__ void round8(const Raw8<float>& f, Raw8<__nv_bfloat16>& r) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.f[2 * i], f.f[2 * i + 1]);
+    r.u[i] = *reinterpret_cast<const unsigned*>(&b);
+  }
+}
+__device__ __forceinline__ void round8(const Raw8<float>& f, Raw8<float>& r) { r = f; }
 // Half-split rotation of elements (a[i], b[i]), i and i + d/2 of one vector: every product and sum rounded to the act dtype
 // (blocks/rope.py:140-173).  bf16: packed arithmetic - one rounding per operation; the fp32 detour rounds the sum twice, which is
 // the same, since two bf16 numbers whose sum has more than 24 bits are too far apart for it to lie near a midpoint.
@@ -294,15 +324,32 @@ __device__ __forceinline__ void rope8(Raw8<float>& a, Raw8<float>& b, const Raw8
   }
 }
 
-// Quotients by a divisor that many elements share: correctly rounded from the correctly rounded reciprocal (Markstein's theorem,
-// Computation of elementary functions on the IBM RISC System/6000 processor, 1990: q' = q + (x - d q) y is the rounded quotient when
-// q is within an ulp of it, which one correction of x y is), two at a time.  Divisors near the ends of the exponent range divide.  An
-// infinite product (of an infinite x, or a quotient beyond the type) stands as it is where MAY_OVERFLOW: it saturates, and its
-// corrections are NaN.
+// Quotients by a divisor that many elements share, from its correctly rounded reciprocal, two at a time: q' = q + (x - d q) y is the
+// rounded quotient when q is within an ulp of it (Markstein's theorem, Computation of elementary functions on the IBM RISC System/6000
+// processor, 1990), which one correction of x y is.  Divisors near the ends of the exponent range divide.
+//   * fp32 elements: corrected twice, correctly rounded.  An infinite product (of an infinite x, or a quotient beyond the type) stands as
+//     it is where MAY_OVERFLOW: it saturates, and its corrections are NaN.
+//   * bf16 elements: corrected once: what is rounded to fp32 is then within 2^-46 of the quotient, and only a quotient that close to
+//     M + half an fp32 ulp, M the midpoint of two codes, could round to another code.  Codes have midpoints of up to eight significant
+//     bits (M = 2 k + 1 for an int8 code k).  With M an odd number of B bits, the divisor as a 24-bit number D and x as X 2^t, X of eight
+//     bits, such an x is M D + c + (less than 2^-18) for c = D 2^(B-25), a whole number below M; so D = c 2^(25-B) + e, |e| <= 8, and
+//     X 2^t = M c 2^(25-B) + M e + c: the first term alone has up to 2 B - 1 bits above 2^(25-B) and X has eight in all, so M e = -c,
+//     which no c between 0 and M is (D = 2^24 - 1, c = M = 1 is one: a divisor of all ones divides).  Quotients that overflow are kept
+//     out by clamping x ahead (FP8: scales from elsewhere).
 struct Divisor {
   float d, y;
   bool slow;
-  template <bool MAY_OVERFLOW> __device__ __forceinline__ void of(float x0, float x1, float& q0, float& q1) const {
+  template <bool TWICE, bool MAY_OVERFLOW> __device__ __forceinline__ void of(float x0, float x1, float& q0, float& q1) const {
+    if (!TWICE) {
+      asm("{\n.reg .b64 x, y, n, p, e;\n"
+          "mov.b64 x, {%2, %3};\nmov.b64 y, {%4, %4};\nmov.b64 n, {%5, %5};\n"
+          "mul.rn.f32x2 p, x, y;\n"
+          "fma.rn.f32x2 e, p, n, x;\nfma.rn.f32x2 p, e, y, p;\n"
+          "mov.b64 {%0, %1}, p;\n}\n"
+          : "=f"(q0), "=f"(q1)
+          : "f"(x0), "f"(x1), "f"(y), "f"(-d));
+      return;
+    }
     float p0, p1;
     asm("{\n.reg .b64 x, y, n, p, q, e;\n"
         "mov.b64 x, {%4, %5};\nmov.b64 y, {%6, %6};\nmov.b64 n, {%7, %7};\n"
@@ -318,16 +365,18 @@ struct Divisor {
     }
   }
 };
-__device__ __forceinline__ Divisor divisor(float v) { return Divisor{v, __frcp_rn(v), !(v >= 1e-18f && v <= 1e18f)}; }
+__device__ __forceinline__ Divisor divisor(float v) {
+  return Divisor{v, __frcp_rn(v), !(v >= 1e-18f && v <= 1e18f) || (__float_as_uint(v) & 0x7fffffu) == 0x7fffffu};
+}
 
 // Codes of one token's eight elements (half a lane's share): two words (8-bit formats) or one (NVFP4).
-template <int FMT, bool SLOW> __device__ __forceinline__ void encode8_by(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
+template <typename T, int FMT, bool SLOW> __device__ __forceinline__ void encode8_by(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
   float q[8];
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
     // FP8: a scale from elsewhere; the other formats' divisors come from the elements' own maximum
     if (SLOW) { q[i] = __fdiv_rn(x[i], d.d); q[i + 1] = __fdiv_rn(x[i + 1], d.d); }
-    else d.of<FMT == TSB200_KV_FP8>(x[i], x[i + 1], q[i], q[i + 1]);
+    else d.of<sizeof(T) == 4, FMT == TSB200_KV_FP8>(x[i], x[i + 1], q[i], q[i + 1]);
   }
   if (FMT == TSB200_KV_FP8) {
     unsigned h[4];
@@ -349,9 +398,9 @@ template <int FMT, bool SLOW> __device__ __forceinline__ void encode8_by(const f
     }
   }
 }
-template <int FMT> __device__ __forceinline__ void encode8(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
-  if (d.slow) encode8_by<FMT, true>(x, d, w0, w1);
-  else encode8_by<FMT, false>(x, d, w0, w1);
+template <typename T, int FMT> __device__ __forceinline__ void encode8(const float (&x)[8], const Divisor& d, unsigned& w0, unsigned& w1) {
+  if (d.slow) encode8_by<T, FMT, true>(x, d, w0, w1);
+  else encode8_by<T, FMT, false>(x, d, w0, w1);
 }
 // 4 x 4 byte transpose: out[j] = byte j of in[0..3]
 __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&out)[4]) {
@@ -370,9 +419,14 @@ __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&o
 //   * V, stored token-minor, is transposed four bytes at a time in registers and leaves through a swizzled tile of shared memory as
 //     16-byte rows, 512 contiguous bytes per warp.
 // Pages that the range covers in part keep their other slots: those go out token by token.  A task is K or V of one head: both at once
-// take 128 registers a thread and leave 24 % of the warps (157 us below).  Instructions and their latencies bound it: 14 an element, the
-// issue slots 58 % busy with the 22 warps that 80 registers a thread leave an SM, memory at 47 %; a further instruction an element costs 2
-// to 4 us.  32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB: 94 us, 242 us with one warp per token vector and a byte-wise transpose.
+// take 128 registers a thread and leave 24 % of the warps.  Instructions and their latencies bound it: a further instruction an element
+// costs 2 to 4 us.  32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB, with the scales' launch (48 us): 141.6 us; 147.6 with loads that a task
+// waits for, two corrections a quotient and selects for what saturates; 290 with one warp per token vector and a byte-wise transpose.
+template <typename T, int D, int FMT> struct AppendSmem {
+  uint4 stage[8][8 * sizeof(T) / 2][32];                                  // per warp: a task's elements, 16-byte pieces by lane
+  T cos[2048 / D][D / 2], sin[2048 / D][D / 2];
+  unsigned v[4][128 / D][(FMT == TSB200_KV_NVFP4 ? D / 2 : D) * 4];       // V records of the warps that have V (the odd ones)
+};
 template <typename T, int D, int FMT>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 1)
 kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,
@@ -383,33 +437,21 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   constexpr int HALF = D / 2, PAGES = 128 / D, TOK = 16 * PAGES;          // tokens of the CTA
   constexpr int EG = HALF / 8;                                            // lanes side by side on a vector
   constexpr int ROWS = FP4 ? D / 2 : D;                                   // 16-byte rows of a V record
-  __shared__ __align__(16) T s_cos[TOK][HALF], s_sin[TOK][HALF];
-  __shared__ __align__(16) unsigned s_v[8][PAGES][ROWS * 4];
+  extern __shared__ __align__(16) uint8_t append_smem[];
+  auto& smem = *reinterpret_cast<AppendSmem<T, D, FMT>*>(append_smem);
   pdl_launch_dependents();
-  pdl_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int eg = lane % EG, tq = lane / EG;                               // elements 8 eg .., tokens 4 tq .. of the CTA's
   const int64_t b = blockIdx.y;
+  pdl_wait();
   const int64_t n_b = new_lens ? min((int64_t)new_lens[b], Tn) : Tn;
   const int64_t start = kv.seq_lens[b];
   const int64_t lp0 = (start >> 4) + (int64_t)blockIdx.x * PAGES;         // first logical page of the CTA
   const int64_t p0 = lp0 * 16;
   if (p0 >= start + n_b) return;
-  if (rope_cos) {
-#pragma unroll
-    for (int i = threadIdx.x; i < TOK * HALF; i += 256) {
-      int64_t p = p0 + i / HALF;
-      p = p < 0 ? 0 : (p >= rope_rows ? rope_rows - 1 : p);
-      s_cos[i / HALF][i % HALF] = from_f32<T>(rope_cos[p * HALF + i % HALF]);
-      s_sin[i / HALF][i % HALF] = from_f32<T>(rope_sin[p * HALF + i % HALF]);
-    }
-    __syncthreads();
-  }
   const int page_of_lane = tq >> 2;                                       // of the CTA's PAGES
   const int slot0 = (tq & 3) * 4;                                         // first of the lane's four slots in that page
   const int64_t lp = lp0 + page_of_lane;
-  int64_t page = lp >= 0 && lp < kv.bt_stride ? (int64_t)kv.block_table[b * kv.bt_stride + lp] : -1;
-  const bool page_ok = page >= 0 && page < kv.num_pages;
   const bool full = lp * 16 >= start && lp * 16 + 16 <= start + n_b;      // every slot of the page is appended
   const int64_t j0 = lp * 16 + slot0 - start;                             // index of the lane's first token in the chunk
   bool tok[4];
@@ -419,43 +461,97 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   const bool vvec = (reinterpret_cast<uintptr_t>(v) & 15) == 0 && vs_ * sizeof(T) % 16 == 0;
   const int lt = page_of_lane * 16 + slot0;                               // the lane's first token in the tables
 
-  // tasks: K or V of a head (half the registers of both at once), then query heads; dealt out over the grid's CTAs of these pages
+  // tasks: K or V of a head (half the registers of both at once; a warp's are all K or all V), then query heads; dealt out over the grid's
+  // CTAs of these pages.  A task's elements are on their way while the task before it is encoded, the first one's while tables and page
+  // numbers are fetched: every lane copies what it will read itself.
   const int tasks = 2 * kv.hkv + (q && rope_cos ? qheads : 0), task_step = 8 * (int)gridDim.z;
   int task = w + 8 * (int)blockIdx.z;
+  auto staged = [&](int i, int half) { return &smem.stage[w][(i * 2 + half) * (int)sizeof(T) / 2][lane]; };   // 16-byte pieces, 32 apart
+  float fp8_scale = 1.f;
+  auto fetch = [&](int t) {
+    if (t >= 2 * kv.hkv) return;
+    const int h = t >> 1;
+    const bool is_v = t & 1, vec = is_v ? vvec : kvec;
+    if (FMT == TSB200_KV_FP8) fp8_scale = (is_v ? kv.v_scale : kv.k_scale)[b * kv.hkv + h];
+    const int64_t stride = is_v ? vs_ : ks;
+    const T* p = (is_v ? v : k) + (b * Tn + j0) * stride + (int64_t)h * D + eg * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, p += stride)
+      if (tok[i]) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (vec) {
+#pragma unroll
+            for (int u = 0; u < (int)sizeof(T) / 2; ++u)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(staged(i, half) + 32 * u)),
+                           "l"(reinterpret_cast<const uint4*>(p + half * HALF) + u) : "memory");
+          } else {
+            Raw8<T> r;
+            r.load(p + half * HALF, false);
+            r.store_strided(staged(i, half));
+          }
+        }
+      }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  fetch(task);
+  int64_t page = lp >= 0 && lp < kv.bt_stride ? (int64_t)kv.block_table[b * kv.bt_stride + lp] : -1;
+  const bool page_ok = page >= 0 && page < kv.num_pages;
+  if (rope_cos) {
+    const bool rvec = ((reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin)) & 15) == 0;
+#pragma unroll 1
+    for (int i = threadIdx.x * 8; i < 2 * TOK * HALF; i += 256 * 8) {      // eight elements of cos, then of sin
+      const int at = i < TOK * HALF ? i : i - TOK * HALF;
+      int64_t p = p0 + at / HALF;
+      p = p < 0 ? 0 : (p >= rope_rows ? rope_rows - 1 : p);
+      Raw8<float> f;
+      f.load((i < TOK * HALF ? rope_cos : rope_sin) + p * HALF + at % HALF, rvec);
+      Raw8<T> r;
+      round8(f, r);
+      r.store(&(i < TOK * HALF ? smem.cos : smem.sin)[at / HALF][at % HALF], true);
+    }
+    __syncthreads();
+  }
   for (; task < 2 * kv.hkv; task += task_step) {
     const int h = task >> 1;
     const bool is_v = task & 1;
     uint8_t* rec = (is_v ? kv.v_pool : kv.k_pool) + ((page_ok ? page : 0) * kv.hkv + h) * rec_bytes;
-    const T* src = (is_v ? v : k) + (int64_t)h * D + eg * 8;
-    const int64_t stride = is_v ? vs_ : ks;
-    const bool vec = is_v ? vvec : kvec;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     Raw8<T> x[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (tok[i] && page_ok) {
-        const T* p = src + (b * Tn + j0 + i) * stride;
-        x[i][0].load(p, vec); x[i][1].load(p + HALF, vec);
+      if (tok[i]) {
+        x[i][0].load_strided(staged(i, 0)); x[i][1].load_strided(staged(i, 1));
       } else {
         x[i][0] = x[i][1] = Raw8<T>{};
       }
     }
-    const Divisor shared = divisor(FMT == TSB200_KV_FP8 ? (is_v ? kv.v_scale : kv.k_scale)[b * kv.hkv + h] : 1.f);
+    const Divisor shared = divisor(fp8_scale);
+    __syncwarp();                              // read: the next task's elements may come
+    fetch(task + task_step);
+    // FP8, bf16: what lies beyond 512 scales saturates as that does (e4m3 ends at 448), without an infinite quotient on the way
+    unsigned bound = 0x7f807f80u;
+    if (FMT == TSB200_KV_FP8 && sizeof(T) == 2 && !shared.slow) {
+      const __nv_bfloat162 c2 = __bfloat162bfloat162(__float2bfloat16_ru(shared.d * 512.0f));
+      bound = *reinterpret_cast<const unsigned*>(&c2);
+    }
     // one vector's codes: per token two words per half (8-bit formats) or one, and its scale(s)
     auto encode = [&](Raw8<T> (&a)[2], unsigned (&c)[4], float& s8, unsigned (&sb)[2]) {
       float f[2][8];
+      if constexpr (FMT == TSB200_KV_FP8 && sizeof(T) == 2) { a[0].clamp(bound); a[1].clamp(bound); }
       a[0].unpack(f[0]);
       a[1].unpack(f[1]);
       if (FMT == TSB200_KV_FP8) {
-        encode8<FMT>(f[0], shared, c[0], c[1]);
-        encode8<FMT>(f[1], shared, c[2], c[3]);
+        encode8<T, FMT>(f[0], shared, c[0], c[1]);
+        encode8<T, FMT>(f[1], shared, c[2], c[3]);
       } else if (FMT == TSB200_KV_INT8) {
         float m = a[1].amax(a[0].amax(0.f));
 #pragma unroll
         for (int o = 1; o < EG; o *= 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         s8 = m > 0.f ? __fdiv_rn(m, 127.0f) : 0.f;         // 0 (slots outside the chunk) takes the division's slow path
         const Divisor d = divisor(__fadd_rn(s8, 1e-6f));
-        encode8<FMT>(f[0], d, c[0], c[1]);
-        encode8<FMT>(f[1], d, c[2], c[3]);
+        encode8<T, FMT>(f[0], d, c[0], c[1]);
+        encode8<T, FMT>(f[1], d, c[2], c[3]);
       } else {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
@@ -465,7 +561,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
           sb[g] = m > 0.f ? (unsigned)__nv_cvt_float_to_fp8(__fdiv_rn(m, 6.0f), __NV_SATFINITE, __NV_E4M3) : 0u;
           Divisor d = divisor(e4m3_to_f32((unsigned char)sb[g]));
           d.slow = m > 3.4028235e38f;                                    // the scale is one of e4m3's, or 0 and not divided by
-          encode8<FMT>(f[g], d, c[2 * g], c[2 * g + 1]);
+          encode8<T, FMT>(f[g], d, c[2 * g], c[2 * g + 1]);
         }
       }
     };
@@ -474,8 +570,8 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
       for (int i = 0; i < 4; ++i) {
         if (rope_cos) {
           Raw8<T> cc, ss;
-          cc.load_shared(&s_cos[lt + i][eg * 8]);
-          ss.load_shared(&s_sin[lt + i][eg * 8]);
+          cc.load_shared(&smem.cos[lt + i][eg * 8]);
+          ss.load_shared(&smem.sin[lt + i][eg * 8]);
           rope8(x[i][0], x[i][1], cc, ss);
         }
         unsigned c[4], sb[2];
@@ -514,9 +610,10 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
     }
     // row of word (g, j): 8-bit: element g / 2 * HALF + 8 eg + 4 (g & 1) + j; NVFP4: pair g * HALF / 2 + 4 eg + j
     auto row_of = [&](int g, int j) { return FP4 ? g * (HALF / 2) + eg * 4 + j : (g >> 1) * HALF + eg * 8 + (g & 1) * 4 + j; };
-    auto swz = [](int r) { return (r & ~7) | ((r ^ (r >> 3)) & 7); };     // rows that a store meets fall into different banks
+    // rows that a store meets fall into different banks: the low three bits of a row are exchanged by the next three
+    auto swz = [](int r) { return (r & ~7) | ((r ^ (r >> 3)) & 7); };
     if (__any_sync(0xffffffffu, full && page_ok)) {
-      unsigned* sv = s_v[w][page_of_lane];
+      unsigned* sv = smem.v[w >> 1][page_of_lane];
       __syncwarp();
 #pragma unroll
       for (int g = 0; g < GROUPS; ++g)
@@ -532,7 +629,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
         if (go) {
 #pragma unroll
           for (int r = lane; r < ROWS; r += 32)
-            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>((uintptr_t)dst) + r * 16) = *reinterpret_cast<const uint4*>(&s_v[w][pg][swz(r) * 4]);
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>((uintptr_t)dst) + r * 16) = *reinterpret_cast<const uint4*>(&smem.v[w >> 1][pg][swz(r) * 4]);
         }
       }
     }
@@ -574,8 +671,8 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
       if (tok[i]) {
         T* qp = q + (b * Tn + j0 + i) * qs + (int64_t)h * D + eg * 8;
         Raw8<T> cc, ss;
-        cc.load_shared(&s_cos[lt + i][eg * 8]);
-        ss.load_shared(&s_sin[lt + i][eg * 8]);
+        cc.load_shared(&smem.cos[lt + i][eg * 8]);
+        ss.load_shared(&smem.sin[lt + i][eg * 8]);
         rope8(x[i][0], x[i][1], cc, ss);
         x[i][0].store(qp, qvec); x[i][1].store(qp + HALF, qvec);
       }
@@ -630,17 +727,8 @@ kv_fp8_scales_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k
       Raw8<float> c, s;
       c.load(rope_cos + p * HALF + eg * 8, rvec);
       s.load(rope_sin + p * HALF + eg * 8, rvec);
-      if constexpr (sizeof(T) == 2) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const __nv_bfloat162 c2 = __floats2bfloat162_rn(c.f[2 * i], c.f[2 * i + 1]), s2 = __floats2bfloat162_rn(s.f[2 * i], s.f[2 * i + 1]);
-          cc.u[i] = *reinterpret_cast<const unsigned*>(&c2);
-          ss.u[i] = *reinterpret_cast<const unsigned*>(&s2);
-        }
-      } else {
-        cc = *reinterpret_cast<Raw8<T>*>(&c);
-        ss = *reinterpret_cast<Raw8<T>*>(&s);
-      }
+      round8(c, cc);
+      round8(s, ss);
 #pragma unroll
       for (int h = 0; h < G; ++h) rope8(x[h][0], x[h][1], cc, ss);
     }
@@ -692,16 +780,24 @@ int launch_append(const tsb200_kv_desc& kv, void* q, int64_t qs, int qheads, con
     int64_t z = 444 / (groups * B);
     if (z > (tasks + 7) / 8) z = (tasks + 7) / 8;
     const dim3 grid((unsigned)groups, (unsigned)B, (unsigned)(z < 1 ? 1 : z));
-    switch (kv.format) {
-      case TSB200_KV_INT8:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_INT8>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
-        break;
-      case TSB200_KV_FP8:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_FP8>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
-        break;
-      default:
-        TSB_CUDA(launch_kernel(kv_append_pages_kernel<T, D, TSB200_KV_NVFP4>, grid, dim3(256), 0, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec));
-    }
+    auto go = [&](auto fmt) {
+      constexpr int FMT = decltype(fmt)::value;
+      constexpr size_t smem = sizeof(AppendSmem<T, D, FMT>);
+      static bool configured[64] = {false};
+      int dev = 0;
+      cudaError_t e = cudaGetDevice(&dev);
+      if (e != cudaSuccess) return e;
+      if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+      if (!configured[dev]) {
+        e = cudaFuncSetAttribute(kv_append_pages_kernel<T, D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+      }
+      return launch_kernel(kv_append_pages_kernel<T, D, FMT>, grid, dim3(256), smem, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec);
+    };
+    if (kv.format == TSB200_KV_INT8) TSB_CUDA(go(std::integral_constant<int, TSB200_KV_INT8>{}));
+    else if (kv.format == TSB200_KV_FP8) TSB_CUDA(go(std::integral_constant<int, TSB200_KV_FP8>{}));
+    else TSB_CUDA(go(std::integral_constant<int, TSB200_KV_NVFP4>{}));
     TSB_LAUNCH_CHECK();
     return TSB200_OK;
   }
