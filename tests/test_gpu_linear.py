@@ -515,3 +515,30 @@ def test_argmax_of_rows(cuda, name, M, N):
         y[2, 0] = -0.0
         y[2, N - 1] = float("nan") if N > 5 else 0.0
     assert torch.equal(ops.argmax(y.to(cuda)).cpu(), torch.argmax(y.float(), -1))
+
+
+@pytest.mark.parametrize("M,K,N,r", [(16, 64, 33, 0), (31, 72, 31, 0), (33, 328, 100, 0), (64, 1032, 40, 0),      # one K rank, two, eight (the last two of which have nothing)
+                                     (65, 4872, 129, 0), (128, 896, 4864, 128), (130, 136, 9480, 0), (300, 264, 4100, 40)])   # 32 x 32 and 64 x 64 tiles
+def test_fp32_prompt_tiles(cuda, M, K, N, r):
+    """Dense fp32 layers at prompt sizes: ragged tiles in both directions, K split over a cluster; single layers, a group and the gated pair.
+    A sum of K products in fp32 is within about K^0.5 2^-24 of its terms' size of the exact one: 1e-5 of the largest output covers K = 4872."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(52)
+    def layer(o, i):
+        f = lambda a, b: ops.Factor.dense(torch.randn((a, b), generator=g, device=cuda) * b ** -0.5)
+        return ops.PackedLinear(f(o, r or i), f(r, i) if r else None, torch.randn(o, generator=g, device=cuda), torch.float32)
+    def exact(l, x):
+        h = x.double() @ l.v.data.double().T if l.v is not None else x.double()
+        return h @ l.u.data.double().T + l.bias.double()
+    a, b = layer(N, K), layer(N, K)
+    x = torch.randn((M, K), generator=g, device=cuda)
+    y = a(x)
+    assert rel_err(y.cpu(), exact(a, x).cpu()) < 1e-5
+    assert torch.equal(y, a(x))
+    for o, l in zip(ops.LinearGroup([a, layer(7, K), b])(x), (a, None, b)):
+        if l is not None:
+            assert rel_err(o.cpu(), exact(l, x).cpu()) < 1e-5
+    I = (N + 7) // 8 * 8                                     # (the down projection reads whole 16-byte pieces)
+    gate, up, down = layer(I, K), layer(I, K), layer(K, I)
+    ref = exact(down, torch.nn.functional.silu(exact(gate, x)) * exact(up, x))
+    assert rel_err(ops.GatedMLP(gate, up, down)(x).cpu(), ref.cpu()) < 2e-5

@@ -30,6 +30,7 @@ struct Seg {
 struct F32Params {
   Seg seg[kMaxSegs];
   int nseg, M, K, ks_log2;
+  int k_rank;                                // tiles: columns of a cluster rank
   int64_t row_bytes;
 };
 
@@ -222,87 +223,180 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
   }
 }
 
-// Prompt-sized token counts on dense factors: 64 tokens x 64 rows per CTA, 4 x 4 sums per thread, K in steps of 32 through shared
-// memory (k-major, so that a thread's operands are two 16-byte reads per k and matrix); the next step is fetched into registers
-// while this one is used.  The kernel above reduces over the lanes and pays 31 shuffles per 32 sums, which at a rank of 128 is as
-// much as the products: 128 tokens, gate | up 4864 x 128: 120 us there, 16 here.
-constexpr int kTM = 64, kTN = 64, kTK = 32;
-template <bool GATED>
-__global__ void __launch_bounds__(256) linear_f32_tile_kernel(const __grid_constant__ F32Params p) {
-  constexpr int MATS = GATED ? 2 : 1;
-  __shared__ __align__(16) float sx[MATS][kTK][kTM + 4], sw[MATS][kTK][kTN + 4];
+// Prompt-sized token counts on dense factors: TM tokens x TN rows per CTA, 4 x 4 sums per thread, K in steps of 64 through a ring of
+// shared memory filled by cp.async (rows as they lie in memory; the pitch of 68 floats puts the eight rows of a read into different
+// banks).  Bound by FMAs where the tiles fill the machine, by their number otherwise: with 32 x 32 tiles a CTA's four groups of 64
+// threads take 16 of every step's 64 columns each, and where even those tiles are few a cluster of up to eight CTAs splits K and adds
+// its partial tiles through distributed shared memory.
+//
+// Cold weights, both factors of a layer (before: 64 x 64 tiles transposed on their way into shared memory from 64 tokens on, the lane
+// kernel below that and for few rows): 128 tokens, 896 -> 128 -> 4864 28.2 -> 14.9 us, 4864 -> 128 -> 896 43.2 -> 19.2; 64 tokens, 3584 -> 224 ->
+// 3584 43.8 -> 17.9; full rank, 16 tokens, 4096 -> 6144 273 -> 77, 48 tokens, 14336 -> 4096 492 -> 262, 128 tokens, 18944 -> 3584 1249 -> 677 (26
+// of the 70 TFLOP/s of the FMA pipe: eight 16-byte reads of shared memory to 64 FMAs).
+constexpr int kTK = 64, kTPitch = kTK + 4;
+template <bool GATED> struct TileCfg {
+  static constexpr int kMats = GATED ? 2 : 1, kStages = GATED ? 2 : 3;
+};
+template <bool GATED, int TM, int TN> constexpr int tile_smem() { return TileCfg<GATED>::kStages * TileCfg<GATED>::kMats * (TM + TN) * kTPitch * 4; }
+
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool in) {   // !in: zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+template <bool GATED, int TM, int TN>
+__global__ void __launch_bounds__(256, 2) linear_f32_tile_kernel(const __grid_constant__ F32Params p) {
+  constexpr int MATS = TileCfg<GATED>::kMats, STAGES = TileCfg<GATED>::kStages;
+  constexpr int TX = TN / 4, TY = TM / 4, KG = 256 / (TX * TY), KK = kTK / KG;
+  constexpr int RP = TN + 8;                                         // pitch of a partial tile
+  static_assert(KG * MATS * TM * RP * 4 <= tile_smem<GATED, TM, TN>(), "partial tiles replace the ring");
+  extern __shared__ __align__(16) float tile_ring[];                 // [stage][matrix][x rows, then w rows][kTPitch]
   int si = 0;
   while (si + 1 < p.nseg && (int)blockIdx.x >= p.seg[si + 1].cta0) ++si;
   const Seg& sg = p.seg[si];
-  const int n0 = ((int)blockIdx.x - sg.cta0) * kTN, m0 = blockIdx.y * kTM;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;         // rows 4 tx .., tokens 4 ty ..
+  const int n0 = ((int)blockIdx.x - sg.cta0) * TN, m0 = blockIdx.y * TM;
+  const int tid = threadIdx.x, kg = tid / (TX * TY), tx = tid % TX, ty = tid / TX % TY;
+  const int rank = blockIdx.z, ranks = gridDim.z;
+  const int k_beg = rank * p.k_rank, k_end = min(p.K, k_beg + p.k_rank);   // (may be empty)
+  const int steps = k_end > k_beg ? (k_end - k_beg + kTK - 1) / kTK : 0;
   pdl_launch_dependents();
-  // a thread fetches 16-byte pieces lk of tile rows lr and lr + 32, of x and of W
-  const int lk = (tid & 7) * 4, lr = tid >> 3;
-  float4 fx[MATS][2], fw[MATS][2];
-  auto fetch_w = [&](int k0) {
+  auto stage_at = [&](int slot, int mat, int row) { return tile_ring + ((slot * MATS + mat) * (TM + TN) + row) * kTPitch; };
+  auto copy_w = [&](int st) {
 #pragma unroll
     for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float* w = reinterpret_cast<const float*>(mat ? sg.w2 : sg.w) + (int64_t)min(n0 + lr + 32 * h, sg.n - 1) * p.K;
-        fw[mat][h] = k0 + lk < p.K ? __ldg(reinterpret_cast<const float4*>(w + k0 + lk)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = tid; i < TN * (kTK / 4); i += 256) {
+        const int row = i / (kTK / 4), k = k_beg + st * kTK + i % (kTK / 4) * 4;
+        const float* w = reinterpret_cast<const float*>(mat ? sg.w2 : sg.w);
+        const bool in = k < k_end && n0 + row < sg.n;
+        cp_async16(stage_at(st % STAGES, mat, TM + row) + i % (kTK / 4) * 4, in ? w + (int64_t)(n0 + row) * p.K + k : w, in);
       }
   };
-  auto fetch_x = [&](int k0) {
+  auto copy_x = [&](int st) {
 #pragma unroll
     for (int mat = 0; mat < MATS; ++mat)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float* x = (mat ? sg.x2 : sg.x) + (int64_t)min(m0 + lr + 32 * h, p.M - 1) * p.K;
-        fx[mat][h] = k0 + lk < p.K ? *reinterpret_cast<const float4*>(x + k0 + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = tid; i < TM * (kTK / 4); i += 256) {
+        const int row = i / (kTK / 4), k = k_beg + st * kTK + i % (kTK / 4) * 4;
+        const float* x = mat ? sg.x2 : sg.x;
+        const bool in = k < k_end && m0 + row < p.M;
+        cp_async16(stage_at(st % STAGES, mat, row) + i % (kTK / 4) * 4, in ? x + (int64_t)(m0 + row) * p.K + k : x, in);
       }
   };
-  fetch_w(0);
+#pragma unroll
+  for (int st = 0; st < STAGES - 1; ++st)
+    if (st < steps) copy_w(st);                                      // constants: ahead of the dependency wait
   pdl_wait();
-  fetch_x(0);
+#pragma unroll
+  for (int st = 0; st < STAGES - 1; ++st) {
+    if (st < steps) copy_x(st);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
   float acc[MATS][4][4] = {};
-  for (int k0 = 0; k0 < p.K; k0 += kTK) {
-    __syncthreads();
+  for (int st = 0; st < steps; ++st) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                                 // the step has landed; every warp is done with the one before
+    if (st + STAGES - 1 < steps) { copy_w(st + STAGES - 1); copy_x(st + STAGES - 1); }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 #pragma unroll
-    for (int mat = 0; mat < MATS; ++mat)
+    for (int mat = 0; mat < MATS; ++mat) {
+      const float* xs = stage_at(st % STAGES, mat, ty) + kg * KK;
+      const float* ws = stage_at(st % STAGES, mat, TM + tx) + kg * KK;
+#pragma unroll 1
+      for (int k0 = 0; k0 < KK; k0 += 16) {                          // sums of 8 products, added in pairs: chains of 8 and K / 16 additions, not of K
+        float pair[4][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float a[4] = {fx[mat][h].x, fx[mat][h].y, fx[mat][h].z, fx[mat][h].w};
-        const float b[4] = {fw[mat][h].x, fw[mat][h].y, fw[mat][h].z, fw[mat][h].w};
+        for (int half = 0; half < 2; ++half) {
+          float part[4][4] = {};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          sx[mat][lk + j][lr + 32 * h] = a[j];
-          sw[mat][lk + j][lr + 32 * h] = b[j];
+          for (int k = k0 + 8 * half; k < k0 + 8 * half + 8; k += 4) {
+            float4 xv[4], wv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              xv[i] = *reinterpret_cast<const float4*>(xs + i * TY * kTPitch + k);
+              wv[i] = *reinterpret_cast<const float4*>(ws + i * TX * kTPitch + k);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                part[i][j] += xv[i].x * wv[j].x;
+                part[i][j] += xv[i].y * wv[j].y;
+                part[i][j] += xv[i].z * wv[j].z;
+                part[i][j] += xv[i].w * wv[j].w;
+              }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (half == 0) pair[i][j] = part[i][j];
+              else acc[mat][i][j] += pair[i][j] + part[i][j];
+            }
         }
       }
-    __syncthreads();
-    if (k0 + kTK < p.K) { fetch_w(k0 + kTK); fetch_x(k0 + kTK); }
-#pragma unroll
-    for (int k = 0; k < kTK; ++k)
-#pragma unroll
-      for (int mat = 0; mat < MATS; ++mat) {
-        const float4 xa = *reinterpret_cast<const float4*>(&sx[mat][k][ty * 4]), wa = *reinterpret_cast<const float4*>(&sw[mat][k][tx * 4]);
-        const float xv[4] = {xa.x, xa.y, xa.z, xa.w}, wv[4] = {wa.x, wa.y, wa.z, wa.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[mat][i][j] += xv[i] * wv[j];
-      }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= p.M) break;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= sg.n) break;
-      float v = acc[0][i][j] + (sg.bias ? sg.bias[n] : 0.f);
-      if (GATED) v = __fmul_rn(v / (1.0f + expf(-v)), acc[MATS - 1][i][j] + (sg.bias2 ? sg.bias2[n] : 0.f));
-      sg.y[(int64_t)m * sg.n + n] = v;
     }
   }
+  // ---- partial tiles [group][matrix][token][row], then one value per (matrix, token, row)
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tile_ring[((kg * MATS + mat) * TM + ty + TY * i) * RP + tx + TX * j] = acc[mat][i][j];
+  __syncthreads();
+  auto sum_groups = [&](int mat, int at) {
+    static_assert(KG == 1 || KG == 4, "groups");
+    auto part = [&](int g) { return tile_ring[((g * MATS + mat) * TM) * RP + at]; };
+    return KG == 1 ? part(0) : (part(0) + part(1)) + (part(2) + part(3));
+  };
+  auto store = [&](int idx, float v, float u) {
+    const int m = m0 + idx / TN, n = n0 + idx % TN;
+    if (m >= p.M || n >= sg.n) return;
+    v += sg.bias ? sg.bias[n] : 0.f;
+    if (GATED) v = __fmul_rn(v / (1.0f + expf(-v)), u + (sg.bias2 ? sg.bias2[n] : 0.f));
+    sg.y[(int64_t)m * sg.n + n] = v;
+  };
+  if (ranks == 1) {
+#pragma unroll
+    for (int idx = tid; idx < TM * TN; idx += 256) {
+      const int at = idx / TN * RP + idx % TN;
+      store(idx, sum_groups(0, at), GATED ? sum_groups(MATS - 1, at) : 0.f);
+    }
+    return;
+  }
+  if (KG > 1) {
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat)
+#pragma unroll
+      for (int idx = tid; idx < TM * TN; idx += 256) {
+        const int at = idx / TN * RP + idx % TN;
+        tile_ring[(mat * TM) * RP + at] = sum_groups(mat, at);       // read and written by this thread alone
+      }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  for (int idx = rank * (TM * TN / ranks) + tid; idx < (rank + 1) * (TM * TN / ranks); idx += 256) {
+    float v[MATS];
+#pragma unroll
+    for (int mat = 0; mat < MATS; ++mat) {
+      const unsigned own = tc::smem_u32(&tile_ring[(mat * TM + idx / TN) * RP + idx % TN]);
+      float f[8];                                                    // of the ranks, added in pairs
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        f[r] = 0.f;
+        if (r < ranks) {
+          unsigned a;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(own), "r"(r));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(f[r]) : "r"(a) : "memory");
+        }
+      }
+      v[mat] = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+    }
+    store(idx, v[0], v[MATS - 1]);
+  }
+  // no CTA leaves while another one may still read its tile
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 template <int BITS, int MT, int R, bool GATED>
@@ -351,36 +445,73 @@ int launch_bits(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
   return launch_cfg<BITS, 8, 4, false>(p, pdl, s);
 }
 
-// Tiles pay where K is short (up to two staged steps of the lanes) or where they fill most of the machine: with few tiles and a long
-// K the lane kernel has more warps (128 tokens, 384 x 896: 13 us there, 20 in 12 tiles).
+// Whether the tiles take a call: dense factors and at least 16 tokens.  Where the lane kernel stages a row's activations once (K <= 1024) and a
+// cluster cannot split K (many rows), only if the tokens, in the eights that it takes, fill more than three quarters of the tiles, which take
+// as long for one token of their 32 as for all (896 -> 4864, tiles / lane kernel: 32 tokens 18.6 / 22.8 us, 24 tokens - / 17.0, 56 tokens 29.4 /
+// 31.1, 40 tokens - / 24.2).  Elsewhere the lane kernel is the slower one by far (24 tokens, 4096 -> 14336 409 us, tiles 150; 3584 -> 3584 67, 41).
 bool use_tiles(const F32Params& p, int bits) {
-  if (bits != 32 || p.M < 16) return false;
+  if (bits != 32 || p.M < 16 || p.K % 4) return false;
   int64_t tiles = 0;
   for (int i = 0; i < p.nseg; ++i) {
-    tiles += (p.seg[i].n + kTN - 1) / kTN;
     if (!aligned(p.seg[i].x, 16) || (p.seg[i].x2 && !aligned(p.seg[i].x2, 16))) return false;
+    tiles += (p.seg[i].n + 31) / 32;
   }
-  return p.K <= 256 || tiles * ((p.M + kTM - 1) / kTM) >= 96;
+  return p.K <= 256 || p.K > kXFloats / 8 || tiles <= 148 || (p.M + 7) / 8 * 4 > (p.M + 31) / 32 * 12;
 }
-int launch_tiles(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
+template <bool GATED, int TM, int TN> int launch_tile(F32Params& p, int ranks, bool pdl, cudaStream_t s) {
+  constexpr int smem = tile_smem<GATED, TM, TN>();
+  static bool configured[64] = {false};
+  int dev = 0;
+  TSB_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return TSB200_ERR_DEVICE;
+  if (!configured[dev]) {
+    TSB_CUDA(cudaFuncSetAttribute(linear_f32_tile_kernel<GATED, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    configured[dev] = true;
+  }
   int ctas = 0;
   for (int i = 0; i < p.nseg; ++i) {
     p.seg[i].cta0 = ctas;
-    ctas += (p.seg[i].n + kTN - 1) / kTN;
+    ctas += (p.seg[i].n + TN - 1) / TN;
   }
-  const int groups = (p.M + kTM - 1) / kTM;
+  const int groups = (p.M + TM - 1) / TM;
   if (groups > 65535) return TSB200_ERR_UNSUPPORTED;
+  p.k_rank = ((p.K + kTK - 1) / kTK + ranks - 1) / ranks * kTK;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas, (unsigned)groups);
+  cfg.gridDim = dim3((unsigned)ctas, (unsigned)groups, (unsigned)ranks);
   cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (ranks > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = (unsigned)ranks;
+  }
+  if (pdl) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  TSB_CUDA(gated ? cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<true>, p) : cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<false>, p));
+  cfg.numAttrs = na;
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<GATED, TM, TN>, p));
   return TSB200_OK;
+}
+// 64 x 64 tiles where they give every SM two CTAs (half the shared-memory reads a sum), else 32 x 32, and K split over a cluster as long as
+// the two CTAs an SM holds still go round once and every rank keeps a step.
+int launch_tiles(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
+  int64_t t64 = 0, t32 = 0;
+  for (int i = 0; i < p.nseg; ++i) {
+    t64 += (p.seg[i].n + 63) / 64;
+    t32 += (p.seg[i].n + 31) / 32;
+  }
+  t64 *= (p.M + 63) / 64;
+  t32 *= (p.M + 31) / 32;
+  if (t64 >= 296) return gated ? launch_tile<true, 64, 64>(p, 1, pdl, s) : launch_tile<false, 64, 64>(p, 1, pdl, s);
+  int ranks = 1;
+  while (ranks < 8 && t32 * ranks * 2 <= 296 && p.K >= 2 * ranks * kTK) ranks *= 2;
+  return gated ? launch_tile<true, 32, 32>(p, ranks, pdl, s) : launch_tile<false, 32, 32>(p, ranks, pdl, s);
 }
 
 int launch_any(F32Params& p, int bits, bool gated, bool pdl, cudaStream_t s) {
