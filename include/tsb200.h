@@ -160,6 +160,20 @@ size_t tsb200_linear_group_workspace_bytes(const tsb200_linear_desc* const* d, i
 int tsb200_linear_group(const tsb200_linear_desc* const* d, int n, const void* x, void* const* y, int64_t M,
                         void* workspace, size_t workspace_bytes, void* stream);
 
+/* Normalised activations of a decode step: x = RMSNorm(residual + delta) * weight as tsb200_add_rmsnorm (variant 0) makes it, without its
+ * launch.  delta may be NULL; residual_out [M, in] takes residual + delta and must not overlap residual or delta. */
+typedef struct {
+  const void* residual;
+  const void* delta;
+  const void* weight;
+  void* residual_out;
+  float eps;
+} tsb200_norm_desc;
+/* tsb200_add_rmsnorm and tsb200_linear_group on its result, the same bits, for fp32 layers with alike factors (n <= 4, M <= 4, rows of at most
+ * 8192 / M elements, M = 3 counting as 4).  TSB200_ERR_UNSUPPORTED for others, before anything is launched. */
+int tsb200_norm_linear_group(const tsb200_norm_desc* norm, const tsb200_linear_desc* const* d, int n, void* const* y, int64_t M,
+                             void* workspace, size_t workspace_bytes, void* stream);
+
 /* Greedy head: tokens[m] = argmax_n (x . W^T + bias)[m, n] with the logits rounded to the act dtype first, i.e. the
  * token torch.argmax would pick from tsb200_linear's output (the first maximum on ties).
  * Replaces the final layer + argmax of a greedy decode step (export/common.py:167,175 for the blocks path; the
@@ -186,6 +200,10 @@ size_t tsb200_mlp_gated_workspace_bytes(const tsb200_linear_desc* gate, const ts
 int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* up,
                      const tsb200_linear_desc* down, const void* x, void* y, int64_t M,
                      void* workspace, size_t workspace_bytes, void* stream);
+/* The same behind a normalisation (see tsb200_norm_linear_group): fp32 layers, gate and up alike, M <= 4, rows of at most 8192 / M elements
+ * (4096 / M where gate and up have full rank); otherwise TSB200_ERR_UNSUPPORTED, before anything is launched. */
+int tsb200_norm_mlp_gated(const tsb200_norm_desc* norm, const tsb200_linear_desc* gate, const tsb200_linear_desc* up,
+                          const tsb200_linear_desc* down, void* y, int64_t M, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------
  * Quantized paged KV cache

@@ -542,3 +542,42 @@ def test_fp32_prompt_tiles(cuda, M, K, N, r):
     gate, up, down = layer(I, K), layer(I, K), layer(K, I)
     ref = exact(down, torch.nn.functional.silu(exact(gate, x)) * exact(up, x))
     assert rel_err(ops.GatedMLP(gate, up, down)(x).cpu(), ref.cpu()) < 2e-5
+
+
+@pytest.mark.parametrize("p", [None, 8, 4, 2, "binary"])
+@pytest.mark.parametrize("M,K,I,r", [(1, 896, 4864, 128), (2, 1000, 304, 0), (3, 72, 1024, 40), (4, 2048, 96, 24), (4, 1024, 96, 0), (1, 8192, 64, 8), (1, 4, 40, 0)])
+def test_fp32_projections_normalise_their_input(cuda, p, M, K, I, r):
+    """Groups and the gated block that take residual + delta: the bits of add_rmsnorm and of the separate calls, the residual included.  Rows
+    beyond one staged K tile and more than four tokens are declined."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(54)
+    def layer(o, i):
+        f = lambda a, b: (ops.Factor.dense if p is None else lambda w: ops.Factor.quantize(w, p))(torch.randn((a, b), generator=g, device=cuda) * b ** -0.5)
+        return ops.PackedLinear(f(o, r or i), f(r, i) if r else None, torch.randn(o, generator=g, device=cuda), torch.float32)
+    if p is None and K % 8:
+        K = 8
+    group = ops.LinearGroup([layer(33, K), layer(8, K), layer(40, K)])
+    mlp = ops.GatedMLP(layer(I, K), layer(I, K), layer(K, I))
+    residual, delta, w = (torch.randn(s, generator=g, device=cuda) for s in ((M, K), (M, K), (K,)))
+    ws = torch.zeros(max(group.workspace_bytes(8), mlp.workspace_bytes(8)), dtype=torch.uint8, device=cuda)
+    for d in (delta, None):
+        after = residual.clone()
+        xn = ops.add_rmsnorm(after, d, w, 1e-6)
+        for name in ("group", "mlp"):
+            kept = torch.empty_like(residual)
+            norm = ops.normalisation(residual, d, w, kept, 1e-6)
+            if name == "group":
+                outs, ref = [torch.empty((M, l.out_features), device=cuda) for l in group.layers], group(xn)
+                assert group.after_norm(norm, M, outs, ws)
+            else:
+                outs, ref = [torch.empty((M, K), device=cuda)], [mlp(xn)]
+                assert mlp.after_norm(norm, M, outs[0], ws)
+            assert torch.equal(kept, after)
+            assert all(torch.equal(a, b) for a, b in zip(outs, ref))
+    big = torch.randn((5, K), generator=g, device=cuda)
+    outs = [torch.zeros((5, l.out_features), device=cuda) for l in group.layers]
+    assert not group.after_norm(ops.normalisation(big, None, w, torch.empty_like(big), 1e-6), 5, outs, ws)
+    assert not any(o.any() for o in outs)
+    for l in group.layers:
+        l.force_simt = True
+    assert not group.after_norm(ops.normalisation(residual, None, w, torch.empty_like(residual), 1e-6), M, outs, ws)

@@ -40,8 +40,12 @@ class PeerDesc(C.Structure):
                 ("epoch", C.c_void_p), ("status", C.c_void_p)]
 
 
+class NormDesc(C.Structure):
+    _fields_ = [("residual", C.c_void_p), ("delta", C.c_void_p), ("weight", C.c_void_p), ("residual_out", C.c_void_p), ("eps", C.c_float)]
+
+
 _i64, _i32, _f32, _vp, _sz = C.c_int64, C.c_int, C.c_float, C.c_void_p, C.c_size_t
-_LD, _KD, _PD = C.POINTER(LinearDesc), C.POINTER(KVDesc), C.POINTER(PeerDesc)
+_LD, _KD, _PD, _ND = C.POINTER(LinearDesc), C.POINTER(KVDesc), C.POINTER(PeerDesc), C.POINTER(NormDesc)
 
 # name -> (restype, argtypes); mirrors include/tsb200.h one to one.
 SIGNATURES = {
@@ -61,11 +65,13 @@ SIGNATURES = {
     "tsb200_linear_simt": (_i32, [_LD, _vp, _vp, _i64, _vp, _sz, _vp]),
     "tsb200_linear_group_workspace_bytes": (_sz, [C.POINTER(_LD), _i32, _i64]),
     "tsb200_linear_group": (_i32, [C.POINTER(_LD), _i32, _vp, C.POINTER(_vp), _i64, _vp, _sz, _vp]),
+    "tsb200_norm_linear_group": (_i32, [_ND, C.POINTER(_LD), _i32, C.POINTER(_vp), _i64, _vp, _sz, _vp]),
     "tsb200_linear_argmax_workspace_bytes": (_sz, [_LD, _i64]),
     "tsb200_linear_argmax": (_i32, [_LD, _vp, _vp, _i64, _vp, _sz, _vp]),
     "tsb200_argmax": (_i32, [_vp, _i32, _i64, _i64, _vp, _vp]),
     "tsb200_mlp_gated_workspace_bytes": (_sz, [_LD, _LD, _LD, _i64]),
     "tsb200_mlp_gated": (_i32, [_LD, _LD, _LD, _vp, _vp, _i64, _vp, _sz, _vp]),
+    "tsb200_norm_mlp_gated": (_i32, [_ND, _LD, _LD, _LD, _vp, _i64, _vp, _sz, _vp]),
     "tsb200_kv_record_bytes": (_sz, [_i32, _i32]),
     "tsb200_kv_fp8_scales": (_i32, [_vp, _vp, _i32, _i64, _i64, _i32, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp]),
     "tsb200_kv_fp8_scales_strided": (_i32, [_vp, _vp, _i32, _i64, _i64, _i64, _i64, _i32, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp]),

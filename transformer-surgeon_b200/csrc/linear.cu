@@ -56,7 +56,8 @@ bool f32_factor(int bits) { return bits == 32 || (bits <= 8); }
 
 // fp32 activations: both factors on the FMA kernel, the second launch chained to the first; n layers that read the same x go
 // through together when their factors are alike.  h: the rank-r intermediates, one behind the other.
-int linear_f32(const tsb200_linear_desc* const* d, int n, const void* x, void* const* y, int64_t M, float* h, cudaStream_t s) {
+int linear_f32(const tsb200_linear_desc* const* d, int n, const void* x, void* const* y, int64_t M, float* h, cudaStream_t s,
+               const tsb200_norm_desc* norm = nullptr) {
   GemmSpec v[4], u[4];
   const bool low = d[0]->rank > 0;
   for (int i = 0; i < n; ++i) {
@@ -67,10 +68,10 @@ int linear_f32(const tsb200_linear_desc* const* d, int n, const void* x, void* c
     h += M * d[i]->rank;
   }
   if (low) {
-    const int st = gemm_f32(v, n, d[0]->v_bits, M, g_pdl != 0, s);
+    const int st = gemm_f32(v, n, d[0]->v_bits, M, g_pdl != 0, s, norm);
     if (st != TSB200_OK) return st;
   }
-  return gemm_f32(u, n, d[0]->u_bits, M, low || g_pdl, s);
+  return gemm_f32(u, n, d[0]->u_bits, M, low || g_pdl, s, low ? nullptr : norm);
 }
 
 bool alike(const tsb200_linear_desc* a, const tsb200_linear_desc* b) {
@@ -119,6 +120,23 @@ extern "C" int tsb200_linear_group(const tsb200_linear_desc* const* d, int n, co
     if (st != TSB200_OK) return st;
   }
   return TSB200_OK;
+}
+
+extern "C" int tsb200_norm_linear_group(const tsb200_norm_desc* norm, const tsb200_linear_desc* const* d, int n, void* const* y, int64_t M, void* workspace,
+                                        size_t workspace_bytes, void* stream) {
+  TSB_REQUIRE_DEVICE();
+  if (!norm || !norm->residual || !norm->weight || !norm->residual_out || norm->residual_out == norm->residual || !d || !y || n < 1) return TSB200_ERR_ARG;
+  bool noop = false;
+  for (int i = 0; i < n; ++i) {
+    const int st = validate_linear(d[i], norm->residual, y[i], M, noop);
+    if (st != TSB200_OK) return st;
+    if (!alike(d[0], d[i])) return TSB200_ERR_UNSUPPORTED;
+  }
+  if (noop) return TSB200_OK;
+  if (n > 4 || d[0]->act_dtype != TSB200_F32) return TSB200_ERR_UNSUPPORTED;
+  if (!workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
+  if (workspace_bytes < tsb200_linear_group_workspace_bytes(d, n, M)) return TSB200_ERR_WORKSPACE;
+  return linear_f32(d, n, nullptr, y, M, (float*)((uint8_t*)workspace + tc::kWsHeader), as_stream(stream), norm);
 }
 
 extern "C" int tsb200_linear(const tsb200_linear_desc* d, const void* x, void* y, int64_t M, void* workspace,

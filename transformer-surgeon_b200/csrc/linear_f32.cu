@@ -10,6 +10,7 @@
 //
 // Up to four matrices that share the reduction length run as one launch (q | k | v, gate | up), and the second factors of a gate /
 // up pair end in SiLU(g) * u (blocks/mlp.py:181-183).
+#include <type_traits>
 #include "tc_common.cuh"
 
 namespace tsb {
@@ -27,8 +28,14 @@ struct Seg {
   float* y;
   int n, cta0;                               // rows; first CTA
 };
+struct Norm {                                // x = RMSNorm(residual + delta) * w; w: null where x is given
+  const float *residual, *delta, *w;
+  float* out;                                // residual + delta
+  float eps;
+};
 struct F32Params {
   Seg seg[kMaxSegs];
+  Norm norm;
   int nseg, M, K, ks_log2;
   int k_rank;                                // tiles: columns of a cluster rank
   int64_t row_bytes;
@@ -88,7 +95,61 @@ template <int V> __device__ __forceinline__ float reduce_scatter(float (&v)[V]) 
   return s;
 }
 
-template <int BITS, int MT, int R, bool GATED>
+// Activations that are the RMSNorm of residual + delta, staged by every CTA for itself (rows of one K tile): a decode step's separate
+// normalisation is a launch of its own in the chain, ~2.3 us, of which this adds back a reduction over the CTA.  The arithmetic and the
+// order of its sums are add_rmsnorm_hf_kernel's (elementwise.cu): the same bits.  The first CTA keeps the new residual.
+template <int MATS, int MT, int KT>
+__device__ __forceinline__ void stage_normalised(const F32Params& p, const float4& nw, float (&xs)[MATS][MT][KT], float (&red)[kWarps][32]) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float ss[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) ss[m] = 0.f;
+  for (int i = tid * 4; i < ((p.K + 31) & ~31); i += kWarps * 128)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m < p.M && i < p.K) {
+        const int64_t at = (int64_t)m * p.K + i;
+        v = *reinterpret_cast<const float4*>(p.norm.residual + at);
+        if (p.norm.delta) {
+          const float4 d = *reinterpret_cast<const float4*>(p.norm.delta + at);
+          v.x = __fadd_rn(v.x, d.x); v.y = __fadd_rn(v.y, d.y); v.z = __fadd_rn(v.z, d.z); v.w = __fadd_rn(v.w, d.w);
+        }
+        if (blockIdx.x == 0) *reinterpret_cast<float4*>(p.norm.out + at) = v;
+        ss[m] += v.x * v.x; ss[m] += v.y * v.y; ss[m] += v.z * v.z; ss[m] += v.w * v.w;
+      }
+      *reinterpret_cast<float4*>(&xs[0][m][i]) = v;
+    }
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    ss[m] = warp_sum(ss[m]);
+    if (lane == 0) red[warp][m] = ss[m];
+  }
+  __syncthreads();
+  float inv[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const float var = warp_sum(lane < kWarps ? red[lane][m] : 0.f) / (float)p.K;
+    inv[m] = 1.0f / sqrtf(var + p.norm.eps);
+  }
+  for (int i = tid * 4; i < p.K; i += kWarps * 128) {                 // the pieces that this thread has staged
+    const float4 w = i == tid * 4 ? nw : __ldg(reinterpret_cast<const float4*>(p.norm.w + i));
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      float4 v = *reinterpret_cast<const float4*>(&xs[0][m][i]);
+      v.x = __fmul_rn(w.x, __fmul_rn(v.x, inv[m])); v.y = __fmul_rn(w.y, __fmul_rn(v.y, inv[m]));
+      v.z = __fmul_rn(w.z, __fmul_rn(v.z, inv[m])); v.w = __fmul_rn(w.w, __fmul_rn(v.w, inv[m]));
+#pragma unroll
+      for (int mat = 0; mat < MATS; ++mat) *reinterpret_cast<float4*>(&xs[mat][m][i]) = v;
+    }
+  }
+  if (MATS > 1)
+    for (int i = p.K + tid; i < ((p.K + 31) & ~31); i += kWarps * 32)
+#pragma unroll
+      for (int m = 0; m < MT; ++m) xs[MATS - 1][m][i] = 0.f;
+}
+
+template <int BITS, int MT, int R, bool GATED, bool NORM>
 __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_constant__ F32Params p) {
   constexpr int MATS = GATED ? 2 : 1;
   using P = Piece<BITS, MT>;
@@ -135,16 +196,20 @@ __global__ void __launch_bounds__(kWarps * 32) linear_f32_kernel(const __grid_co
     const uintptr_t a = (reinterpret_cast<uintptr_t>(q) + 15) & ~(uintptr_t)15, e = (reinterpret_cast<uintptr_t>(q) + p.row_bytes) & ~(uintptr_t)15;
     if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
   }
+  float4 nw = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (NORM && tid * 4 < p.K) nw = __ldg(reinterpret_cast<const float4*>(p.norm.w + tid * 4));
   pdl_wait();
 
   float acc[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = 0.f;
+  if constexpr (NORM) stage_normalised<MATS, MT, kKT>(p, nw, xs, red);
   for (int k0 = 0; k0 < p.K; k0 += kKT) {
     const int kt = min(kKT, p.K - k0);
     __syncthreads();
 #pragma unroll
     for (int mat = 0; mat < MATS; ++mat) {
+      if (NORM) break;
       const float* x = mat ? sg.x2 : sg.x;
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
@@ -399,7 +464,7 @@ __global__ void __launch_bounds__(256, 2) linear_f32_tile_kernel(const __grid_co
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <int BITS, int MT, int R, bool GATED>
+template <int BITS, int MT, int R, bool GATED, bool NORM>
 int launch_cfg(F32Params& p, bool pdl, cudaStream_t s) {
   // K split: enough CTAs for the machine with one token (148 SMs x 2), at least one piece per lane and warp
   int rows = 0;
@@ -426,23 +491,28 @@ int launch_cfg(F32Params& p, bool pdl, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  TSB_CUDA(cudaLaunchKernelEx(&cfg, linear_f32_kernel<BITS, MT, R, GATED>, p));
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, linear_f32_kernel<BITS, MT, R, GATED, NORM>, p));
   return TSB200_OK;
 }
 
 template <int BITS>
 int launch_bits(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
+  if (p.norm.w && (p.M > 4 || p.K > kXFloats / ((gated ? 2 : 1) * (p.M == 1 ? 1 : (p.M == 2 ? 2 : 4))))) return TSB200_ERR_UNSUPPORTED;   // rows of one K tile
   // tokens per warp, and rows so that 32 sums fill the lanes where the tokens do not (few tokens: fewer rows, more warps)
-  if (gated) {
-    if (p.M == 1) return launch_cfg<BITS, 1, 2, true>(p, pdl, s);
-    if (p.M <= 2) return launch_cfg<BITS, 2, 2, true>(p, pdl, s);
-    if (p.M <= 4) return launch_cfg<BITS, 4, 2, true>(p, pdl, s);
-    return launch_cfg<BITS, 8, 2, true>(p, pdl, s);
-  }
-  if (p.M == 1) return launch_cfg<BITS, 1, 2, false>(p, pdl, s);
-  if (p.M <= 2) return launch_cfg<BITS, 2, 2, false>(p, pdl, s);
-  if (p.M <= 4) return launch_cfg<BITS, 4, 4, false>(p, pdl, s);
-  return launch_cfg<BITS, 8, 4, false>(p, pdl, s);
+  auto go = [&](auto norm) {
+    constexpr bool N = decltype(norm)::value;
+    if (gated) {
+      if (p.M == 1) return launch_cfg<BITS, 1, 2, true, N>(p, pdl, s);
+      if (p.M <= 2) return launch_cfg<BITS, 2, 2, true, N>(p, pdl, s);
+      return launch_cfg<BITS, 4, 2, true, N>(p, pdl, s);
+    }
+    if (p.M == 1) return launch_cfg<BITS, 1, 2, false, N>(p, pdl, s);
+    if (p.M <= 2) return launch_cfg<BITS, 2, 2, false, N>(p, pdl, s);
+    return launch_cfg<BITS, 4, 4, false, N>(p, pdl, s);
+  };
+  if (p.norm.w) return go(std::true_type{});
+  if (p.M <= 4) return go(std::false_type{});
+  return gated ? launch_cfg<BITS, 8, 2, true, false>(p, pdl, s) : launch_cfg<BITS, 8, 4, false, false>(p, pdl, s);
 }
 
 // Whether the tiles take a call: dense factors and at least 16 tokens.  Where the lane kernel stages a row's activations once (K <= 1024) and a
@@ -515,7 +585,7 @@ int launch_tiles(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
 }
 
 int launch_any(F32Params& p, int bits, bool gated, bool pdl, cudaStream_t s) {
-  if (use_tiles(p, bits)) return launch_tiles(p, gated, pdl, s);
+  if (!p.norm.w && use_tiles(p, bits)) return launch_tiles(p, gated, pdl, s);
   switch (bits) {
     case 1: return launch_bits<1>(p, gated, pdl, s);
     case 2: return launch_bits<2>(p, gated, pdl, s);
@@ -525,12 +595,19 @@ int launch_any(F32Params& p, int bits, bool gated, bool pdl, cudaStream_t s) {
   }
 }
 
+int take_norm(F32Params& p, const tsb200_norm_desc* norm) {
+  if (!norm) return TSB200_OK;
+  if (p.K % 4 || !aligned(norm->residual, 16) || !aligned(norm->residual_out, 16) || !aligned(norm->weight, 16) || !aligned(norm->delta, 16))
+    return TSB200_ERR_UNSUPPORTED;
+  p.norm = Norm{(const float*)norm->residual, (const float*)norm->delta, (const float*)norm->weight, (float*)norm->residual_out, norm->eps};
+  return TSB200_OK;
+}
 int64_t row_bytes(int64_t K, int bits) { return bits == 32 ? K * 4 : (int64_t)tsb200_packed_row_bytes(K, bits); }
 
 }  // namespace
 
 // n matrices [N_i, K] of one container as one launch; x[i] [M, K], y[i] [M, N_i].
-int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s) {
+int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s, const tsb200_norm_desc* norm) {
   F32Params p = {};
   if (n < 1 || n > kMaxSegs || M < 1 || M > 65535 * 8 || g[0].K > (1 << 30)) return TSB200_ERR_UNSUPPORTED;
   for (int i = 0; i < n; ++i) {
@@ -547,11 +624,13 @@ int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream
   p.M = (int)M;
   p.K = (int)g[0].K;
   p.row_bytes = row_bytes(g[0].K, bits);
+  const int st = take_norm(p, norm);
+  if (st != TSB200_OK) return st;
   return launch_any(p, bits, false, pdl, s);
 }
 
 // y = silu(x_gate . gate^T) * (x_up . up^T), both [N, K] of one container.
-int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s) {
+int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s, const tsb200_norm_desc* norm) {
   F32Params p = {};
   if (gate.K != up.K || gate.N != up.N || M < 1 || M > 65535 * 8 || gate.K > (1 << 30) || gate.N > (1 << 28)) return TSB200_ERR_UNSUPPORTED;
   Seg& sg = p.seg[0];
@@ -565,6 +644,8 @@ int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M
   p.M = (int)M;
   p.K = (int)gate.K;
   p.row_bytes = row_bytes(gate.K, bits);
+  const int st = take_norm(p, norm);
+  if (st != TSB200_OK) return st;
   return launch_any(p, bits, true, pdl, s);
 }
 

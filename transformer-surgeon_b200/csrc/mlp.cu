@@ -65,6 +65,33 @@ bool f32_chainable(const tsb200_linear_desc* g, const tsb200_linear_desc* u, con
   };
   return ok(g) && ok(u) && ok(d) && g->u_bits == u->u_bits && g->rank == u->rank && (g->rank == 0 || g->v_bits == u->v_bits);
 }
+// fp32: [gate V | up V] -> gated U -> down V -> down U on the FMA kernel, chained.  x: given, or normalised on the way in (norm).
+struct F32Buffers {
+  void *h0, *h1, *h2, *act;
+};
+int f32_chain(const tsb200_linear_desc* gate, const tsb200_linear_desc* up, const tsb200_linear_desc* down, const void* x, const tsb200_norm_desc* norm,
+              void* y, int64_t M, const F32Buffers& b, cudaStream_t s) {
+  const bool low = gate->rank > 0;
+  const int64_t kgu = low ? gate->rank : gate->in_features;
+  GemmSpec v[2] = {GemmSpec{gate->v, gate->v_scale, nullptr, x, b.h0, gate->rank, gate->in_features},
+                   GemmSpec{up->v, up->v_scale, nullptr, x, b.h1, up->rank, up->in_features}};
+  int st = low ? gemm_f32(v, 2, gate->v_bits, M, g_pdl != 0, s, norm) : TSB200_OK;
+  if (st == TSB200_OK)
+    st = gemm_f32_gated(GemmSpec{gate->u, gate->u_scale, gate->bias, low ? b.h0 : x, b.act, gate->out_features, kgu},
+                        GemmSpec{up->u, up->u_scale, up->bias, low ? b.h1 : x, b.act, up->out_features, kgu}, gate->u_bits, M, low || g_pdl, s,
+                        low ? nullptr : norm);
+  const void* dx = b.act;
+  if (st == TSB200_OK && down->rank > 0) {
+    const GemmSpec dv{down->v, down->v_scale, nullptr, b.act, b.h2, down->rank, down->in_features};
+    st = gemm_f32(&dv, 1, down->v_bits, M, true, s);
+    dx = b.h2;
+  }
+  if (st == TSB200_OK) {
+    const GemmSpec du{down->u, down->u_scale, down->bias, dx, y, down->out_features, down->rank > 0 ? down->rank : down->in_features};
+    st = gemm_f32(&du, 1, down->u_bits, M, true, s);
+  }
+  return st;
+}
 }  // namespace
 
 // Workspace layout: [region 0 | gate out | up out | act | h0 | h1 | h2].  Region 0 starts with the
@@ -94,6 +121,30 @@ static size_t region0_bytes(const tsb200_linear_desc* gate, const tsb200_linear_
   return align256(r0);
 }
 
+namespace {
+struct Buffers {
+  uint8_t *g, *u, *a;                           // gate out (composed path) / act (fused path), up out, act (composed path)
+  uint8_t *h0, *h1, *h2;
+};
+Buffers buffers(const tsb200_linear_desc* gate, const tsb200_linear_desc* up, const tsb200_linear_desc* down, int64_t M, uint8_t* ws) {
+  const size_t elt = gate->act_dtype == TSB200_F32 ? 4 : 2;
+  const size_t inter_b = align256((size_t)M * (size_t)gate->out_features * elt);
+  const size_t r_b = align256((size_t)M * (size_t)(gate->rank > down->rank ? gate->rank : down->rank) * elt);
+  Buffers b;
+  b.g = ws + region0_bytes(gate, up, down, M);
+  b.u = b.g + inter_b;
+  b.a = b.u + inter_b;
+  b.h0 = b.a + inter_b;
+  b.h1 = b.h0 + r_b;
+  b.h2 = b.h1 + r_b;
+  return b;
+}
+bool block_ok(const tsb200_linear_desc* gate, const tsb200_linear_desc* up, const tsb200_linear_desc* down, int64_t M) {
+  return gate && up && down && M >= 0 && gate->in_features == up->in_features && gate->out_features == up->out_features &&
+         down->in_features == gate->out_features && gate->act_dtype == up->act_dtype && gate->act_dtype == down->act_dtype;
+}
+}  // namespace
+
 extern "C" {
 
 size_t tsb200_mlp_gated_workspace_bytes(const tsb200_linear_desc* gate, const tsb200_linear_desc* up,
@@ -109,26 +160,15 @@ size_t tsb200_mlp_gated_workspace_bytes(const tsb200_linear_desc* gate, const ts
 int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* up, const tsb200_linear_desc* down,
                      const void* x, void* y, int64_t M, void* workspace, size_t workspace_bytes, void* stream) {
   TSB_REQUIRE_DEVICE();
-  if (!gate || !up || !down || M < 0) return TSB200_ERR_ARG;
-  if (gate->in_features != up->in_features || gate->out_features != up->out_features ||
-      down->in_features != gate->out_features)
-    return TSB200_ERR_ARG;
-  if (gate->act_dtype != up->act_dtype || gate->act_dtype != down->act_dtype) return TSB200_ERR_ARG;
+  if (!block_ok(gate, up, down, M)) return TSB200_ERR_ARG;
   if (M == 0) return TSB200_OK;
   if (!x || !y || !workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
   if (workspace_bytes < tsb200_mlp_gated_workspace_bytes(gate, up, down, M)) return TSB200_ERR_WORKSPACE;
   cudaStream_t s = as_stream(stream);
   uint8_t* ws = (uint8_t*)workspace;
-  const size_t elt = gate->act_dtype == TSB200_F32 ? 4 : 2;
   const size_t r0 = region0_bytes(gate, up, down, M);
-  const size_t inter_b = align256((size_t)M * (size_t)gate->out_features * elt);
-  const size_t r_b = align256((size_t)M * (size_t)(gate->rank > down->rank ? gate->rank : down->rank) * elt);
-  uint8_t* buf_g = ws + r0;                     // gate out (composed path) / act (fused path)
-  uint8_t* buf_u = buf_g + inter_b;
-  uint8_t* buf_a = buf_u + inter_b;
-  uint8_t* h0 = buf_a + inter_b;
-  uint8_t* h1 = h0 + r_b;
-  uint8_t* h2 = h1 + r_b;
+  const Buffers bufs = buffers(gate, up, down, M, ws);
+  uint8_t *buf_g = bufs.g, *buf_u = bufs.u, *buf_a = bufs.a, *h0 = bufs.h0, *h1 = bufs.h1, *h2 = bufs.h2;
 
   if (fusable(gate, up, down, M)) {
     PhaseSpec ps[4];
@@ -180,25 +220,7 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
     if (st != TSB200_ERR_UNSUPPORTED) return st;
   }
   if (f32_chainable(gate, up, down)) {
-    // fp32: [gate V | up V] -> gated U -> down V -> down U on the FMA kernel, chained
-    const bool low = gate->rank > 0;
-    const int64_t kgu = low ? gate->rank : gate->in_features;
-    GemmSpec v[2] = {GemmSpec{gate->v, gate->v_scale, nullptr, x, h0, gate->rank, gate->in_features},
-                     GemmSpec{up->v, up->v_scale, nullptr, x, h1, up->rank, up->in_features}};
-    int st = low ? gemm_f32(v, 2, gate->v_bits, M, g_pdl != 0, s) : TSB200_OK;
-    if (st == TSB200_OK)
-      st = gemm_f32_gated(GemmSpec{gate->u, gate->u_scale, gate->bias, low ? h0 : x, buf_g, gate->out_features, kgu},
-                          GemmSpec{up->u, up->u_scale, up->bias, low ? h1 : x, buf_g, up->out_features, kgu}, gate->u_bits, M, low || g_pdl, s);
-    const void* dx = buf_g;
-    if (st == TSB200_OK && down->rank > 0) {
-      const GemmSpec dv{down->v, down->v_scale, nullptr, buf_g, h2, down->rank, down->in_features};
-      st = gemm_f32(&dv, 1, down->v_bits, M, true, s);
-      dx = h2;
-    }
-    if (st == TSB200_OK) {
-      const GemmSpec du{down->u, down->u_scale, down->bias, dx, y, down->out_features, down->rank > 0 ? down->rank : down->in_features};
-      st = gemm_f32(&du, 1, down->u_bits, M, true, s);
-    }
+    const int st = f32_chain(gate, up, down, x, nullptr, y, M, F32Buffers{h0, h1, h2, buf_g}, s);
     if (st != TSB200_ERR_UNSUPPORTED) return st;
   }
   bool noop_g = false, noop_u = false;
@@ -241,6 +263,19 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
   st = tsb200_swiglu(buf_g, buf_u, buf_a, gate->act_dtype, M, inter, inter, inter, inter, stream);
   if (st != TSB200_OK) return st;
   return tsb200_linear(down, buf_a, y, M, ws, r0, stream);
+}
+
+int tsb200_norm_mlp_gated(const tsb200_norm_desc* norm, const tsb200_linear_desc* gate, const tsb200_linear_desc* up,
+                          const tsb200_linear_desc* down, void* y, int64_t M, void* workspace, size_t workspace_bytes, void* stream) {
+  TSB_REQUIRE_DEVICE();
+  if (!norm || !norm->residual || !norm->weight || !norm->residual_out || norm->residual_out == norm->residual) return TSB200_ERR_ARG;
+  if (!block_ok(gate, up, down, M)) return TSB200_ERR_ARG;
+  if (M == 0) return TSB200_OK;
+  if (!y || !workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
+  if (workspace_bytes < tsb200_mlp_gated_workspace_bytes(gate, up, down, M)) return TSB200_ERR_WORKSPACE;
+  if (!f32_chainable(gate, up, down)) return TSB200_ERR_UNSUPPORTED;
+  const Buffers b = buffers(gate, up, down, M, (uint8_t*)workspace);
+  return f32_chain(gate, up, down, nullptr, norm, y, M, F32Buffers{b.h0, b.h1, b.h2, b.g}, as_stream(stream));
 }
 
 }  // extern "C"

@@ -254,9 +254,10 @@ struct GvSpan {
 bool gv_supported(int bits, int64_t M, int64_t N, int64_t K);
 // Whether n phases, one launch each, are modelled to take less time here than in linear_tcq.cu (they are the same bits).
 bool gv_faster(const PhaseSpec* ps, const int* bits, int n, int64_t M);
-// fp32 activations (linear_f32.cu): n <= 4 matrices of one container and reduction length in one launch; a gate / up pair.
-int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s);
-int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s);
+// fp32 activations (linear_f32.cu): n <= 4 matrices of one container and reduction length in one launch; a gate / up pair.  With `norm`
+// (few tokens; else TSB200_ERR_UNSUPPORTED) the matrices' x is what tsb200_add_rmsnorm makes of its residual and delta.
+int gemm_f32(const GemmSpec* g, int n, int bits, int64_t M, bool pdl, cudaStream_t s, const tsb200_norm_desc* norm = nullptr);
+int gemm_f32_gated(const GemmSpec& gate, const GemmSpec& up, int bits, int64_t M, bool pdl, cudaStream_t s, const tsb200_norm_desc* norm = nullptr);
 int gv_gemm(const PhaseSpec& ps, int bits, int64_t M, bool pdl, const GvSpan* ahead, int n_ahead, cudaStream_t s);
 
 }  // namespace tsb

@@ -111,6 +111,7 @@ class CompressedDecoder:
         # persistent activation buffers (stable addresses -> the step can be captured in a CUDA graph)
         self.tokens = torch.zeros(B, dtype=torch.int64, device=device)
         self.resid = torch.zeros((B, c.hidden), dtype=dt, device=device)
+        self.resid_next = torch.empty_like(self.resid)      # where a projection that normalises its own input leaves residual + delta
         self.xn = torch.empty((B, c.hidden), dtype=dt, device=device)
         self.qkv = torch.empty((B, (H + 2 * Hkv) * d), dtype=dt, device=device)
         self.qb = torch.empty((B, H * d), dtype=dt, device=device)
@@ -181,40 +182,55 @@ class CompressedDecoder:
         delta = None
         rope = (self.cos, self.sin)
         peer = self.peer if tp_on else None
+        # fp32: q, k, v and the MLP take residual and delta and normalise them themselves, two launches a layer fewer
+        # (the residual then alternates between two buffers)
+        own_norm = c.dtype == torch.float32 and c.norm_variant == 0 and not tp_on
+        resid, resid_next = self.resid, self.resid_next
         for li, L in enumerate(self.layers):
-            if peer is not None and li > 0:      # the previous layer's down_proj partials: summed, added, normalised
-                peer.allreduce_add_rmsnorm(1, self.resid, L.ln1, c.rms_eps, out=self.xn); n += 1
+            group = L.qkv_group
+            outs = (self.qkv,) if group is None else (self.qb, self.kb, self.vb)
+            if own_norm and (group or ops.LinearGroup([L.qkv])).after_norm(ops.normalisation(resid, delta, L.ln1, resid_next, c.rms_eps), B, outs, self.lin_ws):
+                resid, resid_next = resid_next, resid
+                n += 1 if group is None else 2 if L.q.rank else 1
             else:
-                ops.add_rmsnorm(self.resid, delta, L.ln1, c.rms_eps, c.norm_variant, out=self.xn); n += 1
-            if L.qkv is not None:
-                L.qkv(self.xn, out=self.qkv, ws=self.lin_ws); n += 1
+                if peer is not None and li > 0:      # the previous layer's down_proj partials: summed, added, normalised
+                    peer.allreduce_add_rmsnorm(1, resid, L.ln1, c.rms_eps, out=self.xn); n += 1
+                else:
+                    ops.add_rmsnorm(resid, delta, L.ln1, c.rms_eps, c.norm_variant, out=self.xn); n += 1
+                if group is None:
+                    L.qkv(self.xn, out=self.qkv, ws=self.lin_ws); n += 1
+                else:
+                    group(self.xn, outs, ws=self.lin_ws)
+                    n += sum(2 if l.rank else 1 for l in (L.q, L.k, L.v))
+            if group is None:
                 q4 = self.qkv[:, :H * d].unflatten(1, (H, d)).unsqueeze(1)                   # [B,1,H,d] views
                 k4 = self.qkv[:, H * d:(H + Hkv) * d].unflatten(1, (Hkv, d)).unsqueeze(1)
                 v4 = self.qkv[:, (H + Hkv) * d:].unflatten(1, (Hkv, d)).unsqueeze(1)
             else:
-                L.qkv_group(self.xn, (self.qb, self.kb, self.vb), ws=self.lin_ws)
-                n += sum(2 if l.rank else 1 for l in (L.q, L.k, L.v))
                 q4, k4, v4 = self.qb.view(B, 1, H, d), self.kb.view(B, 1, Hkv, d), self.vb.view(B, 1, Hkv, d)
             self.kv[li].rope_append(q4, k4, v4, rope, seq_lens=self.write_pos); n += 1
             ops.paged_decode_attention(self.kv[li], q4[:, 0], self.max_seq_len, out=self.attn.view(B, H, d),
                                        ws=self.attn_ws, seq_lens=self.seq_lens); n += 2
             if peer is not None:
                 L.o(self.attn, out=peer.partial(0), ws=self.lin_ws); n += 1
-                peer.allreduce_add_rmsnorm(0, self.resid, L.ln2, c.rms_eps, out=self.xn); n += 1
+                peer.allreduce_add_rmsnorm(0, resid, L.ln2, c.rms_eps, out=self.xn); n += 1
                 L.mlp(self.xn, out=peer.partial(1), ws=self.mlp_ws); n += 1
                 continue
             L.o(self.attn, out=self.delta, ws=self.lin_ws); n += 1
             if tp_on:
                 all_reduce_sum(self.delta, self.tp_group)       # row-parallel o_proj: sum of the partial outputs
-            ops.add_rmsnorm(self.resid, self.delta, L.ln2, c.rms_eps, c.norm_variant, out=self.xn); n += 1
-            L.mlp(self.xn, out=self.delta, ws=self.mlp_ws); n += 1
+            if own_norm and L.mlp.after_norm(ops.normalisation(resid, self.delta, L.ln2, resid_next, c.rms_eps), B, self.delta, self.mlp_ws):
+                resid, resid_next = resid_next, resid; n += 1
+            else:
+                ops.add_rmsnorm(resid, self.delta, L.ln2, c.rms_eps, c.norm_variant, out=self.xn); n += 1
+                L.mlp(self.xn, out=self.delta, ws=self.mlp_ws); n += 1
             if tp_on:
                 all_reduce_sum(self.delta, self.tp_group)       # row-parallel down_proj
             delta = self.delta
         if peer is not None:
-            peer.allreduce_add_rmsnorm(1, self.resid, self.final_norm, c.rms_eps, out=self.xn); n += 1
+            peer.allreduce_add_rmsnorm(1, resid, self.final_norm, c.rms_eps, out=self.xn); n += 1
         else:
-            ops.add_rmsnorm(self.resid, delta, self.final_norm, c.rms_eps, c.norm_variant, out=self.xn); n += 1
+            ops.add_rmsnorm(resid, delta, self.final_norm, c.rms_eps, c.norm_variant, out=self.xn); n += 1
         if self.greedy_head:
             if self.head_ws is None:
                 self.head_ws = torch.zeros(self.lm_head.argmax_workspace_bytes(B), dtype=torch.uint8, device=self.device)

@@ -8,7 +8,7 @@ import ctypes as C
 import torch
 
 from . import _lib
-from ._lib import F32, BF16, KV_INT8, KV_FP8, KV_NVFP4, KV_F32, KV_BF16, LinearDesc, KVDesc, check
+from ._lib import F32, BF16, KV_INT8, KV_FP8, KV_NVFP4, KV_F32, KV_BF16, LinearDesc, KVDesc, NormDesc, check
 
 from ._lib import Tsb200Error  # noqa: F401  (re-exported)
 
@@ -361,6 +361,28 @@ class LinearGroup:
         return outs
 
 
+    def after_norm(self, norm, M, outs, ws):
+        """The layers of RMSNorm(residual + delta) * weight, [M, in] fp32 (norm: normalisation()): the bits of add_rmsnorm and of a call, without
+        the launch in between.  False, with nothing done, where the library has no such form."""
+        if any(l.act_dtype != torch.float32 or l.force_simt for l in self.layers):
+            return False
+        ptrs = self._ptrs(*(o.data_ptr() for o in outs))
+        return _fused(_lib.load().tsb200_norm_linear_group(C.byref(norm), self._descs, len(self.layers), ptrs, M, ws.data_ptr(), ws.numel(), _stream()),
+                      "tsb200_norm_linear_group")
+
+
+def normalisation(residual, delta, weight, residual_out, eps):
+    """What LinearGroup.after_norm and GatedMLP.after_norm normalise: residual + delta (kept in residual_out, a buffer of its own)."""
+    return NormDesc(_cuda(residual, "residual").data_ptr(), _p(delta), _cuda(weight, "weight").data_ptr(), _cuda(residual_out, "residual_out").data_ptr(), float(eps))
+
+
+def _fused(status, what):
+    if status == _lib.ERR_UNSUPPORTED:
+        return False
+    check(status, what)
+    return True
+
+
 class GatedMLP:
     """down(silu(gate(x)) * up(x)): MLPGated.forward (blocks/mlp.py:171-185) on three PackedLinear."""
 
@@ -384,6 +406,14 @@ class GatedMLP:
         check(lib.tsb200_mlp_gated(C.byref(self.gate.desc), C.byref(self.up.desc), C.byref(self.down.desc), _p(x2),
                                    _p(out), M, _p(ws), ws.numel(), _stream()), "tsb200_mlp_gated")
         return out.reshape(*lead, self.down.out_features)
+
+
+    def after_norm(self, norm, M, out, ws):
+        """The block of RMSNorm(residual + delta) * weight: as LinearGroup.after_norm."""
+        if self.gate.act_dtype != torch.float32:
+            return False
+        return _fused(_lib.load().tsb200_norm_mlp_gated(C.byref(norm), C.byref(self.gate.desc), C.byref(self.up.desc), C.byref(self.down.desc),
+                                                        out.data_ptr(), M, ws.data_ptr(), ws.numel(), _stream()), "tsb200_norm_mlp_gated")
 
 
 # ---------------------------------------------------------------- KV cache ---------
