@@ -617,3 +617,25 @@ def test_append_of_quotients_at_the_midpoints_of_codes(cuda, fmt, name):
         single.seq_lens += 1
     assert torch.equal(bulk.k_pool, single.k_pool)
     assert torch.equal(bulk.v_pool, single.v_pool)
+
+
+@pytest.mark.parametrize("fmt,H,Hkv,d", [("int8", 16, 8, 128), ("nvfp4", 56, 8, 64), ("fp8", 64, 8, 128)])
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+def test_splits_merge_alike_in_a_cluster_and_in_a_launch(cuda, fmt, H, Hkv, d, name):
+    """Four splits of up to 19 pages: 16 sequences merge in clusters, 40 in a launch of their own.  The first 16 of the 40 are the same bits."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(57)
+    B, pages = 40, 19
+    bt = torch.randperm(B * pages, generator=g, device=cuda).to(torch.int32).reshape(B, pages)
+    kv = ops.PagedKV(fmt, B * pages, Hkv, d, bt, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+    if fmt == "fp8":
+        kv.fill_fp8_scales(6.0 / 448, 6.0 / 448)
+    kv.append(*(torch.randn((B, pages * 16, Hkv, d), generator=g, device=cuda).to(DT[name]) for _ in range(2)))
+    kv.seq_lens = (torch.arange(B, device=cuda) * 20 % 304).to(torch.int32)
+    q = torch.randn((B, H, d), generator=g, device=cuda).to(DT[name])
+    every = ops.paged_decode_attention(kv, q, pages * 16)
+    few = ops.PagedKV(fmt, B * pages, Hkv, d, bt[:16].contiguous(), kv.seq_lens[:16].contiguous(), cuda)
+    few.k_pool, few.v_pool = kv.k_pool, kv.v_pool
+    if fmt == "fp8":
+        few.fill_fp8_scales(6.0 / 448, 6.0 / 448)
+    assert torch.equal(ops.paged_decode_attention(few, q[:16].contiguous(), pages * 16), every[:16])

@@ -55,8 +55,8 @@ inline int choose_splits_fp8(int64_t B, int hkv, int64_t max_seq_len) {
   return (int)s;
 }
 
-// Whether the last CTA of a (sequence, kv head, head chunk) of unquantized pages merges its splits (the quantized formats always launch the
-// reduction).  That takes ~80 cycles per (head, split) row - 35 k
+// Whether the last CTA of a (sequence, kv head, head chunk) of unquantized pages merges its splits (the quantized formats: a cluster or
+// the reduction launch).  That takes ~80 cycles per (head, split) row - 35 k
 // cycles, 20 us, at 7 heads and 63 splits -, a reduction launch that is resident before the partials are complete ~3 us whatever the
 // shape: the launch from 64 rows on.
 inline bool last_cta_merges(int splits, int H, int hkv) { return splits == 1 || splits * (H / hkv < 8 ? H / hkv : 8) < 64; }
@@ -102,6 +102,72 @@ __device__ __forceinline__ float v_elem(const uint8_t* __restrict__ rec, int fmt
   if (fmt == TSB200_KV_FP8) return e4m3_byte_to_f32(rec[e * 16 + t]);
   const unsigned b = rec[(e >> 1) * 16 + t];
   return e2m1_nibble_to_f32(b >> ((e & 1) * 4)) * e4m3_byte_to_f32(rec[16 * (D / 2) + (e >> 4) * 16 + t]);
+}
+
+// Splits of quantized pages whose CTAs are a cluster (1, S, 1) merge through distributed shared memory: `part` = this
+// split's partials ([heads][2 + D], shared memory), `out` = the heads' outputs.  The arithmetic is decode_attn_reduce_kernel's, in its order: the
+// same bits, without its launch.  No CTA leaves while another one may still read its partials.
+constexpr int kMaxCluster = 8;
+__device__ __forceinline__ bool splits_are_cluster() {
+  unsigned n;
+  asm("mov.u32 %0, %%cluster_nctaid.y;\n" : "=r"(n));
+  return n > 1;
+}
+template <typename T, int D>
+__device__ __forceinline__ void merge_cluster(const float* part, int heads, int S, T* __restrict__ out) {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  const unsigned own = (unsigned)__cvta_generic_to_shared(part);
+  for (int idx = (int)(blockIdx.y * blockDim.x + threadIdx.x); idx < heads * (D / 2); idx += S * (int)blockDim.x) {
+    const int h = idx / (D / 2), e = idx % (D / 2) * 2;
+    float2 ml[kMaxCluster], v[kMaxCluster];
+#pragma unroll
+    for (int s = 0; s < kMaxCluster; ++s)
+      if (s < S) {
+        unsigned a;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(own + h * (2 + D) * 4), "r"(s));
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(ml[s].x), "=f"(ml[s].y) : "r"(a) : "memory");
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v[s].x), "=f"(v[s].y) : "r"(a + (2 + e) * 4) : "memory");
+      }
+    float mm = -INFINITY, ll = 0.f, a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int s = 0; s < kMaxCluster; ++s)
+      if (s < S) mm = fmaxf(mm, ml[s].x);
+#pragma unroll
+    for (int s = 0; s < kMaxCluster; ++s)
+      if (s < S) {
+        const float c = ml[s].x == -INFINITY ? 0.f : __expf(ml[s].x - mm);
+        ll += ml[s].y * c;
+        a0 += v[s].x * c;
+        a1 += v[s].y * c;
+      }
+    out[h * D + e] = from_f32<T>(ll > 0.f ? a0 / ll : 0.f);
+    out[h * D + e + 1] = from_f32<T>(ll > 0.f ? a1 / ll : 0.f);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// Launch of grid (pairs, S, chunks); `clusters`: one per (pair, chunk), its CTAs merge the splits themselves.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_splits(bool overlap, bool clusters, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (overlap) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (clusters) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = 1;
+    attr[n].val.clusterDim.y = grid.y;
+    attr[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 // The last CTA of a (sequence, kv head, head chunk) merges its S partials, in split order:

@@ -13,9 +13,9 @@
 // an e2m1 code times its e4m3 block scale is exact in f16 (2 x 4 significant bits), so K goes to
 // the MMA as code * scale; for V the block scale of a token is folded into that token's softmax
 // weight (one product per 16-dim block and token instead of one per element).
-// Several splits leave partials (m, l, acc) in the workspace for decode_attn_reduce_kernel: that launch is resident before the last
-// partial is there, and 3-5 us faster than a merge by the last CTA of a pair, whatever the number of splits (int8, 2 sequences x 32 / 8
-// heads x 500 tokens 8.2 -> 5.5 us, NVFP4, 1 x 32 / 8 x 1000 9.6 -> 6.2).
+// Several splits leave partials (m, l, acc): in shared memory where a cluster merges them (launch_mma says when), else in the workspace for
+// decode_attn_reduce_kernel.  That launch is resident before the last partial is there, and 3-5 us faster than a merge by the last CTA of a
+// pair, whatever the number of splits (captured: int8, 2 sequences x 32 / 8 heads x 500 tokens 8.2 -> 5.5 us, NVFP4, 1 x 32 / 8 x 1000 9.6 -> 6.2).
 //
 // Bound by the page loop's instructions.  Against copies by all 32 lanes (cp.async, 4 to 9 a lane and page), block scales widened by every
 // lane and a rescale of the accumulators on every page, half to all of the stated tokens: int8, 64 x 8 kv heads x 4096 95.1 -> 89.6 us, 16 x 4 x
@@ -375,12 +375,14 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
     l0 += __shfl_xor_sync(0xffffffffu, l0, o);
     l1 += __shfl_xor_sync(0xffffffffu, l1, o);
   }
+  const bool clustered = splits_are_cluster();
   __syncthreads();   // every warp is done with its ring; reuse shared memory for the merge
   constexpr int AR = D + 4;                                  // row pitch: the fragments' four head rows fall into different banks
   float* sm_m = reinterpret_cast<float*>(smem + kBarBytes);  // [warps][8]
   float* sm_l = sm_m + kWarps * 8;                           // [warps][8]
   float* sm_c = sm_l + kWarps * 8;                           // [warps][8]
   float* sm_acc = sm_c + kWarps * 8;                         // [warps][8][AR]
+  float* sm_part = sm_acc + kWarps * 8 * AR;                 // [8][2 + D]: this split's partials where a cluster merges
   if (gid == 0) {
     sm_m[w * 8 + 2 * tid] = m0; sm_m[w * 8 + 2 * tid + 1] = m1;
     sm_l[w * 8 + 2 * tid] = l0; sm_l[w * 8 + 2 * tid + 1] = l1;
@@ -422,7 +424,7 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       out[bh * D + e] = from_f32<T>(ll > 0.f ? a0 * vscale / ll : 0.f);
       out[bh * D + e + 1] = from_f32<T>(ll > 0.f ? a1 * vscale / ll : 0.f);
     } else {
-      float* o = ws + (bh * S + s) * (2 + D);
+      float* o = clustered ? sm_part + i * (2 + D) : ws + (bh * S + s) * (2 + D);
       if (e == 0) {                                          // natural-log domain (shared with the reducer kernel)
         float mm = -INFINITY;
 #pragma unroll
@@ -432,6 +434,7 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
       *reinterpret_cast<float2*>(o + 2 + e) = make_float2(a0 * vscale, a1 * vscale);
     }
   }
+  if (clustered) merge_cluster<T, D>(sm_part, gn, S, out + ((int64_t)b * H + hk * g + g0) * D);
 }
 
 template <typename T, int D, int FMT>
@@ -441,7 +444,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   constexpr int kWarps = AttnCfg<FMT, D>::kWarps, kStages = AttnCfg<FMT, D>::kStages;
   static_assert(kWarps * kStages * 8 <= kBarBytes, "barriers");
   constexpr size_t pipe = (size_t)kWarps * (kStages * 2 * REC + (FMT == TSB200_KV_NVFP4 ? D * 2 : 0));
-  constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4)) * sizeof(float);
+  constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4) + 8 * (2 + D)) * sizeof(float);
   constexpr size_t smem = kBarBytes + (pipe > merge ? pipe : merge);
   static bool configured[64] = {false};   // per device: the attribute lives in the device's context
   int dev = 0;
@@ -453,9 +456,14 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   }
   const int g = H / kv.hkv, S = choose_splits(B, kv.hkv, max_seq_len);
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((g + 7) / 8));
-  TSB_CUDA(launch_kernel_if(attn_overlaps(kv), decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
+  // Few splits of short sequences merge in a cluster, which spares the host a launch (a call by itself, 33 sequences x 8 kv heads x 83-166
+  // tokens, int8: 14.2 us with the launch, 12.3); clusters wait until an SM group has room for all their CTAs, so that longer work, which
+  // hides the host's time, is faster with the launch (captured: 64 x 8 x 4096, int8, 4 splits 89.6 us, clusters 97.7; 16 x 8 x 2000, NVFP4 19.2,
+  // 23.1; 32 x 8 x 200, NVFP4 11.8, 11.6).
+  const bool clusters = S > 1 && S <= kMaxCluster && B * kv.hkv * ((max_seq_len + 15) / 16) <= 4096;
+  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, (T*)out, status));
-  return S == 1 ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
+  return S == 1 || clusters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }
 
 }  // namespace
@@ -494,7 +502,7 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
     const int S8 = choose_splits_fp8(B, kv->hkv, max_seq_len);   // never more than choose_splits(): the workspace fits
     const int r = dtype == TSB200_F32 ? launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s)
                                       : launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s);
-    if (r != TSB200_OK || S8 == 1) return r;
+    if (r != TSB200_OK || S8 <= kMaxCluster) return r;
     return dtype == TSB200_F32 ? launch_reduce<float, 128>(ws, B * H, S8, out, s) : launch_reduce<__nv_bfloat16, 128>(ws, B * H, S8, out, s);
   }
 #define TSB_GO(TT, DD, FF) return launch_mma<TT, DD, FF>(*kv, q, qs, H, sm_scale, max_seq_len, B, ws, out, status, s)
