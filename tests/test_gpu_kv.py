@@ -639,3 +639,19 @@ def test_splits_merge_alike_in_a_cluster_and_in_a_launch(cuda, fmt, H, Hkv, d, n
     if fmt == "fp8":
         few.fill_fp8_scales(6.0 / 448, 6.0 / 448)
     assert torch.equal(ops.paged_decode_attention(few, q[:16].contiguous(), pages * 16), every[:16])
+
+
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+def test_long_splits_have_the_bits_of_shorter_ones(cuda, name):
+    """NVFP4, four splits: deeper rings from 64 pages a split on (a context limit of 4096), the same bits as below (4080)."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(58)
+    B, H, Hkv, d, pages = 40, 16, 8, 128, 256
+    bt = torch.arange(B * pages, device=cuda).flip(0).to(torch.int32).reshape(B, pages)
+    kv = ops.PagedKV("nvfp4", B * pages, Hkv, d, bt, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+    for _ in range(4):
+        kv.append(*(torch.randn((B, 1020, Hkv, d), generator=g, device=cuda).to(DT[name]) for _ in range(2)))
+        kv.seq_lens += 1020
+    kv.seq_lens -= (torch.arange(B, device=cuda) * 97).to(torch.int32)
+    q = torch.randn((B, H, d), generator=g, device=cuda).to(DT[name])
+    assert torch.equal(ops.paged_decode_attention(kv, q, 4096), ops.paged_decode_attention(kv, q, 4080))

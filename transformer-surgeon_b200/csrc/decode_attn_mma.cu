@@ -19,7 +19,7 @@
 //
 // Bound by the page loop's instructions.  Against copies by all 32 lanes (cp.async, 4 to 9 a lane and page), block scales widened by every
 // lane and a rescale of the accumulators on every page, half to all of the stated tokens: int8, 64 x 8 kv heads x 4096 95.1 -> 89.6 us, 16 x 4 x
-// 8192 35.7 -> 33.6; NVFP4, 64 x 8 x 4096 96.9 -> 90.8, 30 x 4 x 3000 31.3 -> 26.6, 8 x 4 x 32768 58.8 -> 57.3.
+// 8192 35.7 -> 33.6; NVFP4, 64 x 8 x 4096 96.9 -> 86.9, 30 x 4 x 3000 31.3 -> 26.6, 8 x 4 x 32768 58.8 -> 54.3.
 #include "tc_common.cuh"
 #include "decode_attn_common.cuh"
 
@@ -45,11 +45,13 @@ constexpr unsigned kWaitLimit = 1u << 22;
 // Warps per CTA, ring stages (pages) per warp, CTAs per SM that registers are to allow.  What counts is how many CTAs an SM holds: the page
 // loop is bound by the instructions that widen codes and by the chain of a page's softmax, and the warps of other CTAs fill its gaps.  int8,
 // head_dim 64: 30 sequences x 2 kv heads x 1.5k-3k tokens 12.4 us at 5 CTAs, 13.5 at 4; head_dim 128 is limited by registers (3).  NVFP4, 128:
-// 5 CTAs of 3 stages against 4 of 4: 16 x 4 x 1k-2k tokens 14.2 us to 15.1, 16 x 8 x 1k-2k 19.2 to 21.4; 8 x 4 x 16k-32k 57.3 to 54.0.
-template <int FMT, int D> struct AttnCfg {
+// 5 CTAs of 3 stages against 4 of 4: 16 x 4 x 1k-2k tokens 14.2 us to 15.1, 16 x 8 x 1k-2k 19.2 to 21.4, 16 x 4 x 6k-12k (62 pages a split)
+// 43.1 to 44.6; 64 x 8 x 2k-4k (64 pages) 91.7 to 86.9, 8 x 4 x 16k-32k (85) 57.4 to 54.3.
+// Hence LONG: splits of 64 pages and more, whose warps stream 16 and more.
+template <int FMT, int D, bool LONG> struct AttnCfg {
   static constexpr int kWarps = FMT == TSB200_KV_INT8 ? 6 : 4;
-  static constexpr int kStages = FMT == TSB200_KV_INT8 && D == 128 ? 2 : 3;
-  static constexpr int kCtas = FMT == TSB200_KV_INT8 ? (D == 128 ? 3 : 5) : (FMT == TSB200_KV_NVFP4 && D == 128 ? 5 : 4);
+  static constexpr int kStages = FMT == TSB200_KV_INT8 && D == 128 ? 2 : (LONG ? 4 : 3);
+  static constexpr int kCtas = FMT == TSB200_KV_INT8 ? (D == 128 ? 3 : 5) : (FMT == TSB200_KV_NVFP4 && D == 128 && !LONG ? 5 : 4);
 };
 
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -126,13 +128,13 @@ template <int FMT, int D> struct RecBytes {
   static constexpr int value = FMT == TSB200_KV_INT8 ? 16 * D + 64 : (FMT == TSB200_KV_NVFP4 ? 9 * D : 16 * D);
 };
 
-template <typename T, int D, int FMT>
-__global__ void __launch_bounds__(AttnCfg<FMT, D>::kWarps * 32, AttnCfg<FMT, D>::kCtas)
+template <typename T, int D, int FMT, bool LONG>
+__global__ void __launch_bounds__(AttnCfg<FMT, D, LONG>::kWarps * 32, AttnCfg<FMT, D, LONG>::kCtas)
 decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
                        float* __restrict__ ws, T* __restrict__ out, int* __restrict__ status) {
   constexpr bool FP4 = FMT == TSB200_KV_NVFP4;
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int kWarps = AttnCfg<FMT, D>::kWarps, kStages = AttnCfg<FMT, D>::kStages;
+  constexpr int kWarps = AttnCfg<FMT, D, LONG>::kWarps, kStages = AttnCfg<FMT, D, LONG>::kStages;
   constexpr int STAGE = 2 * REC;                // K and V of a page
   constexpr int NC = D / 16;                    // k-steps of QK, m-tiles of PV
   extern __shared__ __align__(128) uint8_t smem[];
@@ -437,11 +439,11 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   if (clustered) merge_cluster<T, D>(sm_part, gn, S, out + ((int64_t)b * H + hk * g + g0) * D);
 }
 
-template <typename T, int D, int FMT>
-int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int64_t B, float* ws, void* out,
+template <typename T, int D, int FMT, bool LONG>
+int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S, int64_t B, float* ws, void* out,
                int* status, cudaStream_t st) {
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int kWarps = AttnCfg<FMT, D>::kWarps, kStages = AttnCfg<FMT, D>::kStages;
+  constexpr int kWarps = AttnCfg<FMT, D, LONG>::kWarps, kStages = AttnCfg<FMT, D, LONG>::kStages;
   static_assert(kWarps * kStages * 8 <= kBarBytes, "barriers");
   constexpr size_t pipe = (size_t)kWarps * (kStages * 2 * REC + (FMT == TSB200_KV_NVFP4 ? D * 2 : 0));
   constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4) + 8 * (2 + D)) * sizeof(float);
@@ -451,17 +453,17 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   TSB_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return TSB200_ERR_DEVICE;
   if (!configured[dev]) {
-    TSB_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<T, D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TSB_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<T, D, FMT, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev] = true;
   }
-  const int g = H / kv.hkv, S = choose_splits(B, kv.hkv, max_seq_len);
+  const int g = H / kv.hkv;
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((g + 7) / 8));
   // Few splits of short sequences merge in a cluster, which spares the host a launch (a call by itself, 33 sequences x 8 kv heads x 83-166
   // tokens, int8: 14.2 us with the launch, 12.3); clusters wait until an SM group has room for all their CTAs, so that longer work, which
   // hides the host's time, is faster with the launch (captured: 64 x 8 x 4096, int8, 4 splits 89.6 us, clusters 97.7; 16 x 8 x 2000, NVFP4 19.2,
   // 23.1; 32 x 8 x 200, NVFP4 11.8, 11.6).
   const bool clusters = S > 1 && S <= kMaxCluster && B * kv.hkv * ((max_seq_len + 15) / 16) <= 4096;
-  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
+  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT, LONG>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, (T*)out, status));
   return S == 1 || clusters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }
@@ -505,10 +507,15 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
     if (r != TSB200_OK || S8 <= kMaxCluster) return r;
     return dtype == TSB200_F32 ? launch_reduce<float, 128>(ws, B * H, S8, out, s) : launch_reduce<__nv_bfloat16, 128>(ws, B * H, S8, out, s);
   }
-#define TSB_GO(TT, DD, FF) return launch_mma<TT, DD, FF>(*kv, q, qs, H, sm_scale, max_seq_len, B, ws, out, status, s)
+  const int S = choose_splits(B, kv->hkv, max_seq_len);
+  const bool long_splits = kv->format == TSB200_KV_NVFP4 && D == 128 && (max_seq_len + 15) / 16 >= 64 * S;
+#define TSB_GO(TT, DD, FF)                                                                                                        \
+  if (FF == TSB200_KV_NVFP4 && DD == 128 && long_splits)                                                                          \
+    return launch_mma<TT, DD, FF, (FF == TSB200_KV_NVFP4 && DD == 128)>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s); \
+  return launch_mma<TT, DD, FF, false>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s)
 #define TSB_FMT(FF)                                                                                                       \
-  if (dtype == TSB200_F32) { if (D == 64) TSB_GO(float, 64, FF); TSB_GO(float, 128, FF); }                               \
-  if (D == 64) TSB_GO(__nv_bfloat16, 64, FF);                                                                             \
+  if (dtype == TSB200_F32) { if (D == 64) { TSB_GO(float, 64, FF); } TSB_GO(float, 128, FF); }                               \
+  if (D == 64) { TSB_GO(__nv_bfloat16, 64, FF); }                                                                            \
   TSB_GO(__nv_bfloat16, 128, FF)
   if (kv->format == TSB200_KV_NVFP4) { TSB_FMT(TSB200_KV_NVFP4); }
   if (kv->format == TSB200_KV_INT8) { TSB_FMT(TSB200_KV_INT8); }
