@@ -581,3 +581,21 @@ def test_fp32_projections_normalise_their_input(cuda, p, M, K, I, r):
     for l in group.layers:
         l.force_simt = True
     assert not group.after_norm(ops.normalisation(residual, None, w, torch.empty_like(residual), 1e-6), M, outs, ws)
+
+
+@pytest.mark.parametrize("K", [4096, 4100, 5000, 8192])
+def test_long_rows_are_normalised_as_add_rmsnorm_does(cuda, K):
+    """One token, rows on both sides of 16 KB, where add_rmsnorm changes the order of its sum: 48 rows each, since two orders of 8192 squares
+    often round to the same number."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(55)
+    layer = ops.PackedLinear(ops.Factor.dense(torch.randn((16, K), generator=g, device=cuda) * K ** -0.5), None, None, torch.float32)
+    group = ops.LinearGroup([layer])
+    ws = torch.zeros(group.workspace_bytes(1), dtype=torch.uint8, device=cuda)
+    for _ in range(48):
+        residual, delta, w = (torch.randn(s, generator=g, device=cuda) for s in ((1, K), (1, K), (K,)))
+        after, kept, out = residual.clone(), torch.empty_like(residual), torch.empty((1, 16), device=cuda)
+        xn = ops.add_rmsnorm(after, delta, w, 1e-6)
+        assert group.after_norm(ops.normalisation(residual, delta, w, kept, 1e-6), 1, [out], ws)
+        assert torch.equal(kept, after)
+        assert torch.equal(out, group(xn)[0])

@@ -64,6 +64,9 @@ int check_device_cached();   // TSB200_OK iff current device is CC 10.0
     if (_s != TSB200_OK) return _s;             \
   } while (0)
 
+// RMSNorm rows of up to this many bytes (whole 16-byte pieces, aligned) are summed piece by piece, longer ones element by element.
+constexpr int kNormPieceRow = 16384;
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

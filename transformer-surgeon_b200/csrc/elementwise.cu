@@ -280,7 +280,7 @@ int tsb200_add_rmsnorm(void* residual, const void* delta, const void* w, void* y
   if (!residual || !w || !y) return TSB200_ERR_ARG;
   if (M > 0x7fffffffLL) return TSB200_ERR_UNSUPPORTED;
   const int64_t elt = dtype == TSB200_F32 ? 4 : 2;
-  if ((dtype == TSB200_F32 || dtype == TSB200_BF16) && variant == 0 && hidden * elt % 16 == 0 && hidden * elt <= 16384 && aligned(residual, 16) &&
+  if ((dtype == TSB200_F32 || dtype == TSB200_BF16) && variant == 0 && hidden * elt % 16 == 0 && hidden * elt <= kNormPieceRow && aligned(residual, 16) &&
       aligned(y, 16) && aligned(w, 16) && (!delta || aligned(delta, 16)))
     return dtype == TSB200_F32 ? launch_rmsnorm_hf<float>(residual, delta, w, y, M, hidden, eps, as_stream(stream))
                                : launch_rmsnorm_hf<__nv_bfloat16>(residual, delta, w, y, M, hidden, eps, as_stream(stream));

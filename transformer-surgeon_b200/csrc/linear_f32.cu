@@ -97,7 +97,9 @@ template <int V> __device__ __forceinline__ float reduce_scatter(float (&v)[V]) 
 
 // Activations that are the RMSNorm of residual + delta, staged by every CTA for itself (rows of one K tile): a decode step's separate
 // normalisation is a launch of its own in the chain, ~2.3 us, of which this adds back a reduction over the CTA.  The arithmetic and the
-// order of its sums are add_rmsnorm_hf_kernel's (elementwise.cu): the same bits.  The first CTA keeps the new residual.
+// order of its sums are tsb200_add_rmsnorm's (elementwise.cu): the same bits.  That order depends on the row: pieces of 16 bytes up to
+// kNormPieceRow bytes (add_rmsnorm_hf_kernel), single elements beyond (add_rmsnorm_kernel; here only one token's row is that long).  The first
+// CTA keeps the new residual.
 template <int MATS, int MT, int KT>
 __device__ __forceinline__ void stage_normalised(const F32Params& p, const float4& nw, float (&xs)[MATS][MT][KT], float (&red)[kWarps][32]) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -120,6 +122,16 @@ __device__ __forceinline__ void stage_normalised(const F32Params& p, const float
       }
       *reinterpret_cast<float4*>(&xs[0][m][i]) = v;
     }
+  if constexpr (KT * 4 > kNormPieceRow) {
+    if (p.K * 4 > kNormPieceRow) {
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        ss[m] = 0.f;
+        for (int i = tid; i < p.K; i += kWarps * 32) ss[m] += xs[0][m][i] * xs[0][m][i];
+      }
+    }
+  }
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
     ss[m] = warp_sum(ss[m]);
