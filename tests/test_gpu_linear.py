@@ -599,3 +599,28 @@ def test_long_rows_are_normalised_as_add_rmsnorm_does(cuda, K):
         assert group.after_norm(ops.normalisation(residual, delta, w, kept, 1e-6), 1, [out], ws)
         assert torch.equal(kept, after)
         assert torch.equal(out, group(xn)[0])
+
+
+def test_a_residual_over_its_own_terms_is_refused(cuda):
+    """residual_out sharing memory with residual or delta, whole or in part: an error from both entry points, nothing written.  Neighbours are fine."""
+    from transformer_surgeon_b200 import ops
+    M, K = 2, 64
+    g = torch.Generator(device=cuda).manual_seed(56)
+    dense = lambda o, i: ops.PackedLinear(ops.Factor.dense(torch.randn((o, i), generator=g, device=cuda)), None, None, torch.float32)
+    group, mlp = ops.LinearGroup([dense(8, K)]), ops.GatedMLP(dense(32, K), dense(32, K), dense(K, 32))
+    ws = torch.zeros(max(group.workspace_bytes(M), mlp.workspace_bytes(M)), dtype=torch.uint8, device=cuda)
+    rows = torch.randn((5 * M, K), generator=g, device=cuda)
+    w, outs = torch.ones(K, device=cuda), (torch.zeros((M, 8), device=cuda), torch.zeros((M, K), device=cuda))
+    before = rows.clone()
+    def both(residual, delta, kept):
+        norm = ops.normalisation(residual, delta, w, kept, 1e-6)
+        return lambda: group.after_norm(norm, M, [outs[0]], ws), lambda: mlp.after_norm(norm, M, outs[1], ws)
+    a, b, c = rows[:M], rows[M:2 * M], rows[M + 1:2 * M + 1]
+    for residual, delta, kept in ((a, b, a), (a, b, b), (a, b, c), (c, a, b), (a, None, a)):
+        for call in both(residual, delta, kept):
+            with pytest.raises(ops.Tsb200Error):
+                call()
+    assert torch.equal(rows, before) and not outs[0].any() and not outs[1].any()
+    for call in both(a, b, rows[2 * M:3 * M]):
+        assert call()
+    assert torch.equal(rows[2 * M:3 * M], a + b)

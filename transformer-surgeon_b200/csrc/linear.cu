@@ -125,7 +125,7 @@ extern "C" int tsb200_linear_group(const tsb200_linear_desc* const* d, int n, co
 extern "C" int tsb200_norm_linear_group(const tsb200_norm_desc* norm, const tsb200_linear_desc* const* d, int n, void* const* y, int64_t M, void* workspace,
                                         size_t workspace_bytes, void* stream) {
   TSB_REQUIRE_DEVICE();
-  if (!norm || !norm->residual || !norm->weight || !norm->residual_out || norm->residual_out == norm->residual || !d || !y || n < 1) return TSB200_ERR_ARG;
+  if (!norm || !norm->residual || !norm->weight || !norm->residual_out || !d || !y || n < 1) return TSB200_ERR_ARG;
   bool noop = false;
   for (int i = 0; i < n; ++i) {
     const int st = validate_linear(d[i], norm->residual, y[i], M, noop);

@@ -607,8 +607,15 @@ int launch_any(F32Params& p, int bits, bool gated, bool pdl, cudaStream_t s) {
   }
 }
 
+// The first CTA stores the residual while others still read what it is the sum of: none of the two may share a byte with it.
+bool overlap(const void* a, const void* b, int64_t bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return (x < y ? y - x : x - y) < (uintptr_t)bytes;
+}
 int take_norm(F32Params& p, const tsb200_norm_desc* norm) {
   if (!norm) return TSB200_OK;
+  const int64_t bytes = (int64_t)p.M * p.K * 4;
+  if (overlap(norm->residual_out, norm->residual, bytes) || (norm->delta && overlap(norm->residual_out, norm->delta, bytes))) return TSB200_ERR_ARG;
   if (p.K % 4 || !aligned(norm->residual, 16) || !aligned(norm->residual_out, 16) || !aligned(norm->weight, 16) || !aligned(norm->delta, 16))
     return TSB200_ERR_UNSUPPORTED;
   p.norm = Norm{(const float*)norm->residual, (const float*)norm->delta, (const float*)norm->weight, (float*)norm->residual_out, norm->eps};

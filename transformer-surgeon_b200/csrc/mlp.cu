@@ -268,7 +268,7 @@ int tsb200_mlp_gated(const tsb200_linear_desc* gate, const tsb200_linear_desc* u
 int tsb200_norm_mlp_gated(const tsb200_norm_desc* norm, const tsb200_linear_desc* gate, const tsb200_linear_desc* up,
                           const tsb200_linear_desc* down, void* y, int64_t M, void* workspace, size_t workspace_bytes, void* stream) {
   TSB_REQUIRE_DEVICE();
-  if (!norm || !norm->residual || !norm->weight || !norm->residual_out || norm->residual_out == norm->residual) return TSB200_ERR_ARG;
+  if (!norm || !norm->residual || !norm->weight || !norm->residual_out) return TSB200_ERR_ARG;
   if (!block_ok(gate, up, down, M)) return TSB200_ERR_ARG;
   if (M == 0) return TSB200_OK;
   if (!y || !workspace || !aligned(workspace, 256)) return TSB200_ERR_ARG;
