@@ -624,3 +624,15 @@ def test_a_residual_over_its_own_terms_is_refused(cuda):
     for call in both(a, b, rows[2 * M:3 * M]):
         assert call()
     assert torch.equal(rows[2 * M:3 * M], a + b)
+
+
+def test_normalisation_of_other_types_and_sizes_is_refused(cuda):
+    from transformer_surgeon_b200 import ops
+    r, w = torch.zeros((2, 64), device=cuda), torch.ones(64, device=cuda)
+    ops.normalisation(r, r, w, torch.empty_like(r), 1e-6)
+    for args in ((r.bfloat16(), None, w, r), (r, r.bfloat16(), w, r), (r, None, w.bfloat16(), r), (r, None, w, r.bfloat16())):
+        with pytest.raises(TypeError):
+            ops.normalisation(*args, 1e-6)
+    for args in ((r, r[:1], w, r), (r, None, w[:32], r), (r, None, w, r[:1]), (r, r.cpu(), w, r), (r, r.t().contiguous().t(), w, r)):
+        with pytest.raises(ValueError):
+            ops.normalisation(*args, 1e-6)

@@ -372,8 +372,15 @@ class LinearGroup:
 
 
 def normalisation(residual, delta, weight, residual_out, eps):
-    """What LinearGroup.after_norm and GatedMLP.after_norm normalise: residual + delta (kept in residual_out, a buffer of its own)."""
-    return NormDesc(_cuda(residual, "residual").data_ptr(), _p(delta), _cuda(weight, "weight").data_ptr(), _cuda(residual_out, "residual_out").data_ptr(), float(eps))
+    """What LinearGroup.after_norm and GatedMLP.after_norm normalise: residual + delta (kept in residual_out, a buffer of its own), fp32."""
+    for t, name in ((delta, "delta"), (residual_out, "residual_out")):
+        if t is not None and _cuda(t, name).numel() != residual.numel():
+            raise ValueError(f"{name} must have residual's size")
+    if weight.numel() != residual.shape[-1]:
+        raise ValueError("weight must have one element per column")
+    if any(t is not None and t.dtype != torch.float32 for t in (residual, delta, weight, residual_out)):
+        raise TypeError("layers that normalise their own input take fp32 tensors")
+    return NormDesc(_cuda(residual, "residual").data_ptr(), _p(delta), _cuda(weight, "weight").data_ptr(), residual_out.data_ptr(), float(eps))
 
 
 def _fused(status, what):
