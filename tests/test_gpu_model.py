@@ -258,3 +258,22 @@ def test_batched_prefill_matches_stepwise(cuda, family, dtype, kv):
     if kv == "int8" and dtype == torch.float32:
         for a, kvl in zip(pools_s, dec.kv):
             assert torch.equal(a, kvl.k_pool)
+
+
+@pytest.mark.parametrize("batch", [4, 5])
+def test_eager_fp32_steps_set_nothing_up(cuda, monkeypatch, batch):
+    """Uncaptured fp32 steps after the first: no layer group is built, and with more sequences than the normalising projections take they
+    are not asked."""
+    from transformer_surgeon_b200 import ops
+    _, eng = build("qwen2", cuda, "fp32", batch=batch)
+    tokens = torch.zeros(batch, dtype=torch.int64, device=cuda)
+    eng.step(tokens)
+    calls = []
+    for cls, name in ((ops.LinearGroup, "__init__"), (ops.LinearGroup, "after_norm"), (ops.GatedMLP, "after_norm")):
+        def counted(self, *a, _f=getattr(cls, name), _name=name, **k):
+            calls.append(_name)
+            return _f(self, *a, **k)
+        monkeypatch.setattr(cls, name, counted)
+    eng.step(tokens)
+    assert "__init__" not in calls
+    assert calls == ["after_norm"] * (2 * len(eng.layers) if batch == 4 else 0)

@@ -51,13 +51,17 @@ class LayerWeights:
         self._group = None
 
     @property
+    def projections(self):
+        """q, k and v, or the one layer they are packed as, behind one call."""
+        layers = [self.q, self.k, self.v] if self.qkv is None else [self.qkv]
+        if self._group is None or self._group.layers != layers:      # a layer may have been replaced
+            self._group = ops.LinearGroup(layers)
+        return self._group
+
+    @property
     def qkv_group(self):
         """q, k and v behind one call (None where they are packed as one layer)."""
-        if self.qkv is not None:
-            return None
-        if self._group is None or self._group.layers != [self.q, self.k, self.v]:      # a layer may have been replaced
-            self._group = ops.LinearGroup([self.q, self.k, self.v])
-        return self._group
+        return self.projections if self.qkv is None else None
 
 
 def fuse_rows(factors, biases, act_dtype):
@@ -182,14 +186,14 @@ class CompressedDecoder:
         delta = None
         rope = (self.cos, self.sin)
         peer = self.peer if tp_on else None
-        # fp32: q, k, v and the MLP take residual and delta and normalise them themselves, two launches a layer fewer
-        # (the residual then alternates between two buffers)
-        own_norm = c.dtype == torch.float32 and c.norm_variant == 0 and not tp_on
+        # fp32, few sequences: q, k, v and the MLP take residual and delta and normalise them themselves, two launches a layer
+        # fewer (the residual then alternates between two buffers)
+        own_norm = c.dtype == torch.float32 and c.norm_variant == 0 and not tp_on and B <= ops.NORM_TOKENS
         resid, resid_next = self.resid, self.resid_next
         for li, L in enumerate(self.layers):
             group = L.qkv_group
             outs = (self.qkv,) if group is None else (self.qb, self.kb, self.vb)
-            if own_norm and (group or ops.LinearGroup([L.qkv])).after_norm(ops.normalisation(resid, delta, L.ln1, resid_next, c.rms_eps), B, outs, self.lin_ws):
+            if own_norm and L.projections.after_norm(ops.normalisation(resid, delta, L.ln1, resid_next, c.rms_eps), B, outs, self.lin_ws):
                 resid, resid_next = resid_next, resid
                 n += 1 if group is None else 2 if L.q.rank else 1
             else:

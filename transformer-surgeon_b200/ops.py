@@ -371,6 +371,9 @@ class LinearGroup:
                       "tsb200_norm_linear_group")
 
 
+NORM_TOKENS = 4      # layers take their input through after_norm up to this many tokens
+
+
 def normalisation(residual, delta, weight, residual_out, eps):
     """What LinearGroup.after_norm and GatedMLP.after_norm normalise: residual + delta (kept in residual_out, a buffer of its own), fp32."""
     for t, name in ((delta, "delta"), (residual_out, "residual_out")):
