@@ -218,9 +218,6 @@ template <> struct Raw8<__nv_bfloat16> {
     }
   }
   __device__ __forceinline__ void load_shared(const __nv_bfloat16* p) { load(p, true); }
-  // 16-byte pieces 32 apart in shared memory
-  __device__ __forceinline__ void load_strided(const uint4* p) { load(reinterpret_cast<const __nv_bfloat16*>(p), true); }
-  __device__ __forceinline__ void store_strided(uint4* p) const { store(reinterpret_cast<__nv_bfloat16*>(p), true); }
   __device__ __forceinline__ void store(__nv_bfloat16* p, bool vec) const {
     if (vec) {
       *reinterpret_cast<uint4*>(p) = make_uint4(u[0], u[1], u[2], u[3]);
@@ -266,14 +263,6 @@ template <> struct Raw8<float> {
     }
   }
   __device__ __forceinline__ void load_shared(const float* p) { load(p, true); }
-  __device__ __forceinline__ void load_strided(const uint4* p) {
-    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 32);
-    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-  }
-  __device__ __forceinline__ void store_strided(uint4* p) const {
-    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
-    *reinterpret_cast<float4*>(p + 32) = make_float4(f[4], f[5], f[6], f[7]);
-  }
   __device__ __forceinline__ void store(float* p, bool vec) const {
     if (vec) {
       *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
@@ -422,12 +411,12 @@ __device__ __forceinline__ void transpose4(const unsigned (&in)[4], unsigned (&o
 // take 128 registers a thread and leave 24 % of the warps.  Instructions and their latencies bound it: a further instruction an element
 // costs 2 to 4 us.  32 x 2048 tokens, 8 heads, d 128, FP8, 402 MB, with the scales' launch (48 us): 141.6 us; 147.6 with loads that a task
 // waits for, two corrections a quotient and selects for what saturates; 290 with one warp per token vector and a byte-wise transpose.
-template <typename T, int D, int FMT> struct AppendSmem {
-  uint4 stage[8][8 * sizeof(T) / 2][32];                                  // per warp: a task's elements, 16-byte pieces by lane
+template <typename T, int D, int FMT, bool AHEAD> struct AppendSmem {
+  uint4 stage[8][AHEAD ? 8 : 1][32];                                      // per warp: a task's elements, 16-byte pieces by lane (bf16)
   T cos[2048 / D][D / 2], sin[2048 / D][D / 2];
   unsigned v[4][128 / D][(FMT == TSB200_KV_NVFP4 ? D / 2 : D) * 4];       // V records of the warps that have V (the odd ones)
 };
-template <typename T, int D, int FMT>
+template <typename T, int D, int FMT, bool AHEAD>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 1)
 kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qheads, const T* __restrict__ k,
                        const T* __restrict__ v, int64_t ks, int64_t vs_, int64_t Tn, const int32_t* __restrict__ new_lens,
@@ -438,7 +427,7 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   constexpr int EG = HALF / 8;                                            // lanes side by side on a vector
   constexpr int ROWS = FP4 ? D / 2 : D;                                   // 16-byte rows of a V record
   extern __shared__ __align__(16) uint8_t append_smem[];
-  auto& smem = *reinterpret_cast<AppendSmem<T, D, FMT>*>(append_smem);
+  auto& smem = *reinterpret_cast<AppendSmem<T, D, FMT, AHEAD>*>(append_smem);
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int eg = lane % EG, tq = lane / EG;                               // elements 8 eg .., tokens 4 tq .. of the CTA's
@@ -462,11 +451,13 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
   const int lt = page_of_lane * 16 + slot0;                               // the lane's first token in the tables
 
   // tasks: K or V of a head (half the registers of both at once; a warp's are all K or all V), then query heads; dealt out over the grid's
-  // CTAs of these pages.  A task's elements are on their way while the task before it is encoded, the first one's while tables and page
-  // numbers are fetched: every lane copies what it will read itself.
+  // CTAs of these pages.  AHEAD: a task's elements are on their way while the task before it is encoded, the first one's while tables and page
+  // numbers are fetched: every lane copies what it will read itself.  Not so with one task to a warp, which nothing hides the detour of
+  // (NVFP4, 4 x 2048 tokens, 4 heads of 128: 12.5 us, 10.2 without), nor for fp32: a lane's 32 bytes would come from the L2 as two halves of a sector
+  // (FP8, 32 x 2048 tokens, 4 heads of 128: 185 us, 118 without).
   const int tasks = 2 * kv.hkv + (q && rope_cos ? qheads : 0), task_step = 8 * (int)gridDim.z;
   int task = w + 8 * (int)blockIdx.z;
-  auto staged = [&](int i, int half) { return &smem.stage[w][(i * 2 + half) * (int)sizeof(T) / 2][lane]; };   // 16-byte pieces, 32 apart
+  auto staged = [&](int i, int half) { return &smem.stage[w][i * 2 + half][lane]; };
   float fp8_scale = 1.f;
   auto fetch = [&](int t) {
     if (t >= 2 * kv.hkv) return;
@@ -481,20 +472,18 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           if (vec) {
-#pragma unroll
-            for (int u = 0; u < (int)sizeof(T) / 2; ++u)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(staged(i, half) + 32 * u)),
-                           "l"(reinterpret_cast<const uint4*>(p + half * HALF) + u) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(staged(i, half))),
+                         "l"(reinterpret_cast<const uint4*>(p + half * HALF)) : "memory");
           } else {
             Raw8<T> r;
             r.load(p + half * HALF, false);
-            r.store_strided(staged(i, half));
+            r.store(reinterpret_cast<T*>(staged(i, half)), true);
           }
         }
       }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  fetch(task);
+  if constexpr (AHEAD) fetch(task);
   int64_t page = lp >= 0 && lp < kv.bt_stride ? (int64_t)kv.block_table[b * kv.bt_stride + lp] : -1;
   const bool page_ok = page >= 0 && page < kv.num_pages;
   if (rope_cos) {
@@ -516,19 +505,36 @@ kv_append_pages_kernel(tsb200_kv_desc kv, T* __restrict__ q, int64_t qs, int qhe
     const int h = task >> 1;
     const bool is_v = task & 1;
     uint8_t* rec = (is_v ? kv.v_pool : kv.k_pool) + ((page_ok ? page : 0) * kv.hkv + h) * rec_bytes;
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     Raw8<T> x[4][2];
+    if constexpr (AHEAD) {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (tok[i]) {
-        x[i][0].load_strided(staged(i, 0)); x[i][1].load_strided(staged(i, 1));
-      } else {
-        x[i][0] = x[i][1] = Raw8<T>{};
+      for (int i = 0; i < 4; ++i) {
+        if (tok[i]) {
+          x[i][0].load_shared(reinterpret_cast<const T*>(staged(i, 0))); x[i][1].load_shared(reinterpret_cast<const T*>(staged(i, 1)));
+        } else {
+          x[i][0] = x[i][1] = Raw8<T>{};
+        }
       }
+    } else {
+      const int64_t stride = is_v ? vs_ : ks;
+      const T* p = (is_v ? v : k) + (b * Tn + j0) * stride + (int64_t)h * D + eg * 8;
+      const bool vec = is_v ? vvec : kvec;
+#pragma unroll
+      for (int i = 0; i < 4; ++i, p += stride) {
+        if (tok[i] && page_ok) {
+          x[i][0].load(p, vec); x[i][1].load(p + HALF, vec);
+        } else {
+          x[i][0] = x[i][1] = Raw8<T>{};
+        }
+      }
+      if (FMT == TSB200_KV_FP8) fp8_scale = (is_v ? kv.v_scale : kv.k_scale)[b * kv.hkv + h];
     }
     const Divisor shared = divisor(fp8_scale);
-    __syncwarp();                              // read: the next task's elements may come
-    fetch(task + task_step);
+    if constexpr (AHEAD) {
+      __syncwarp();                            // read: the next task's elements may come
+      fetch(task + task_step);
+    }
     // FP8, bf16: what lies beyond 512 scales saturates as that does (e4m3 ends at 448), without an infinite quotient on the way
     unsigned bound = 0x7f807f80u;
     if (FMT == TSB200_KV_FP8 && sizeof(T) == 2 && !shared.slow) {
@@ -780,24 +786,30 @@ int launch_append(const tsb200_kv_desc& kv, void* q, int64_t qs, int qheads, con
     int64_t z = 444 / (groups * B);
     if (z > (tasks + 7) / 8) z = (tasks + 7) / 8;
     const dim3 grid((unsigned)groups, (unsigned)B, (unsigned)(z < 1 ? 1 : z));
-    auto go = [&](auto fmt) {
+    auto go = [&](auto fmt, auto ahead) {
       constexpr int FMT = decltype(fmt)::value;
-      constexpr size_t smem = sizeof(AppendSmem<T, D, FMT>);
+      constexpr bool AHEAD = decltype(ahead)::value;
+      constexpr size_t smem = sizeof(AppendSmem<T, D, FMT, AHEAD>);
       static bool configured[64] = {false};
       int dev = 0;
       cudaError_t e = cudaGetDevice(&dev);
       if (e != cudaSuccess) return e;
       if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
       if (!configured[dev]) {
-        e = cudaFuncSetAttribute(kv_append_pages_kernel<T, D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(kv_append_pages_kernel<T, D, FMT, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
       }
-      return launch_kernel(kv_append_pages_kernel<T, D, FMT>, grid, dim3(256), smem, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec);
+      return launch_kernel(kv_append_pages_kernel<T, D, FMT, AHEAD>, grid, dim3(256), smem, s, kv, (T*)q, qs, qheads, (const T*)k, (const T*)v, ks, vs, Tn, new_lens, rc, rs, rr, rec);
     };
-    if (kv.format == TSB200_KV_INT8) TSB_CUDA(go(std::integral_constant<int, TSB200_KV_INT8>{}));
-    else if (kv.format == TSB200_KV_FP8) TSB_CUDA(go(std::integral_constant<int, TSB200_KV_FP8>{}));
-    else TSB_CUDA(go(std::integral_constant<int, TSB200_KV_NVFP4>{}));
+    auto pick = [&](auto fmt) {
+      if constexpr (sizeof(T) == 2)
+        if (8 * (int)grid.z < 2 * kv.hkv) return go(fmt, std::true_type{});      // several tasks to a warp
+      return go(fmt, std::false_type{});
+    };
+    if (kv.format == TSB200_KV_INT8) TSB_CUDA(pick(std::integral_constant<int, TSB200_KV_INT8>{}));
+    else if (kv.format == TSB200_KV_FP8) TSB_CUDA(pick(std::integral_constant<int, TSB200_KV_FP8>{}));
+    else TSB_CUDA(pick(std::integral_constant<int, TSB200_KV_NVFP4>{}));
     TSB_LAUNCH_CHECK();
     return TSB200_OK;
   }
