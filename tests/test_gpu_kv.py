@@ -655,3 +655,39 @@ def test_long_splits_have_the_bits_of_shorter_ones(cuda, name):
     kv.seq_lens -= (torch.arange(B, device=cuda) * 97).to(torch.int32)
     q = torch.randn((B, H, d), generator=g, device=cuda).to(DT[name])
     assert torch.equal(ops.paged_decode_attention(kv, q, 4096), ops.paged_decode_attention(kv, q, 4080))
+
+
+def filled_cache(fmt, B, pages, Hkv, d, name, cuda, g):
+    """B sequences of pages * 16 tokens over scattered pages, and a function for the first n of them."""
+    from transformer_surgeon_b200 import ops
+    bt = torch.randperm(B * pages, generator=g, device=cuda).to(torch.int32).reshape(B, pages)
+    kv = ops.PagedKV(fmt, B * pages, Hkv, d, bt, torch.zeros(B, dtype=torch.int32, device=cuda), cuda)
+    if fmt == "fp8":
+        kv.fill_fp8_scales(6.0 / 448, 6.0 / 448)
+    kv.append(*(torch.randn((B, pages * 16, Hkv, d), generator=g, device=cuda).to(DT[name]) for _ in range(2)))
+
+    def first(n):
+        few = ops.PagedKV(fmt, B * pages, Hkv, d, bt[:n].contiguous(), kv.seq_lens[:n].contiguous(), cuda)
+        few.k_pool, few.v_pool = kv.k_pool, kv.v_pool
+        if fmt == "fp8":
+            few.fill_fp8_scales(6.0 / 448, 6.0 / 448)
+        return few
+    return kv, first
+
+
+@pytest.mark.parametrize("fmt,H,Hkv,B,few,S", [("fp8", 4, 1, 33, 33, 2)] + [("fp8", 4, 1, B, 33, S) for S, B in ((3, 96), (4, 73), (5, 58), (6, 48), (7, 40), (8, 37))])
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+def test_clusters_of_every_size_merge_as_a_launch_does(cuda, fmt, H, Hkv, B, few, S, name):
+    """Two to eight splits of a sequence: so many pairs that the clusters would not fit the device at once take the reduction launch, the first few
+    of the same sequences clusters, with the same bits.  Both against the one-lane-per-element kernel (bound: attn_tol's)."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(61)
+    pages = 24 * S if fmt == "fp8" and H // Hkv <= 4 else 4 * S + 1          # as many as give S splits
+    kv, first = filled_cache(fmt, B, pages, Hkv, 128, name, cuda, g)
+    kv.seq_lens = (pages * 16 - torch.arange(B, device=cuda) * 37 % (pages * 16 + 1)).to(torch.int32)
+    q = torch.randn((B, H, 128), generator=g, device=cuda).to(DT[name])
+    out = ops.paged_decode_attention(kv, q, pages * 16)
+    assert torch.equal(ops.paged_decode_attention(first(few), q[:few].contiguous(), pages * 16), out[:few])
+    ref = ops.paged_decode_attention(kv, q, pages * 16, simt=True).float()
+    scale = 6.0 if fmt == "fp8" else 5.0                                    # |V| of N(0, 1)
+    assert torch.all((out.float() - ref).abs() <= C_P_TC * scale + 2 * C_OUT[name] * ref.abs() + 1e-6)

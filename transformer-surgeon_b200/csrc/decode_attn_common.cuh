@@ -145,6 +145,30 @@ __device__ __forceinline__ void merge_cluster(const float* part, int heads, int 
   }
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
+// Clusters (1, S, 1) of `kernel` that the device holds at a time (0: none).  `cache`: of one instance and device, by S; 0 = not asked yet.
+template <typename K>
+inline int active_clusters(K* kernel, dim3 grid, int threads, size_t smem, int (&cache)[kMaxCluster + 1]) {
+  if (cache[grid.y]) return cache[grid.y] - 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = grid.y;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  cache[grid.y] = n + 1;
+  return n;
+}
+
 // Launch of grid (pairs, S, chunks); `clusters`: one per (pair, chunk), its CTAs merge the splits themselves.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_splits(bool overlap, bool clusters, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
@@ -228,6 +252,8 @@ __device__ __forceinline__ void merge_splits(const float* __restrict__ part, int
   }
 }
 
+// Merges partials (decode_attn_simt.cu), chained to the attention launch.
+template <typename T, int D> int launch_reduce(const float* ws, int64_t BH, int S, void* out, cudaStream_t st);
 int validate_kv(const tsb200_kv_desc* kv, bool need_table);
 
 }  // namespace tsb

@@ -18,8 +18,6 @@
 
 namespace tsb {
 
-template <typename T, int D> int launch_reduce(const float* ws, int64_t BH, int S, void* out, cudaStream_t st);
-
 namespace {
 
 using tc::mbar_arrive;
@@ -396,8 +394,8 @@ decode_attn_fp8_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
 }  // namespace
 
 // FP8 pages, head_dim 128, group <= 4: returns TSB200_ERR_UNSUPPORTED otherwise (the caller then
-// uses the f16 tensor-core kernel).  Up to eight splits merge in a cluster; more leave their
-// partials to a reduction launch.
+// uses the f16 tensor-core kernel).  Up to eight splits merge in a cluster where all clusters fit the
+// device at once; otherwise their partials are left to a reduction launch.
 template <typename T>
 int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
                     int64_t B, float* ws, void* out, int* status, cudaStream_t st) {
@@ -413,10 +411,14 @@ int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, 
     configured[dev] = true;
   }
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, 1);
-  // (the grid is one wave: clusters wait for nobody; 8 sequences x 8 kv heads x 4k-8k tokens, 4 splits: 29.9 us, 32.1 with the reduction launch)
-  TSB_CUDA(launch_splits(attn_overlaps(kv), S > 1 && S <= kMaxCluster, decode_attn_fp8_kernel<T>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
+  // The CTAs of a cluster share a group of SMs, so that the 296 slots hold fewer than 296 / S clusters (148, 93, 71, 56, 45, 37, 33 of two to eight); the
+  // rest would start when a whole one has ended.  9 sequences x 4 kv heads x 2k-4k tokens, 8 splits: 20.1 us in clusters, 14.0 with the launch; 12 x 8 x
+  // 4k-8k, 3 splits 49.2 / 37.3; where they fit, 8 x 8 x 4k-8k, 4 splits 29.9 / 30.6, 16 x 8 x 1k-2k, 2 splits 18.1 / 19.9.
+  static int held[64][kMaxCluster + 1] = {};
+  const bool clusters = S > 1 && S <= kMaxCluster && (int64_t)grid.x <= active_clusters(decode_attn_fp8_kernel<T>, grid, kWarps * 32, smem, held[dev]);
+  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_fp8_kernel<T>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale, max_seq_len,
                          S, ws, (T*)out, status));
-  return TSB200_OK;
+  return S == 1 || clusters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }
 template int launch_attn_fp8<float>(const tsb200_kv_desc&, const void*, int64_t, int, float, int64_t, int, int64_t, float*, void*, int*,
                                     cudaStream_t);

@@ -25,7 +25,6 @@
 
 namespace tsb {
 
-template <typename T, int D> int launch_reduce(const float* ws, int64_t BH, int S, void* out, cudaStream_t st);
 template <typename T>
 int launch_attn_fp8(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
                     int64_t B, float* ws, void* out, int* status, cudaStream_t st);
@@ -502,10 +501,8 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   if (kv->format == TSB200_KV_FP8 && D == 128 && H / kv->hkv <= 4) {
     // e4m3 pages go to the tensor cores as FP8 (decode_attn_fp8.cu)
     const int S8 = choose_splits_fp8(B, kv->hkv, max_seq_len);   // never more than choose_splits(): the workspace fits
-    const int r = dtype == TSB200_F32 ? launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s)
-                                      : launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s);
-    if (r != TSB200_OK || S8 <= kMaxCluster) return r;
-    return dtype == TSB200_F32 ? launch_reduce<float, 128>(ws, B * H, S8, out, s) : launch_reduce<__nv_bfloat16, 128>(ws, B * H, S8, out, s);
+    return dtype == TSB200_F32 ? launch_attn_fp8<float>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s)
+                               : launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s);
   }
   const int S = choose_splits(B, kv->hkv, max_seq_len);
   const bool long_splits = kv->format == TSB200_KV_NVFP4 && D == 128 && (max_seq_len + 15) / 16 >= 64 * S;
