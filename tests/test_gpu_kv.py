@@ -675,7 +675,8 @@ def filled_cache(fmt, B, pages, Hkv, d, name, cuda, g):
     return kv, first
 
 
-@pytest.mark.parametrize("fmt,H,Hkv,B,few,S", [("fp8", 4, 1, 33, 33, 2)] + [("fp8", 4, 1, B, 33, S) for S, B in ((3, 96), (4, 73), (5, 58), (6, 48), (7, 40), (8, 37))])
+@pytest.mark.parametrize("fmt,H,Hkv,B,few,S", [("fp8", 4, 1, 33, 33, 2)] + [("fp8", 4, 1, B, 33, S) for S, B in ((3, 96), (4, 73), (5, 58), (6, 48), (7, 40), (8, 37))]
+                         + [(f, 8, 2, 128 if S == 3 else 75, 10, S) for f in ("int8", "nvfp4") for S in (3, 5, 6, 7)] + [("fp8", 10, 2, 75, 10, S) for S in (5, 6, 7)])
 @pytest.mark.parametrize("name", ["fp32", "bf16"])
 def test_clusters_of_every_size_merge_as_a_launch_does(cuda, fmt, H, Hkv, B, few, S, name):
     """Two to eight splits of a sequence: so many pairs that the clusters would not fit the device at once take the reduction launch, the first few

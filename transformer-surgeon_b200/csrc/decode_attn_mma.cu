@@ -457,11 +457,16 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   }
   const int g = H / kv.hkv;
   dim3 grid((unsigned)(B * kv.hkv), (unsigned)S, (unsigned)((g + 7) / 8));
-  // Few splits of short sequences merge in a cluster, which spares the host a launch (a call by itself, 33 sequences x 8 kv heads x 83-166
-  // tokens, int8: 14.2 us with the launch, 12.3); clusters wait until an SM group has room for all their CTAs, so that longer work, which
-  // hides the host's time, is faster with the launch (captured: 64 x 8 x 4096, int8, 4 splits 89.6 us, clusters 97.7; 16 x 8 x 2000, NVFP4 19.2,
-  // 23.1; 32 x 8 x 200, NVFP4 11.8, 11.6).
-  const bool clusters = S > 1 && S <= kMaxCluster && B * kv.hkv * ((max_seq_len + 15) / 16) <= 4096;
+  // A cluster merges without another launch, but its CTAs start together, in one group of SMs, and none leaves before the last: it is the faster
+  // one as long as all of them fit the device at once (captured, NVFP4, head_dim 128: 16 sequences x 8 kv heads x 65-130 tokens, 2 splits, 6.3 us,
+  // launch 7.7; 12 x 8 x 500-1000, 8 splits, one CTA in twenty-five too many, 14.9 / 11.9; int8, 64 x 8 x 1k-2k, 4 splits 67.8 / 58.7).  Beyond that it
+  // depends on the outputs: the launch has a CTA per sequence and query head.  Two splits, more than one head to a CTA: 128 x 8 x 100-200, 8
+  // heads 27.7 / 46.2; one head 21.7 / 20.8.  Up to four splits, more than four heads: 64 x 8 x 250-500, 8 heads 27.6 / 34.4, 4 heads 35.4 / 35.3.  Over
+  // 2204 calls of several splits this choice is 0.7 % from the better of the two.
+  static int held[64][kMaxCluster + 1] = {};
+  const bool clusters = S > 1 && S <= kMaxCluster &&
+                        ((S == 2 && g > 1) || (S <= 4 && g > 4) ||
+                         (int64_t)grid.x * grid.z <= active_clusters(decode_attn_mma_kernel<T, D, FMT, LONG>, grid, kWarps * 32, smem, held[dev]));
   TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT, LONG>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, (T*)out, status));
   return S == 1 || clusters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
