@@ -692,3 +692,19 @@ def test_clusters_of_every_size_merge_as_a_launch_does(cuda, fmt, H, Hkv, B, few
     ref = ops.paged_decode_attention(kv, q, pages * 16, simt=True).float()
     scale = 6.0 if fmt == "fp8" else 5.0                                    # |V| of N(0, 1)
     assert torch.all((out.float() - ref).abs() <= C_P_TC * scale + 2 * C_OUT[name] * ref.abs() + 1e-6)
+
+
+@pytest.mark.parametrize("fmt,d,B,Hkv,pages", [("nvfp4", 64, 90, 12, 7), ("nvfp4", 64, 64, 12, 2), ("fp8", 64, 90, 12, 7), ("fp8", 64, 64, 12, 1),
+                                               ("nvfp4", 128, 40, 16, 3)])
+@pytest.mark.parametrize("name", ["fp32", "bf16"])
+def test_attention_of_many_and_of_few_ctas(cuda, fmt, d, B, Hkv, pages, name):
+    """The instances for more CTAs than the GPU holds and for fewer (more warps against more registers; rings of four pages where all CTAs of
+    them fit): the first sequences of many are the same bits by themselves."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(62)
+    kv, first = filled_cache(fmt, B, pages, Hkv, d, name, cuda, g)
+    kv.seq_lens = (torch.arange(B, device=cuda) * 13 % (pages * 16 + 1)).to(torch.int32)
+    q = torch.randn((B, 2 * Hkv, d), generator=g, device=cuda).to(DT[name])
+    n = 9                                                       # (fewer than eight pages: one split, however few the sequences)
+    out = ops.paged_decode_attention(kv, q, pages * 16)
+    assert torch.equal(ops.paged_decode_attention(first(n), q[:n].contiguous(), pages * 16), out[:n])

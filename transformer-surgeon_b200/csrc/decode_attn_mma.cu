@@ -44,13 +44,18 @@ constexpr unsigned kWaitLimit = 1u << 22;
 // Warps per CTA, ring stages (pages) per warp, CTAs per SM that registers are to allow.  What counts is how many CTAs an SM holds: the page
 // loop is bound by the instructions that widen codes and by the chain of a page's softmax, and the warps of other CTAs fill its gaps.  int8,
 // head_dim 64: 30 sequences x 2 kv heads x 1.5k-3k tokens 12.4 us at 5 CTAs, 13.5 at 4; head_dim 128 is limited by registers (3).  NVFP4, 128:
-// 5 CTAs of 3 stages against 4 of 4: 16 x 4 x 1k-2k tokens 14.2 us to 15.1, 16 x 8 x 1k-2k 19.2 to 21.4, 16 x 4 x 6k-12k (62 pages a split)
-// 43.1 to 44.6; 64 x 8 x 2k-4k (64 pages) 91.7 to 86.9, 8 x 4 x 16k-32k (85) 57.4 to 54.3.
-// Hence LONG: splits of 64 pages and more, whose warps stream 16 and more.
-template <int FMT, int D, bool LONG> struct AttnCfg {
+// VAR is another instance for some grids (the dispatch at the end counts CTAs; times of 1100 grids, captured):
+//   * NVFP4, 128: 3 stages and 5 CTAs, or (VAR) 4 and 4, which has the registers for it.  VAR for up to 512 CTAs, which it holds at once too (1 x 8 x 16k-32k
+//     tokens, 64 splits: 17.9 -> 15.1 us; none slower by more than runs differ), and for splits of 64 pages and more: on grids of two waves of
+//     either 2-5 % faster, on 768 CTAs, one and a bit, 5 % faster to 4 % slower.  Shorter splits want the fifth CTA (16 x 8 x 250-500,
+//     5 pages a split: 10.4 us, VAR 11.8; 21 pages 20.0 / 20.1).
+//   * NVFP4 and FP8, 64: 88 registers and 5 CTAs, or (VAR) 64 and 8 (FP8: 24 bytes spilled).  VAR where there are more CTAs than the first holds and few
+//     pages to each, so that what counts is how many start at a time (NVFP4, 128 x 12 x 32-64 tokens 9.5 -> 7.8 us, 128 x 4 x 65-130, 8
+//     heads 11.6 -> 9.1); with long splits or few CTAs it is up to a third slower.
+template <int FMT, int D, bool VAR> struct AttnCfg {
   static constexpr int kWarps = FMT == TSB200_KV_INT8 ? 6 : 4;
-  static constexpr int kStages = FMT == TSB200_KV_INT8 && D == 128 ? 2 : (LONG ? 4 : 3);
-  static constexpr int kCtas = FMT == TSB200_KV_INT8 ? (D == 128 ? 3 : 5) : (FMT == TSB200_KV_NVFP4 && D == 128 && !LONG ? 5 : 4);
+  static constexpr int kStages = FMT == TSB200_KV_INT8 && D == 128 ? 2 : (D == 128 && VAR ? 4 : 3);
+  static constexpr int kCtas = FMT == TSB200_KV_INT8 ? (D == 128 ? 3 : 5) : D == 64 && VAR ? 8 : (FMT == TSB200_KV_NVFP4 && D == 128 && !VAR ? 5 : 4);
 };
 
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -127,13 +132,13 @@ template <int FMT, int D> struct RecBytes {
   static constexpr int value = FMT == TSB200_KV_INT8 ? 16 * D + 64 : (FMT == TSB200_KV_NVFP4 ? 9 * D : 16 * D);
 };
 
-template <typename T, int D, int FMT, bool LONG>
-__global__ void __launch_bounds__(AttnCfg<FMT, D, LONG>::kWarps * 32, AttnCfg<FMT, D, LONG>::kCtas)
+template <typename T, int D, int FMT, bool VAR>
+__global__ void __launch_bounds__(AttnCfg<FMT, D, VAR>::kWarps * 32, AttnCfg<FMT, D, VAR>::kCtas)
 decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S,
                        float* __restrict__ ws, T* __restrict__ out, int* __restrict__ status) {
   constexpr bool FP4 = FMT == TSB200_KV_NVFP4;
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int kWarps = AttnCfg<FMT, D, LONG>::kWarps, kStages = AttnCfg<FMT, D, LONG>::kStages;
+  constexpr int kWarps = AttnCfg<FMT, D, VAR>::kWarps, kStages = AttnCfg<FMT, D, VAR>::kStages;
   constexpr int STAGE = 2 * REC;                // K and V of a page
   constexpr int NC = D / 16;                    // k-steps of QK, m-tiles of PV
   extern __shared__ __align__(128) uint8_t smem[];
@@ -147,13 +152,13 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   uint8_t* ring = smem + kBarBytes + (size_t)w * kStages * STAGE;
   uint2* vscales = reinterpret_cast<uint2*>(smem + kBarBytes + (size_t)kWarps * kStages * STAGE) + w * (D / 4);    // NVFP4
   const unsigned ring_a = smem_u32(ring), bar_a = smem_u32(smem) + w * kStages * 8;
+  // lengths and block table do not come from the preceding launch (see tsb200_set_pdl): looked up ahead of the dependency wait
+  int len = kv.seq_lens[b];
   if (lane == 0) {
     for (int i = 0; i < kStages; ++i) mbar_init(reinterpret_cast<unsigned long long*>(smem) + w * kStages + i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncwarp();
-  // lengths and block table do not come from the preceding launch (see tsb200_set_pdl): looked up ahead of the dependency wait
-  int len = kv.seq_lens[b];
   len = len < 0 ? 0 : (len > max_seq_len ? (int)max_seq_len : len);
   int pb, pe;
   split_range(len, s, S, pb, pe);
@@ -438,11 +443,11 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   if (clustered) merge_cluster<T, D>(sm_part, gn, S, out + ((int64_t)b * H + hk * g + g0) * D);
 }
 
-template <typename T, int D, int FMT, bool LONG>
+template <typename T, int D, int FMT, bool VAR>
 int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float sm_scale, int64_t max_seq_len, int S, int64_t B, float* ws, void* out,
                int* status, cudaStream_t st) {
   constexpr int REC = RecBytes<FMT, D>::value;
-  constexpr int kWarps = AttnCfg<FMT, D, LONG>::kWarps, kStages = AttnCfg<FMT, D, LONG>::kStages;
+  constexpr int kWarps = AttnCfg<FMT, D, VAR>::kWarps, kStages = AttnCfg<FMT, D, VAR>::kStages;
   static_assert(kWarps * kStages * 8 <= kBarBytes, "barriers");
   constexpr size_t pipe = (size_t)kWarps * (kStages * 2 * REC + (FMT == TSB200_KV_NVFP4 ? D * 2 : 0));
   constexpr size_t merge = (size_t)(kWarps * 24 + kWarps * 8 * (D + 4) + 8 * (2 + D)) * sizeof(float);
@@ -452,7 +457,7 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   TSB_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return TSB200_ERR_DEVICE;
   if (!configured[dev]) {
-    TSB_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<T, D, FMT, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TSB_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<T, D, FMT, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev] = true;
   }
   const int g = H / kv.hkv;
@@ -466,8 +471,8 @@ int launch_mma(const tsb200_kv_desc& kv, const void* q, int64_t qs, int H, float
   static int held[64][kMaxCluster + 1] = {};
   const bool clusters = S > 1 && S <= kMaxCluster &&
                         ((S == 2 && g > 1) || (S <= 4 && g > 4) ||
-                         (int64_t)grid.x * grid.z <= active_clusters(decode_attn_mma_kernel<T, D, FMT, LONG>, grid, kWarps * 32, smem, held[dev]));
-  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT, LONG>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
+                         (int64_t)grid.x * grid.z <= active_clusters(decode_attn_mma_kernel<T, D, FMT, VAR>, grid, kWarps * 32, smem, held[dev]));
+  TSB_CUDA(launch_splits(attn_overlaps(kv), clusters, decode_attn_mma_kernel<T, D, FMT, VAR>, grid, dim3(kWarps * 32), smem, st, kv, (const T*)q, qs, H, sm_scale,
                          max_seq_len, S, ws, (T*)out, status));
   return S == 1 || clusters ? TSB200_OK : launch_reduce<T, D>(ws, B * H, S, out, st);
 }
@@ -510,10 +515,14 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
                                : launch_attn_fp8<__nv_bfloat16>(*kv, q, qs, H, sm_scale, max_seq_len, S8, B, ws, out, status, s);
   }
   const int S = choose_splits(B, kv->hkv, max_seq_len);
-  const bool long_splits = kv->format == TSB200_KV_NVFP4 && D == 128 && (max_seq_len + 15) / 16 >= 64 * S;
-#define TSB_GO(TT, DD, FF)                                                                                                        \
-  if (FF == TSB200_KV_NVFP4 && DD == 128 && long_splits)                                                                          \
-    return launch_mma<TT, DD, FF, (FF == TSB200_KV_NVFP4 && DD == 128)>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s); \
+  // Instances: see AttnCfg
+  const int64_t pages = (max_seq_len + 15) / 16, ctas = n_ctr * S;
+  const bool var = kv->format != TSB200_KV_INT8 &&
+                   (D == 64 ? (ctas > 5 * 148 && pages <= 2 * S) || (ctas > 6 * 148 && pages <= (kv->format == TSB200_KV_NVFP4 ? 16 : 8) * S)
+                            : kv->format == TSB200_KV_NVFP4 && (ctas <= 512 || pages >= 64 * S));
+#define TSB_GO(TT, DD, FF)                                                                                                       \
+  if (var && FF != TSB200_KV_INT8 && (DD == 64 || FF == TSB200_KV_NVFP4))                                                        \
+    return launch_mma<TT, DD, FF, (FF != TSB200_KV_INT8 && (DD == 64 || FF == TSB200_KV_NVFP4))>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s); \
   return launch_mma<TT, DD, FF, false>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s)
 #define TSB_FMT(FF)                                                                                                       \
   if (dtype == TSB200_F32) { if (D == 64) { TSB_GO(float, 64, FF); } TSB_GO(float, 128, FF); }                               \
