@@ -185,8 +185,8 @@ def test_decode_attention_against_oracle(cuda, fmt, name, H, Hkv, d, simt):
 @pytest.mark.parametrize("name", ["fp32", "bf16"])
 @pytest.mark.parametrize("H,Hkv,d,cap,qpad", [(7, 1, 128, 576, 0), (7, 1, 128, 640, 3), (14, 2, 64, 3968, 8), (4, 1, 128, 4400, 0), (9, 1, 128, 520, 0)])
 def test_decode_attention_split_merges(cuda, fmt, name, H, Hkv, d, cap, qpad):
-    """Splits merged by the last CTA (63 rows) and by the chained reduction (70 rows, 62 splits, short and empty sequences, two head
-    chunks); queries off a 16-byte boundary and strided."""
+    """Eight to 62 splits (the FP8 kernel of up to four heads: eleven) of full, short and empty sequences, one and two head chunks, put together
+    by a cluster or the chained reduction; queries off a 16-byte boundary and strided."""
     from transformer_surgeon_b200 import ops
     rng = np.random.default_rng(29)
     B = 3
@@ -708,3 +708,31 @@ def test_attention_of_many_and_of_few_ctas(cuda, fmt, d, B, Hkv, pages, name):
     n = 9                                                       # (fewer than eight pages: one split, however few the sequences)
     out = ops.paged_decode_attention(kv, q, pages * 16)
     assert torch.equal(ops.paged_decode_attention(first(n), q[:n].contiguous(), pages * 16), out[:n])
+
+
+@pytest.mark.parametrize("fmt,H,Hkv,d", [("int8", 16, 4, 128), ("nvfp4", 16, 4, 128), ("fp8", 20, 4, 128), ("fp8", 8, 4, 64)])
+@pytest.mark.parametrize("limit", [48, 448, 4096])
+def test_attention_after_append_under_dependent_launch(cuda, fmt, H, Hkv, d, limit):
+    """As the test above for the other kernel, which looks lengths and pages up ahead of its wait: the token of the append before it is in the
+    result, with one split, a cluster and a reduction launch."""
+    from transformer_surgeon_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(63)
+    B = 6
+    kv, _ = filled_cache(fmt, B, limit // 16, Hkv, d, "bf16", cuda, g)
+    lens = torch.tensor([0, 15, 16, limit - 1, limit // 2, 31], dtype=torch.int32, device=cuda)
+    k, v = (torch.randn((B, 1, Hkv, d), generator=g, device=cuda).bfloat16() for _ in range(2))
+    q = torch.randn((B, H, d), generator=g, device=cuda).bfloat16()
+    after, outs = lens + 1, []
+    for pdl in (False, True):
+        old = ops.set_pdl(pdl)
+        try:
+            for sign in (-1, 1):                                 # another token into the same slot first
+                kv.append(sign * k, sign * v, seq_lens=lens)
+                out = ops.paged_decode_attention(kv, q, limit, seq_lens=after)
+            torch.cuda.synchronize()
+        finally:
+            ops.set_pdl(old)
+        outs.append(out.clone())
+    assert torch.equal(outs[0], outs[1])
+    ref = ops.paged_decode_attention(kv, q, limit, seq_lens=lens + 1, simt=True)
+    assert torch.all((outs[1].float() - ref.float()).abs() <= C_P_TC * 6.0 + 2 * C_OUT["bf16"] * ref.float().abs() + 1e-6)
