@@ -19,8 +19,9 @@ inline int choose_splits(int64_t B, int hkv, int64_t max_seq_len) {
   const int64_t base = B * hkv;
   const int64_t pages = (max_seq_len + 15) / 16;
   int64_t s = (148 * 8 + base - 1) / (base > 0 ? base : 1);
-  // few (sequence, kv head) pairs, long contexts: about 768 CTAs measured fastest while the last CTA merged the splits (8 sequences x
-  // 4 kv heads x 32k tokens, NVFP4 pages: 24 splits 99 us, 37 splits 115 us, 13 splits 128 us; 24 splits and the merge launch: 61)
+  // few (sequence, kv head) pairs, long contexts: about 768 CTAs.  Fitted while the last CTA merged the splits and an SM held four CTAs (8 sequences x
+  // 4 kv heads x 32k tokens, NVFP4 pages: 24 splits 99 us, 37 splits 115 us, 13 splits 128 us) and not since: 768 are 1.04 to 1.7 waves of
+  // the 740 to 444 that fit now.  Another number would change the order of the sums.
   if (base > 0 && base < 148) {
     s = (768 + base - 1) / base;
   } else if (s >= 3) {

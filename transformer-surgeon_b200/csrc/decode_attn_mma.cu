@@ -14,8 +14,9 @@
 // the MMA as code * scale; for V the block scale of a token is folded into that token's softmax
 // weight (one product per 16-dim block and token instead of one per element).
 // Several splits leave partials (m, l, acc): in shared memory where a cluster merges them (launch_mma says when), else in the workspace for
-// decode_attn_reduce_kernel.  That launch is resident before the last partial is there, and 3-5 us faster than a merge by the last CTA of a
-// pair, whatever the number of splits (captured: int8, 2 sequences x 32 / 8 heads x 500 tokens 8.2 -> 5.5 us, NVFP4, 1 x 32 / 8 x 1000 9.6 -> 6.2).
+// decode_attn_reduce_kernel.  That launch is resident before the last partial is there, and for few outputs 3-5 us faster than a merge by the
+// last CTA of a pair (captured: int8, 2 sequences x 32 / 8 heads x 500 tokens 8.2 -> 5.5 us, NVFP4, 1 x 32 / 8 x 1000 9.6 -> 6.2); a
+// call that is not captured pays 2 us for it on the host (1 x 12 x 1000, head_dim 64: 9.3 -> 11.2).
 //
 // Bound by the page loop's instructions.  Against copies by all 32 lanes (cp.async, 4 to 9 a lane and page), block scales widened by every
 // lane and a rescale of the accumulators on every page, half to all of the stated tokens: int8, 64 x 8 kv heads x 4096 95.1 -> 89.6 us, 16 x 4 x

@@ -580,8 +580,10 @@ template <bool GATED, int TM, int TN> int launch_tile(F32Params& p, int ranks, b
   TSB_CUDA(cudaLaunchKernelEx(&cfg, linear_f32_tile_kernel<GATED, TM, TN>, p));
   return TSB200_OK;
 }
-// 64 x 64 tiles where they give every SM two CTAs (half the shared-memory reads a sum), else 32 x 32, and K split over a cluster as long as
-// the two CTAs an SM holds still go round once and every rank keeps a step.
+// 64 x 64 tiles (half the shared-memory reads a sum) from 296 of them on, two for every SM: at a time without a pair, whose 104 KB rings leave room for
+// two CTAs, one after the other with one (139 KB).  Else 32 x 32, and K split over a cluster as long as the two CTAs an SM holds still go
+// round once and K has a step for every rank; ranks take whole steps, the same number each, so that the last ones may have none (9
+// steps: five ranks of eight work - as long as five would take).
 int launch_tiles(F32Params& p, bool gated, bool pdl, cudaStream_t s) {
   int64_t t64 = 0, t32 = 0;
   for (int i = 0; i < p.nseg; ++i) {
