@@ -695,11 +695,11 @@ def test_clusters_of_every_size_merge_as_a_launch_does(cuda, fmt, H, Hkv, B, few
 
 
 @pytest.mark.parametrize("fmt,d,B,Hkv,pages", [("nvfp4", 64, 90, 12, 7), ("nvfp4", 64, 64, 12, 2), ("fp8", 64, 90, 12, 7), ("fp8", 64, 64, 12, 1),
-                                               ("nvfp4", 128, 40, 16, 3)])
+                                               ("nvfp4", 128, 40, 16, 3), ("nvfp4", 128, 30, 16, 3)])
 @pytest.mark.parametrize("name", ["fp32", "bf16"])
 def test_attention_of_many_and_of_few_ctas(cuda, fmt, d, B, Hkv, pages, name):
-    """The instances for more CTAs than the GPU holds and for fewer (more warps against more registers; rings of four pages where all CTAs of
-    them fit): the first sequences of many are the same bits by themselves."""
+    """The instances for more CTAs than the GPU holds and for fewer (more warps against more registers; rings of four pages where more than two CTAs an SM
+    and all of them fit): the first sequences of many are the same bits by themselves."""
     from transformer_surgeon_b200 import ops
     g = torch.Generator(device=cuda).manual_seed(62)
     kv, first = filled_cache(fmt, B, pages, Hkv, d, name, cuda, g)

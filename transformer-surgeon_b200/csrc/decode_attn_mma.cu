@@ -44,10 +44,11 @@ using tc::smem_u32;
 constexpr unsigned kWaitLimit = 1u << 22;
 // Warps per CTA, ring stages (pages) per warp, CTAs per SM that registers are to allow.  What counts is how many CTAs an SM holds: the page
 // loop is bound by the instructions that widen codes and by the chain of a page's softmax, and the warps of other CTAs fill its gaps.  int8,
-// head_dim 64: 30 sequences x 2 kv heads x 1.5k-3k tokens 12.4 us at 5 CTAs, 13.5 at 4; head_dim 128 is limited by registers (3).  NVFP4, 128:
+// head_dim 64: 30 sequences x 2 kv heads x 1.5k-3k tokens 12.4 us at 5 CTAs, 13.5 at 4; head_dim 128 is limited by registers (3).
 // VAR is another instance for some grids (the dispatch at the end counts CTAs; times of 1100 grids, captured):
-//   * NVFP4, 128: 3 stages and 5 CTAs, or (VAR) 4 and 4, which has the registers for it.  VAR for up to 512 CTAs, which it holds at once too (1 x 8 x 16k-32k
-//     tokens, 64 splits: 17.9 -> 15.1 us; none slower by more than runs differ), and for splits of 64 pages and more: on grids of two waves of
+//   * NVFP4, 128: 3 stages and 5 CTAs, or (VAR) 4 and 4, which has the registers for it.  VAR for up to 512 CTAs, which it holds at once too, from two an SM or
+//     eight pages a split on (1 x 8 x 16k-32k tokens, 64 splits: 17.9 -> 15.1 us, 32 x 16 x 32-64, one split 0.91 of the time; below both
+//     0.87 to 1.11, 64 x 4 x 32-64 5.0 -> 5.4), and for splits of 64 pages and more: on grids of two waves of
 //     either 2-5 % faster, on 768 CTAs, one and a bit, 5 % faster to 4 % slower.  Shorter splits want the fifth CTA (16 x 8 x 250-500,
 //     5 pages a split: 10.4 us, VAR 11.8; 21 pages 20.0 / 20.1).
 //   * NVFP4 and FP8, 64: 88 registers and 5 CTAs, or (VAR) 64 and 8 (FP8: 24 bytes spilled).  VAR where there are more CTAs than the first holds and few
@@ -520,7 +521,7 @@ static int decode_attn_dispatch(const tsb200_kv_desc* kv, const void* q, void* o
   const int64_t pages = (max_seq_len + 15) / 16, ctas = n_ctr * S;
   const bool var = kv->format != TSB200_KV_INT8 &&
                    (D == 64 ? (ctas > 5 * 148 && pages <= 2 * S) || (ctas > 6 * 148 && pages <= (kv->format == TSB200_KV_NVFP4 ? 16 : 8) * S)
-                            : kv->format == TSB200_KV_NVFP4 && (ctas <= 512 || pages >= 64 * S));
+                            : kv->format == TSB200_KV_NVFP4 && ((ctas <= 512 && (ctas > 2 * 148 || pages >= 8 * S)) || pages >= 64 * S));
 #define TSB_GO(TT, DD, FF)                                                                                                       \
   if (var && FF != TSB200_KV_INT8 && (DD == 64 || FF == TSB200_KV_NVFP4))                                                        \
     return launch_mma<TT, DD, FF, (FF != TSB200_KV_INT8 && (DD == 64 || FF == TSB200_KV_NVFP4))>(*kv, q, qs, H, sm_scale, max_seq_len, S, B, ws, out, status, s); \
