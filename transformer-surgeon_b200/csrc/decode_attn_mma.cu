@@ -154,13 +154,13 @@ decode_attn_mma_kernel(tsb200_kv_desc kv, const T* __restrict__ q, int64_t qs, i
   uint8_t* ring = smem + kBarBytes + (size_t)w * kStages * STAGE;
   uint2* vscales = reinterpret_cast<uint2*>(smem + kBarBytes + (size_t)kWarps * kStages * STAGE) + w * (D / 4);    // NVFP4
   const unsigned ring_a = smem_u32(ring), bar_a = smem_u32(smem) + w * kStages * 8;
-  // lengths and block table do not come from the preceding launch (see tsb200_set_pdl): looked up ahead of the dependency wait
-  int len = kv.seq_lens[b];
   if (lane == 0) {
     for (int i = 0; i < kStages; ++i) mbar_init(reinterpret_cast<unsigned long long*>(smem) + w * kStages + i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncwarp();
+  // lengths and block table do not come from the preceding launch (see tsb200_set_pdl): looked up ahead of the dependency wait
+  int len = kv.seq_lens[b];
   len = len < 0 ? 0 : (len > max_seq_len ? (int)max_seq_len : len);
   int pb, pe;
   split_range(len, s, S, pb, pe);
